@@ -69,6 +69,13 @@ cudaError_t rd_launch_mh_jump(int prec, int geometry_mask, int grid, cudaStream_
                               const int* ch_off, const double* wtab, const int* step_ptr,
                               int it_idx, double* partial, int* tickets, double kscale, int* queue,
                               int part = 0, int nparts = 1, int form = 0);
+cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
+                                 const Pool& pool, const PlanEntry* sup_plan, const PlanHeader* sup_ph,
+                                 const float4* qpp, const double* qF, const NearState& nr, double kscale);
+cudaError_t rd_launch_mh_jumps_near(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
+                                    const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
+                                    const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
+                                    int jumps, const NearState& nr, double kscale, int* gave_up, bool lone);
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                            const Pool& pool, const ChainState& cs, const int* ch_off,
                            const double* work, const int* step_ptr, const EventLog& ev);
@@ -239,6 +246,7 @@ struct rd_engine {
   double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr, *qF = nullptr, *qfx = nullptr, *qfy = nullptr;
   float4* qpp = nullptr;   // planar quadrature points in the FP32 frame
   ChainState cs{};
+  NearState nr{};
   int *d_choff = nullptr, *d_qoff = nullptr, *d_npts = nullptr, *d_zero_off = nullptr;
   PlanEntry* plan[PM_COUNT] = {};
   PlanHeader* ph[PM_COUNT] = {};
@@ -251,7 +259,8 @@ struct rd_engine {
   EventLog evlog{nullptr, nullptr, 0};   // emission / absorption records (rd_events_take)
   int *ccnt = nullptr, *cpre = nullptr, *cflag = nullptr;   // compaction: per 256-particle unit survivors,
                                                             // first destinations and load flags
-  int* cq = nullptr;      // compaction: [0] tile counter, [1] blocks left, [2] waits that gave up
+  int* cq = nullptr;      // compaction: [0] tile counter, [1] blocks left, [2] waits that gave up; [3] waits of the MH jumps
+                          // (k_mh_jumps_near) that gave up
   double* ramo = nullptr;   // velocity-pass item partials (10 per 128-particle item)
   int* life = nullptr;
   int* d_step = nullptr;
@@ -335,6 +344,31 @@ static int supply_panels(double Lx, double Ly, int emitter_type, double ring_rmi
   return std::min(256, std::max(16, P));
 }
 
+// Bins of the near / far split (rd_near.cuh): a diode with P x P supply panels
+// (16 P^2 points, P >= 16) takes (P + 6) (P + 7) / 2 + 1 of them, fewer than the
+// 3 P^2 from 3/16 of its first point on.
+static size_t near_bins(long long qcap) { return 3 * ((size_t)qcap / 16 + 1) + 16; }
+
+// All of the split's arrays in one allocation (256-byte aligned parts).
+static cudaError_t alloc_near(rd_engine* e, long long cap, long long qcap, int S) {
+  size_t at = 0;
+  auto part = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t low = part(sizeof(float4) * cap), hi = part(sizeof(float4) * cap), lo = part(sizeof(float2) * cap),
+               rank = part(sizeof(int) * cap), cnt = part(sizeof(int) * near_bins(qcap)),
+               start = part(sizeof(int) * near_bins(qcap)), count = part(sizeof(unsigned long long) * S),
+               progress = part(sizeof(unsigned long long) * S),
+               rec = part(sizeof(float) * RD_NEAR_REC * ((size_t)qcap / 16 + 1));
+  unsigned char* base = nullptr;
+  const cudaError_t ce = e->dalloc(&base, at);
+  if (ce != cudaSuccess) return ce;
+  NearState& n = e->nr;
+  n.low = (float4*)(base + low); n.hi = (float4*)(base + hi); n.lo = (float2*)(base + lo);
+  n.rank = (int*)(base + rank); n.cnt = (int*)(base + cnt); n.start = (int*)(base + start);
+  n.count = (unsigned long long*)(base + count); n.progress = (unsigned long long*)(base + progress);
+  n.rec = (float*)(base + rec);
+  return cudaSuccess;
+}
+
 static int alloc_pool(rd_engine* e, Pool& P, long long cap) {
   double** dbl[] = {&P.x, &P.y, &P.z, &P.vx, &P.vy, &P.vz, &P.ax, &P.ay, &P.az,
                     &P.bx, &P.by, &P.bz, &P.cx, &P.cy, &P.cz, &P.q, &P.m};
@@ -347,12 +381,13 @@ static int alloc_pool(rd_engine* e, Pool& P, long long cap) {
 }
 
 // ---- pipeline pieces ----------------------------------------------------------------
-static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) {
+static cudaError_t plan_on(rd_engine* e, int mode, cudaStream_t st, const int* npts = nullptr) {
   e->kernels_in_step++;
   const int slot = mode & 0xff;
-  return rd_launch_plan(e->st, e->dP, e->dD, e->nslots_hw(), mode, rd_chunk_rule(e->clen_min, e->nch_max),
+  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), mode, rd_chunk_rule(e->clen_min, e->nch_max),
                         e->max_items, npts, e->plan[slot], e->ph[slot]);
 }
+static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) { return plan_on(e, mode, e->st, npts); }
 
 static bool valid_chunking(int clen_min, int nch_max) {
   return clen_min >= RD_TILE && clen_min <= 65536 && clen_min % RD_TILE == 0 && nch_max >= 1 &&
@@ -366,6 +401,8 @@ struct Sig {
   bool tts = false;           // some diode uses the two-time-step integrator
   int jumps = 0;
   int mh_planar = 0;          // planar diodes with batched MH chains
+  int mh_near = 0;            // of these, the diodes whose jumps take the near / far split
+  bool mh_slow() const { return mh_planar > mh_near || emit_tip; }
 };
 static Sig signature(const rd_engine* e) {
   Sig s;
@@ -380,6 +417,7 @@ static Sig signature(const rd_engine* e) {
       if (p.geometry != RD_G_TIP && !p.image_charge) s.emit_lat = true;
       if (p.geometry != RD_G_TIP && p.mh_serial) s.emit_serial = true;
       if (p.geometry != RD_G_TIP && !p.mh_serial) s.mh_planar++;
+      if (p.mh_fast) s.mh_near++;
       s.jumps = std::max(s.jumps, p.mh_jumps);
     }
   }
@@ -388,7 +426,7 @@ static Sig signature(const rd_engine* e) {
 
 // MH launch shape of the planar jumps for the resident mix: parts of the plan
 // (one launch and one stream each; one diode cannot be split) and the FP32
-// thread form.  Neither changes a result: each diode's chains and counters sit
+// thread form.  (Jumps by the near / far split have one shape.)  Neither changes a result: each diode's chains and counters sit
 // in one part, and both forms do the same lane arithmetic in the same order.
 static int mh_parts_for(const rd_engine* e, const Sig& s) {
   if (s.mh_planar <= 1) return 1;
@@ -399,11 +437,12 @@ static int mh_form_for(const rd_engine* e, const Sig& s) {
   return s.mh_planar == 1 ? 1 : 0;
 }
 
-static int planar_mh_launch(rd_engine* e, const Sig& s, int it, int parts, int form, cudaStream_t main) {
+static int planar_mh_launch(rd_engine* e, const Sig& s, int it, int parts, int form, cudaStream_t main,
+                            int pm = PM_MH) {
   for (int q = 0; q < parts; ++q) {
     cudaStream_t sq = q == 0 ? main : e->stp[q];
     int* queue = q == 0 ? e->item_queue : e->item_queue + 6 + 2 * (q + 1);
-    CK(rd_launch_mh_jump(e->cfg.precision, 1, e->grid, sq, e->dP, e->dD, e->pool, e->plan[PM_MH], e->ph[PM_MH],
+    CK(rd_launch_mh_jump(e->cfg.precision, 1, e->grid, sq, e->dP, e->dD, e->pool, e->plan[pm], e->ph[pm],
                          e->cs, e->d_choff, e->wtab, e->d_step, it, e->partial, e->tickets, e->kscale, queue,
                          parts > 1 ? q + 1 : 0, parts, form));
   }
@@ -431,12 +470,30 @@ static int mh_join(rd_engine* e, int parts, cudaStream_t main) {
 // fill the idle SMs.  Results do not depend on it.
 static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
   const int prec = e->cfg.precision;
-  const int parts = mh_parts_for(e, s), form = mh_form_for(e, s);
-  int rc = mh_fork(e, parts, main);
-  if (rc) return rc;
-  for (int it = 1; it <= s.jumps; ++it) {
-    if (s.emit_planar) {
-      if ((rc = planar_mh_launch(e, s, it, parts, form, main))) return rc;
+  const bool slow = s.mh_planar > s.mh_near, near = s.mh_near > 0;
+  const int parts = slow ? mh_parts_for(e, s) : 1, form = mh_form_for(e, s);
+  int pm = PM_MH, rc;
+  if (near) {
+    CK(rd_launch_near_setup(e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_SUPPLY_PLANAR],
+                            e->ph[PM_SUPPLY_PLANAR], e->qpp, e->qF, e->nr, e->kscale));
+    e->kernels_in_step += 4;
+    CK(plan_on(e, PM_MH_NEAR, main));
+    if (slow) {
+      pm = PM_MH_SLOW;
+      CK(plan_on(e, pm, main));
+    }
+  }
+  if (near) {
+    CK(rd_launch_mh_jumps_near(e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
+                               e->plan[PM_MH], e->cs, e->d_choff, e->wtab, e->d_step, s.jumps, e->nr, e->kscale,
+                               e->cq + 3, s.mh_near == 1));
+    e->kernels_in_step += s.mh_near == 1 ? 2 : 1;
+  }
+  const int tiled_jumps = slow || s.emit_tip ? s.jumps : 0;
+  if ((rc = mh_fork(e, parts, main))) return rc;
+  for (int it = 1; it <= tiled_jumps; ++it) {
+    if (slow) {
+      if ((rc = planar_mh_launch(e, s, it, parts, form, main, pm))) return rc;
       e->kernels_in_step += parts;
     }
     if (s.emit_tip) {   // tip propose + jump
@@ -445,7 +502,12 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
       e->kernels_in_step += 2;
     }
   }
-  return mh_join(e, parts, main);
+  if ((rc = mh_join(e, parts, main))) return rc;
+  if (near) {   // the pair sums at the chains' last points, for the emission test
+    if ((rc = planar_mh_launch(e, s, RD_MH_FINAL, 1, form, main))) return rc;
+    e->kernels_in_step++;
+  }
+  return RD_OK;
 }
 
 // The tiled MH chains of a step on stream `main`: round 0 of the start (tiled
@@ -594,13 +656,15 @@ static int launch_update_position(rd_engine* e) {
 }
 
 // Waits of the in-place compaction (k_compact_move) that gave up: each is a
-// tile that stored nothing, so the particle state is no longer valid.  Read
-// after the engine stream has drained.
+// tile that stored nothing, so the particle state is no longer valid; and waits
+// of the Metropolis-Hastings jumps (k_mh_jumps_near).  Read after the engine stream
+// has drained.
 static int compaction_check(rd_engine* e) {
-  int bad = 0;
-  CK(cudaMemcpyAsync(&bad, e->cq + 2, sizeof(int), cudaMemcpyDeviceToHost, e->st));
+  int gave_up[2] = {0, 0};
+  CK(cudaMemcpyAsync(gave_up, e->cq + 2, sizeof gave_up, cudaMemcpyDeviceToHost, e->st));
   CK(cudaStreamSynchronize(e->st));
-  if (bad) return fail(RD_ERR_STATE, "compaction: a wait on an earlier tile gave up; the particle state is not valid");
+  if (gave_up[1]) return fail(RD_ERR_STATE, "emission: a wait on a diode's last jump gave up; the chain state is not valid");
+  if (gave_up[0]) return fail(RD_ERR_STATE, "compaction: a wait on an earlier tile gave up; the particle state is not valid");
   return RD_OK;
 }
 
@@ -628,9 +692,9 @@ static int launch_step_body(rd_engine* e) {
 static std::string sig_string(rd_engine* e) {
   Sig s = signature(e);
   char b[128];
-  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
-           s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.jumps, e->clen_min, e->nch_max,
-           mh_parts_for(e, s), mh_form_for(e, s));
+  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
+           s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.mh_near > 1 ? 2 : s.mh_near, s.mh_planar > s.mh_near,
+           s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
   return b;
 }
 
@@ -774,9 +838,10 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
       e->dalloc(&e->qw, qcap) || e->dalloc(&e->qF, qcap) || e->dalloc(&e->qfx, qcap) ||
       e->dalloc(&e->qfy, qcap) || e->dalloc(&e->qpp, qcap) || e->dalloc(&e->cs.gx, chcap) || e->dalloc(&e->cs.gy, chcap) ||
       e->dalloc(&e->cs.fx, chcap) || e->dalloc(&e->cs.fy, chcap) || e->dalloc(&e->cs.fsup, chcap) ||
-      e->dalloc(&e->cs.fF, chcap) ||
+      e->dalloc(&e->cs.fF, chcap) || e->dalloc(&e->cs.fe, chcap) ||
       e->dalloc(&e->cs.fgx, chcap) || e->dalloc(&e->cs.fgy, chcap) ||
       e->dalloc(&e->cs.pph, chcap) || e->dalloc(&e->cs.pih, chcap) ||
+      (cfg->precision == RD_PREC_FP32C && alloc_near(e, cap, qcap, S)) ||
       e->dalloc(&e->d_choff, S) || e->dalloc(&e->d_qoff, S) ||
       e->dalloc(&e->d_npts, S) || e->dalloc(&e->d_zero_off, S) ||
       e->dalloc(&e->partial, (size_t)e->max_items * 3 * RD_ITILE) ||
@@ -806,6 +871,10 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
   if (e->evlog.count) cudaMemsetAsync(e->evlog.count, 0, sizeof(int), e->st);
   e->evlog.cap = cfg->event_capacity > 0 ? cfg->event_capacity : 0;
   cudaMemsetAsync(e->life, 0, sizeof(int) * (size_t)S * RD_MAX_LIFE, e->st);
+  if (e->nr.cnt) {
+    cudaMemsetAsync(e->nr.cnt, 0, sizeof(int) * near_bins(qcap), e->st);
+    cudaMemsetAsync(e->nr.count, 0, sizeof(unsigned long long) * S, e->st);
+  }
   cudaMemsetAsync(e->d_npts, 0, sizeof(int) * S, e->st);
   cudaMemsetAsync(e->d_zero_off, 0, sizeof(int) * S, e->st);
   cudaMemsetAsync(e->d_step, 0, sizeof(int), e->st);
@@ -921,6 +990,42 @@ static int flush_admissions(rd_engine* e) {
   if (e->pending.empty()) return RD_OK;
   int rc = activate_pending(e);
   if (rc) return rc;
+  CK(cudaStreamSynchronize(e->st));
+  return RD_OK;
+}
+
+// The near / far split of the FP32 chains' field for a new planar diode.  It wants
+// the 4-node supply rule (its panels carry the far part), one image partner
+// (every term of the sum has one sign), panels that are about square (the two
+// axes share the near region) and enough of them that the near region is a
+// part of the emitter (P >= 16; the default rule gives that).  Everything else
+// keeps the pair-sum jumps, as do diodes that are given ions or atoms later.
+static void near_params(const rd_engine* e, DiodeParams& p, int P, int Q) {
+  p.mh_fast = 0;
+  if (e->cfg.precision != RD_PREC_FP32C || p.geometry != RD_G_PLANAR || p.mh_serial || p.emitter_type == 4 ||
+      !p.image_charge || p.N_ic_max != 0 || Q != 4 || P < 16 || P > 1024 || p.max_chains >= 1 << 22)
+    return;
+  const double ax = 0.5e9 * p.em_Lx / P, ay = 0.5e9 * p.em_Ly / P;
+  if (ax > 2.0 * ay || ay > 2.0 * ax) return;
+  p.mh_fast = 1;
+  p.nr_P = P;
+  p.nr_boff = p.q_off / 16 * 3;
+  p.nr_bx = P + 2 * RD_NEAR_M;
+  p.nr_by = (P + 2 * RD_NEAR_M + 1) / 2;
+  p.nr_Z = (float)(5.0 * std::max(ax, ay));
+  p.nr_Ez = (float)p.E_z;
+  p.nr_ax = (float)ax; p.nr_ay = (float)ay;
+  p.nr_iax = (float)(1.0 / ax); p.nr_iay = (float)(1.0 / ay);
+  p.nr_iwx = (float)(0.5 / ax); p.nr_iwy = (float)(0.5 / ay);
+}
+
+// A diode that holds anything but electrons keeps the pair-sum jumps from now on.
+static int keep_pair_sum(rd_engine* e, int d) {
+  DiodeParams& p = e->slots[d].p;
+  if (!p.mh_fast) return RD_OK;
+  p.mh_fast = 0;
+  e->act_P[d].mh_fast = 0;
+  CK(cudaMemcpyAsync(e->dP + d, &e->act_P[d], sizeof(DiodeParams), cudaMemcpyHostToDevice, e->st));
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }
@@ -1073,6 +1178,7 @@ static int diode_add_impl(rd_engine* e, const rd_diode_config* c, int* diode, cu
     qs.ring_rmin = p.ring_rmin; qs.ring_thick = p.ring_thick; qs.org_x = p.org_x; qs.org_y = p.org_y;
     qs.a_foci = p.a_foci; qs.eta_1 = p.eta_1; qs.max_xi = p.max_xi; qs.shift_z = p.shift_z;
     if (c->geometry == RD_GEOM_PLANAR) gauss_legendre(Q, qs.gx, qs.gw);
+    near_params(e, p, P_, Q);
     CK(rd_launch_quad_fill(us, qs, e->qx, e->qy, e->qz, e->qw, e->qpp));
   }
   CK(upload(e, e->work + sl.w_off, wv.data(), sl.w_len * sizeof(double), us, deferred));
@@ -1170,6 +1276,9 @@ int rd_add_particles(rd_engine* e, int d, int n, const double* pos, const double
   if (n < 0 || (n > 0 && !pos)) return fail(RD_ERR_INVALID, "bad particle arrays");
   int rc = stage(e, 6LL * n, n);
   if (rc) return rc;
+  if (species && std::any_of(species, species + n, [](int s) { return s != RD_SPECIES_ELEC; }) &&
+      (rc = keep_pair_sum(e, d)))
+    return rc;
   if (n > 0) {
     // the previous upload from the pinned stage has completed (every call ends with a
     // stream synchronize), so the stage can be refilled
@@ -1499,7 +1608,8 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   CK(cudaMemcpyAsync(e->save_ax, e->pool.ax, bytes, cudaMemcpyDeviceToDevice, e->st));
   CK(cudaMemcpyAsync(e->save_ay, e->pool.ay, bytes, cudaMemcpyDeviceToDevice, e->st));
   CK(cudaMemcpyAsync(e->save_az, e->pool.az, bytes, cudaMemcpyDeviceToDevice, e->st));
-  const int jumps = std::max(signature(e).jumps, 1);
+  // jumps that take the pair sums (near / far split: only the start and the last points)
+  const int jumps = signature(e).mh_slow() ? std::max(signature(e).jumps, 1) : 2;
   const int saved_min = e->clen_min, saved_max = e->nch_max;
   const int user_parts = e->mh_parts, user_form = e->mh_form;
   e->mh_parts = 0;    // the chunking is searched at the default launch shape
@@ -1634,7 +1744,7 @@ int rd_do_emission(rd_engine* e, int step) {
   int rc = launch_emission(e);
   if (rc) return rc;
   CK(cudaStreamSynchronize(e->st));
-  return RD_OK;
+  return compaction_check(e);
 }
 
 int rd_update_position(rd_engine* e, int step) {
@@ -1833,12 +1943,18 @@ int rd_diode_load(rd_engine* e, int d, const void* buf, long long size) {
   const int off = p.off;
   for (int k = 0; k < kStateDoubles; ++k, in += sizeof(double) * (size_t)h.n)
     if (h.n) CK(cudaMemcpy(state_dbl(e->pool, k) + off, in, sizeof(double) * (size_t)h.n, cudaMemcpyHostToDevice));
+  int rc = RD_OK;   // species is the first of the integer arrays
+  for (int i = 0; i < h.n && rc == RD_OK; ++i) {
+    int sp;
+    std::memcpy(&sp, in + sizeof(int) * (size_t)i, sizeof sp);
+    if (sp != RD_SPECIES_ELEC) { rc = keep_pair_sum(e, d); break; }
+  }
+  if (rc) return rc;
   for (int k = 0; k < kStateInts; ++k, in += sizeof(int) * (size_t)h.n)
     if (h.n) CK(cudaMemcpy(state_int(e->pool, k) + off, in, sizeof(int) * (size_t)h.n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(e->life + (size_t)d * RD_MAX_LIFE, in, sizeof(int) * RD_MAX_LIFE, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(e->dD + d, &y, sizeof y, cudaMemcpyHostToDevice));
-  int rc = repack(e);   // the FP32 packs (and tip image points) of the loaded particles
-  if (rc) return rc;
+  if ((rc = repack(e))) return rc;   // the FP32 packs (and tip image points) of the loaded particles
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }

@@ -807,6 +807,7 @@ __global__ void k_mh_init(const DiodeParams* __restrict__ P, DiodeDyn* __restric
             const float Ff = (float)Fz;
             cs.fsup[k] = rho_xy_f(p, wtab, fx, fy, Ff);
             cs.fF[k] = Ff;
+            cs.fe[k] = 0.0f;
           }
         }
       } else {
@@ -866,6 +867,21 @@ __device__ __forceinline__ void mh_std_step(const DiodeParams& p, double* mh_std
   }
 }
 
+// One tile's acceptance counts into the diode's; the last of its tiles updates MH_std.
+__device__ __forceinline__ void mh_counts_add(const DiodeParams& p, DiodeDyn& y, int tiles, int it_idx,
+                                              int ndim_first, int a, int r) {
+  atomicAdd(&y.mh_acc, a);
+  atomicAdd(&y.mh_rej, r);
+  __threadfence();
+  int prev = atomicAdd(&y.mh_done, 1);
+  if (prev == tiles - 1) {
+    __threadfence();
+    int A = atomicExch(&y.mh_acc, 0), R = atomicExch(&y.mh_rej, 0);
+    y.mh_done = 0;
+    mh_std_step(p, &y.MH_std, &y.a_rate, it_idx, ndim_first, A, R);
+  }
+}
+
 __device__ __forceinline__ void mh_counts_and_update(const DiodeParams& p, DiodeDyn& y, int tiles,
                                                      int it_idx, int ndim_first, int a, int r,
                                                      int* red_i) {
@@ -877,18 +893,7 @@ __device__ __forceinline__ void mh_counts_and_update(const DiodeParams& p, Diode
     if (tid < s) { red_i[tid] += red_i[tid + s]; red_i[RD_ITILE + tid] += red_i[RD_ITILE + tid + s]; }
     __syncthreads();
   }
-  if (tid == 0) {
-    atomicAdd(&y.mh_acc, red_i[0]);
-    atomicAdd(&y.mh_rej, red_i[RD_ITILE]);
-    __threadfence();
-    int prev = atomicAdd(&y.mh_done, 1);
-    if (prev == tiles - 1) {
-      __threadfence();
-      int A = atomicExch(&y.mh_acc, 0), R = atomicExch(&y.mh_rej, 0);
-      y.mh_done = 0;
-      mh_std_step(p, &y.MH_std, &y.a_rate, it_idx, ndim_first, A, R);
-    }
-  }
+  if (tid == 0) mh_counts_add(p, y, tiles, it_idx, ndim_first, red_i[0], red_i[RD_ITILE]);
   __syncthreads();
 }
 
@@ -1073,6 +1078,7 @@ __device__ __forceinline__ void mh_start_f32(const DiodeParams& p, ChainState& c
     const float Ff = (float)F;
     cs.fsup[k] = rho_xy_f(p, wtab, x, y, Ff);
     cs.fF[k] = Ff;
+    cs.fe[k] = 0.0f;
     float g1, g2;
     gauss2f(p.seed, (uint32_t)c, 1u, step, &g1, &g2);
     cs.fgx[k] = g1; cs.fgy[k] = g2;
@@ -1095,7 +1101,8 @@ __device__ __forceinline__ void mh_start_f64(const DiodeParams& p, ChainState& c
 }
 
 // One Metropolis-Hastings jump iteration of the planar chains (it_idx >= 1),
-// or round 0 of their uniform start (it_idx == 0: every chain of the step
+// the pair sums at the last points of the chains that jump by the near / far
+// split (RD_MH_FINAL), or round 0 of their uniform start (it_idx == 0: every chain of the step
 // evaluates its first uniform draw here, tiled like a jump; the chains that
 // drew an unfavourable point continue in k_mh_init from round 1), or a dry
 // pass for the autotuner (it_idx < 0: the field at every chain's current
@@ -1127,13 +1134,14 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
   const int nt = blockDim.x;
   const int total = ph->total_items, nd = ph->n_diodes, tid = threadIdx.x;
   const bool init = it_idx == 0;
-  const bool dry = it_idx < 0;   // timing pass: field at the current points, nothing written
+  const bool fin = it_idx == RD_MH_FINAL;   // the field at the last points of the chains of rd_near.cuh
+  const bool dry = it_idx < 0 && !fin;      // timing pass: field at the current points, nothing written
   int lo, hi;   // this launch's part of the plan (part_range)
   part_range(plan, nd, total, part, nparts, &lo, &hi);
   for (int g = queue_first(lo, hi); g < hi; g = queue_next(queue, &s_item, lo, hi)) {
     ItemRef it = decode_item(plan, nd, g);
     const DiodeParams& p = P[it.d];
-    if (p.geometry != RD_G_PLANAR || it_idx > p.mh_jumps) continue;
+    if (p.geometry != RD_G_PLANAR || it_idx > p.mh_jumps || (fin && !p.mh_fast)) continue;
     DiodeDyn& y = Dy[it.d];
     const int ndim_first = (p.mh_jumps + 2) / 4;   // nint(0.25 mh_jumps), :1141
     const int M = plan[it.d].n_i;
@@ -1150,7 +1158,7 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
         const int c = it.i0 + tid + q * nt;
         kk[q] = ch_off[it.d] + c;
         ok[q] = (c < M) ? (init ? 1 : cs.ok[kk[q]]) : 0;
-        mh_propose_f32(p, cs, kk[q], c, ok[q], init, dry, step, sx, sy, hx, hy, &fwx[q], &fwy[q]);
+        mh_propose_f32(p, cs, kk[q], c, ok[q], init, dry || fin, step, sx, sy, hx, hy, &fwx[q], &fwy[q]);
       }
     } else {
       const double mhs = y.MH_std;
@@ -1186,6 +1194,17 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
     }
     // epilogue of the completed tile
     if (dry) continue;
+    if constexpr (PREC == 1) {
+      if (fin) {   // the field and the point in metres that the emission test reads
+        for (int q = 0; q < CPT; ++q) {
+          if (!ok[q]) continue;
+          cs.F[kk[q]] = z0_finish<PREC>(p, s[q], kscale);
+          cs.x[kk[q]] = p.org_x + (double)fwx[q] * 1.0e-9;
+          cs.y[kk[q]] = p.org_y + (double)fwy[q] * 1.0e-9;
+        }
+        continue;
+      }
+    }
     if (init) {   // a favourable start (F < 0) makes the chain; the others go to k_mh_init
       for (int q = 0; q < CPT; ++q) {
         if (!ok[q]) continue;
@@ -1211,6 +1230,8 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
   }
   queue_leave(queue, lo, hi);
 }
+
+#include "rd_near.cuh"
 
 // mh_decide_f for a vacuum-field chain (F_n = F_c), out of line: k_mh_vacuum
 // reaches it only for a proposal into another work-function cell.
@@ -2413,6 +2434,49 @@ cudaError_t rd_launch_mh_jump(int prec, int geometry_mask, int grid, cudaStream_
     else k_mh_jump_tip<0><<<rd_grid(k_mh_jump_tip<0>, RD_ITILE, grid), RD_ITILE, 0, st>>>(P, Dy, pool, plan, ph, cs, ch_off, step_ptr, it_idx, partial, tickets, kscale, queue + 2);
   }
   return cudaGetLastError();
+}
+
+// Bins, near electrons and panel records of the step's chains (rd_near.cuh), from the
+// supply field qF.
+cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
+                                 const Pool& pool, const PlanEntry* sup_plan, const PlanHeader* sup_ph,
+                                 const float4* qpp, const double* qF, const NearState& nr, double kscale) {
+  k_near_count<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
+  k_near_scan<<<nslots, 1024, 0, st>>>(P, Dy, nr);
+  k_near_scatter<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
+  k_near_panels<<<rd_grid(k_near_panels, 256, grid), 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
+  return cudaGetLastError();
+}
+
+// All jumps of those chains: cooperative launches (the blocks wait for one another's
+// counts), one block per resident slot of the GPU at most.  A lone diode gets both
+// kernels; the device's item count says which of them runs it.
+template <class... A>
+static cudaError_t launch_coop(void (*kernel)(A...), int block, int grid, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = st;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, args...);
+}
+cudaError_t rd_launch_mh_jumps_near(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
+                                    const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
+                                    const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
+                                    int jumps, const NearState& nr, double kscale, int* gave_up, bool lone) {
+  const int most = rd_grid(k_mh_jumps_near, 128, 0), most1 = rd_grid(k_mh_jumps_near_one, 256, 0);
+  const int g = grid > 0 && grid < most ? grid : most, g1 = grid > 0 && grid < most1 ? grid : most1;
+  if (lone) {
+    const cudaError_t e = launch_coop(k_mh_jumps_near_one, 256, g1, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab,
+                                      step_ptr, jumps, nr, kscale, gave_up);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_coop(k_mh_jumps_near, 128, g, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr,
+                     kscale, gave_up, lone ? g1 : 0);
 }
 
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,

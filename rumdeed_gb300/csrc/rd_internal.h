@@ -40,6 +40,13 @@
 inline int rd_chunk_rule(int clen_min, int nch_max) { return clen_min | (nch_max << 16); }
 #define RD_MAX_LIFE 1000
 #define RD_COMPACT_SPIN (1 << 22)   // polls (64 ns sleeps) of a compaction tile waiting on an earlier one
+#define RD_MH_FINAL (-2)      // k_mh_jump_planar: pair sums at the chains' last points (rd_near.cuh)
+#define RD_NEAR_SPIN (1 << 22)   // polls of a block waiting for a diode's last jump (about a second or more)
+#define RD_NEAR_M 3           // near region of a panel: this many panels on every side
+#define RD_NEAR_CPB 32        // chains per item of k_mh_jumps_near
+#define RD_NEAR_W (2 * RD_NEAR_M + 1)   // panels across the near region
+#define RD_NEAR_ROWS (RD_NEAR_M + 1)    // rows of bins (two panels high) that cover it
+#define RD_NEAR_REC 32        // words of a panel record (a multiple of 4)
 #define RD_MAX_WORK 4096      // max checkerboard cells per diode (64x64)
 
 enum { RD_G_PLANAR = 1, RD_G_TIP = 2 };
@@ -89,11 +96,21 @@ struct DiodeParams {
   double planes_z[10];
   int tts;               // two-time-step interval T (atom_time_interval); 0 off
   double ramo_uz;        // -1 / d: z of the planar unit field E_zunit_planar
+  // near / far split of the FP32 chains' field (rd_near.cuh)
+  int mh_fast;           // 1: the diode's jumps take it
+  int nr_P;              // panels per side of the supply rule
+  int nr_boff;           // first bin of this diode
+  int nr_bx, nr_by;      // bins along x (one panel wide) and y (two panels high)
+  float nr_Z;            // near electrons are lower than this (nm)
+  float nr_Ez;           // E_z
+  float nr_ax, nr_ay, nr_iax, nr_iay, nr_iwx, nr_iwy;   // panel half widths (nm), 1 / half width, 1 / width
 };
 
 // Planner modes (k_plan): which i-set of each diode a pair-sum plan covers.
-// Modes up to PM_SUPPLY_LAT are pair sums (tiles x j-chunks), the two PM_PART
-// modes per-particle index spaces.  PM_SUPPLY_PLANAR: the supply points of
+// Modes up to PM_SUPPLY_LAT and PM_MH_SLOW are pair sums (tiles x j-chunks), the
+// two PM_PART modes per-particle index spaces, PM_MH_NEAR tiles of RD_NEAR_CPB
+// chains.  PM_MH: all batched chains of the tiled kernels (start rounds, last
+// points); their jumps split into PM_MH_NEAR (rd_near.cuh) and PM_MH_SLOW.  PM_SUPPLY_PLANAR: the supply points of
 // planar diodes with image charges (F_z only: the lateral components cancel
 // at the cathode); PM_SUPPLY_LAT: those of planar diodes without (all three
 // components, for the mean field of field.dt).  PM_ALL_DIODES added to PM_FORCE_PLANAR or
@@ -101,7 +118,7 @@ struct DiodeParams {
 // Calculate_Acceleration_Particles pass, which ignores two_time_step).
 enum { PM_FORCE_PLANAR = 0, PM_FORCE_TIP = 1, PM_FIELD = 2, PM_SUPPLY_PLANAR = 3,
        PM_SUPPLY_TIP = 4, PM_MH = 5, PM_FORCE_TTS = 6, PM_SUPPLY_LAT = 7, PM_PART = 8, PM_PART1024 = 9,
-       PM_COUNT = 10, PM_ALL_DIODES = 0x100 };
+       PM_MH_SLOW = 10, PM_MH_NEAR = 11, PM_COUNT = 12, PM_ALL_DIODES = 0x100 };
 
 // Supply quadrature grid of one diode, filled on the device (k_quad_fill):
 // planar, quad_n x quad_n Gauss-Legendre nodes (P panels of Q nodes per side)
@@ -204,8 +221,23 @@ struct ChainState {
   // emitter centre (the chain lives on that grid), the target's rho and the
   // field as floats (mh_decide_f), Gaussian pair
   float *fx, *fy, *fsup, *fF, *fgx, *fgy;
+  float* fe;             // bound on |fF - field|; 0: fF is the pair sum's (rd_near.cuh)
   // FP32-compensated tip chains: the proposal packed once per jump for the
   // field tiles (the point on the FP32 nm grid and the high words of its
   // apex-sphere image)
   float4 *pph, *pih;
+};
+
+// Near / far split of the cathode field (rd_near.cuh): per particle slot (x, y, z,
+// bin) and its rank in the bin; the near electrons in bin order; per bin the count
+// and first slot; per supply panel the record.
+struct NearState {
+  float4* low;
+  int* rank;
+  float4* hi;
+  float2* lo;
+  int *cnt, *start;
+  float* rec;
+  unsigned long long *count, *progress;   // per slot: tiles done, accepted, rejected of a jump; jumps
+                                          // done and step size (near_counts)
 };

@@ -1,0 +1,775 @@
+// rd_near.cuh -- the jumps of the FP32 planar Metropolis-Hastings chains from a
+// near / far split of the cathode field (included by rd_field.cu, in its
+// anonymous namespace).
+//
+// A jump needs the field at its proposal only to compare two targets, and the
+// FP32 chains already decide from FP32 estimates of the targets wherever those
+// are certain (mh_decide_f).  The same holds for the field itself: an estimate
+// with a bound on how far it can lie from the value the pair-sum kernel
+// (k_mh_jump_planar) computes decides every jump outside that bound, and the few
+// jumps inside it take the pair sum.  So the decisions, and with them the
+// chains, are those of the pair-sum kernel, bit for bit, and the field that
+// emission reads is the pair sum at each chain's last point (one pass after the
+// last jump, RD_MH_FINAL).
+//
+// The estimate.  The step's supply integral has just evaluated the pair sum S at
+// 4 x 4 Gauss-Legendre nodes of each of the emitter's P x P panels.  Electrons
+// lower than nr_Z and within RD_NEAR_M panels of a panel (in whole bins) are near it; the others
+// are far, and their part of S is smooth over the panel:
+//   S(p) = I[S(nodes) - sum_near g(nodes)](p) + sum_near g(p),
+// I the interpolation in the nodes, g_j(p) = q z / (rho^2 + z^2)^{3/2}.  A jump
+// then costs 16 coefficients and the near electrons (tens to a few hundred)
+// instead of all of them.
+//
+// The bound.  With a the panel's half widths and D the distance from a far
+// electron to the panel, the Taylor coefficients of g along an axis are
+// Gegenbauer polynomials of its direction cosine c, d^4 g / 4! = C_4^{3/2}(c) z / R^7,
+// at most K z / D^7 with K = 15 (c = 1), or 2.5 where c^2 <= 0.68, so
+//   |I g - g|(t) <= T_x |w(t_x)| a_x^4 + T_y L(t_x) |w(t_y)| a_y^4,
+//   T = sum_far K z / D^7,  w(t) = prod (t - node),  L the Lebesgue function.
+// The rounding of the pair sum itself (tiles of 128 terms added one after
+// another: 128 u of the tile's sum of magnitudes, 25 u of each term), of the
+// node values carried through I (L(t_x) L(t_y) times theirs), and of this
+// kernel's own sums is bounded by multiples of u = 2^-24 times the sum of
+// magnitudes, which is |S| because every charge has one sign (diodes that hold
+// ions or atoms keep the pair-sum kernel).  nr_guard has the multiples.
+//
+// Measured (GB300, jumps of one step, the split's set-up and last pass included):
+//   one diode, 4500 electrons, 3800 chains, 100 jumps      6.13 -> 0.79 ms
+//   24 diodes of 256-4096 electrons, 30,000 chains, 200    15.9 -> 2.3 ms
+//   128 diodes of 256-32768 electrons, 353,000 chains, 200  276 -> 26.4 ms
+// Open after the estimate: one jump in 10^5; the estimate lay within 0.08 of its
+// bound in every jump checked.  What is left is latency (one near list, one far
+// record, three logarithms and one counter per jump), not arithmetic.
+//
+// Near region: RD_NEAR_M = 3 panels and nr_Z = 5 half widths.  5 panels and 8 half
+// widths make the bound's T ten times smaller and leave half as many jumps open,
+// but the near list more than twice as long: 31 -> 42 ms on the 128 diodes.
+
+
+// Does the diode's step run its jumps here?  (planner mode PM_MH_NEAR)
+__device__ __forceinline__ bool near_live(const DiodeParams& p, const DiodeDyn& y) {
+  return p.active && p.emission && p.mh_fast && y.chains > 0 && !rd_mh_vacuum(p, y);
+}
+
+// Bin of a low electron: row << 16 | column, or -1 for one that is far from every
+// panel.  Bins are one panel wide and two high, RD_NEAR_M panels more than the
+// emitter on every side; the near region of panel (x, y) is the columns x .. x + 2 M
+// and the RD_NEAR_ROWS rows from y / 2 on.
+__device__ __forceinline__ int near_bin(const DiodeParams& p, float x, float y, float z) {
+  if (!(z < p.nr_Z)) return -1;
+  const float fx = floorf((x + p.em_hx) * p.nr_iwx), fy = floorf((y + p.em_hy) * p.nr_iwy);
+  if (!(fabsf(fx) < 4096.0f) || !(fabsf(fy) < 4096.0f)) return -1;
+  const int bx = (int)fx + RD_NEAR_M, y2 = (int)fy + RD_NEAR_M;
+  if (bx < 0 || bx >= p.nr_bx || y2 < 0 || y2 >= 2 * p.nr_by) return -1;
+  return ((y2 >> 1) << 16) | bx;
+}
+
+// A diode's progress through its jumps, written by the last tile of each jump: the
+// number done, whether the step size is at its upper clamp (bit 31), and the step
+// size as a float (high word).
+#define RD_NEAR_CLAMPED 0x80000000u
+__device__ __forceinline__ unsigned long long near_progress(const DiodeParams& p, int done, double mh_std) {
+  return ((unsigned long long)__float_as_uint((float)mh_std) << 32) |
+         ((unsigned)done | (mh_std == p.mh_hi ? RD_NEAR_CLAMPED : 0u));
+}
+
+// Electrons into bins: each electron's bin and its rank among the bin's.
+__global__ void __launch_bounds__(256)
+k_near_count(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, NearState nr) {
+  const int d = blockIdx.y;
+  const DiodeParams& p = P[d];
+  if (!near_live(p, Dy[d])) return;
+  const int n = Dy[d].n, nb = p.nr_bx;
+  int* cnt = nr.cnt + p.nr_boff;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const float4 h = pool.zk_hi[p.off + j];
+    const float z = pool.zk_lo[p.off + j].z;
+    const int code = near_bin(p, h.x, h.y, z);
+    nr.low[p.off + j] = make_float4(h.x, h.y, z, __int_as_float(code));
+    if (code >= 0) nr.rank[p.off + j] = atomicAdd(&cnt[(code >> 16) * nb + (code & 0xffff)], 1);
+  }
+}
+
+// First slot of each bin (one block per diode); the counts are left at zero for
+// the next step.
+__global__ void __launch_bounds__(1024)
+k_near_scan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, NearState nr) {
+  __shared__ int wsum[32];
+  const int d = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const DiodeParams& p = P[d];
+  if (!near_live(p, Dy[d])) return;
+  const int bins = p.nr_bx * p.nr_by, per = (bins + 1023) / 1024;
+  int* cnt = nr.cnt + p.nr_boff;
+  int* start = nr.start + p.nr_boff;
+  const int b0 = min(tid * per, bins), b1 = min(b0 + per, bins);
+  int s = 0;
+  for (int b = b0; b < b1; ++b) s += cnt[b];
+  int x = s;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += v;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int t = wsum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += v;
+    }
+    wsum[lane] = t;
+  }
+  __syncthreads();
+  int at = (w > 0 ? wsum[w - 1] : 0) + x - s;
+  for (int b = b0; b < b1; ++b) {
+    const int c = cnt[b];
+    start[b] = at;
+    cnt[b] = 0;
+    at += c;
+  }
+  if (tid == 1023) start[bins] = at;   // the last thread's range ends at the last bin
+  if (tid == 0) nr.progress[d] = near_progress(p, 0, Dy[d].MH_std);   // no jump of this step done
+}
+
+// The near electrons in bin order: (x_hi, y_hi, z^2, q z) and (x_lo, y_lo).
+__global__ void __launch_bounds__(256)
+k_near_scatter(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, NearState nr) {
+  const int d = blockIdx.y;
+  const DiodeParams& p = P[d];
+  if (!near_live(p, Dy[d])) return;
+  const int n = Dy[d].n, nb = p.nr_bx;
+  const int* start = nr.start + p.nr_boff;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const int code = __float_as_int(nr.low[p.off + j].w);
+    if (code < 0) continue;
+    const int k = p.off + start[(code >> 16) * nb + (code & 0xffff)] + nr.rank[p.off + j];
+    const float4 l = pool.zk_lo[p.off + j];
+    nr.hi[k] = pool.zk_hi[p.off + j];
+    nr.lo[k] = make_float2(l.x, l.y);
+  }
+}
+
+__device__ __forceinline__ float near_term(float4 h, float2 l, float px, float py) {
+  const float dx = (px - h.x) - l.x, dy = (py - h.y) - l.y;
+  const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, h.z)));
+  return h.w * ((inv * inv) * inv);
+}
+
+// Inverse Vandermonde matrix of the four Gauss-Legendre nodes: coefficients of
+// the interpolating cubic from the node values.
+__device__ const float c_gl4_inv[4][4] = {
+    {-0.0923265988f, 0.592326599f, 0.592326599f, -0.0923265988f},
+    {0.107214846f, -1.74223419f, 1.74223419f, -0.107214846f},
+    {0.798762056f, -0.798762056f, -0.798762056f, 0.798762056f},
+    {-0.927567512f, 2.34943118f, -2.34943118f, 0.927567512f}};
+
+// Panel records, one warp per panel: the far part's interpolation coefficients
+// (powers of t_x fastest), the panel's centre, T and the largest |S| of its
+// nodes, and where its near electrons are.  The supply plan's tiles of 128 points cover eight panels each.
+__global__ void __launch_bounds__(256)
+k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, const PlanEntry* __restrict__ plan,
+              const PlanHeader* __restrict__ ph, const float4* __restrict__ qpp, const double* __restrict__ qF,
+              NearState nr, double kscale) {
+  const int total = ph->total_items, nd = ph->n_diodes, lane = threadIdx.x & 31;
+  for (int g = blockIdx.x; g < total; g += gridDim.x) {
+    const ItemRef it = decode_item(plan, nd, g);
+    if (it.chunk != 0) continue;
+    const DiodeParams& p = P[it.d];
+    if (!near_live(p, Dy[it.d])) continue;
+    const int NP = p.nr_P, pan = it.tile * 8 + (threadIdx.x >> 5);
+    if (pan >= NP * NP) continue;
+    const int ppy = pan / NP, ppx = pan - ppy * NP, nb = p.nr_bx, r0 = ppy >> 1;
+    const int* start = nr.start + p.nr_boff;
+    // the node of this lane (lanes l and l + 16 share one and take every other near electron)
+    const int k = p.q_off + (ppy * 4 + ((lane >> 2) & 3)) * p.quad_n + ppx * 4 + (lane & 3);
+    const float4 pp = qpp[k];
+    const float S = (float)((qF[k] - p.E_z) / (-2.0 * kscale));
+    float near = 0.0f;
+    for (int r = 0; r < RD_NEAR_ROWS; ++r) {
+      const int row = (r0 + r) * nb + ppx;   // bins ppx .. ppx + 2 M of this row
+      const int e1 = start[row + RD_NEAR_W];
+      for (int e0 = start[row]; e0 < e1; e0 += 64) {   // short runs: the sums stay accurate
+        float s = 0.0f;
+        for (int e = e0 + (lane >> 4); e < min(e0 + 64, e1); e += 2)
+          s += near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z);
+        near += s;
+      }
+    }
+    near += __shfl_xor_sync(0xffffffffu, near, 16);
+    float big = fabsf(S);
+    for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+    // tensor coefficients of the far part, about the value at the first node
+    const float far = S - near, base = __shfl_sync(0xffffffffu, far, 0), v = far - base;
+    float cx = 0.0f, c = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) cx = fmaf(c_gl4_inv[lane & 3][q], __shfl_sync(0xffffffffu, v, (lane & 12) + q), cx);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c = fmaf(c_gl4_inv[(lane >> 2) & 3][q], __shfl_sync(0xffffffffu, cx, 4 * q + (lane & 3)), c);
+    if (lane == 0) c += base;
+    // T over the far electrons, as seen from the panel's rectangle
+    const double wx = p.em_Lx * 1.0e9 / NP, wy = p.em_Ly * 1.0e9 / NP;
+    const float ox = (float)((ppx + 0.5) * wx - 0.5e9 * p.em_Lx), oy = (float)((ppy + 0.5) * wy - 0.5e9 * p.em_Ly);
+    const float ax = p.nr_ax, ay = p.nr_ay;
+    float Tx = 0.0f, Ty = 0.0f;
+    const int n = Dy[it.d].n;
+    for (int j = lane; j < n; j += 32) {
+      const float4 e = nr.low[p.off + j];
+      const int code = __float_as_int(e.w);
+      const bool is_near = code >= 0 && (unsigned)((code & 0xffff) - ppx) < RD_NEAR_W &&
+                           (unsigned)((code >> 16) - r0) < RD_NEAR_ROWS;
+      // least and largest lateral distances to the panel's points
+      const float ux = fabsf(e.x - ox), uy = fabsf(e.y - oy), z2 = fmaf(e.z, e.z, 1e-20f);
+      const float bx = fmaxf(ux - ax, 0.0f), by = fmaxf(uy - ay, 0.0f), tx = ux + ax, ty = uy + ay;
+      const float inv = rsqrtf(fmaf(bx, bx, fmaf(by, by, z2)));
+      const float i2 = inv * inv, v7 = is_near ? 0.0f : (e.z * inv) * (i2 * i2 * i2);
+      // c_x^2 <= 0.68 over the panel: 0.32 x^2 <= 0.68 (y^2 + z^2)
+      Tx = fmaf(0.32f * tx * tx <= 0.68f * fmaf(by, by, z2) ? 2.5f : 15.0f, v7, Tx);
+      Ty = fmaf(0.32f * ty * ty <= 0.68f * fmaf(bx, bx, z2) ? 2.5f : 15.0f, v7, Ty);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      Tx += __shfl_xor_sync(0xffffffffu, Tx, o);
+      Ty += __shfl_xor_sync(0xffffffffu, Ty, o);
+    }
+    float* rec = nr.rec + (size_t)(p.q_off / 16 + pan) * RD_NEAR_REC;
+    if (lane < 16) rec[lane] = c;
+    // the rows of near electrons end to end: what turns a list index into an electron, and the row's end
+    int a0 = 0, len = 0;
+    if (lane < RD_NEAR_ROWS) {
+      const int row = (r0 + lane) * nb + ppx;
+      a0 = start[row];
+      len = start[row + RD_NEAR_W] - a0;
+    }
+    int end = len;
+    for (int o = 1; o < RD_NEAR_ROWS; o <<= 1) {
+      const int v2 = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v2;
+    }
+    if (lane < RD_NEAR_ROWS) {
+      reinterpret_cast<int*>(rec)[20 + lane] = end;
+      reinterpret_cast<int*>(rec)[20 + RD_NEAR_ROWS + lane] = a0 - (end - len);
+    }
+    if (lane == 0) *reinterpret_cast<float4*>(rec + 16) = make_float4(ox, oy, 1.03f * Tx, big);
+    if (lane == 1) rec[28] = 1.03f * Ty;
+  }
+}
+
+// Bound on |estimate - pair sum| at (tx, ty) of a panel: the interpolation's
+// error, and the roundings of the pair sum (153 u of the sum of magnitudes A at
+// the point, the same of the nodes' `big` carried through the interpolation),
+// of the near sums (at most ~60 u each), of the points' own coordinates (half
+// an ulp of the emitter's half width, against the distance 5 a to the nearest
+// far electron: 0.6 P u) and of the evaluation (~30 u).
+// near_bound0 is the part that does not depend on A (factor near_boundA).
+__device__ __forceinline__ float near_bound0(const DiodeParams& p, float tx, float ty, float Tx, float Ty, float big) {
+  const float x2 = tx * tx, y2 = ty * ty;
+  const float wx = fabsf((x2 - 0.741555748f) * (x2 - 0.115587109f)), wy = fabsf((y2 - 0.741555748f) * (y2 - 0.115587109f));
+  const float lx = 1.48f + 14.0f * fmaxf(fabsf(tx) - 0.9f, 0.0f), ly = 1.48f + 14.0f * fmaxf(fabsf(ty) - 0.9f, 0.0f);
+  const float ax2 = p.nr_ax * p.nr_ax, ay2 = p.nr_ay * p.nr_ay;
+  const float u = 5.97e-8f, c = 0.6f * (float)p.nr_P;
+  return Tx * ((wx + 1e-5f) * (ax2 * ax2)) + Ty * (lx * (wy + 1e-5f) * (ay2 * ay2)) + u * (lx * ly * (250.0f + c) * big);
+}
+__device__ __forceinline__ float near_boundA(const DiodeParams& p) { return 5.97e-8f * (250.0f + 0.6f * (float)p.nr_P); }
+
+// The pair sums of k_mh_jump_planar at two points, by the NT threads of a block,
+// bit for bit.  A warp takes two j-tiles at a time: its lanes form the factors
+// 1/r^3 of both points (the part that can run in parallel), four lanes add them up,
+// one (tile, point) each, in the tile kernel's order from zero; then the tile sums
+// of a chunk are folded in order with two-sum and the chunks added in order with
+// pair_add (pair_partials).  out[0], out[1]: the sums before z0_finish.
+// 4800 electrons: ~3 us (40 us with one thread per tile, whose strided loads and
+// reciprocal roots all sit on the sum's chain).
+#define RD_NEAR_PASS 128      // tiles per pass over the electrons
+template <int NT>
+struct NearExact {
+  float4 f[NT / 32][2][2][RD_TILE / 4];   // 1/r^3 of (tile, point), by warp
+  float4 q[NT / 32][2][RD_TILE / 4];      // q z of the tile
+  float t[2][RD_NEAR_PASS];
+  float h[2][RD_NCH_MAX], l[2][RD_NCH_MAX];
+  double out[2];
+  int still;
+};
+template <int NT>
+__device__ __forceinline__ void near_exact2(const float4* __restrict__ zhi, const float4* __restrict__ zlo, int n,
+                                            int clen, int nch, float x0, float y0, float x1, float y1,
+                                            NearExact<NT>* s) {
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int tiles = (n + RD_TILE - 1) / RD_TILE, tpc = clen / RD_TILE;
+  float ch = 0.0f, cl = 0.0f;   // the open chunk of point tid (threads 0 and 1)
+  int in_chunk = 0, chunk = 0;
+  for (int base = 0; base < tiles; base += RD_NEAR_PASS) {
+    const int here = min(RD_NEAR_PASS, tiles - base);
+    for (int t2 = 2 * w; t2 < here; t2 += NT / 16) {
+      float4 h[2][RD_TILE / 32];
+      float2 l[2][RD_TILE / 32];
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int v = 0; v < RD_TILE / 32; ++v) {   // all loads in flight; past the electrons q z = 0
+          const int j = (base + t2 + b) * RD_TILE + lane + 32 * v;
+          h[b][v] = j < n ? zhi[j] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+          l[b][v] = j < n ? *reinterpret_cast<const float2*>(&zlo[j]) : make_float2(0.0f, 0.0f);
+        }
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int v = 0; v < RD_TILE / 32; ++v) {
+          const int k = lane + 32 * v;
+          const float dx0 = (x0 - h[b][v].x) - l[b][v].x, dy0 = (y0 - h[b][v].y) - l[b][v].y;
+          const float dx1 = (x1 - h[b][v].x) - l[b][v].x, dy1 = (y1 - h[b][v].y) - l[b][v].y;
+          const float i0 = rsqrtf(fmaf(dx0, dx0, fmaf(dy0, dy0, h[b][v].z)));
+          const float i1 = rsqrtf(fmaf(dx1, dx1, fmaf(dy1, dy1, h[b][v].z)));
+          reinterpret_cast<float*>(s->q[w][b])[k] = h[b][v].w;
+          reinterpret_cast<float*>(s->f[w][b][0])[k] = (i0 * i0) * i0;
+          reinterpret_cast<float*>(s->f[w][b][1])[k] = (i1 * i1) * i1;
+        }
+      __syncwarp();
+      if (lane < 4 && t2 + (lane >> 1) < here) {   // a term with q z = 0 adds nothing
+        const int b = lane >> 1, pt = lane & 1;
+        float a = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < RD_TILE / 4; ++k) {
+          const float4 q = s->q[w][b][k], f = s->f[w][b][pt][k];
+          a = fmaf(q.x, f.x, a);
+          a = fmaf(q.y, f.y, a);
+          a = fmaf(q.z, f.z, a);
+          a = fmaf(q.w, f.w, a);
+        }
+        s->t[pt][t2 + b] = a;
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    if (tid < 2) {   // RD_NEAR_PASS need not hold whole chunks: the open one carries over
+      for (int i = 0; i < here; ++i) {
+        two_sum_acc(ch, cl, s->t[tid][i]);
+        if (++in_chunk == tpc || base + i + 1 == tiles) {
+          s->h[tid][chunk] = ch;
+          s->l[tid][chunk] = cl;
+          ch = cl = 0.0f;
+          in_chunk = 0;
+          ++chunk;
+        }
+      }
+    }
+    if (base + RD_NEAR_PASS < tiles) __syncthreads();
+  }
+  if (tid < 2) {
+    float H = 0.0f, L = 0.0f;
+    if (tiles > 0 && nch == 1) {
+      H = s->h[tid][0];
+      L = s->l[tid][0];
+    } else {
+      for (int c = 0; c < nch && tiles > 0; ++c) pair_add(H, L, s->h[tid][c], s->l[tid][c]);
+    }
+    s->out[tid] = (double)H + (double)L;
+  }
+  __syncthreads();
+}
+
+// The bound on mh_decide_f's FP32 evaluation (7.3e-7 + 3.0e-7 S, see mh_guard, which
+// takes ten times it) and a tenth more.
+__device__ __forceinline__ float near_guard(float S) { return 8.0e-7f + 3.3e-7f * S; }
+
+// The decision of mh_decide_f from estimated fields: the proposal's Fn within dF of
+// the pair sum's, the chain's Fc within fe; t0, t2 the proposal's work-function
+// entry, lu the accept test's log u.  The fields' errors widen the guard: each
+// relative error is at most 1/4 and enters 2 log(-F) - rho at most 2.5-fold.
+// Returns 1 taken, 0 rejected, -1 open; *rn the proposal's rho (if taken).
+__device__ __forceinline__ int near_decide(const DiodeParams& p, float Fn, float dF, float Fc, float fe, float rc,
+                                           float t0, float t2, float lu, float* rn) {
+  if (Fn - dF > 0.0f) return 0;   // F >= 0: rejected
+  if (!(Fn < 0.0f && 4.0f * dF <= -Fn)) return -1;
+  *rn = rho_entry_f(p, t0, t2, Fn);
+  const float l2 = 2.0f * logf(Fn / Fc), df = l2 - (*rn - rc);
+  const float St = fabsf(l2) + fabsf(*rn) + fabsf(rc);
+  const float eps = 2.5f * (dF / -Fn + fe / -Fc);
+  if (!(isfinite(df) && isfinite(eps) && isfinite(lu))) return -1;
+  const float gd = near_guard(St + fabsf(lu)) + eps;
+  if (df >= near_guard(St) + eps || lu <= df - gd) return 1;
+  return lu > df + gd ? 0 : -1;
+}
+
+// Field from a sum, and the rounding of that step.
+__device__ __forceinline__ float near_field(const DiodeParams& p, float ksc, float S, float dS, float* dF) {
+  const float A0 = -2.0f * ksc;
+  *dF = fabsf(A0) * dS + 2.4e-7f * (fabsf(p.nr_Ez) + fabsf(A0 * S));
+  return fmaf(A0, S, p.nr_Ez);
+}
+
+// A jump that the interpolated estimate leaves open (rare; out of line so that it
+// costs the others no registers).  First the direct sums at the proposal (px, py)
+// and at the chain's point (cx, cy) by the whole block, in any order: they lie
+// within the roundings of the two sums (153 u for the pair sum, 25 u a term and at
+// most 60 u for the order here) of the pair sums, some twenty times closer than the
+// estimate, and let the targets be compared in FP64; what even they leave open takes
+// the pair sums (near_exact2) and
+// mh_accept_one_f's test.  The thread that holds the chain (mine) decides and
+// updates it; returns 1 there if the proposal is taken.
+template <int NT>
+__device__ __noinline__ int near_open(const DiodeParams& p, const Pool& pool, const ChainState& cs,
+                                      const double* __restrict__ wtab, const PlanEntry& e, double kscale, bool mine,
+                                      int c, int k, int it_idx, uint32_t step, float px, float py, float cx, float cy,
+                                      float lu, NearExact<NT>* s) {
+  const float4* zhi = pool.zk_hi + p.off;
+  const float4* zlo = pool.zk_lo + p.off;
+  const int n = e.n_j, tid = threadIdx.x;
+  float sn = 0.0f, sc = 0.0f, rn = 0.0f, rc = 0.0f;
+  for (int j0 = 0; j0 < n; j0 += 8 * NT) {   // eight loads in flight, runs of eight terms
+    float4 h[8];
+    float2 l[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int j = j0 + q * NT + tid;
+      h[q] = j < n ? zhi[j] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+      l[q] = j < n ? *reinterpret_cast<const float2*>(&zlo[j]) : make_float2(0.0f, 0.0f);
+    }
+    rn = rc = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { rn += near_term(h[q], l[q], px, py); rc += near_term(h[q], l[q], cx, cy); }
+    sn += rn;
+    sc += rc;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sn += __shfl_xor_sync(0xffffffffu, sn, o);
+    sc += __shfl_xor_sync(0xffffffffu, sc, o);
+  }
+  if ((tid & 31) == 0) { s->t[0][tid >> 5] = sn; s->t[1][tid >> 5] = sc; }
+  if (tid == 0) s->still = 0;
+  __syncthreads();
+  int a = 0;
+  if (mine) {
+    sn = sc = 0.0f;
+    for (int w = 0; w < NT / 32; ++w) { sn += s->t[0][w]; sc += s->t[1][w]; }
+    const float u = 5.97e-8f;
+    float dFn, dFc, t0, t2, r;
+    const float Fn = near_field(p, (float)kscale, sn, 250.0f * u * fabsf(sn), &dFn);
+    work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
+    float Fc = cs.fF[k], fe = cs.fe[k], rho = cs.fsup[k];
+    if (fe != 0.0f) {
+      const float F2 = near_field(p, (float)kscale, sc, 250.0f * u * fabsf(sc), &dFc);
+      if (dFc < fe && F2 < 0.0f && 4.0f * dFc <= -F2) {
+        Fc = F2; fe = dFc;
+        rho = rho_xy_f(p, wtab, cx, cy, F2);
+        cs.fF[k] = Fc; cs.fe[k] = fe; cs.fsup[k] = rho;
+      }
+    }
+    int take = near_decide(p, Fn, dFn, Fc, fe, rho, t0, t2, lu, &r);
+    const double Dn = p.E_z - 2.0 * kscale * (double)sn, Dc = p.E_z - 2.0 * kscale * (double)sc;
+    if (take < 0 && Dn < 0.0 && Dc < 0.0) {   // the targets in FP64: only the sums' own bounds remain
+      const double en = 2.0 * kscale * 250.0 * (double)u * fabs((double)sn), ec = 2.0 * kscale * 250.0 * (double)u * fabs((double)sc);
+      if (4.0 * en <= -Dn && 4.0 * ec <= -Dc) {
+        uint32_t o[4];
+        philox4x32((uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), o);
+        const double d = (supply_log_chain_d(p, wtab, px, py, Dn) - supply_log_chain_d(p, wtab, cx, cy, Dc)) -
+                         log(u01_words(o[0], o[1]));
+        const double eps = 2.5 * (en / -Dn + ec / -Dc) + 1.0e-11;   // take iff d >= 0 (or s_n >= s_c, where log u <= 0)
+        if (d > eps) take = 1;
+        else if (d < -eps) take = 0;
+        r = rho_entry_f(p, t0, t2, Fn);
+      }
+    }
+    if (take == 1) {
+      cs.fx[k] = px; cs.fy[k] = py; cs.fsup[k] = r; cs.fF[k] = Fn; cs.fe[k] = dFn;
+      a = 1;
+    }
+    s->still = take < 0;
+  }
+  __syncthreads();
+  if (!s->still) return a;   // block-uniform
+  near_exact2<NT>(zhi, zlo, n, e.clen, e.nch, px, py, cx, cy, s);
+  if (mine) {
+    const double F = z0_finish<1>(p, s->out[0], kscale);
+    if (cs.fe[k] != 0.0f) {   // the current point's field was an estimate
+      const double Fc = z0_finish<1>(p, s->out[1], kscale);
+      const float Fcf = (float)Fc;
+      cs.F[k] = Fc; cs.fF[k] = Fcf; cs.fe[k] = 0.0f;
+      cs.fsup[k] = rho_xy_f(p, wtab, cx, cy, Fcf);
+    }
+    if (F < 0.0) {
+      const float Ff = (float)F;
+      const float r = rho_xy_f(p, wtab, px, py, Ff);
+      if (mh_decide_f(p, wtab, c, it_idx, step, F, Ff, r, px, py, cx, cy, cs.F[k], cs.fF[k], cs.fsup[k])) {
+        cs.fx[k] = px; cs.fy[k] = py; cs.fsup[k] = r; cs.fF[k] = Ff; cs.F[k] = F; cs.fe[k] = 0.0f;
+        a = 1;
+      }
+    }
+  }
+  __syncthreads();
+  return a;
+}
+
+// The plan entry of item g: two rounds of 32 slots each instead of a binary search's
+// chain of loads (more than 1024 slots take decode_item).
+__device__ __forceinline__ int near_entry(const PlanEntry* __restrict__ plan, int nd, int g, int lane) {
+  if (nd == 1) return 0;
+  if (nd > 1024) return decode_item(plan, nd, g).d;
+  const int step = (nd + 31) / 32;
+  const int i = lane * step;
+  const int seg = __popc(__ballot_sync(0xffffffffu, i < nd && plan[i].item_off <= g)) - 1;
+  const int j = seg * step + lane;
+  return seg * step + __popc(__ballot_sync(0xffffffffu, lane < step && j < nd && plan[j].item_off <= g)) - 1;
+}
+
+// The acceptance counts of one tile; the diode's last tile updates MH_std
+// (MH_std_update :603-612, as mh_std_step) and lets the next jump go.  One packed
+// atomic carries the tile count and both sums, so its answer tells the last tile
+// the diode's totals.  At the upper clamp with a rate above 0.35 the product stays
+// clamped, whatever the factor: no FP64 exponential on the jump's critical path;
+// the rate itself is only kept at the last jump (every jump counts the same chains).
+__device__ __forceinline__ void near_counts(const DiodeParams& p, DiodeDyn& y, unsigned long long* count,
+                                            unsigned long long* progress, unsigned long long last, int tiles, int it_idx,
+                                            int ndim_first, int a, int r) {
+  const unsigned long long add = (1ull << 44) | ((unsigned long long)a << 22) | (unsigned long long)r;
+  const unsigned long long now = atomicAdd(count, add) + add;
+  if ((int)(now >> 44) != tiles) return;
+  __stcg(count, 0ull);
+  const int A = (int)(now >> 22) & 0x3fffff, R = (int)now & 0x3fffff;
+  unsigned long long next = last + 1;   // the step size stays
+  if (it_idx > ndim_first && A + R > 0 &&
+      (it_idx == p.mh_jumps || !((unsigned)last & RD_NEAR_CLAMPED) || 20ll * A <= 7ll * (A + R))) {
+    const double g = mh_std_gain(A, R, &y.a_rate);
+    const double m = mh_std_clamp(p, __ldcg(&y.MH_std) * g);
+    __stcg(&y.MH_std, m);
+    next = near_progress(p, it_idx, m);
+  }
+  __threadfence();
+  *reinterpret_cast<volatile unsigned long long*>(progress) = next;
+}
+
+// Every jump of every chain of the diodes with the near / far split, in one
+// cooperative launch.  A block of NW warps takes 32 chains at a time (an item of the
+// PM_MH_NEAR plan) through a jump: warp 0 proposes and evaluates the far part, one
+// chain per lane, while other warps draw log u and the next Gaussian pairs; every
+// chain's near electrons are summed by eight lanes (loads of four electrons in
+// flight per lane); warp 0 decides; the jumps left open take the pair sums
+// (near_open).  A jump needs the acceptance counts of the whole diode's last one
+// (MH_std), nothing of any other diode: a block walks its items jump by jump and
+// waits only for the diode's progress word.  All blocks are resident (cooperative
+// launch) and an item waits only for items of earlier jumps, so every wait ends;
+// each still polls at most RD_NEAR_SPIN times (about a second), after which the
+// block counts in *gave_up and leaves (rd_run reports it).
+// ONE: every block has at most one item; its chains stay in registers.
+template <int NW>
+struct NearShared {
+  float x[32], y[32], near[32], lu[32], g[2][32];   // proposal, near sum, log u, next Gaussian pair
+  int pan[32];                                      // the chain's panel; -1: no chain
+  float cx[32], cy[32];                             // the chains' points, where a jump is left open
+  unsigned open;
+  int dead;
+  NearExact<32 * NW> ex;
+};
+
+// The far part at a point: a panel's record, then its value and bound (c0.x, c0.y).
+struct NearFar {
+  float4 c0, c1, c2, c3, cm;
+  float ty;
+  __device__ __forceinline__ void load(const float4* rec) {
+    c0 = rec[0]; c1 = rec[1]; c2 = rec[2]; c3 = rec[3]; cm = rec[4];
+    ty = reinterpret_cast<const float*>(rec)[28];
+  }
+  __device__ __forceinline__ void eval(const DiodeParams& p, float px, float py) {
+    const float x = (px - cm.x) * p.nr_iax, y = (py - cm.y) * p.nr_iay;
+    const float r0 = fmaf(fmaf(fmaf(c0.w, x, c0.z), x, c0.y), x, c0.x);
+    const float r1 = fmaf(fmaf(fmaf(c1.w, x, c1.z), x, c1.y), x, c1.x);
+    const float r2 = fmaf(fmaf(fmaf(c2.w, x, c2.z), x, c2.y), x, c2.x);
+    const float r3 = fmaf(fmaf(fmaf(c3.w, x, c3.z), x, c3.y), x, c3.x);
+    c0.y = near_bound0(p, x, y, cm.z, ty, cm.w);
+    c0.x = fmaf(fmaf(fmaf(r3, y, r2), y, r1), y, r0);
+  }
+};
+
+template <int NW, bool ONE>
+__device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const Pool& pool,
+                                           const PlanEntry* __restrict__ plan, int total, int nd,
+                                           const PlanEntry* __restrict__ plan_mh, const ChainState& cs,
+                                           const int* __restrict__ ch_off, const double* __restrict__ wtab,
+                                           int engine_step, int jumps, const NearState& nr, double kscale, int* gave_up) {
+  constexpr int NT = 32 * NW, ROUNDS = 8 / NW;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  if (tid == 0) sh.dead = 0;
+  const float ksc = (float)kscale;
+  // the chains of the block's item (ONE; warp 0)
+  float fx = 0.0f, fy = 0.0f, gx = 0.0f, gy = 0.0f, Fc = 0.0f, rc = 0.0f, fe = 0.0f;
+  int ok = 0, d = 0;
+  for (int it = 1; it <= jumps; ++it) {
+    for (int g = blockIdx.x; g < total; g += gridDim.x) {
+      if (!ONE || it == 1) d = near_entry(plan, nd, g, lane);
+      const DiodeParams& p = P[d];
+      if (it > p.mh_jumps) continue;
+      DiodeDyn& y = Dy[d];
+      const int ndim_first = (p.mh_jumps + 2) / 4;   // nint(0.25 mh_jumps), :1141
+      const int M = plan[d].n_i, c = (g - plan[d].item_off) * 32 + lane, k = ch_off[d] + c;
+      const uint32_t step = (uint32_t)(engine_step - y.step_offset);
+      const float* recs = nr.rec + (size_t)(p.q_off / 16) * RD_NEAR_REC;
+      float px = 0.0f, py = 0.0f, t0 = 0.0f, t2 = 0.0f;
+      NearFar far_part;
+      unsigned long long pr = 0;
+      if (NW > 1 ? w == NW - 1 : true) {   // the next proposal's Gaussian pair
+        if (c < M && it < p.mh_jumps && cs.ok[k]) {
+          float g1, g2;
+          gauss2f(p.seed, (uint32_t)c, (uint32_t)(it + 1), step, &g1, &g2);
+          sh.g[0][lane] = g1;
+          sh.g[1][lane] = g2;
+        }
+      }
+      if (w == (NW > 1 ? 1 : 0) && c < M) {   // log u of the accept test, as mh_decide_f forms it
+        uint32_t o[4];
+        philox4x32((uint32_t)c, (uint32_t)it, step, RNG_ACCEPT, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), o);
+        sh.lu[lane] = logf(fmaf((float)(o[1] >> 11), 1.1102230246251565e-16f, (float)o[0] * 2.3283064365386963e-10f));
+      }
+      if (w == 0) {
+        if (!ONE || it == 1) {
+          ok = c < M ? cs.ok[k] : 0;
+          if (ok) {
+            fx = cs.fx[k]; fy = cs.fy[k]; gx = cs.fgx[k]; gy = cs.fgy[k];
+            Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k];
+          }
+        }
+        // the step size: fixed during the warm-up jumps, then MH_std after the last jump
+        if (lane == 0) {
+          const volatile unsigned long long* prog = nr.progress + d;
+          pr = *prog;
+          for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1 && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
+          if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
+        }
+        pr = __shfl_sync(0xffffffffu, pr, 0);
+        const float mhs = __uint_as_float((unsigned)(pr >> 32));
+        const float sx = (it > ndim_first) ? p.em_wx * mhs : p.em_wx * 0.10f;
+        const float sy = (it > ndim_first) ? p.em_wy * mhs : p.em_wy * 0.10f;
+        if (ok) {   // mh_propose_f32
+          const float hx = p.em_hx, hy = p.em_hy;
+          px = fmaf(gx, sx, fx);
+          py = fmaf(gy, sy, fy);
+          if (px > hx) px = hx - (px - hx); else if (px < -hx) px = -hx - (px + hx);
+          if (py > hy) py = hy - (py - hy); else if (py < -hy) py = -hy - (py + hy);
+        }
+        const int NP = p.nr_P;
+        const int ppx = min(max((int)floorf((px + p.em_hx) * p.nr_iwx), 0), NP - 1);
+        const int ppy = min(max((int)floorf((py + p.em_hy) * p.nr_iwy), 0), NP - 1);
+        const int pan = ppy * NP + ppx;
+        sh.x[lane] = px; sh.y[lane] = py;
+        sh.pan[lane] = ok ? pan : -1;
+        if (NW > 1) __syncthreads(); else __syncwarp();
+        const float4* rec = reinterpret_cast<const float4*>(recs + (size_t)pan * RD_NEAR_REC);
+        far_part.load(rec);
+        if (!ONE) far_part.eval(p, px, py);   // (ONE: evaluated after the near sums, the loads in flight meanwhile)
+        if (ok) work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
+      } else {
+        __syncthreads();
+      }
+      if (sh.dead) {   // block-uniform
+        if (tid == 0) atomicAdd(gave_up, 1);
+        return;
+      }
+      // near electrons
+      for (int r8 = 0; r8 < ROUNDS; ++r8) {
+        const int l = lane & 7, q = (w * ROUNDS + r8) * 4 + (lane >> 3), pan = sh.pan[q];
+        float s = 0.0f;
+        if (pan >= 0) {
+          // the list's rows: their ends in it, and what turns an index of it into an electron
+          const int4* rt = reinterpret_cast<const int4*>(recs + (size_t)pan * RD_NEAR_REC + 20);
+          const int4 end = rt[0], at = rt[1];
+          const float x = sh.x[q], yv = sh.y[q];
+          const float4* nh = nr.hi + p.off;
+          const float2* nl = nr.lo + p.off;
+          float run = 0.0f;
+          int m = 0;
+          for (int e = l; e < end.w; e += 32) {
+            float4 h[4];
+            float2 lo[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int ee = e + 8 * u;
+              const int k2 = ee + (ee < end.x ? at.x : ee < end.y ? at.y : ee < end.z ? at.z : at.w);
+              const bool in = ee < end.w;
+              h[u] = in ? nh[k2] : make_float4(0.0f, 0.0f, 1.0f, 0.0f);
+              lo[u] = in ? nl[k2] : make_float2(0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) run += near_term(h[u], lo[u], x, yv);
+            if (++m == 8) { s += run; run = 0.0f; m = 0; }   // short runs: the sum stays accurate
+          }
+          s += run;
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (l == 0) sh.near[q] = s;
+      }
+      if (NW > 1) __syncthreads(); else __syncwarp();
+      int a = 0;
+      if (w == 0) {   // the decisions (mh_decide_f with the field's bound added to its guard)
+        int open = 0;
+        const float cx = fx, cy = fy;
+        if (ok) {
+          if (ONE) far_part.eval(p, px, py);
+          const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y;
+          float dF, rn;
+          const float Fn = near_field(p, ksc, S, fmaf(near_boundA(p), 1.01f * fabsf(S), b0), &dF);
+          const int take = near_decide(p, Fn, dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
+          open = take < 0;
+          if (take == 1) {
+            fx = px; fy = py; rc = rn; Fc = Fn; fe = dF;
+            a = 1;
+          }
+        }
+        const unsigned mask = __ballot_sync(0xffffffffu, open);
+        if (mask) { sh.cx[lane] = cx; sh.cy[lane] = cy; }
+        if (lane == 0) sh.open = mask;
+        if (ok && ((!ONE && a) || open)) {
+          cs.fx[k] = fx; cs.fy[k] = fy; cs.fF[k] = Fc; cs.fsup[k] = rc; cs.fe[k] = fe;
+        }
+        if (ok && it < p.mh_jumps) {
+          gx = sh.g[0][lane];
+          gy = sh.g[1][lane];
+          if (!ONE) { cs.fgx[k] = gx; cs.fgy[k] = gy; }
+        }
+      }
+      if (NW > 1) __syncthreads(); else __syncwarp();
+      const unsigned open = sh.open;
+      for (unsigned o = open; o; o &= o - 1) {   // block-uniform
+        const int q = __ffs(o) - 1;
+        a += near_open<NT>(p, pool, cs, wtab, plan_mh[d], kscale, tid == q, c, k, it, step, sh.x[q], sh.y[q], sh.cx[q],
+                           sh.cy[q], sh.lu[q], &sh.ex);
+        if (ONE && tid == q) { fx = cs.fx[k]; fy = cs.fy[k]; Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k]; }
+      }
+      if (w == 0) {
+        const int acc = __popc(__ballot_sync(0xffffffffu, a)), rej = __popc(__ballot_sync(0xffffffffu, ok && !a));
+        if (lane == 0)
+          near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, ndim_first, acc, rej);
+        if (ONE && ok && it == p.mh_jumps) { cs.fx[k] = fx; cs.fy[k] = fy; }   // the last points (RD_MH_FINAL)
+      }
+    }
+  }
+}
+
+// A lone diode's few items: eight warps each, the chains in registers (at most two
+// blocks per SM; leaves larger diodes to k_mh_jumps_near).
+__global__ void __launch_bounds__(256, 2)
+k_mh_jumps_near_one(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const __grid_constant__ Pool pool,
+                    const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
+                    const PlanEntry* __restrict__ plan_mh, const __grid_constant__ ChainState cs,
+                    const int* __restrict__ ch_off, const double* __restrict__ wtab, const int* __restrict__ step_ptr,
+                    int jumps, const __grid_constant__ NearState nr, double kscale, int* gave_up) {
+  __shared__ NearShared<8> sh;
+  const int total = ph->total_items;
+  if ((int)blockIdx.x >= total || total > (int)gridDim.x) return;
+  near_jumps<8, true>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
+                      gave_up);
+}
+
+// Any number of items, four warps each; above: leaves plans of at most that many
+// items to k_mh_jumps_near_one.
+__global__ void __launch_bounds__(128, 8)
+k_mh_jumps_near(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const __grid_constant__ Pool pool,
+                const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
+                const PlanEntry* __restrict__ plan_mh, const __grid_constant__ ChainState cs,
+                const int* __restrict__ ch_off, const double* __restrict__ wtab, const int* __restrict__ step_ptr,
+                int jumps, const __grid_constant__ NearState nr, double kscale, int* gave_up, int above) {
+  __shared__ NearShared<4> sh;
+  const int total = ph->total_items;
+  if ((int)blockIdx.x >= total || total <= above) return;
+  near_jumps<4, false>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
+                       gave_up);
+}

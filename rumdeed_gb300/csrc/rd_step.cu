@@ -115,6 +115,8 @@ __device__ __forceinline__ int plan_ni(const DiodeParams& p, const DiodeDyn& y, 
     case PM_SUPPLY_TIP: return (p.emission && p.geometry == RD_G_TIP) ? 10000 : 0;
     // serial diodes: k_mh_serial; diodes with no particle in flight: k_mh_vacuum
     case PM_MH: return (p.emission && !p.mh_serial && !rd_mh_vacuum(p, y)) ? y.chains : 0;
+    case PM_MH_SLOW: return (p.emission && !p.mh_serial && !p.mh_fast && !rd_mh_vacuum(p, y)) ? y.chains : 0;
+    case PM_MH_NEAR: return (p.emission && p.mh_fast && !rd_mh_vacuum(p, y)) ? y.chains : 0;
     default: return nj;
   }
 }
@@ -149,8 +151,8 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
   __shared__ int s_items[32], s_chains[32];
   __shared__ int s_run_items, s_run_chains;
   const int tid = threadIdx.x;
-  const int tsize = (mode == PM_PART1024) ? 1024 : RD_ITILE;
-  const bool pair = ((mode & 0xff) <= PM_SUPPLY_LAT);
+  const int tsize = (mode == PM_PART1024) ? 1024 : (mode == PM_MH_NEAR) ? RD_NEAR_CPB : RD_ITILE;
+  const bool pair = (mode & 0xff) <= PM_SUPPLY_LAT || mode == PM_MH_SLOW;
   const int clen_min = chunk_rule & 0xffff, nch_max = chunk_rule >> 16;   // see rd_chunk_rule
   // the planar supply points are many tiles already: at most RD_SUP_NCH chunks per tile
   const int nch_eff = ((mode & 0xff) == PM_SUPPLY_PLANAR || (mode & 0xff) == PM_SUPPLY_LAT)
