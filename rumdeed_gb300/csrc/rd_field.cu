@@ -106,6 +106,8 @@ k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __
       fx *= kscale; fy *= kscale; fz *= kscale;
     } else {
       const double L2 = c_k.L2, dfc = c_k.div_fac_c;
+      rd_d4 im1 = make_d4(0.0, 0.0, 0.0, 0.0);
+      if (GEOM == RD_G_TIP && p.image_charge) im1 = tip_image_d4(p, X, Y, Z);
       fx = fy = fz = 0.0;
       for (int jt = it.j0; jt < it.j1; jt += RD_TILE) {
         __syncthreads();
@@ -114,7 +116,7 @@ k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __
         __syncthreads();
         int kmax = min(RD_TILE, it.j1 - jt);
         if (GEOM == RD_G_TIP)
-          tip_tile_f64<T_UPPER>(sj, kmax, X, Y, Z, dfc, -1, p.image_charge, p, L2, c_k.tip_K, fx, fy, fz);
+          tip_tile_f64<T_UPPER>(sj, nullptr, im1, kmax, X, Y, Z, dfc, -1, p.image_charge, L2, c_k.tip_K, fx, fy, fz);
         else
           planar_tile_f64<T_UPPER>(sj, kmax, X, Y, Z, dfc, -1, p.N_ic_max, p.d, p.image_charge, L2, fx, fy, fz);
       }
@@ -410,19 +412,19 @@ __device__ __forceinline__ void z0_item_sumN(const DiodeParams& p, const Pool& p
   for (int i = 0; i < CPT; ++i) { out_hi[i] = hi[i]; out_lo[i] = lo[i]; }
 }
 
+// The FP64 tile sum of q_j sum_h h / (r_h + l^2)^3: 13 FP64 operations a term.
 __device__ __forceinline__ double z0_tile_f64(const rd_d4* __restrict__ sj, int kmax, double px,
                                               double py, int nic, double d, double L2) {
+  const float L2x3 = (float)(3.0 * L2);
   double s = 0.0;
   for (int k = 0; k < kmax; ++k) {
-    rd_d4 pj = sj[k];
-    double dx = px - pj.x, dy = py - pj.y, dxy2 = dx * dx + dy * dy;
-    double r = sqrt(dxy2 + pj.z * pj.z) + L2;
-    s += (pj.w * pj.z) / ((r * r) * r);
+    const rd_d4 pj = sj[k];
+    const double dx = px - pj.x, dy = py - pj.y, dxy2 = fma(dx, dx, dy * dy);
+    s = fma(pj.w * pj.z, planar_inv_f64(fma(pj.z, pj.z, dxy2), L2, L2x3), s);
     for (int n = 1; n <= nic; ++n) {
-      double h1 = pj.z + (2.0 * n) * d, h2 = pj.z - (2.0 * n) * d;
-      double r1 = sqrt(dxy2 + h1 * h1) + L2, r2 = sqrt(dxy2 + h2 * h2) + L2;
-      s += (pj.w * h1) / ((r1 * r1) * r1);
-      s += (pj.w * h2) / ((r2 * r2) * r2);
+      const double h1 = pj.z + (2.0 * n) * d, h2 = pj.z - (2.0 * n) * d;
+      s = fma(pj.w * h1, planar_inv_f64(fma(h1, h1, dxy2), L2, L2x3), s);
+      s = fma(pj.w * h2, planar_inv_f64(fma(h2, h2, dxy2), L2, L2x3), s);
     }
   }
   return s;
@@ -737,10 +739,12 @@ __device__ void warp_field_general(const DiodeParams& p, const Pool& pool, int n
     if (p.geometry == RD_G_TIP) tip_split_finish(fx, fy, fz, ts, iih.w, p.image_charge, c_k.tip_K, &fx, &fy, &fz);
     fx *= kscale; fy *= kscale; fz *= kscale;
   } else {
+    rd_d4 im1 = make_d4(0.0, 0.0, 0.0, 0.0);
+    if (p.geometry == RD_G_TIP && p.image_charge) im1 = tip_image_d4(p, X, Y, Z);
     for (int j = lane; j < n; j += 32) {
       rd_d4 pj = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
       if (p.geometry == RD_G_TIP)
-        tip_tile_f64<T_UPPER>(&pj, 1, X, Y, Z, c_k.div_fac_c, -1, p.image_charge, p, c_k.L2, c_k.tip_K, fx, fy, fz);
+        tip_tile_f64<T_UPPER>(&pj, nullptr, im1, 1, X, Y, Z, c_k.div_fac_c, -1, p.image_charge, c_k.L2, c_k.tip_K, fx, fy, fz);
       else
         planar_tile_f64<T_UPPER>(&pj, 1, X, Y, Z, c_k.div_fac_c, -1, p.N_ic_max, p.d, p.image_charge, c_k.L2, fx, fy, fz);
     }
@@ -1797,13 +1801,15 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
       if (ok[0]) { X = cs.pxx[kk[0]]; Y = cs.pyy[kk[0]]; Z = cs.pzz[kk[0]]; }
       else tip_xyz(p, 1.5, p.eta_1, 0.0, &X, &Y, &Z);
       double fx = 0, fy = 0, fz = 0;
+      rd_d4 im1 = make_d4(0.0, 0.0, 0.0, 0.0);
+      if (p.image_charge) im1 = tip_image_d4(p, X, Y, Z);
       for (int jt = it.j0; jt < it.j1; jt += RD_TILE) {
         __syncthreads();
         int j = jt + tid;
         if (j < it.j1) sj[tid] = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
         __syncthreads();
-        tip_tile_f64<T_UPPER>(sj, min(RD_TILE, it.j1 - jt), X, Y, Z, c_k.div_fac_c, -1,
-                              p.image_charge, p, c_k.L2, c_k.tip_K, fx, fy, fz);
+        tip_tile_f64<T_UPPER>(sj, nullptr, im1, min(RD_TILE, it.j1 - jt), X, Y, Z, c_k.div_fac_c, -1,
+                              p.image_charge, c_k.L2, c_k.tip_K, fx, fy, fz);
       }
       f3[0][0] = fx; f3[0][1] = fy; f3[0][2] = fz;
     }

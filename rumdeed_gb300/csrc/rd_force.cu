@@ -8,7 +8,7 @@
 // higher-indexed one (:1303-1323, :1372-1402).
 //
 // Two precisions:
-//  * FP64 ("plain"): the reference's arithmetic in SI units.
+//  * FP64 ("plain"): SI units, the inverse cubes of rd_f64.cuh.
 //  * FP32 compensated: positions as (hi, lo) float pairs in nm, rsqrt and
 //    per-j-tile float accumulation, tile sums folded into (hi, lo) pairs with
 //    two-sum, the final sum and all prefactors in FP64.  The image partner
@@ -356,7 +356,7 @@ k_force_tip_f64(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
                 const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
                 double* __restrict__ partial, int* __restrict__ tickets, int* __restrict__ queue) {
   __shared__ int s_item;
-  __shared__ rd_d4 sj[RD_TILE];
+  __shared__ rd_d4 sj[RD_TILE], sim[RD_TILE];
   const int total = ph->total_items, nd = ph->n_diodes;
   const int tid = threadIdx.x;
   const double L2 = c_k.L2, dfc = c_k.div_fac_c, K = c_k.tip_K;
@@ -369,19 +369,25 @@ k_force_tip_f64(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
     double x1 = 0, y1 = 0, z1 = 0, q1 = 0;
     if (valid) { x1 = pool.x[off + i]; y1 = pool.y[off + i]; z1 = pool.z[off + i]; q1 = pool.q[off + i]; }
     const double qd1 = q1 * dfc;
+    const bool ic = p.image_charge != 0;
+    rd_d4 im1 = make_d4(0.0, 0.0, 0.0, 0.0);
+    if (ic && valid) im1 = tip_image_d4(p, x1, y1, z1);
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int jt = it.j0; jt < it.j1; jt += RD_TILE) {
       __syncthreads();
       int j = jt + tid;
-      if (j < it.j1) sj[tid] = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
+      if (j < it.j1) {
+        sj[tid] = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
+        if (ic && jt <= it.i0) sim[tid] = tip_image_d4(p, sj[tid].x, sj[tid].y, sj[tid].z);
+      }
       __syncthreads();
       int kmax = min(RD_TILE, it.j1 - jt);
       if (jt == it.i0)
-        tip_tile_f64<T_DIAG>(sj, kmax, x1, y1, z1, qd1, tid, p.image_charge, p, L2, K, ax, ay, az);
+        tip_tile_f64<T_DIAG>(sj, sim, im1, kmax, x1, y1, z1, qd1, tid, p.image_charge, L2, K, ax, ay, az);
       else if (jt > it.i0)
-        tip_tile_f64<T_UPPER>(sj, kmax, x1, y1, z1, qd1, -1, p.image_charge, p, L2, K, ax, ay, az);
+        tip_tile_f64<T_UPPER>(sj, sim, im1, kmax, x1, y1, z1, qd1, -1, p.image_charge, L2, K, ax, ay, az);
       else
-        tip_tile_f64<T_LOWER>(sj, kmax, x1, y1, z1, qd1, -1, p.image_charge, p, L2, K, ax, ay, az);
+        tip_tile_f64<T_LOWER>(sj, sim, im1, kmax, x1, y1, z1, qd1, -1, p.image_charge, L2, K, ax, ay, az);
     }
     if (it.nch > 1) {
       double* pp = partial + (size_t)g * 3 * RD_ITILE;
@@ -443,6 +449,9 @@ k_force_tts_f64(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
       si = pool.species[off + i];
     }
     const double qd1 = q1 * dfc;
+    const float L2x3 = (float)(3.0 * L2);
+    rd_d4 im1 = make_d4(0.0, 0.0, 0.0, 0.0);
+    if (tip && p.image_charge && valid) im1 = tip_image_d4(p, x1, y1, z1);
     double ax = 0.0, ay = 0.0, az = 0.0;
     for (int jt = it.j0; jt < it.j1; jt += RD_TILE) {
       __syncthreads();
@@ -460,12 +469,15 @@ k_force_tts_f64(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
                           (si == 2 && (sjk == 1 || (sjk == 2 && ion_step)));
         if (!take) continue;
         const bool upper = (si != sjk) ? (si == 1) : (jj > i);
-        if (tip)
-          tip_pair_f64(sj[k], x1, y1, z1, qd1, upper, p.image_charge, p, L2, K, ax, ay, az);
-        else
-          planar_pair_f64(sj[k], x1, y1, z1, qd1, upper, p.N_ic_max, p.d, p.image_charge, L2, ax, ay, az);
+        if (tip) {
+          const rd_d4 im = !p.image_charge ? im1 : upper ? im1 : tip_image_d4(p, sj[k].x, sj[k].y, sj[k].z);
+          tip_pair_f64(sj[k], im, x1, y1, z1, upper, p.image_charge, L2, L2x3, K, ax, ay, az);
+        } else {
+          planar_pair_f64(sj[k], x1, y1, z1, upper, p.N_ic_max, p.d, p.image_charge, L2, L2x3, ax, ay, az);
+        }
       }
     }
+    ax *= qd1; ay *= qd1; az *= qd1;
     if (it.nch > 1) {
       double* pp = partial + (size_t)g * 3 * RD_ITILE;
       pp[tid] = ax; pp[RD_ITILE + tid] = ay; pp[2 * RD_ITILE + tid] = az;

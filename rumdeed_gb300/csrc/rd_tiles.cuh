@@ -3,6 +3,7 @@
 // point, always in the upper role: the point images / is imaged as the "a"
 // argument of the reference image functions).
 #pragma once
+#include "rd_f64.cuh"
 #include "rd_pair.cuh"
 
 enum { T_UPPER = 0, T_LOWER = 1, T_DIAG = 2 };
@@ -86,44 +87,51 @@ __device__ __forceinline__ void planar_tile_f32(const float4* __restrict__ sh, c
   tx += sx; ty += sy; tz += sz;
 }
 
-// ---- planar, FP64 (reference arithmetic) ---------------------------------------
-// One pair (i, j): Coulomb term plus, with image charges on, the planar
-// series of acc_ic_planar_series.inc with i in the "a" role when upper and j
-// in it otherwise (the x, y parts then change sign: force_ic_N).
-__device__ __forceinline__ void planar_pair_f64(const rd_d4& pj, double x1, double y1, double z1,
-                                                double qd1, bool upper, int nic, double d, int ic,
-                                                double L2, double& ax, double& ay, double& az) {
-  double pre = qd1 * pj.w;
-  double dx = x1 - pj.x, dy = y1 - pj.y, dz = z1 - pj.z;
-  double dxy2 = dx * dx + dy * dy;
-  double r = sqrt(dxy2 + dz * dz) + L2;
-  double inv = 1.0 / ((r * r) * r);
-  ax = ax + (pre * inv) * dx;
-  ay = ay + (pre * inv) * dy;
-  az = az + (pre * inv) * dz;
+// ---- planar, FP64 --------------------------------------------------------------
+// One pair (i, j) of acc_ic_planar_series.inc's sum, without the factor q_i k: the
+// Coulomb term plus, with image charges on, the partners' with i in the "a" role
+// when upper and j in it otherwise (the x, y parts then change sign: force_ic_N).
+// Every term shares dx, dy, so their inverse cubes are added up first.  25 FP64
+// operations with one image partner (50 with sqrt and division, rd_f64.cuh).
+__device__ __forceinline__ double planar_inv_f64(double s, double L2, float L2x3) {
+  return rd_cube_ok(s) ? rd_inv_cube(s, L2x3) : rd_inv_cube_any(s, L2);
+}
+__device__ __forceinline__ void planar_pair_f64(const rd_d4& pj, double x1, double y1, double z1, bool upper, int nic,
+                                                double d, int ic, double L2, float L2x3, double& ax, double& ay,
+                                                double& az) {
+  const double dx = x1 - pj.x, dy = y1 - pj.y, dz = z1 - pj.z;
+  const double dxy2 = fma(dx, dx, dy * dy);
+  const double r2 = fma(dz, dz, dxy2);
+  double t, tz;
   if (ic) {
-    double za = upper ? z1 : pj.z, zb = upper ? pj.z : z1;
-    // acc_ic_planar_series.inc
-    double zic = -1.0 * zb, dzi = za - zic;
-    r = sqrt(dxy2 + dzi * dzi) + L2;
-    inv = 1.0 / ((r * r) * r);
-    double icx = -dx * inv, icy = -dy * inv, icz = -dzi * inv;
-    for (int n = 1; n <= nic; ++n) {
-      double zz0 = (2.0 * n) * d - zb, zz1 = (-2.0 * n) * d - zb;
-      double zz2 = (2.0 * n) * d + zb, zz3 = (-2.0 * n) * d + zb;
-      dzi = za - zz0; r = sqrt(dxy2 + dzi * dzi) + L2; inv = 1.0 / ((r * r) * r);
-      icx = icx - dx * inv; icy = icy - dy * inv; icz = icz - dzi * inv;
-      dzi = za - zz1; r = sqrt(dxy2 + dzi * dzi) + L2; inv = 1.0 / ((r * r) * r);
-      icx = icx - dx * inv; icy = icy - dy * inv; icz = icz - dzi * inv;
-      dzi = za - zz2; r = sqrt(dxy2 + dzi * dzi) + L2; inv = 1.0 / ((r * r) * r);
-      icx = icx + dx * inv; icy = icy + dy * inv; icz = icz + dzi * inv;
-      dzi = za - zz3; r = sqrt(dxy2 + dzi * dzi) + L2; inv = 1.0 / ((r * r) * r);
-      icx = icx + dx * inv; icy = icy + dy * inv; icz = icz + dzi * inv;
+    const double zs = z1 + pj.z, s2 = fma(zs, zs, dxy2);   // the n = 0 partner at -z
+    double inv, ini;
+    if (rd_cube_ok(r2) && rd_cube_ok(s2)) {
+      inv = rd_inv_cube(r2, L2x3);
+      ini = rd_inv_cube(s2, L2x3);
+    } else {
+      inv = rd_inv_cube_any(r2, L2);
+      ini = rd_inv_cube_any(s2, L2);
     }
-    ax = ax + pre * icx;
-    ay = ay + pre * icy;
-    az = az + pre * icz;
+    t = inv - ini;
+    tz = fma(inv, dz, -(ini * zs));
+    const double da = upper ? dz : -dz;
+    for (int n = 1; n <= nic; ++n) {
+      const double nd = (2.0 * n) * d;
+      const double h0 = zs - nd, h1 = zs + nd, h2 = da - nd, h3 = da + nd;   // partners at 2nd - z, -2nd - z, 2nd + z, -2nd + z
+      const double i0 = planar_inv_f64(fma(h0, h0, dxy2), L2, L2x3), i1 = planar_inv_f64(fma(h1, h1, dxy2), L2, L2x3);
+      const double i2 = planar_inv_f64(fma(h2, h2, dxy2), L2, L2x3), i3 = planar_inv_f64(fma(h3, h3, dxy2), L2, L2x3);
+      t += (i2 + i3) - (i0 + i1);
+      tz = fma(i2, h2, fma(i3, h3, fma(-i0, h0, fma(-i1, h1, tz))));
+    }
+  } else {
+    t = planar_inv_f64(r2, L2, L2x3);
+    tz = t * dz;
   }
+  const double w = pj.w * t;
+  ax = fma(w, dx, ax);
+  ay = fma(w, dy, ay);
+  az = fma(pj.w, tz, az);
 }
 
 template <int MODE>
@@ -131,11 +139,16 @@ __device__ __forceinline__ void planar_tile_f64(const rd_d4* __restrict__ sj, in
                                                 double y1, double z1, double qd1, int self_k,
                                                 int nic, double d, int ic, double L2,
                                                 double& ax, double& ay, double& az) {
+  const float L2x3 = (float)(3.0 * L2);
+  double tx = 0.0, ty = 0.0, tz = 0.0;
   for (int k = 0; k < kmax; ++k) {
     if (MODE == T_DIAG && k == self_k) continue;
     const bool upper = (MODE == T_UPPER) || (MODE == T_DIAG && k > self_k);
-    planar_pair_f64(sj[k], x1, y1, z1, qd1, upper, nic, d, ic, L2, ax, ay, az);
+    planar_pair_f64(sj[k], x1, y1, z1, upper, nic, d, ic, L2, L2x3, tx, ty, tz);
   }
+  ax = fma(qd1, tx, ax);
+  ay = fma(qd1, ty, ay);
+  az = fma(qd1, tz, az);
 }
 
 // ---- hyperboloid tip -------------------------------------------------------------
@@ -211,47 +224,62 @@ __device__ __forceinline__ void tip_split_finish(double Dx, double Dy, double Dz
   *fz = (1.0 + K) * Dz + K * (((double)t.wz - c * (double)t.uz) - 2.0 * (double)t.lz);
 }
 
-// FP64 tip gather: Calculate_Acceleration_Particles_ACC tip branch (:1344-1426).
-// One pair (i, j); upper: i is the lower-indexed ("a") particle.
-__device__ __forceinline__ void tip_pair_f64(const rd_d4& pj, double x1, double y1, double z1,
-                                             double qd1, bool upper, int ic, const DiodeParams& p,
-                                             double L2, double K, double& ax, double& ay,
-                                             double& az) {
-  const double z0 = p.h_tip - p.r_tip, R = p.r_tip;
-  double pre = qd1 * pj.w;
-  double dx = x1 - pj.x, dy = y1 - pj.y, dz = z1 - pj.z;
-  double r = sqrt(dx * dx + dy * dy + dz * dz) + L2;
-  double inv = 1.0 / ((r * r) * r);
-  ax = ax + (pre * inv) * dx;
-  ay = ay + (pre * inv) * dy;
-  az = az + (pre * inv) * dz;
-  if (ic) {
-    double xa = upper ? x1 : pj.x, ya = upper ? y1 : pj.y, za = upper ? z1 : pj.z;
-    double xb = upper ? pj.x : x1, yb = upper ? pj.y : y1, zb = upper ? pj.z : z1;
-    double sgn = upper ? 1.0 : -1.0;
-    double dza = za - z0;
-    double dis = sqrt(xa * xa + ya * ya + dza * dza);
-    double zim = z0 + (R * R) / (sqrt((1.0 + (xa * xa) / (dza * dza)) + (ya * ya) / (dza * dza)) * dis);
-    double xim = ((zim - z0) * xa) / dza, yim = ((zim - z0) * ya) / dza;
-    double tda = pow((xb - xa) * (xb - xa) + (yb - ya) * (yb - ya) + (zb - za) * (zb - za), 1.5);
-    double tdb = pow((xb - xim) * (xb - xim) + (yb - yim) * (yb - yim) + (zb - zim) * (zb - zim), 1.5);
-    double icx = K * ((xa - xb) / tda - (R * (xim - xb)) / (dis * tdb));
-    double icy = K * ((ya - yb) / tda - (R * (yim - yb)) / (dis * tdb));
-    double icz = K * ((za - zb) / tda - (R * (zim - zb)) / (dis * tdb));
-    ax = ax + pre * sgn * icx;
-    ay = ay + pre * sgn * icy;
-    az = az + pre * icz;
+// FP64 tip gather: Calculate_Acceleration_Particles_ACC tip branch (:1344-1426),
+// without the factor q_i k.  One pair (i, j); upper: i is the lower-indexed ("a")
+// particle.  im: the image point of the "a" particle in the apex sphere and c = R /
+// dis_a (tip_image_d4), the same for every pair a particle has that role in.  The
+// image term's two distances to the power 3/2 are inverse cubes without the l^2, the
+// first of them the Coulomb term's distance.  36 FP64 operations; with the image
+// point formed per pair and pow(., 1.5) for the cubes a pair took several hundred.
+__device__ __forceinline__ rd_d4 tip_image_d4(const DiodeParams& p, double xa, double ya, double za) {
+  double xi, yi, zi;
+  const double dis = tip_image_point(p, xa, ya, za, &xi, &yi, &zi);
+  return make_d4(xi, yi, zi, p.r_tip / dis);
+}
+__device__ __forceinline__ void tip_pair_f64(const rd_d4& pj, const rd_d4& im, double x1, double y1, double z1,
+                                             bool upper, int ic, double L2, float L2x3, double K, double& ax,
+                                             double& ay, double& az) {
+  const double dx = x1 - pj.x, dy = y1 - pj.y, dz = z1 - pj.z;
+  const double r2 = fma(dz, dz, fma(dx, dx, dy * dy));
+  double inv, ina;
+  if (rd_cube_ok(r2)) {
+    inv = rd_inv_cube<true>(r2, L2x3, &ina);
+  } else {
+    inv = rd_inv_cube_any(r2, L2);
+    ina = rd_inv_cube_any(r2, 0.0);
   }
+  if (!ic) {
+    const double w = pj.w * inv;
+    ax = fma(w, dx, ax); ay = fma(w, dy, ay); az = fma(w, dz, az);
+    return;
+  }
+  // b: the particle that is not the "a" one.  x, y of the image term change sign for it.
+  const double ex = im.x - (upper ? pj.x : x1), ey = im.y - (upper ? pj.y : y1), ez = im.z - (upper ? pj.z : z1);
+  const double s2 = fma(ez, ez, fma(ex, ex, ey * ey));
+  const double inb = rd_cube_ok(s2) ? rd_inv_cube0(s2) : rd_inv_cube_any(s2, 0.0);
+  const double kb = K * (im.w * inb), ka = K * ina, kbs = upper ? kb : -kb;
+  // upper: a - b = d; lower: a - b = -d, x and y mirrored
+  const double wd = inv + ka, wz = upper ? wd : inv - ka;
+  ax = fma(pj.w, fma(wd, dx, -(kbs * ex)), ax);
+  ay = fma(pj.w, fma(wd, dy, -(kbs * ey)), ay);
+  az = fma(pj.w, fma(wz, dz, -(kb * ez)), az);
 }
 
+// im1: the point's own image (it is the "a" particle of the pairs with j above);
+// sim: the images of the tile's particles (not read in T_UPPER).
 template <int MODE>
-__device__ __forceinline__ void tip_tile_f64(const rd_d4* __restrict__ sj, int kmax, double x1,
-                                             double y1, double z1, double qd1, int self_k, int ic,
-                                             const DiodeParams& p, double L2, double K,
-                                             double& ax, double& ay, double& az) {
+__device__ __forceinline__ void tip_tile_f64(const rd_d4* __restrict__ sj, const rd_d4* __restrict__ sim,
+                                             const rd_d4& im1, int kmax, double x1, double y1, double z1, double qd1,
+                                             int self_k, int ic, double L2, double K, double& ax, double& ay,
+                                             double& az) {
+  const float L2x3 = (float)(3.0 * L2);
+  double tx = 0.0, ty = 0.0, tz = 0.0;
   for (int k = 0; k < kmax; ++k) {
     if (MODE == T_DIAG && k == self_k) continue;
     const bool upper = (MODE == T_UPPER) || (MODE == T_DIAG && k > self_k);
-    tip_pair_f64(sj[k], x1, y1, z1, qd1, upper, ic, p, L2, K, ax, ay, az);
+    tip_pair_f64(sj[k], upper ? im1 : sim[k], x1, y1, z1, upper, ic, L2, L2x3, K, tx, ty, tz);
   }
+  ax = fma(qd1, tx, ax);
+  ay = fma(qd1, ty, ay);
+  az = fma(qd1, tz, az);
 }
