@@ -235,6 +235,7 @@ struct rd_engine {
   double kscale = 0.0;
   int max_items = 0;
   int clen_min = RD_CLEN_MIN, nch_max = RD_NCH_MAX;   // chunk rule of the pair sums
+  bool chunk_auto = true;                             // no chunking set: shorter chunks for small systems
   // device memory
   DiodeParams* dP = nullptr;
   DiodeDyn* dD = nullptr;
@@ -381,10 +382,14 @@ static int alloc_pool(rd_engine* e, Pool& P, long long cap) {
 }
 
 // ---- pipeline pieces ----------------------------------------------------------------
+static int chunk_rule(const rd_engine* e) {
+  return rd_chunk_rule(e->clen_min, e->nch_max, e->chunk_auto ? RD_ITEMS : 0);
+}
+
 static cudaError_t plan_on(rd_engine* e, int mode, cudaStream_t st, const int* npts = nullptr) {
   e->kernels_in_step++;
   const int slot = mode & 0xff;
-  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), mode, rd_chunk_rule(e->clen_min, e->nch_max),
+  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), mode, chunk_rule(e),
                         e->max_items, npts, e->plan[slot], e->ph[slot]);
 }
 static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) { return plan_on(e, mode, e->st, npts); }
@@ -692,9 +697,9 @@ static int launch_step_body(rd_engine* e) {
 static std::string sig_string(rd_engine* e) {
   Sig s = signature(e);
   char b[128];
-  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
+  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
            s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.mh_near > 1 ? 2 : s.mh_near, s.mh_planar > s.mh_near,
-           s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
+           e->chunk_auto, s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
   return b;
 }
 
@@ -767,7 +772,7 @@ int rd_engine_view(rd_engine* e, int diode, const DiodeParams** P, const DiodeDy
 }
 
 int rd_engine_repack(rd_engine* e) { return repack(e); }
-int rd_engine_chunk_rule(rd_engine* e) { return rd_chunk_rule(e->clen_min, e->nch_max); }
+int rd_engine_chunk_rule(rd_engine* e) { return chunk_rule(e); }
 
 // ---- C ABI ----------------------------------------------------------------------------
 extern "C" {
@@ -797,6 +802,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
   e->grid = cfg->grid_blocks > 0 ? cfg->grid_blocks : 0;   // 0: occupancy-based per kernel
   e->clen_min = cfg->chunk_min > 0 ? cfg->chunk_min : RD_CLEN_MIN;
   e->nch_max = cfg->chunk_count_max > 0 ? cfg->chunk_count_max : RD_NCH_MAX;
+  e->chunk_auto = cfg->chunk_min <= 0 && cfg->chunk_count_max <= 0;
   if ((ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking)) != cudaSuccess ||
       (ce = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming)) != cudaSuccess)
     return bail(fail(RD_ERR_CUDA, cudaGetErrorString(ce)));
@@ -1611,6 +1617,8 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   // jumps that take the pair sums (near / far split: only the start and the last points)
   const int jumps = signature(e).mh_slow() ? std::max(signature(e).jumps, 1) : 2;
   const int saved_min = e->clen_min, saved_max = e->nch_max;
+  const bool saved_auto = e->chunk_auto;
+  e->chunk_auto = false;
   const int user_parts = e->mh_parts, user_form = e->mh_form;
   e->mh_parts = 0;    // the chunking is searched at the default launch shape
   e->mh_form = -1;
@@ -1624,7 +1632,7 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
       e->nch_max = b;
       double fms = 0.0, mms = 0.0;
       if ((rc = time_pair_passes(e, 2, &fms, &mms))) {
-        e->clen_min = saved_min; e->nch_max = saved_max; e->mh_parts = user_parts; e->mh_form = user_form;
+        e->clen_min = saved_min; e->nch_max = saved_max; e->chunk_auto = saved_auto; e->mh_parts = user_parts; e->mh_form = user_form;
         return rc;
       }
       const double est = fms + jumps * mms;
@@ -1717,6 +1725,7 @@ int rd_set_chunking(rd_engine* e, int chunk_min, int chunk_count_max) {
     return fail(RD_ERR_INVALID, "chunk_min must be a multiple of 128 in [128, 65536], chunk_count_max in [1, 32]");
   e->clen_min = a;
   e->nch_max = b;
+  e->chunk_auto = chunk_min <= 0 && chunk_count_max <= 0;
   return RD_OK;
 }
 

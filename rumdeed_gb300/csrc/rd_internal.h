@@ -36,8 +36,18 @@
 // RD_NCH_MAX chunks per i-tile
 #define RD_CLEN_MIN 1024
 #define RD_NCH_MAX 32
-// the planner's chunk rule argument: clen_min | nch_max << 16
-inline int rd_chunk_rule(int clen_min, int nch_max) { return clen_min | (nch_max << 16); }
+// Without a chunking set by hand, a pair sum of fewer tiles than the GPU has room for
+// takes shorter chunks (down to one j-tile), enough for RD_ITEMS items: 16 per SM.
+// The rule looks only at the diode's own counts.  Measured with 0 (chunks of 1024) /
+// 640 / 1216 / 2432 / 4864 items: forces of 6000 electrons in FP64 2.88 / 2.42 / 2.04 /
+// 2.03 / 2.04 ms, of 8191 with 29 image partners 1.12 / 1.00 / 0.84 / 0.75 / 0.76 ms;
+// a step with 1300 electrons and 960 FP64 chains 55.0 / 9.3 / 9.3 / 9.3 / 9.3 ms;
+// 128 diodes of 256-32768 electrons unchanged.
+#define RD_ITEMS 2432
+// the planner's chunk rule argument: clen_min | nch_max << 16 | (target items / 64) << 24
+inline int rd_chunk_rule(int clen_min, int nch_max, int target) {
+  return clen_min | (nch_max << 16) | ((target / 64) << 24);
+}
 #define RD_MAX_LIFE 1000
 #define RD_COMPACT_SPIN (1 << 22)   // polls (64 ns sleeps) of a compaction tile waiting on an earlier one
 #define RD_MH_FINAL (-2)      // k_mh_jump_planar: pair sums at the chains' last points (rd_near.cuh)

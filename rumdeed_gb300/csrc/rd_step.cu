@@ -129,12 +129,16 @@ __device__ __forceinline__ int plan_ni(const DiodeParams& p, const DiodeDyn& y, 
 // at most ~1024 particles also bound the cost of one work item, so the last
 // items of a launch end soon after the others.
 __device__ __forceinline__ void plan_split(int ni, int nj, int tsize, bool pair, int grow, int clen_min,
-                                           int nch_max, int* tiles, int* nch, int* clen) {
+                                           int nch_max, int target, int* tiles, int* nch, int* clen) {
   *tiles = (ni + tsize - 1) / tsize;
   *nch = 1;
   *clen = RD_TILE;
   if (pair && *tiles > 0) {
     int c = (nj + nch_max - 1) / nch_max;
+    if (target > 0) {   // a small system: short enough chunks for `target` items
+      const long long len = ((long long)nj * *tiles + target - 1) / target;
+      if (len < clen_min) clen_min = (int)len;
+    }
     if (c < clen_min) c = clen_min;
     c = ((c + RD_TILE - 1) / RD_TILE) * RD_TILE;
     c <<= grow;   // only if the scratch bound is ever hit (never by construction)
@@ -153,7 +157,7 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
   const int tid = threadIdx.x;
   const int tsize = (mode == PM_PART1024) ? 1024 : (mode == PM_MH_NEAR) ? RD_NEAR_CPB : RD_ITILE;
   const bool pair = (mode & 0xff) <= PM_SUPPLY_LAT || mode == PM_MH_SLOW;
-  const int clen_min = chunk_rule & 0xffff, nch_max = chunk_rule >> 16;   // see rd_chunk_rule
+  const int clen_min = chunk_rule & 0xffff, nch_max = (chunk_rule >> 16) & 0xff, target = (chunk_rule >> 24) * 64;   // rd_chunk_rule
   // the planar supply points are many tiles already: at most RD_SUP_NCH chunks per tile
   const int nch_eff = ((mode & 0xff) == PM_SUPPLY_PLANAR || (mode & 0xff) == PM_SUPPLY_LAT)
                           ? min(nch_max, RD_SUP_NCH) : nch_max;
@@ -167,7 +171,7 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
     for (int d = tid; d < nslots; d += blockDim.x) {
       if (!P[d].active) continue;
       int tiles, nch, clen;
-      plan_split(plan_ni(P[d], Dy[d], mode, npts, d), Dy[d].n, tsize, pair, grow, clen_min, nch_eff, &tiles,
+      plan_split(plan_ni(P[d], Dy[d], mode, npts, d), Dy[d].n, tsize, pair, grow, clen_min, nch_eff, target, &tiles,
                  &nch, &clen);
       cnt += (double)tiles * nch;
     }
@@ -194,7 +198,7 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
       nj = Dy[d].n;
       ni = plan_ni(P[d], Dy[d], mode, npts, d);
       if (mode == PM_MH) chains = ni;
-      plan_split(ni, nj, tsize, pair, grow, clen_min, nch_eff, &tiles, &nch, &clen);
+      plan_split(ni, nj, tsize, pair, grow, clen_min, nch_eff, target, &tiles, &nch, &clen);
       items = tiles * nch;
     }
     int lane = tid & 31, w = tid >> 5;
