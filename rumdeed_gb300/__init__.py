@@ -513,7 +513,9 @@ class Diode:
 
     @property
     def n(self):
-        return self.counters()["n"]
+        n = C.c_int()
+        _check(self.L.rd_get_particles(self.e.h, self.index, 0, None, None, None, None, None, None, C.byref(n)))
+        return n.value
 
     def particles(self):
         n = self.n

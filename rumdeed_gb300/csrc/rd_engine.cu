@@ -102,6 +102,14 @@ cudaError_t rd_launch_add_particles(cudaStream_t st, const DiodeParams* P, Diode
                                     const double* vel, const int* species, int step, int section);
 cudaError_t rd_launch_quad_fill(cudaStream_t st, const QuadSpec& q, double* qx, double* qy, double* qz,
                                 double* qw, float4* qpp);
+cudaError_t rd_launch_rows_out(cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy, const Pool& pool, int d,
+                               int r0, int rows, const RowsOut& o, unsigned char* out);
+cudaError_t rd_launch_points_in(cudaStream_t st, const double* in, int M, double* x, double* y, double* z, int* npts,
+                                int nslots, int d);
+cudaError_t rd_launch_points_out(cudaStream_t st, const double* x, const double* y, const double* z, int M,
+                                 double* out);
+cudaError_t rd_launch_state_in(cudaStream_t st, const DiodeParams* P, const Pool& pool, int d, int r0, int rows,
+                               const double* dbl, const int* in);
 cudaError_t rd_launch_mark(cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
                            int d, int i, int why);
 cudaError_t rd_launch_validate(int nslots, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
@@ -272,6 +280,9 @@ struct rd_engine {
   double* stage_hd = nullptr;   // pinned host mirrors of stage_d / stage_i: uploads are DMA
   int* stage_hi = nullptr;      // copies from page-locked memory
   long long stage_cap = 0;
+  unsigned char* io_h = nullptr;   // pinned buffer of the particle and point transfers
+  size_t io_cap = 0;
+  bool packs_stale = false;        // electrons emitted since the last pack (rd_do_emission alone)
   // overlapped admission (rd_serve): uploads on stream sa from a pinned arena into a device
   // arena, slots activated on st before the next step (activate_pending)
   cudaStream_t sa = nullptr;
@@ -724,6 +735,37 @@ static int ensure_graph(rd_engine* e) {
 static int repack(rd_engine* e) {
   CK(plan(e, PM_PART));
   CK(rd_launch_pack(e->grid, e->st, e->dP, e->pool, e->plan[PM_PART], e->ph[PM_PART]));
+  e->packs_stale = false;
+  return RD_OK;
+}
+
+// The FP32 packs follow every change of a position or charge (added, moved, marked,
+// loaded or compacted particles); only the electrons of an emission that no position
+// update has followed yet are without.
+static int fresh_packs(rd_engine* e) { return e->packs_stale ? repack(e) : RD_OK; }
+
+// Pinned space for a transfer of `want` bytes in one or more parts: the upload stage
+// where it holds a quarter of it, else a buffer of the engine's own (RD_IO_MAX at most).
+// Both are free here: every call that uses them waits for its kernels.
+#define RD_IO_MAX ((size_t)64 << 20)
+static int io_space(rd_engine* e, size_t want, unsigned char** buf, size_t* have) {
+  const size_t staged = sizeof(double) * (size_t)e->stage_cap;
+  if (want > e->io_cap && want <= 4 * staged) {
+    *buf = reinterpret_cast<unsigned char*>(e->stage_hd);
+    *have = staged;
+    return RD_OK;
+  }
+  if (want > e->io_cap && e->io_cap < RD_IO_MAX) {
+    if (e->io_h) cudaFreeHost(e->io_h);
+    e->io_h = nullptr;
+    e->io_cap = 0;
+    size_t cap = 1 << 19;
+    while (cap < want && cap < RD_IO_MAX) cap *= 2;
+    CK(cudaHostAlloc((void**)&e->io_h, cap, cudaHostAllocDefault));
+    e->io_cap = cap;
+  }
+  *buf = e->io_h;
+  *have = e->io_cap;
   return RD_OK;
 }
 
@@ -907,6 +949,7 @@ int rd_engine_destroy(rd_engine* e) {
   if (e->stage_i) cudaFree(e->stage_i);
   if (e->stage_hd) cudaFreeHost(e->stage_hd);
   if (e->stage_hi) cudaFreeHost(e->stage_hi);
+  if (e->io_h) cudaFreeHost(e->io_h);
   if (e->fpx) { cudaFree(e->fpx); cudaFree(e->fpy); cudaFree(e->fpz); cudaFree(e->ffx); cudaFree(e->ffy); cudaFree(e->ffz); }
   if (e->ev0) cudaEventDestroy(e->ev0);
   if (e->ev1) cudaEventDestroy(e->ev1);
@@ -1312,28 +1355,37 @@ int rd_get_particles(rd_engine* e, int d, int cap, double* pos, double* vel, dou
                      double* charge, int* id, int* section, int* n_out) {
   if (e) { const int rcf = flush_admissions(e); if (rcf) return rcf; }
   if (!valid_diode(e, d)) return fail(RD_ERR_NOTFOUND, "unknown diode");
-  DiodeDyn y;
-  int rc = read_dyn(e, d, &y);
+  double* vecs[3] = {pos, vel, acc};
+  const size_t row = 24 * ((pos != nullptr) + (vel != nullptr) + (acc != nullptr)) + 8 * (charge != nullptr) +
+                     4 * ((id != nullptr) + (section != nullptr));
+  // rows the arrays can take; the particle count comes with the first part
+  const int limit = row ? std::max(0, std::min(cap, e->slots[d].p.cap)) : 0;
+  unsigned char* io = nullptr;
+  size_t have = 0;
+  int rc = io_space(e, 64 + row * (size_t)limit, &io, &have);
   if (rc) return rc;
-  if (n_out) *n_out = y.n;
-  int n = std::min(y.n, cap);
-  if (n <= 0) return RD_OK;
-  const int off = e->slots[d].p.off;
-  std::vector<double> buf(n);
-  auto get3 = [&](double* dst, double* a, double* b, double* c2) -> int {
-    double* src[3] = {a, b, c2};
-    for (int k2 = 0; k2 < 3; ++k2) {
-      CK(cudaMemcpy(buf.data(), src[k2] + off, sizeof(double) * n, cudaMemcpyDeviceToHost));
-      for (int i = 0; i < n; ++i) dst[3 * i + k2] = buf[i];
-    }
-    return RD_OK;
-  };
-  if (pos && (rc = get3(pos, e->pool.x, e->pool.y, e->pool.z))) return rc;
-  if (vel && (rc = get3(vel, e->pool.vx, e->pool.vy, e->pool.vz))) return rc;
-  if (acc && (rc = get3(acc, e->pool.ax, e->pool.ay, e->pool.az))) return rc;
-  if (charge) CK(cudaMemcpy(charge, e->pool.q + off, sizeof(double) * n, cudaMemcpyDeviceToHost));
-  if (id) CK(cudaMemcpy(id, e->pool.id + off, sizeof(int) * n, cudaMemcpyDeviceToHost));
-  if (section) CK(cudaMemcpy(section, e->pool.section + off, sizeof(int) * n, cudaMemcpyDeviceToHost));
+  const int part = row ? (int)std::min<size_t>(std::max(limit, 1), (have - 64) / row) : 0;
+  int n = 0;
+  for (int r0 = 0; r0 == 0 || r0 < std::min(n, limit); r0 += std::max(part, 1)) {
+    const int rows = std::max(0, std::min(part, limit - r0));
+    RowsOut o;
+    long long at = 64;
+    auto take = [&](bool want, int bytes) { const long long k = want ? at : -1; if (want) at += (long long)bytes * rows; return k; };
+    for (int v = 0; v < 3; ++v) o.vec[v] = take(vecs[v] != nullptr, 24);
+    o.charge = take(charge != nullptr, 8);
+    o.id = take(id != nullptr, 4);
+    o.section = take(section != nullptr, 4);
+    CK(rd_launch_rows_out(e->st, e->dP, e->dD, e->pool, d, r0, rows, o, io));
+    CK(cudaStreamSynchronize(e->st));
+    n = *reinterpret_cast<const int*>(io);
+    const size_t m = (size_t)std::max(0, std::min(rows, n - r0));
+    for (int v = 0; v < 3; ++v)
+      if (vecs[v]) std::memcpy(vecs[v] + 3 * (size_t)r0, io + o.vec[v], 24 * m);
+    if (charge) std::memcpy(charge + r0, io + o.charge, 8 * m);
+    if (id) std::memcpy(id + r0, io + o.id, 4 * m);
+    if (section) std::memcpy(section + r0, io + o.section, 4 * m);
+  }
+  if (n_out) *n_out = n;
   return RD_OK;
 }
 
@@ -1371,30 +1423,35 @@ int rd_accel(rd_engine* e, int d, double* acc3n) {
   if (e) { const int rcf = flush_admissions(e); if (rcf) return rcf; }
   NvtxRange nvtx_range("rd_accel");
   if (!valid_diode(e, d)) return fail(RD_ERR_NOTFOUND, "unknown diode");
-  int rc = repack(e);
+  int rc = fresh_packs(e);
   if (rc) return rc;
   if ((rc = launch_force(e))) return rc;
-  CK(cudaStreamSynchronize(e->st));
   if (acc3n) return rd_get_particles(e, d, 1 << 30, nullptr, nullptr, acc3n, nullptr, nullptr, nullptr, nullptr);
+  CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }
 
-static int field_at_batch(rd_engine* e, int d, int M, const double* pos, double* field);
+static int field_at_batch(rd_engine* e, int d, int M, const double* pos, double* field, double* io);
 
 int rd_field_at(rd_engine* e, int d, int M, const double* pos, double* field) {
   if (e) { const int rcf = flush_admissions(e); if (rcf) return rcf; }
   NvtxRange nvtx_range("rd_field_at");
   if (!valid_diode(e, d)) return fail(RD_ERR_NOTFOUND, "unknown diode");
   if (M < 0 || (M > 0 && (!pos || !field))) return fail(RD_ERR_INVALID, "bad point arrays");
-  const int chunk = (e->max_items / 2) * RD_ITILE;
-  for (int m0 = 0; m0 < M; m0 += chunk) {
-    int rc = field_at_batch(e, d, std::min(chunk, M - m0), pos + 3LL * m0, field + 3LL * m0);
-    if (rc) return rc;
-  }
+  unsigned char* io = nullptr;
+  size_t have = 0;
+  int rc = io_space(e, 24 * (size_t)M, &io, &have);
+  if (rc) return rc;
+  const int chunk = (int)std::min<size_t>((size_t)(e->max_items / 2) * RD_ITILE, have / 24);
+  for (int m0 = 0; m0 < M; m0 += chunk)
+    if ((rc = field_at_batch(e, d, std::min(chunk, M - m0), pos + 3LL * m0, field + 3LL * m0,
+                             reinterpret_cast<double*>(io))))
+      return rc;
   return RD_OK;
 }
 
-static int field_at_batch(rd_engine* e, int d, int M, const double* pos, double* field) {
+// io: pinned space for 3 M doubles
+static int field_at_batch(rd_engine* e, int d, int M, const double* pos, double* field, double* io) {
   if (M == 0) return RD_OK;
   if (M > e->fcap) {
     if (e->fpx) { cudaFree(e->fpx); cudaFree(e->fpy); cudaFree(e->fpz); cudaFree(e->ffx); cudaFree(e->ffy); cudaFree(e->ffz); }
@@ -1403,28 +1460,17 @@ static int field_at_batch(rd_engine* e, int d, int M, const double* pos, double*
     for (auto b : bufs) CK(cudaMalloc(b, cap * sizeof(double)));
     e->fcap = cap;
   }
-  std::vector<double> h(M);
-  double* dsts[3] = {e->fpx, e->fpy, e->fpz};
-  for (int k2 = 0; k2 < 3; ++k2) {
-    for (int i = 0; i < M; ++i) h[i] = pos[3 * i + k2];
-    CK(cudaMemcpyAsync(dsts[k2], h.data(), sizeof(double) * M, cudaMemcpyHostToDevice, e->st));
-    CK(cudaStreamSynchronize(e->st));
-  }
-  std::vector<int> np(e->slots.size(), 0);
-  np[d] = M;
-  CK(cudaMemcpyAsync(e->d_npts, np.data(), sizeof(int) * np.size(), cudaMemcpyHostToDevice, e->st));
-  int rc = repack(e);
+  std::memcpy(io, pos, 24 * (size_t)M);
+  CK(rd_launch_points_in(e->st, io, M, e->fpx, e->fpy, e->fpz, e->d_npts, (int)e->slots.size(), d));
+  int rc = fresh_packs(e);
   if (rc) return rc;
   CK(plan(e, PM_FIELD, e->d_npts));
   PointSet pts{e->fpx, e->fpy, e->fpz, e->ffx, e->ffy, e->ffz, e->d_zero_off};
   CK(rd_launch_field_points(e->cfg.precision, e->slots[d].p.geometry, e->grid, e->st, e->dP, e->pool,
                             e->plan[PM_FIELD], e->ph[PM_FIELD], pts, e->partial, e->tickets, e->kscale));
-  double* srcs[3] = {e->ffx, e->ffy, e->ffz};
-  for (int k2 = 0; k2 < 3; ++k2) {
-    CK(cudaMemcpyAsync(h.data(), srcs[k2], sizeof(double) * M, cudaMemcpyDeviceToHost, e->st));
-    CK(cudaStreamSynchronize(e->st));
-    for (int i = 0; i < M; ++i) field[3 * i + k2] = h[i];
-  }
+  CK(rd_launch_points_out(e->st, e->ffx, e->ffy, e->ffz, M, io));
+  CK(cudaStreamSynchronize(e->st));
+  std::memcpy(field, io, 24 * (size_t)M);
   return RD_OK;
 }
 
@@ -1516,7 +1562,10 @@ int rd_time_field_at(rd_engine* e, int d, int M, const double* pos, int reps, do
   if (M <= 0 || !pos || !ms_per_eval || reps <= 0) return fail(RD_ERR_INVALID, "bad argument");
   if (M > (e->max_items / 2) * RD_ITILE) return fail(RD_ERR_CAPACITY, "too many points for one evaluation");
   std::vector<double> field(3LL * M);
-  int rc = field_at_batch(e, d, M, pos, field.data());   // uploads the points; warm-up
+  double* io = nullptr;
+  CK(cudaHostAlloc((void**)&io, 24 * (size_t)M, cudaHostAllocDefault));
+  const int rc = field_at_batch(e, d, M, pos, field.data(), io);   // uploads the points; warm-up
+  cudaFreeHost(io);
   if (rc) return rc;
   PointSet pts{e->fpx, e->fpy, e->fpz, e->ffx, e->ffy, e->ffz, e->d_zero_off};
   CK(cudaEventRecord(e->ev0, e->st));
@@ -1750,6 +1799,7 @@ int rd_do_emission(rd_engine* e, int step) {
   NvtxRange nvtx_range("rd_do_emission");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   CK(rd_launch_step_set(e->st, e->d_step, step));
+  e->packs_stale = true;
   int rc = launch_emission(e);
   if (rc) return rc;
   CK(cudaStreamSynchronize(e->st));
@@ -1761,8 +1811,9 @@ int rd_update_position(rd_engine* e, int step) {
   NvtxRange nvtx_range("rd_update_position");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   CK(rd_launch_step_set(e->st, e->d_step, step));
-  int rc = launch_update_position(e);
+  int rc = launch_update_position(e);   // packs every particle
   if (rc) return rc;
+  e->packs_stale = false;
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }
@@ -1793,6 +1844,7 @@ int rd_run(rd_engine* e, int first_step, int nsteps) {
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
   e->last_ms = ms;
+  if (nsteps > 0) e->packs_stale = false;
   return compaction_check(e);
 }
 
@@ -1944,26 +1996,44 @@ int rd_diode_load(rd_engine* e, int d, const void* buf, long long size) {
   if (size < state_bytes(h.n)) return fail(RD_ERR_INVALID, "diode state truncated");
   const DiodeParams& p = e->slots[d].p;
   if (h.n > p.cap) return fail(RD_ERR_CAPACITY, "saved particles exceed the slot's capacity");
-  CK(cudaStreamSynchronize(e->st));
   in += sizeof h;
   DiodeDyn y;
   std::memcpy(&y, in, sizeof y);
   in += sizeof y;
-  const int off = p.off;
-  for (int k = 0; k < kStateDoubles; ++k, in += sizeof(double) * (size_t)h.n)
-    if (h.n) CK(cudaMemcpy(state_dbl(e->pool, k) + off, in, sizeof(double) * (size_t)h.n, cudaMemcpyHostToDevice));
+  const char* ints = in + kStateDoubles * sizeof(double) * (size_t)h.n;
+  const char* life = ints + kStateInts * sizeof(int) * (size_t)h.n;
   int rc = RD_OK;   // species is the first of the integer arrays
-  for (int i = 0; i < h.n && rc == RD_OK; ++i) {
+  for (int i = 0; i < h.n; ++i) {
     int sp;
-    std::memcpy(&sp, in + sizeof(int) * (size_t)i, sizeof sp);
-    if (sp != RD_SPECIES_ELEC) { rc = keep_pair_sum(e, d); break; }
+    std::memcpy(&sp, ints + sizeof(int) * (size_t)i, sizeof sp);
+    if (sp != RD_SPECIES_ELEC) {
+      if ((rc = keep_pair_sum(e, d))) return rc;
+      break;
+    }
   }
-  if (rc) return rc;
-  for (int k = 0; k < kStateInts; ++k, in += sizeof(int) * (size_t)h.n)
-    if (h.n) CK(cudaMemcpy(state_int(e->pool, k) + off, in, sizeof(int) * (size_t)h.n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(e->life + (size_t)d * RD_MAX_LIFE, in, sizeof(int) * RD_MAX_LIFE, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(e->dD + d, &y, sizeof y, cudaMemcpyHostToDevice));
-  if ((rc = repack(e))) return rc;   // the FP32 packs (and tip image points) of the loaded particles
+  const size_t row = kStateDoubles * sizeof(double) + kStateInts * sizeof(int);
+  const size_t head = sizeof(DiodeDyn) + sizeof(int) * RD_MAX_LIFE + 64;
+  unsigned char* io = nullptr;
+  size_t have = 0;
+  if ((rc = io_space(e, head + 16 + row * (size_t)h.n, &io, &have))) return rc;
+  const int part = (int)std::min<size_t>(std::max(h.n, 1), (have - head - 16) / row);
+  CK(cudaStreamSynchronize(e->st));
+  for (int r0 = 0; r0 < h.n; r0 += part) {
+    const int rows = std::min(part, h.n - r0);
+    double* hd = reinterpret_cast<double*>(io + ((head + 15) & ~(size_t)15));
+    int* hi = reinterpret_cast<int*>(hd + (size_t)kStateDoubles * rows);
+    for (int k = 0; k < kStateDoubles; ++k)
+      std::memcpy(hd + (size_t)k * rows, in + sizeof(double) * ((size_t)k * h.n + r0), sizeof(double) * (size_t)rows);
+    for (int k = 0; k < kStateInts; ++k)
+      std::memcpy(hi + (size_t)k * rows, ints + sizeof(int) * ((size_t)k * h.n + r0), sizeof(int) * (size_t)rows);
+    CK(rd_launch_state_in(e->st, e->dP, e->pool, d, r0, rows, hd, hi));   // with the FP32 packs
+    if (r0 + rows < h.n) CK(cudaStreamSynchronize(e->st));
+  }
+  std::memcpy(io, &y, sizeof y);
+  std::memcpy(io + sizeof y, life, sizeof(int) * RD_MAX_LIFE);
+  CK(cudaMemcpyAsync(e->dD + d, io, sizeof y, cudaMemcpyHostToDevice, e->st));
+  CK(cudaMemcpyAsync(e->life + (size_t)d * RD_MAX_LIFE, io + sizeof y, sizeof(int) * RD_MAX_LIFE,
+                     cudaMemcpyHostToDevice, e->st));
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }

@@ -251,3 +251,9 @@ struct NearState {
   unsigned long long *count, *progress;   // per slot: tiles done, accepted, rejected of a jump; jumps
                                           // done and step size (near_counts)
 };
+
+// Where k_rows_out puts a diode's particles in the host buffer (byte offsets; -1: not
+// asked for): positions, velocities, accelerations, charges, ids, sections.
+struct RowsOut {
+  long long vec[3], charge, id, section;
+};

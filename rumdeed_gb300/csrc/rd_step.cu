@@ -16,6 +16,8 @@
 //  * k_compact_*: stable, order-preserving compaction from the first dead
 //    index (Remove_Particles :352-562, compact_array :1180-1223) with the
 //    life-time histogram (record_lifetime :1135-1160).
+#include <algorithm>
+
 #include "rd_pair.cuh"
 
 namespace {
@@ -781,6 +783,107 @@ cudaError_t rd_launch_add_particles(cudaStream_t st, const DiodeParams* P, Diode
     k_add_particles<<<blocks, 256, 0, st>>>(P, Dy, pool, d, cnt, pos, vel, species, step, section);
   }
   k_add_finish<<<1, 1, 0, st>>>(P, Dy, d, cnt);
+  return cudaGetLastError();
+}
+
+// ---- host buffers ---------------------------------------------------------------
+// Particles and points cross to the host through a pinned buffer that these kernels
+// read and write directly (the link to the host is coherent), so a call takes one
+// launch and one synchronisation instead of a pageable copy per array with a strided
+// host loop behind it: the (3, N) layout is formed here, three neighbouring threads
+// writing the components of one row.  Bound by latency up to ~10^4 rows (a launch and
+// the wait), then by the link and the host's own copy.  A small force call, 300
+// electrons: 141 -> 69 us; the field of 65536 at 4096 points: 514 -> 425 us; forces of
+// 65536: 4.07 -> 3.94 ms.
+
+// Rows [r0, r0 + rows) of diode d's particles, at most its n: each array asked for at
+// its offset of `out` (bytes, rows apart by `rows`); n itself at out[0].
+__global__ void __launch_bounds__(256)
+k_rows_out(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, int d, int r0, int rows,
+           RowsOut o, unsigned char* __restrict__ out) {
+  const int n = Dy[d].n, off = P[d].off + r0;
+  const int m = min(rows, n - r0);
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  if (t0 == 0) *reinterpret_cast<int*>(out) = n;
+  const double* const src[3][3] = {{pool.x, pool.y, pool.z}, {pool.vx, pool.vy, pool.vz}, {pool.ax, pool.ay, pool.az}};
+  for (int v = 0; v < 3; ++v) {
+    if (o.vec[v] < 0) continue;
+    double* dst = reinterpret_cast<double*>(out + o.vec[v]);
+    for (int t = t0; t < 3 * m; t += nt) {
+      const int i = t / 3, c = t - 3 * i;
+      dst[t] = (c == 0 ? src[v][0] : c == 1 ? src[v][1] : src[v][2])[off + i];
+    }
+  }
+  if (o.charge >= 0)
+    for (int t = t0; t < m; t += nt) reinterpret_cast<double*>(out + o.charge)[t] = pool.q[off + t];
+  if (o.id >= 0)
+    for (int t = t0; t < m; t += nt) reinterpret_cast<int*>(out + o.id)[t] = pool.id[off + t];
+  if (o.section >= 0)
+    for (int t = t0; t < m; t += nt) reinterpret_cast<int*>(out + o.section)[t] = pool.section[off + t];
+}
+
+cudaError_t rd_launch_rows_out(cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy, const Pool& pool, int d,
+                               int r0, int rows, const RowsOut& o, unsigned char* out) {
+  const int blocks = std::min(608, std::max(1, (3 * rows + 255) / 256));
+  k_rows_out<<<blocks, 256, 0, st>>>(P, Dy, pool, d, r0, rows, o, out);
+  return cudaGetLastError();
+}
+
+// M points, (3, M) in the pinned buffer, to the field kernels' arrays, and the point
+// counts of the slots (M for slot d, 0 for the others).
+__global__ void __launch_bounds__(256)
+k_points_in(const double* __restrict__ in, int M, double* __restrict__ x, double* __restrict__ y,
+            double* __restrict__ z, int* __restrict__ npts, int nslots, int d) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (int s = t0; s < nslots; s += nt) npts[s] = s == d ? M : 0;
+  for (int t = t0; t < 3 * M; t += nt) {
+    const int i = t / 3, c = t - 3 * i;
+    (c == 0 ? x : c == 1 ? y : z)[i] = in[t];
+  }
+}
+__global__ void __launch_bounds__(256)
+k_points_out(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z, int M,
+             double* __restrict__ out) {
+  const int t0 = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (int t = t0; t < 3 * M; t += nt) {
+    const int i = t / 3, c = t - 3 * i;
+    out[t] = (c == 0 ? x : c == 1 ? y : z)[i];
+  }
+}
+
+cudaError_t rd_launch_points_in(cudaStream_t st, const double* in, int M, double* x, double* y, double* z, int* npts,
+                                int nslots, int d) {
+  const int blocks = std::min(608, std::max(1, (std::max(3 * M, nslots) + 255) / 256));
+  k_points_in<<<blocks, 256, 0, st>>>(in, M, x, y, z, npts, nslots, d);
+  return cudaGetLastError();
+}
+cudaError_t rd_launch_points_out(cudaStream_t st, const double* x, const double* y, const double* z, int M,
+                                 double* out) {
+  k_points_out<<<std::min(608, (3 * M + 255) / 256), 256, 0, st>>>(x, y, z, M, out);
+  return cudaGetLastError();
+}
+
+// A checkpoint's particle arrays (17 of doubles, then 5 of ints, n each) from the
+// pinned buffer into diode d's slots [r0, r0 + rows), packed for the FP32 forms.
+__global__ void __launch_bounds__(256)
+k_state_in(const DiodeParams* __restrict__ P, Pool pool, int d, int r0, int rows, const double* __restrict__ dbl,
+           const int* __restrict__ in) {
+  const DiodeParams& p = P[d];
+  double* const a[17] = {pool.x, pool.y, pool.z, pool.vx, pool.vy, pool.vz, pool.ax, pool.ay, pool.az,
+                         pool.bx, pool.by, pool.bz, pool.cx, pool.cy, pool.cz, pool.q, pool.m};
+  int* const b[5] = {pool.species, pool.id, pool.step0, pool.section, pool.mask};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+    const int gi = p.off + r0 + i;
+#pragma unroll
+    for (int k = 0; k < 17; ++k) a[k][gi] = dbl[(size_t)k * rows + i];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) b[k][gi] = in[(size_t)k * rows + i];
+    pack_one(p, pool, gi);
+  }
+}
+cudaError_t rd_launch_state_in(cudaStream_t st, const DiodeParams* P, const Pool& pool, int d, int r0, int rows,
+                               const double* dbl, const int* in) {
+  k_state_in<<<std::min(608, (rows + 255) / 256), 256, 0, st>>>(P, pool, d, r0, rows, dbl, in);
   return cudaGetLastError();
 }
 
