@@ -141,8 +141,12 @@ __device__ __forceinline__ double work_at(const DiodeParams& P, const double* wo
     if (sec) *sec = (int)w[4 * k + 3];
     return w[4 * k + 2];
   }
-  double xs = (x - P.em_x0) / P.em_Lx, ys = (y - P.em_y0) / P.em_Ly;
   int nx = P.work_nx, ny = P.work_ny;
+  if (nx == 1 && ny == 1) {   // one cell, whatever the point: no FP64 divisions
+    if (sec) *sec = 1;
+    return w[0];
+  }
+  double xs = (x - P.em_x0) / P.em_Lx, ys = (y - P.em_y0) / P.em_Ly;
   int xi = (int)floor(xs / (1.0 / nx)) + 1, yi = (int)floor(ys / (1.0 / ny)) + 1;
   xi = xi > nx ? nx : (xi < 1 ? 1 : xi);
   yi = yi > ny ? ny : (yi < 1 ? 1 : yi);

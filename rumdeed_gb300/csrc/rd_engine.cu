@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <chrono>
 #include <deque>
+#include <initializer_list>
 #include <map>
 #include <cmath>
 #include <cstdio>
@@ -50,7 +51,7 @@ cudaError_t rd_launch_z0_points(int prec, int grid, cudaStream_t st, const Diode
                                 double* partial, int* tickets, double kscale, int* queue);
 cudaError_t rd_launch_supply_reduce(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                                     const double* qx, const double* qy, const double* qw,
-                                    const double* qF, const double* qfx, const double* qfy,
+                                    const double* qF, const double* qfx, const double* qfy, double* qS,
                                     const double* work, const int* step_ptr, double* sup_part);
 cudaError_t rd_launch_mh_serial(int prec, int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                                 const Pool& pool, const double* work, const double* wtab,
@@ -80,8 +81,7 @@ cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, Di
                            const Pool& pool, const ChainState& cs, const int* ch_off,
                            const double* work, const int* step_ptr, const EventLog& ev);
 cudaError_t rd_launch_plan(cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy, int nslots,
-                           int mode, int chunk_rule, int max_items, const int* npts,
-                           PlanEntry* plan, PlanHeader* ph);
+                           const PlanJobs& jobs, int chunk_rule, int max_items, const int* npts);
 cudaError_t rd_launch_pack(int grid, cudaStream_t st, const DiodeParams* P, const Pool& pool,
                            const PlanEntry* plan, const PlanHeader* ph);
 cudaError_t rd_launch_position(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
@@ -252,7 +252,8 @@ struct rd_engine {
   std::vector<void*> allocs;
   double* work = nullptr;
   double* wtab = nullptr;   // per work cell: log phi, log(l_const/phi^2), l_const/phi^2
-  double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr, *qF = nullptr, *qfx = nullptr, *qfy = nullptr;
+  double *qx = nullptr, *qy = nullptr, *qz = nullptr, *qw = nullptr, *qF = nullptr, *qfx = nullptr, *qfy = nullptr,
+         *qS = nullptr;   // qS: the points' shares of N_sup
   float4* qpp = nullptr;   // planar quadrature points in the FP32 frame
   ChainState cs{};
   NearState nr{};
@@ -397,13 +398,15 @@ static int chunk_rule(const rd_engine* e) {
   return rd_chunk_rule(e->clen_min, e->nch_max, e->chunk_auto ? RD_ITEMS : 0);
 }
 
-static cudaError_t plan_on(rd_engine* e, int mode, cudaStream_t st, const int* npts = nullptr) {
+// The plans of `modes` in one launch.
+static cudaError_t plans_on(rd_engine* e, std::initializer_list<int> modes, cudaStream_t st,
+                            const int* npts = nullptr) {
   e->kernels_in_step++;
-  const int slot = mode & 0xff;
-  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), mode, chunk_rule(e),
-                        e->max_items, npts, e->plan[slot], e->ph[slot]);
+  PlanJobs jobs{};
+  for (int m : modes) jobs.j[jobs.n++] = PlanJob{m, e->plan[m & 0xff], e->ph[m & 0xff]};
+  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), jobs, chunk_rule(e), e->max_items, npts);
 }
-static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) { return plan_on(e, mode, e->st, npts); }
+static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) { return plans_on(e, {mode}, e->st, npts); }
 
 static bool valid_chunking(int clen_min, int nch_max) {
   return clen_min >= RD_TILE && clen_min <= 65536 && clen_min % RD_TILE == 0 && nch_max >= 1 &&
@@ -438,6 +441,13 @@ static Sig signature(const rd_engine* e) {
     }
   }
   return s;
+}
+
+// The plans of the batched MH chains (counts of this step's supply).
+static cudaError_t plan_chains(rd_engine* e, const Sig& s) {
+  if (s.mh_near == 0) return plan(e, PM_MH);
+  if (s.mh_planar == s.mh_near) return plans_on(e, {PM_MH, PM_MH_NEAR}, e->st);
+  return plans_on(e, {PM_MH, PM_MH_NEAR, PM_MH_SLOW}, e->st);
 }
 
 // MH launch shape of the planar jumps for the resident mix: parts of the plan
@@ -493,11 +503,7 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
     CK(rd_launch_near_setup(e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_SUPPLY_PLANAR],
                             e->ph[PM_SUPPLY_PLANAR], e->qpp, e->qF, e->nr, e->kscale));
     e->kernels_in_step += 4;
-    CK(plan_on(e, PM_MH_NEAR, main));
-    if (slow) {
-      pm = PM_MH_SLOW;
-      CK(plan_on(e, pm, main));
-    }
+    if (slow) pm = PM_MH_SLOW;
   }
   if (near) {
     CK(rd_launch_mh_jumps_near(e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
@@ -608,9 +614,9 @@ static int launch_emission(rd_engine* e) {
     e->kernels_in_step++;
   }
   CK(rd_launch_supply_reduce(ns, e->st, e->dP, e->dD, e->qx, e->qy, e->qw, e->qF, e->qfx, e->qfy,
-                             e->work, e->d_step, e->sup_part));
+                             e->qS, e->work, e->d_step, e->sup_part));
   e->kernels_in_step += 2;
-  CK(plan(e, PM_MH));
+  CK(plan_chains(e, s));
   if (s.emit_planar) {   // diodes with no particle in flight: all their MH sampling in one launch
     CK(rd_launch_mh_vacuum(prec, ns, e->st, e->dP, e->dD, e->cs, e->d_choff, e->wtab, e->d_step, e->kscale));
     e->kernels_in_step += 2;   // uniform work functions, and the others
@@ -634,22 +640,25 @@ static int launch_emission(rd_engine* e) {
 static int launch_force(rd_engine* e, bool step_pass = false) {
   Sig s = signature(e);
   const int all = step_pass ? 0 : PM_ALL_DIODES;
+  if (!step_pass) {   // a step's plans are built with its position pass's (plan_particles)
+    if (s.planar && s.tip) CK(plans_on(e, {PM_FORCE_PLANAR | all, PM_FORCE_TIP | all}, e->st));
+    else if (s.planar) CK(plan(e, PM_FORCE_PLANAR | all));
+    else if (s.tip) CK(plan(e, PM_FORCE_TIP | all));
+  }
   if (s.planar) {
-    CK(plan(e, PM_FORCE_PLANAR | all));
     CK(rd_launch_force(e->cfg.precision, 1, s.nic ? 1 : 0, e->grid, e->st, e->dP, e->dD, e->pool,
                        e->plan[PM_FORCE_PLANAR], e->ph[PM_FORCE_PLANAR], e->partial, e->tickets,
                        e->kscale, e->item_queue + 4));
     e->kernels_in_step++;
   }
   if (s.tip) {
-    CK(plan(e, PM_FORCE_TIP | all));
     CK(rd_launch_force(e->cfg.precision, 2, 0, e->grid, e->st, e->dP, e->dD, e->pool,
                        e->plan[PM_FORCE_TIP], e->ph[PM_FORCE_TIP], e->partial, e->tickets,
                        e->kscale, e->item_queue + 4));
     e->kernels_in_step++;
   }
   if (step_pass && s.tts) {
-    CK(plan(e, PM_FORCE_TTS));
+    if (s.planar && s.tip) CK(plan(e, PM_FORCE_TTS));
     CK(rd_launch_force_tts(e->grid, e->st, e->dP, e->dD, e->pool, e->plan[PM_FORCE_TTS], e->ph[PM_FORCE_TTS],
                            e->partial, e->tickets, e->item_queue + 4, e->d_step));
     e->kernels_in_step++;
@@ -657,9 +666,19 @@ static int launch_force(rd_engine* e, bool step_pass = false) {
   return RD_OK;
 }
 
+// The plans over the particles for the rest of a step (their counts stay until the
+// compaction's end), in one launch.
+static cudaError_t plan_particles(rd_engine* e) {
+  const Sig s = signature(e);
+  const int f = s.planar ? PM_FORCE_PLANAR : PM_FORCE_TIP;
+  if (s.planar && s.tip) return plans_on(e, {PM_PART, PM_PART1024, PM_FORCE_PLANAR, PM_FORCE_TIP}, e->st);
+  if (s.tts) return plans_on(e, {PM_PART, PM_PART1024, f, PM_FORCE_TTS}, e->st);
+  return plans_on(e, {PM_PART, PM_PART1024, f}, e->st);
+}
+
 static int launch_update_position(rd_engine* e) {
   const int ns = e->nslots_hw();
-  CK(plan(e, PM_PART));
+  CK(plan_particles(e));
   CK(rd_launch_position(e->grid, e->st, e->dP, e->dD, e->pool, e->plan[PM_PART], e->ph[PM_PART], e->evlog,
                         e->d_step));
   e->kernels_in_step++;
@@ -684,8 +703,8 @@ static int compaction_check(rd_engine* e) {
   return RD_OK;
 }
 
-static int launch_remove(rd_engine* e) {
-  CK(plan(e, PM_PART1024));
+static int launch_remove(rd_engine* e, bool planned) {
+  if (!planned) CK(plan(e, PM_PART1024));
   CK(rd_launch_compact(e->grid, e->nslots_hw(), e->st, e->dP, e->dD, e->pool, e->plan[PM_PART1024],
                        e->ph[PM_PART1024], e->ccnt, e->cpre, e->cflag, e->cq, e->life, e->d_step));
   e->kernels_in_step += 4;
@@ -698,7 +717,7 @@ static int launch_step_body(rd_engine* e) {
   if (rc) return rc;
   rc = launch_update_position(e);
   if (rc) return rc;
-  rc = launch_remove(e);
+  rc = launch_remove(e, true);
   if (rc) return rc;
   CK(rd_launch_step_inc(e->st, e->d_step));
   e->kernels_in_step++;
@@ -884,7 +903,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
   if (e->dalloc(&e->dP, S) || e->dalloc(&e->dD, S) || e->dalloc(&e->work, (size_t)S * 4 + 4096) || e->dalloc(&e->wtab, 3 * ((size_t)S * 4 + 4096)) ||
       e->dalloc(&e->qx, qcap) || e->dalloc(&e->qy, qcap) || e->dalloc(&e->qz, qcap) ||
       e->dalloc(&e->qw, qcap) || e->dalloc(&e->qF, qcap) || e->dalloc(&e->qfx, qcap) ||
-      e->dalloc(&e->qfy, qcap) || e->dalloc(&e->qpp, qcap) || e->dalloc(&e->cs.gx, chcap) || e->dalloc(&e->cs.gy, chcap) ||
+      e->dalloc(&e->qfy, qcap) || e->dalloc(&e->qS, qcap) || e->dalloc(&e->qpp, qcap) || e->dalloc(&e->cs.gx, chcap) || e->dalloc(&e->cs.gy, chcap) ||
       e->dalloc(&e->cs.fx, chcap) || e->dalloc(&e->cs.fy, chcap) || e->dalloc(&e->cs.fsup, chcap) ||
       e->dalloc(&e->cs.fF, chcap) || e->dalloc(&e->cs.fe, chcap) ||
       e->dalloc(&e->cs.fgx, chcap) || e->dalloc(&e->cs.fgy, chcap) ||
@@ -893,7 +912,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
       e->dalloc(&e->d_choff, S) || e->dalloc(&e->d_qoff, S) ||
       e->dalloc(&e->d_npts, S) || e->dalloc(&e->d_zero_off, S) ||
       e->dalloc(&e->partial, (size_t)e->max_items * 3 * RD_ITILE) ||
-      e->dalloc(&e->tickets, e->max_items) ||
+      e->dalloc(&e->tickets, 3 * (size_t)e->max_items) ||
       e->dalloc(&e->ccnt, cunits) || e->dalloc(&e->cpre, cunits) || e->dalloc(&e->cflag, cunits) ||
       e->dalloc(&e->cq, 4) ||
       e->dalloc(&e->sup_part, (size_t)S * RD_SUP_SPLIT * 4) ||
@@ -913,7 +932,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
       return bail(fail(RD_ERR_NOMEM, "plan allocation failed"));
   cudaMemsetAsync(e->dP, 0, sizeof(DiodeParams) * S, e->st);
   cudaMemsetAsync(e->dD, 0, sizeof(DiodeDyn) * S, e->st);
-  cudaMemsetAsync(e->tickets, 0, sizeof(int) * e->max_items, e->st);
+  cudaMemsetAsync(e->tickets, 0, 3 * sizeof(int) * (size_t)e->max_items, e->st);
   cudaMemsetAsync(e->cq, 0, sizeof(int) * 4, e->st);
   cudaMemsetAsync(e->item_queue, 0, sizeof(int) * (8 + 2 * RD_MH_PARTS_MAX), e->st);
   if (e->evlog.count) cudaMemsetAsync(e->evlog.count, 0, sizeof(int), e->st);
@@ -1062,6 +1081,7 @@ static void near_params(const rd_engine* e, DiodeParams& p, int P, int Q) {
   p.nr_bx = P + 2 * RD_NEAR_M;
   p.nr_by = (P + 2 * RD_NEAR_M + 1) / 2;
   p.nr_Z = (float)(5.0 * std::max(ax, ay));
+  p.nr_hx = ax; p.nr_hy = ay;
   p.nr_Ez = (float)p.E_z;
   p.nr_ax = (float)ax; p.nr_ay = (float)ay;
   p.nr_iax = (float)(1.0 / ax); p.nr_iay = (float)(1.0 / ay);
@@ -1823,7 +1843,7 @@ int rd_remove_particles(rd_engine* e, int step) {
   NvtxRange nvtx_range("rd_remove_particles");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   CK(rd_launch_step_set(e->st, e->d_step, step));
-  int rc = launch_remove(e);
+  int rc = launch_remove(e, false);
   if (rc) return rc;
   CK(cudaStreamSynchronize(e->st));
   return compaction_check(e);
@@ -2087,8 +2107,8 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
       CK(rd_launch_field_points(prec, RD_G_TIP, e->grid, e->st, e->dP, e->pool, e->plan[PM_SUPPLY_TIP],
                                 e->ph[PM_SUPPLY_TIP], pts, e->partial, e->tickets, e->kscale));
     }
-    CK(rd_launch_supply_reduce(S, e->st, e->dP, e->dD, e->qx, e->qy, e->qw, e->qF, e->qfx, e->qfy, e->work,
-                               e->d_step, e->sup_part));
+    CK(rd_launch_supply_reduce(S, e->st, e->dP, e->dD, e->qx, e->qy, e->qw, e->qF, e->qfx, e->qfy, e->qS,
+                               e->work, e->d_step, e->sup_part));
     CK(cudaEventRecord(ev[1], e->st));
     CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
     CK(cudaStreamSynchronize(e->st));
@@ -2099,7 +2119,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
       out->supply_pair_evals += npt * dyn[d].n;
       out->mh_pair_evals += (long long)dyn[d].chains * dyn[d].n * sl.p.mh_jumps;
     }
-    CK(plan(e, PM_MH));
+    CK(plan_chains(e, s));
     if (s.emit_planar)
       CK(rd_launch_mh_vacuum(prec, S, e->st, e->dP, e->dD, e->cs, e->d_choff, e->wtab, e->d_step, e->kscale));
     const int gmask = (s.emit_planar ? 1 : 0) | (s.emit_tip ? 2 : 0);
@@ -2123,7 +2143,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
     CK(cudaEventRecord(ev[3], e->st));
   }
   CK(cudaEventRecord(ev[4], e->st));
-  CK(plan(e, PM_PART));
+  CK(plan_particles(e));
   CK(rd_launch_position(e->grid, e->st, e->dP, e->dD, e->pool, e->plan[PM_PART], e->ph[PM_PART], e->evlog,
                         e->d_step));
   CK(cudaEventRecord(ev[5], e->st));
@@ -2134,7 +2154,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
                         e->d_step));
   CK(cudaEventRecord(ev[7], e->st));
   CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
-  rc = launch_remove(e);
+  rc = launch_remove(e, true);
   if (rc) return rc;
   CK(rd_launch_step_inc(e->st, e->d_step));
   CK(cudaEventRecord(ev[8], e->st));

@@ -20,6 +20,7 @@
 //    streams keyed by the diode seed with counters (chain, iteration, step,
 //    purpose), so every chain is reproducible and independent of scheduling.
 #include <cooperative_groups.h>
+#include <algorithm>
 #include <type_traits>
 
 #include "rd_tiles.cuh"
@@ -498,7 +499,8 @@ __device__ __forceinline__ bool pair_partials(double* partial, int* tickets, con
 #pragma unroll
   for (int q = 0; q < CPT; ++q) {
     float H = 0.0f, L = 0.0f;
-    for (int c = 0; c < it.nch; ++c) {
+#pragma unroll 8
+    for (int c = 0; c < it.nch; ++c) {   // the loads of eight chunks in flight
       const float2 v = __ldcg(pf + (size_t)(it.base + c) * RD_ITILE + tid + q * nt);
       pair_add(H, L, v.x, v.y);
     }
@@ -581,25 +583,68 @@ __device__ __forceinline__ long nint_d(double x) {
 
 // N_sup = sum_k w_k A S(F_k), N_round = nint(N_sup + residual) (planar,
 // Do_Field_Emission_Planar_rectangle :282-285) or nint(N_sup) (tip, :488).
-// The FN supply of a point is FP64 transcendental work, so a diode's points
-// are spread over RD_SUP_SPLIT blocks (contiguous ranges); each block writes
-// its (supply, field) sums and k_supply_finish adds a diode's block sums in
-// block order, so N_sup depends only on the diode's own points.
+// The FN supply of a point is FP64 transcendental work, and an SM's FP64 pipe takes 16
+// clocks per warp instruction: k_supply_points evaluates the points with one thread
+// each over all SMs, k_supply_reduce only adds.  RD_SUP_SPLIT blocks per diode add
+// contiguous ranges, and the diode's last block to finish adds their sums in block
+// order, so N_sup depends only on the diode's own points.  One diode of 40,000 points:
+// 12 us; 51 with the evaluation in the 64 blocks and a second kernel whose one thread
+// added up.
 __device__ __forceinline__ bool supply_live(const DiodeParams& p, const DiodeDyn& y, const int* step_ptr) {
   return p.active && p.emission && *step_ptr - y.step_offset > p.emit_delay;   // emitter on (:181)
 }
 
-__global__ void __launch_bounds__(256)
-k_supply_reduce(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy,
+__global__ void __launch_bounds__(128)
+k_supply_points(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy,
                 const double* __restrict__ qx, const double* __restrict__ qy,
                 const double* __restrict__ qw, const double* __restrict__ qF,
                 const double* __restrict__ qfx, const double* __restrict__ qfy,
-                const double* __restrict__ work, const int* __restrict__ step_ptr,
-                double* __restrict__ sup_part) {
-  __shared__ double red[256];
-  const int d = blockIdx.x, b = blockIdx.y;
+                const double* __restrict__ work, const int* __restrict__ step_ptr, double* __restrict__ qS) {
+  const int d = blockIdx.y;
   const DiodeParams& p = P[d];
   if (!supply_live(p, Dy[d], step_ptr)) return;
+  const int npt = (p.geometry == RD_G_TIP) ? 10000 : p.quad_n * p.quad_n;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
+    const int k = p.q_off + i;
+    double F = qF[k], S = 0.0;
+    if (p.geometry == RD_G_TIP) {   // Field_normal :105-112
+      double nx, ny, nz;
+      tip_normal(p, qx[k], qy[k], &nx, &ny, &nz);
+      F = (nx * qfx[k] + ny * qfy[k]) + nz * F;
+    }
+    if (F < 0.0) {
+      if (p.geometry == RD_G_TIP) {
+        double t = fn_t_y(F, p.tip_phi, p.image_charge);   // Elec_Supply (tip) :1710-1718
+        S = (((qw[k] * c_k.a_FN) * (F * F)) * p.dt) / ((c_k.q0 * p.tip_phi) * (t * t));
+      } else {
+        double phi = work_at(p, work, qx[k], qy[k], nullptr);
+        S = fn_supply_v2(F, phi, p.image_charge, p.dt);   // times its weight in k_supply_reduce
+      }
+    }
+    qS[k] = S;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+k_supply_reduce(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy,
+                const double* __restrict__ qS, const double* __restrict__ qw, const double* __restrict__ qF,
+                const double* __restrict__ qfx, const double* __restrict__ qfy,
+                const int* __restrict__ step_ptr, double* __restrict__ sup_part) {
+  __shared__ double red[256];
+  __shared__ double s_sum[4];
+  __shared__ int s_last;
+  const int d = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  const DiodeParams& p = P[d];
+  if (!p.active || !p.emission) return;
+  DiodeDyn& y = Dy[d];
+  if (!supply_live(p, y, step_ptr)) {   // the emitter is not on yet (:181)
+    if (b == 0 && tid == 0) {
+      y.N_sup = 0.0; y.chains = y.chains_capped = y.chains_failed = 0;
+      y.mh_acc = y.mh_rej = y.mh_done = 0;
+      y.F_avg_z = 0.0; y.F_avg_x = 0.0; y.F_avg_y = 0.0; y.df_avg = 0.0;
+    }
+    return;
+  }
   const int npt = (p.geometry == RD_G_TIP) ? 10000 : p.quad_n * p.quad_n;
   const int per = (npt + RD_SUP_SPLIT - 1) / RD_SUP_SPLIT;
   const int k0 = b * per, k1 = min(npt, k0 + per);
@@ -607,58 +652,42 @@ k_supply_reduce(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
   // their lateral mean goes to field.dt too
   const bool lat = p.geometry == RD_G_PLANAR && !p.image_charge;
   double acc = 0.0, fsum = 0.0, fxs = 0.0, fys = 0.0;
-  for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    double F = qF[p.q_off + k];
-    fsum += F;
+  for (int k = k0 + tid; k < k1; k += blockDim.x) {
+    if (p.geometry == RD_G_TIP) acc += qS[p.q_off + k];   // the cell's area is in its value
+    else acc = fma(qw[p.q_off + k], qS[p.q_off + k], acc);
+    fsum += qF[p.q_off + k];
     if (lat) { fxs += qfx[p.q_off + k]; fys += qfy[p.q_off + k]; }
-    if (p.geometry == RD_G_TIP) {   // Field_normal :105-112
-      double nx, ny, nz;
-      tip_normal(p, qx[p.q_off + k], qy[p.q_off + k], &nx, &ny, &nz);
-      F = (nx * qfx[p.q_off + k] + ny * qfy[p.q_off + k]) + nz * F;
-    }
-    if (F < 0.0) {
-      if (p.geometry == RD_G_TIP) {
-        double t = fn_t_y(F, p.tip_phi, p.image_charge);   // Elec_Supply (tip) :1710-1718
-        acc += (((qw[p.q_off + k] * c_k.a_FN) * (F * F)) * p.dt) / ((c_k.q0 * p.tip_phi) * (t * t));
-      } else {
-        double phi = work_at(p, work, qx[p.q_off + k], qy[p.q_off + k], nullptr);
-        acc += qw[p.q_off + k] * fn_supply_v2(F, phi, p.image_charge, p.dt);
-      }
-    }
   }
-  const double N_sup = block_sum(acc, red);
-  const double F_sum = block_sum(fsum, red);
-  const double Fx_sum = lat ? block_sum(fxs, red) : 0.0;   // block-uniform condition
-  const double Fy_sum = lat ? block_sum(fys, red) : 0.0;
-  if (threadIdx.x == 0) {
-    double* o = sup_part + ((size_t)d * RD_SUP_SPLIT + b) * 4;
-    o[0] = N_sup; o[1] = F_sum; o[2] = Fx_sum; o[3] = Fy_sum;
+  const double N_blk = block_sum(acc, red);
+  const double F_blk = block_sum(fsum, red);
+  const double Fx_blk = lat ? block_sum(fxs, red) : 0.0;   // block-uniform condition
+  const double Fy_blk = lat ? block_sum(fys, red) : 0.0;
+  double* const parts = sup_part + (size_t)d * RD_SUP_SPLIT * 4;
+  if (tid == 0) {
+    double* o = parts + 4 * b;
+    o[0] = N_blk; o[1] = F_blk; o[2] = Fx_blk; o[3] = Fy_blk;
+    __threadfence();
+    s_last = atomicAdd(&y.sup_done, 1) == RD_SUP_SPLIT - 1;
+    if (s_last) y.sup_done = 0;
   }
-}
-
-__global__ void k_supply_finish(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, int nslots,
-                                const int* __restrict__ step_ptr, const double* __restrict__ sup_part) {
-  const int d = blockIdx.x * blockDim.x + threadIdx.x;
-  if (d >= nslots) return;
-  const DiodeParams& p = P[d];
-  if (!p.active || !p.emission) return;
-  DiodeDyn& y = Dy[d];
-  if (!supply_live(p, y, step_ptr)) {   // the emitter is not on yet (:181)
-    y.N_sup = 0.0; y.chains = y.chains_capped = y.chains_failed = 0;
-    y.mh_acc = y.mh_rej = y.mh_done = 0;
-    y.F_avg_z = 0.0; y.F_avg_x = 0.0; y.F_avg_y = 0.0; y.df_avg = 0.0;
-    return;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  __shared__ double s_part[RD_SUP_SPLIT * 4];
+  for (int k = tid; k < RD_SUP_SPLIT * 4; k += blockDim.x) s_part[k] = __ldcg(parts + k);
+  __syncthreads();
+  if (tid < 4) {   // in block order
+    double s = 0.0;
+    for (int q = 0; q < RD_SUP_SPLIT; ++q) s += s_part[4 * q + tid];
+    s_sum[tid] = s;
   }
-  const int npt = (p.geometry == RD_G_TIP) ? 10000 : p.quad_n * p.quad_n;
-  double N_sup = 0.0, F_sum = 0.0, Fx_sum = 0.0, Fy_sum = 0.0;
-  for (int b = 0; b < RD_SUP_SPLIT; ++b) {
-    const double* o = sup_part + ((size_t)d * RD_SUP_SPLIT + b) * 4;
-    N_sup += o[0]; F_sum += o[1]; Fx_sum += o[2]; Fy_sum += o[3];
-  }
+  __syncthreads();
+  if (tid != 0) return;
+  const double N_sup = s_sum[0];
   y.N_sup = N_sup;
-  y.F_avg_z = p.geometry == RD_G_TIP ? 0.0 : F_sum / npt;   // F_avg, :644-651 (planar)
-  y.F_avg_x = p.geometry == RD_G_TIP ? 0.0 : Fx_sum / npt;
-  y.F_avg_y = p.geometry == RD_G_TIP ? 0.0 : Fy_sum / npt;
+  y.F_avg_z = p.geometry == RD_G_TIP ? 0.0 : s_sum[1] / npt;   // F_avg, :644-651 (planar)
+  y.F_avg_x = p.geometry == RD_G_TIP ? 0.0 : s_sum[2] / npt;
+  y.F_avg_y = p.geometry == RD_G_TIP ? 0.0 : s_sum[3] / npt;
   long nr;
   if (p.geometry == RD_G_TIP) {
     nr = nint_d(N_sup);
@@ -689,10 +718,19 @@ __device__ double warp_field_planar_z0(const DiodeParams& p, const Pool& pool, i
     const float4 pp = z0_point(p, px, py);
     const float dnm = (float)(p.d * 1.0e9);
     float hi = 0.f, lo = 0.f;
-    for (int j = lane; j < n; j += 32) {
-      float4 h = pool.zk_hi[off + j], l = pool.zk_lo[off + j];
-      two_sum_acc(hi, lo, nic == 0 ? z0_tile_f32<true>(&h, &l, 1, pp, 0, dnm)
-                                   : z0_tile_f32<false>(&h, &l, 1, pp, nic, dnm));
+    for (int j0 = lane; j0 < n; j0 += 32 * 4) {   // four electrons' loads in flight, added in order
+      float4 h[4], l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = min(j0 + 32 * q, n - 1);
+        h[q] = pool.zk_hi[off + j];
+        l[q] = pool.zk_lo[off + j];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (j0 + 32 * q < n)
+          two_sum_acc(hi, lo, nic == 0 ? z0_tile_f32<true>(&h[q], &l[q], 1, pp, 0, dnm)
+                                       : z0_tile_f32<false>(&h[q], &l[q], 1, pp, nic, dnm));
     }
     s = (double)hi + (double)lo;
   } else {
@@ -1499,8 +1537,8 @@ k_mh_vacuum_uniform(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy
   const int d = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   DiodeDyn& y = Dy[d];
   if (!P[d].active || !rd_mh_vacuum(P[d], y) || y.chains <= 0) return;
-  const int M = y.chains, c0 = blockIdx.x * RD_VU_CHAINS;
-  if (c0 >= M) return;
+  const int M = y.chains;
+  if ((int)blockIdx.x * RD_VU_CHAINS >= M) return;
   {
     const int* src = reinterpret_cast<const int*>(P + d);
     int* dst = reinterpret_cast<int*>(&sp);
@@ -1524,7 +1562,6 @@ k_mh_vacuum_uniform(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy
   const float Ff = (float)F;
   const bool start_ok = F < 0.0 && p.init_rounds > 0;
   const int ndim_first = (J + 2) / 4;
-  const int nc = min(RD_VU_CHAINS, M - c0);   // chains of this block
   if (tid == 0) {   // the schedule
     const int T = start_ok ? M : 0;
     double m = y.MH_std, ar = y.a_rate, rate = 0.0, g = 0.0;
@@ -1547,7 +1584,10 @@ k_mh_vacuum_uniform(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy
     }
     s_end[0] = m; s_end[1] = ar;
   }
-  // the start (round 0) of the block's chains, one per lane of warp 1
+  bool first = true;
+  for (int c0 = blockIdx.x * RD_VU_CHAINS; c0 < M; c0 += gridDim.x * RD_VU_CHAINS) {   // groups of chains
+  const int nc = min(RD_VU_CHAINS, M - c0);
+  // the start (round 0) of the group's chains, one per lane of warp 1
   const int c = c0 + lane;
   const bool mine = w == 1 && lane < nc;
   Real px = 0, py = 0, gx = 0, gy = 0;
@@ -1577,7 +1617,8 @@ k_mh_vacuum_uniform(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy
       const int nj = min(RD_VU_JCHUNK, J - j0 + 1);
       __syncthreads();   // the previous chunk's walk is done with s_g
       // the Gaussian pair of jump it is the draw with counter it (the start's for jump 1)
-      for (int k = tid - (j0 == 1 ? 32 : 0); k < nj * nc; k += blockDim.x - (j0 == 1 ? 32 : 0)) {
+      const int busy = j0 == 1 && first ? 32 : 0;
+      for (int k = tid - busy; k < nj * nc; k += blockDim.x - busy) {
         if (k < 0) break;   // thread 0's warp forms the schedule during the first chunk
         const int jj = k / nc, q = k - jj * nc;
         Real a, b;
@@ -1639,6 +1680,8 @@ k_mh_vacuum_uniform(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy
       y.MH_std = s_end[0];
       y.a_rate = s_end[1];
     }
+  }
+  first = false;
   }
 }
 
@@ -1944,10 +1987,11 @@ __global__ void k_mh_propose(const DiodeParams* __restrict__ P, const DiodeDyn* 
 // drop count, q = -q0, m = m0, the Beeman history seeded with (q/m) E_vac.
 // Accept test of every chain's final state (Escape_Prob_Planar / _Tip and the
 // uniform draw), spread over RD_EMIT_SPLIT blocks per diode: the FN escape
-// exponent is FP64 transcendental work.  Stores the chain's escape
-// probability (cs.df, the term of df_avg) and whether it emits (cs.em);
-// k_emit then appends in chain order.
-__global__ void __launch_bounds__(256)
+// exponent is FP64 transcendental work, and an SM's FP64 pipe takes 16 clocks per warp
+// instruction.  Stores the chain's escape probability (cs.df, the term of df_avg),
+// whether it emits (cs.em) and, if so, its electron's place, section (cs.prop_ok)
+// and vacuum acceleration; k_emit then appends in chain order.
+__global__ void __launch_bounds__(64)
 k_emit_test(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, ChainState cs,
             const int* __restrict__ ch_off, const double* __restrict__ work, const int* __restrict__ step_ptr) {
   const int d = blockIdx.x;
@@ -1962,8 +2006,8 @@ k_emit_test(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, 
     rng2(p.seed, (uint32_t)c, 0u, (uint32_t)step, RNG_EMIT, &u1, &u2);
     const int ok = cs.ok[k];
     const double F = cs.F[k];
-    int e = 0;
-    double df;
+    int e = 0, sec = 1;
+    double df, X = 0.0, Y = 0.0, Z = 0.0;
     if (p.geometry == RD_G_TIP) {
       double Df = 0.0;
       if (ok) {
@@ -1972,15 +2016,32 @@ k_emit_test(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, 
       }
       df = Df;
       e = F < 0.0 && u1 <= Df;
+      if (e) {   // one length scale out along the surface normal
+        double nx, ny, nz;
+        tip_normal(p, cs.tx[k], cs.ty[k], &nx, &ny, &nz);
+        X = cs.tx[k] + nx * c_k.length_scale;
+        Y = cs.ty[k] + ny * c_k.length_scale;
+        Z = cs.tz[k] + nz * c_k.length_scale;
+      }
     } else {
-      const double phi = work_at(p, work, cs.x[k], cs.y[k], nullptr);
+      const double phi = work_at(p, work, cs.x[k], cs.y[k], &sec);
       double D = ok ? fn_escape_log(F, phi, p.image_charge) : -1.79769313486231570e308;
       if (F >= 0.0) D = -1.79769313486231570e308;
       df = exp(D);
       e = log(u1) <= D;
+      X = cs.x[k]; Y = cs.y[k];
+      Z = 1.0 * c_k.length_scale;
     }
     cs.df[k] = df;
     cs.em[k] = e;
+    if (e) {   // where it goes and the vacuum acceleration there (k_emit only copies)
+      double ex, ey, ez;
+      vacuum_field(p, X, Y, Z, &ex, &ey, &ez);
+      const double qm = (-1.0 * c_k.q0) / (1.0 * c_k.m0);
+      cs.pxx[k] = X; cs.pyy[k] = Y; cs.pzz[k] = Z;
+      cs.px[k] = qm * ex; cs.py[k] = qm * ey; cs.pF[k] = qm * ez;
+      cs.prop_ok[k] = sec;
+    }
   }
 }
 
@@ -2008,10 +2069,11 @@ k_emit(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool, 
   int emitted = 0, dropped = 0;
   for (int c0 = 0; c0 < M; c0 += blockDim.x) {
     const int c = c0 + tid, k = ch_off[d] + c;
-    int e = 0;
+    int e = 0, sec = 0;
     if (c < M) {
       df_sum += cs.df[k];
       e = cs.em[k];
+      sec = cs.prop_ok[k];
     }
     // block-wide exclusive scan of e
     unsigned bal = __ballot_sync(0xffffffffu, e);
@@ -2024,27 +2086,13 @@ k_emit(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool, 
     if (e) {
       int i = n0 + slot;
       if (i < p.cap) {
-        double X, Y, Z;
-        int sec = 1;
-        if (p.geometry == RD_G_TIP) {   // one length scale out along the surface normal
-          double nx, ny, nz;
-          tip_normal(p, cs.tx[k], cs.ty[k], &nx, &ny, &nz);
-          X = cs.tx[k] + nx * c_k.length_scale;
-          Y = cs.ty[k] + ny * c_k.length_scale;
-          Z = cs.tz[k] + nz * c_k.length_scale;
-        } else {
-          X = cs.x[k]; Y = cs.y[k];
-          work_at(p, work, X, Y, &sec);
-          Z = 1.0 * c_k.length_scale;
-        }
-        int gi = p.off + i;
-        double qm = (-1.0 * c_k.q0) / (1.0 * c_k.m0), ex, ey, ez;
-        vacuum_field(p, X, Y, Z, &ex, &ey, &ez);
+        const double X = cs.pxx[k], Y = cs.pyy[k], Z = cs.pzz[k];
+        const int gi = p.off + i;
         pool.x[gi] = X; pool.y[gi] = Y; pool.z[gi] = Z;
         pool.vx[gi] = 0.0; pool.vy[gi] = 0.0; pool.vz[gi] = 0.0;
-        pool.ax[gi] = pool.bx[gi] = pool.cx[gi] = qm * ex;
-        pool.ay[gi] = pool.by[gi] = pool.cy[gi] = qm * ey;
-        pool.az[gi] = pool.bz[gi] = pool.cz[gi] = qm * ez;
+        pool.ax[gi] = pool.bx[gi] = pool.cx[gi] = cs.px[k];
+        pool.ay[gi] = pool.by[gi] = pool.cy[gi] = cs.py[k];
+        pool.az[gi] = pool.bz[gi] = pool.cz[gi] = cs.pF[k];
         pool.q[gi] = -1.0 * c_k.q0;
         pool.m[gi] = 1.0 * c_k.m0;
         pool.species[gi] = 1;
@@ -2378,11 +2426,12 @@ cudaError_t rd_launch_z0_points(int prec, int grid, cudaStream_t st, const Diode
 
 cudaError_t rd_launch_supply_reduce(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                                     const double* qx, const double* qy, const double* qw,
-                                    const double* qF, const double* qfx, const double* qfy,
+                                    const double* qF, const double* qfx, const double* qfy, double* qS,
                                     const double* work, const int* step_ptr, double* sup_part) {
-  k_supply_reduce<<<dim3(nslots, RD_SUP_SPLIT), 256, 0, st>>>(P, Dy, qx, qy, qw, qF, qfx, qfy, work, step_ptr,
-                                                              sup_part);
-  k_supply_finish<<<(nslots + 127) / 128, 128, 0, st>>>(P, Dy, nslots, step_ptr, sup_part);
+  // one diode: a thread per point of the default rules; many: a few points per thread
+  const int blocks = std::max(8, 1216 / std::max(nslots, 1));
+  k_supply_points<<<dim3(blocks, nslots), 128, 0, st>>>(P, Dy, qx, qy, qw, qF, qfx, qfy, work, step_ptr, qS);
+  k_supply_reduce<<<dim3(nslots, RD_SUP_SPLIT), 256, 0, st>>>(P, Dy, qS, qw, qF, qfx, qfy, step_ptr, sup_part);
   return cudaGetLastError();
 }
 
@@ -2400,7 +2449,7 @@ cudaError_t rd_launch_mh_vacuum(int prec, int nslots, cudaStream_t st, const Dio
                                 const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
                                 double kscale) {
   const int grid = nslots * RD_VAC_CTAS;
-  const dim3 ugrid(RD_VAC_MAX_CHAINS / RD_VU_CHAINS, nslots);
+  const dim3 ugrid(std::min(RD_VAC_MAX_CHAINS / RD_VU_CHAINS, std::max(16, 4864 / std::max(nslots, 1))), nslots);
   if (prec == 1) {
     k_mh_vacuum_uniform<1><<<ugrid, RD_VU_THREADS, 0, st>>>(P, Dy, cs, ch_off, wtab, step_ptr, kscale);
     k_mh_vacuum<1><<<grid, RD_VAC_THREADS, 0, st>>>(P, Dy, cs, ch_off, wtab, step_ptr, kscale, nslots);
@@ -2450,7 +2499,7 @@ cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const Di
   k_near_count<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
   k_near_scan<<<nslots, 1024, 0, st>>>(P, Dy, nr);
   k_near_scatter<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
-  k_near_panels<<<rd_grid(k_near_panels, 256, grid), 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
+  k_near_panels<<<rd_grid(k_near_panels, 64, grid), 64, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
   return cudaGetLastError();
 }
 
@@ -2488,7 +2537,7 @@ cudaError_t rd_launch_mh_jumps_near(int grid, cudaStream_t st, const DiodeParams
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                            const Pool& pool, const ChainState& cs, const int* ch_off,
                            const double* work, const int* step_ptr, const EventLog& ev) {
-  k_emit_test<<<dim3(nslots, RD_EMIT_SPLIT), 256, 0, st>>>(P, Dy, cs, ch_off, work, step_ptr);
+  k_emit_test<<<dim3(nslots, RD_EMIT_SPLIT), 64, 0, st>>>(P, Dy, cs, ch_off, work, step_ptr);
   k_emit<<<nslots, 1024, 0, st>>>(P, Dy, pool, cs, ch_off, work, step_ptr, ev);
   return cudaGetLastError();
 }
@@ -2518,15 +2567,15 @@ __global__ void __launch_bounds__(RD_VU_THREADS)
 k_mh_serial_vacuum(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const double* __restrict__ work,
                    const double* __restrict__ wtab, const int* __restrict__ step_ptr, double kscale) {
   __shared__ DiodeParams sp;
-  __shared__ double s_mhs[RD_VU_CHAINS];           // MH_std each chain of the block walks with
+  __shared__ double s_mhs[RD_SV_CHAINS];           // MH_std each chain of the block walks with
   __shared__ double s_end;                          // MH_std after the diode's last chain
-  __shared__ double s_g[RD_VU_JCHUNK][RD_VU_CHAINS][2];
+  __shared__ double s_g[RD_VU_JCHUNK][RD_SV_CHAINS][2];
   const int d = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const DiodeParams& pg = P[d];
   if (!pg.active || !pg.emission || !pg.mh_serial || pg.geometry != RD_G_PLANAR || pg.emitter_type == 4) return;
   DiodeDyn& y = Dy[d];
   if (y.n != 0 || y.chains <= 0 || y.chains > RD_VAC_MAX_CHAINS) return;   // the grid covers this many
-  const int M = y.chains, c0 = blockIdx.x * RD_VU_CHAINS;
+  const int M = y.chains, c0 = blockIdx.x * RD_SV_CHAINS;
   if (c0 >= M) return;
   {
     const int* src = reinterpret_cast<const int*>(P + d);
@@ -2547,7 +2596,7 @@ k_mh_serial_vacuum(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy,
   const double F = z0_finish<PREC>(p, 0.0, kscale);   // k_mh_serial's field with no particle: z0_finish of a zero sum
   const bool found = F < 0.0 && p.init_rounds > 0;     // every chain starts at its round-0 draw, or none does
   const bool updates = found && J > ndim_first;        // each chain updates MH_std once, at rate 1
-  const int nc = min(RD_VU_CHAINS, M - c0);
+  const int nc = min(RD_SV_CHAINS, M - c0);
   if (tid == 0) {   // MH_std of chains c0 .. c0 + nc - 1, and after chain M - 1
     const double ar = (double)(J - ndim_first) / (double)(J - ndim_first);   // 1, formed as k_mh_serial forms it
     const double g = exp(0.025 * (ar - 0.35));          // k_mh_serial's factor at that rate
@@ -2618,7 +2667,7 @@ k_mh_serial_vacuum(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy,
   if (tid == 0) {
     if (emits) atomicOr(&y.ser_emit, 1);
     __threadfence();
-    const int nblk = (M + RD_VU_CHAINS - 1) / RD_VU_CHAINS;
+    const int nblk = (M + RD_SV_CHAINS - 1) / RD_SV_CHAINS;
     if (atomicAdd(&y.ser_ticket, 1) == nblk - 1) {   // every block of the diode is done
       __threadfence();
       if (atomicAdd(&y.ser_emit, 0) == 0) {   // no chain emitted: the step's results, as k_mh_serial
@@ -2641,7 +2690,7 @@ k_mh_serial_vacuum(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy,
 cudaError_t rd_launch_mh_serial(int prec, int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                                 const Pool& pool, const double* work, const double* wtab,
                                 const int* step_ptr, double kscale, const EventLog& ev) {
-  const dim3 vgrid(RD_VAC_MAX_CHAINS / RD_VU_CHAINS, nslots);
+  const dim3 vgrid(RD_VAC_MAX_CHAINS / RD_SV_CHAINS, nslots);
   if (prec == 1) {
     k_mh_serial_vacuum<1><<<vgrid, RD_VU_THREADS, 0, st>>>(P, Dy, work, wtab, step_ptr, kscale);
     k_mh_serial<1><<<nslots, 256, 0, st>>>(P, Dy, pool, work, wtab, step_ptr, kscale, ev);

@@ -30,8 +30,9 @@
 #define RD_MH_PARTS 2         // planar MH jump launches per jump, one stream each (default)
 #define RD_MH_PARTS_MAX 4     // at most this many (rd_autotune / rd_set_mh_launch choose)
 #define RD_SUP_SPLIT 64       // blocks per diode in the supply reduction
-#define RD_SUP_NCH 4          // at most this many j-chunks per tile of planar supply points
-#define RD_EMIT_SPLIT 8       // blocks per diode in the emission accept test
+#define RD_SUP_NCH 4          // scratch: j-chunks per tile of planar supply points
+#define RD_SUP_CLEN 512       // their shortest default chunk
+#define RD_EMIT_SPLIT 64      // blocks per diode in the emission accept test (64 threads each)
 // j-chunking of pair sums: at least RD_CLEN_MIN particles per chunk, at most
 // RD_NCH_MAX chunks per i-tile
 #define RD_CLEN_MIN 1024
@@ -112,6 +113,7 @@ struct DiodeParams {
   int nr_boff;           // first bin of this diode
   int nr_bx, nr_by;      // bins along x (one panel wide) and y (two panels high)
   float nr_Z;            // near electrons are lower than this (nm)
+  double nr_hx, nr_hy;   // panel half widths (nm)
   float nr_Ez;           // E_z
   float nr_ax, nr_ay, nr_iax, nr_iay, nr_iwx, nr_iwy;   // panel half widths (nm), 1 / half width, 1 / width
 };
@@ -176,7 +178,9 @@ struct DiodeDyn {
 #define RD_VAC_MAX_CHAINS (RD_VAC_CTAS * RD_VAC_THREADS * RD_VAC_CPT)
 #define RD_VAC_WTAB 512       // supply-target table entries staged in shared memory
 #define RD_VAC_MAXJ 1024      // jumps whose step-size schedule a uniform work function precomputes
-#define RD_VU_CHAINS 32       // chains per block of k_mh_vacuum_uniform (one lane each)
+#define RD_VU_CHAINS 8        // chains k_mh_vacuum_uniform's blocks take at a time (one lane each): the draws,
+                              // not the walk, bound it, and 8 spread one diode over the SMs
+#define RD_SV_CHAINS 32       // chains per block of k_mh_serial_vacuum
 #define RD_VU_THREADS 128     // its threads (all draw the Gaussian pairs)
 #define RD_VU_JCHUNK 64       // jumps whose Gaussian pairs a block holds at once
 #ifdef __CUDACC__

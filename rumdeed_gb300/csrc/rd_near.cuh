@@ -167,24 +167,26 @@ __device__ const float c_gl4_inv[4][4] = {
 // Panel records, one warp per panel: the far part's interpolation coefficients
 // (powers of t_x fastest), the panel's centre, T and the largest |S| of its
 // nodes, and where its near electrons are.  The supply plan's tiles of 128 points cover eight panels each.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(64)
 k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, const PlanEntry* __restrict__ plan,
               const PlanHeader* __restrict__ ph, const float4* __restrict__ qpp, const double* __restrict__ qF,
               NearState nr, double kscale) {
   const int total = ph->total_items, nd = ph->n_diodes, lane = threadIdx.x & 31;
+  const double inv_A0 = 1.0 / (-2.0 * kscale);
   for (int g = blockIdx.x; g < total; g += gridDim.x) {
     const ItemRef it = decode_item(plan, nd, g);
-    if (it.chunk != 0) continue;
     const DiodeParams& p = P[it.d];
     if (!near_live(p, Dy[it.d])) continue;
-    const int NP = p.nr_P, pan = it.tile * 8 + (threadIdx.x >> 5);
-    if (pan >= NP * NP) continue;
+    const int NP = p.nr_P;
+    // the item's share of the tile's eight panels, one warp each
+    for (int pan = it.tile * 8 + 8 * it.chunk / it.nch + (threadIdx.x >> 5);
+         pan < min(NP * NP, it.tile * 8 + 8 * (it.chunk + 1) / it.nch); pan += 2) {
     const int ppy = pan / NP, ppx = pan - ppy * NP, nb = p.nr_bx, r0 = ppy >> 1;
     const int* start = nr.start + p.nr_boff;
     // the node of this lane (lanes l and l + 16 share one and take every other near electron)
     const int k = p.q_off + (ppy * 4 + ((lane >> 2) & 3)) * p.quad_n + ppx * 4 + (lane & 3);
     const float4 pp = qpp[k];
-    const float S = (float)((qF[k] - p.E_z) / (-2.0 * kscale));
+    const float S = (float)((qF[k] - p.E_z) * inv_A0);
     float near = 0.0f;
     for (int r = 0; r < RD_NEAR_ROWS; ++r) {
       const int row = (r0 + r) * nb + ppx;   // bins ppx .. ppx + 2 M of this row
@@ -208,11 +210,11 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     for (int q = 0; q < 4; ++q) c = fmaf(c_gl4_inv[(lane >> 2) & 3][q], __shfl_sync(0xffffffffu, cx, 4 * q + (lane & 3)), c);
     if (lane == 0) c += base;
     // T over the far electrons, as seen from the panel's rectangle
-    const double wx = p.em_Lx * 1.0e9 / NP, wy = p.em_Ly * 1.0e9 / NP;
-    const float ox = (float)((ppx + 0.5) * wx - 0.5e9 * p.em_Lx), oy = (float)((ppy + 0.5) * wy - 0.5e9 * p.em_Ly);
+    const float ox = (float)((2 * ppx + 1 - NP) * p.nr_hx), oy = (float)((2 * ppy + 1 - NP) * p.nr_hy);
     const float ax = p.nr_ax, ay = p.nr_ay;
     float Tx = 0.0f, Ty = 0.0f;
     const int n = Dy[it.d].n;
+#pragma unroll 4
     for (int j = lane; j < n; j += 32) {
       const float4 e = nr.low[p.off + j];
       const int code = __float_as_int(e.w);
@@ -251,6 +253,7 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     }
     if (lane == 0) *reinterpret_cast<float4*>(rec + 16) = make_float4(ox, oy, 1.03f * Tx, big);
     if (lane == 1) rec[28] = 1.03f * Ty;
+    }
   }
 }
 

@@ -64,8 +64,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[RD_NOALLOC_SCRA
 
 // kernels from the other translation units
 cudaError_t rd_launch_plan(cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy, int nslots,
-                           int mode, int chunk_rule, int max_items, const int* npts,
-                           PlanEntry* plan, PlanHeader* ph);
+                           const PlanJobs& jobs, int chunk_rule, int max_items, const int* npts);
 cudaError_t rd_launch_field_points(int prec, int geom, int grid, cudaStream_t st,
                                    const DiodeParams* P, const Pool& pool, const PlanEntry* plan,
                                    const PlanHeader* ph, const PointSet& pts, double* partial,
@@ -189,7 +188,7 @@ extern "C" int rd_field_at_noalloc(rd_engine* e, int diode, int M, const double*
                                  px + RD_NOALLOC_MAX_POINTS, px + 2 * RD_NOALLOC_MAX_POINTS);
   cudaError_t ce = cudaGetLastError();
   if (ce == cudaSuccess)
-    ce = rd_launch_plan(st, P, Dy, 1, PM_FIELD, rd_engine_chunk_rule(e), NA_MAX_ITEMS, ints, plan, ph);
+    ce = rd_launch_plan(st, P, Dy, 1, PlanJobs{1, {{PM_FIELD, plan, ph}}}, rd_engine_chunk_rule(e), NA_MAX_ITEMS, ints);
   PointSet pts{px, px + RD_NOALLOC_MAX_POINTS, px + 2 * RD_NOALLOC_MAX_POINTS,
                fx, fx + RD_NOALLOC_MAX_POINTS, fx + 2 * RD_NOALLOC_MAX_POINTS, ints + 1};
   if (ce == cudaSuccess)

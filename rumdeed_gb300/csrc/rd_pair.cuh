@@ -54,6 +54,17 @@ struct PlanHeader {
   int pad[2];
 };
 
+// Plans that one k_plan launch builds.
+struct PlanJob {
+  int mode;
+  PlanEntry* plan;
+  PlanHeader* ph;
+};
+struct PlanJobs {
+  int n;
+  PlanJob j[4];
+};
+
 struct ItemRef {
   int d;        // plan entry (== diode slot)
   int tile, chunk, nch;

@@ -131,7 +131,7 @@ __device__ __forceinline__ int plan_ni(const DiodeParams& p, const DiodeDyn& y, 
 // at most ~1024 particles also bound the cost of one work item, so the last
 // items of a launch end soon after the others.
 __device__ __forceinline__ void plan_split(int ni, int nj, int tsize, bool pair, int grow, int clen_min,
-                                           int nch_max, int target, int* tiles, int* nch, int* clen) {
+                                           int nch_max, int target, int shortest, int* tiles, int* nch, int* clen) {
   *tiles = (ni + tsize - 1) / tsize;
   *nch = 1;
   *clen = RD_TILE;
@@ -139,7 +139,7 @@ __device__ __forceinline__ void plan_split(int ni, int nj, int tsize, bool pair,
     int c = (nj + nch_max - 1) / nch_max;
     if (target > 0) {   // a small system: short enough chunks for `target` items
       const long long len = ((long long)nj * *tiles + target - 1) / target;
-      if (len < clen_min) clen_min = (int)len;
+      if (len < clen_min) clen_min = min(clen_min, max((int)len, shortest));
     }
     if (c < clen_min) c = clen_min;
     c = ((c + RD_TILE - 1) / RD_TILE) * RD_TILE;
@@ -149,86 +149,86 @@ __device__ __forceinline__ void plan_split(int ni, int nj, int tsize, bool pair,
   }
 }
 
+// One block per plan (PlanJobs), a thread per slot: counts, a block scan of the items
+// (and chains), the entries.  Bound by latency: a step has several plans in a row
+// with its kernels waiting for them.  One warp for up to 32 slots needs no barrier;
+// 1024 threads with a tree of barriers over FP64 counts took 9 us for a single
+// diode, this 3.  The chunks grow only if the items would not fit the scratch (never
+// by construction).
 __global__ void __launch_bounds__(1024)
-k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int nslots, int mode,
-       int chunk_rule, int max_items, const int* __restrict__ npts, PlanEntry* __restrict__ plan,
-       PlanHeader* __restrict__ ph) {
-  __shared__ double red[1024];
-  __shared__ int s_items[32], s_chains[32];
-  __shared__ int s_run_items, s_run_chains;
-  const int tid = threadIdx.x;
+k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int nslots, PlanJobs jobs, int chunk_rule,
+       int max_items, const int* __restrict__ npts) {
+  __shared__ long long s_items[32];
+  __shared__ int s_chains[32];
+  const PlanJob job = jobs.j[blockIdx.x];
+  const int mode = job.mode, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
   const int tsize = (mode == PM_PART1024) ? 1024 : (mode == PM_MH_NEAR) ? RD_NEAR_CPB : RD_ITILE;
   const bool pair = (mode & 0xff) <= PM_SUPPLY_LAT || mode == PM_MH_SLOW;
-  const int clen_min = chunk_rule & 0xffff, nch_max = (chunk_rule >> 16) & 0xff, target = (chunk_rule >> 24) * 64;   // rd_chunk_rule
-  // the planar supply points are many tiles already: at most RD_SUP_NCH chunks per tile
-  const int nch_eff = ((mode & 0xff) == PM_SUPPLY_PLANAR || (mode & 0xff) == PM_SUPPLY_LAT)
-                          ? min(nch_max, RD_SUP_NCH) : nch_max;
-  // grow the chunk length only if the items would not fit the scratch
-  __shared__ int s_grow;
-  if (tid == 0) s_grow = 0;
-  __syncthreads();
-  for (int round = 0; round < 24; ++round) {
-    const int grow = s_grow;
-    double cnt = 0.0;
-    for (int d = tid; d < nslots; d += blockDim.x) {
-      if (!P[d].active) continue;
-      int tiles, nch, clen;
-      plan_split(plan_ni(P[d], Dy[d], mode, npts, d), Dy[d].n, tsize, pair, grow, clen_min, nch_eff, target, &tiles,
-                 &nch, &clen);
-      cnt += (double)tiles * nch;
-    }
-    red[tid] = cnt;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (tid < s) red[tid] += red[tid + s];
-      __syncthreads();
-    }
-    const bool fits = red[0] <= (double)max_items;
-    __syncthreads();
-    if (fits) break;
-    if (tid == 0) s_grow = grow + 1;
-    __syncthreads();
+  const bool supply = (mode & 0xff) == PM_SUPPLY_PLANAR, lat = (mode & 0xff) == PM_SUPPLY_LAT;
+  int clen_min = chunk_rule & 0xffff, target = (chunk_rule >> 24) * 64;   // rd_chunk_rule
+  int nch_max = (chunk_rule >> 16) & 0xff;
+  // the supply points are many tiles already: few chunks per tile.  k_z0_points keeps one
+  // sum per point, a third of an item's scratch: three times the items fit.
+  if (lat) nch_max = min(nch_max, RD_SUP_NCH);
+  if (supply) {
+    nch_max = min(nch_max, 3 * RD_SUP_NCH);
+    target *= 4;   // its items are single warps
+    max_items *= 3;
   }
-  const int grow = s_grow;
-  // pass 3: entries with a running block scan
-  if (tid == 0) { s_run_items = 0; s_run_chains = 0; }
-  __syncthreads();
-  for (int base = 0; base < nslots; base += blockDim.x) {
-    int d = base + tid;
-    int items = 0, ni = 0, nj = 0, tiles = 0, nch = 1, clen = RD_TILE, chains = 0;
-    if (d < nslots && P[d].active) {
-      nj = Dy[d].n;
-      ni = plan_ni(P[d], Dy[d], mode, npts, d);
-      if (mode == PM_MH) chains = ni;
-      plan_split(ni, nj, tsize, pair, grow, clen_min, nch_eff, target, &tiles, &nch, &clen);
-      items = tiles * nch;
+  for (int grow = 0; grow < 24; ++grow) {
+    long long run_i = 0;
+    int run_c = 0;
+    for (int base = 0; base < nslots; base += blockDim.x) {
+      const int d = base + tid;
+      int ni = 0, nj = 0, tiles = 0, nch = 1, clen = RD_TILE, chains = 0;
+      long long items = 0;
+      if (d < nslots && P[d].active) {
+        nj = Dy[d].n;
+        ni = plan_ni(P[d], Dy[d], mode, npts, d);
+        if (mode == PM_MH) chains = ni;
+        plan_split(ni, nj, tsize, pair, grow, clen_min, nch_max, target, supply ? RD_SUP_CLEN : RD_TILE, &tiles, &nch, &clen);
+        items = (long long)tiles * nch;
+      }
+      long long vi = items;
+      int vc = chains;
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long a = __shfl_up_sync(0xffffffffu, vi, o);
+        const int b = __shfl_up_sync(0xffffffffu, vc, o);
+        if (lane >= o) { vi += a; vc += b; }
+      }
+      long long ti = __shfl_sync(0xffffffffu, vi, 31), oi = 0;
+      int tc = __shfl_sync(0xffffffffu, vc, 31), oc = 0;
+      if (nw > 1) {
+        if (lane == 31) { s_items[w] = vi; s_chains[w] = vc; }
+        __syncthreads();
+        ti = 0;
+        tc = 0;
+        for (int q = 0; q < nw; ++q) {
+          if (q == w) { oi = ti; oc = tc; }
+          ti += s_items[q];
+          tc += s_chains[q];
+        }
+        __syncthreads();
+      }
+      if (d < nslots) {
+        PlanEntry e;
+        e.item_off = (int)min(run_i + oi + vi - items, (long long)max_items);
+        e.tiles = tiles; e.nch = nch; e.clen = clen; e.n_i = ni; e.n_j = nj;
+        e.pad0 = run_c + oc + vc - chains;
+        e.tsize = tsize;
+        job.plan[d] = e;
+      }
+      run_i += ti;
+      run_c += tc;
     }
-    int lane = tid & 31, w = tid >> 5;
-    int vi = items, vc = chains;
-    for (int o = 1; o < 32; o <<= 1) {
-      int a = __shfl_up_sync(0xffffffffu, vi, o), b = __shfl_up_sync(0xffffffffu, vc, o);
-      if (lane >= o) { vi += a; vc += b; }
-    }
-    if (lane == 31) { s_items[w] = vi; s_chains[w] = vc; }
-    __syncthreads();
-    int oi = 0, oc = 0;
-    for (int q = 0; q < w; ++q) { oi += s_items[q]; oc += s_chains[q]; }
-    int run_i = s_run_items, run_c = s_run_chains;
-    if (d < nslots) {
-      PlanEntry e;
-      e.item_off = run_i + oi + vi - items;
-      e.tiles = tiles; e.nch = nch; e.clen = clen; e.n_i = ni; e.n_j = nj;
-      e.pad0 = run_c + oc + vc - chains;
-      e.tsize = tsize;
-      plan[d] = e;
+    if (run_i <= max_items || !pair || grow == 23) {
+      if (tid == 0) {
+        job.ph->total_items = (int)min(run_i, (long long)max_items);
+        job.ph->n_diodes = nslots;
+      }
+      return;
     }
     __syncthreads();
-    if (tid == blockDim.x - 1) { s_run_items = run_i + oi + vi; s_run_chains = run_c + oc + vc; }
-    __syncthreads();
-  }
-  if (tid == 0) {
-    ph->total_items = s_run_items < max_items ? s_run_items : max_items;
-    ph->n_diodes = nslots;
   }
 }
 
@@ -417,27 +417,33 @@ k_velocity(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, P
 // moved, divided by the particle counts before removal) and the
 // electron-step count, per diode: the diode's item partials (k_velocity)
 // added in a fixed order.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * RD_VEL_NV)
 k_ramo(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const PlanEntry* __restrict__ plan,
        const double* __restrict__ part) {
-  __shared__ double red[RD_VEL_NV][256];
-  const int d = blockIdx.x;
+  __shared__ double red[RD_VEL_NV][1];
+  const int d = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const DiodeParams& p = P[d];
   if (!p.active) return;
   DiodeDyn& y = Dy[d];
   const int n = y.n;
   const int g0 = plan[d].item_off, items = plan[d].tiles;
-  double v[RD_VEL_NV];
-  for (int k = 0; k < RD_VEL_NV; ++k) v[k] = 0.0;
-  for (int t = threadIdx.x; t < items; t += blockDim.x)
-    for (int k = 0; k < RD_VEL_NV; ++k) v[k] += part[(size_t)(g0 + t) * RD_VEL_NV + k];
-  for (int k = 0; k < RD_VEL_NV; ++k) red[k][threadIdx.x] = v[k];
+  // warp k adds value k: 256 strided partial sums, eight per lane, then their tree
+  double v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = 0.0;
+  for (int t0 = 0; t0 < items; t0 += 256)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int t = t0 + lane + 32 * q;
+      if (t < items) v[q] += part[(size_t)(g0 + t) * RD_VEL_NV + k];
+    }
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int q = 0; q < h; ++q) v[q] += v[q + h];
+  for (int h = 16; h > 0; h >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], h);
+  if (lane == 0) red[k][0] = v[0];
   __syncthreads();
-  for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h)
-      for (int k = 0; k < RD_VEL_NV; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + h];
-    __syncthreads();
-  }
   if (threadIdx.x == 0) {
     const double ne = red[8][0], ni = red[9][0];
     y.ramo_current = red[0][0];
@@ -673,9 +679,9 @@ __global__ void k_step_inc(int* step_ptr) { *step_ptr += 1; }
 
 // ---- launch wrappers ------------------------------------------------------------------
 cudaError_t rd_launch_plan(cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy, int nslots,
-                           int mode, int chunk_rule, int max_items, const int* npts,
-                           PlanEntry* plan, PlanHeader* ph) {
-  k_plan<<<1, 1024, 0, st>>>(P, Dy, nslots, mode, chunk_rule, max_items, npts, plan, ph);
+                           const PlanJobs& jobs, int chunk_rule, int max_items, const int* npts) {
+  const int threads = nslots >= 1024 ? 1024 : ((nslots + 31) / 32) * 32;
+  k_plan<<<jobs.n, threads > 0 ? threads : 32, 0, st>>>(P, Dy, nslots, jobs, chunk_rule, max_items, npts);
   return cudaGetLastError();
 }
 // Loads the planner and the pack kernel into the current context now (they
@@ -702,7 +708,7 @@ cudaError_t rd_launch_velocity(int grid, int nslots, cudaStream_t st, const Diod
                                DiodeDyn* Dy, const Pool& pool, const PlanEntry* plan,
                                const PlanHeader* ph, double* part, const int* step_ptr) {
   k_velocity<<<rd_grid(k_velocity, RD_ITILE, grid), RD_ITILE, 0, st>>>(P, Dy, pool, plan, ph, part, step_ptr);
-  k_ramo<<<nslots, 256, 0, st>>>(P, Dy, plan, part);
+  k_ramo<<<nslots, 32 * RD_VEL_NV, 0, st>>>(P, Dy, plan, part);
   return cudaGetLastError();
 }
 cudaError_t rd_launch_compact(int grid, int nslots, cudaStream_t st, const DiodeParams* P,
