@@ -2130,33 +2130,109 @@ k_emit(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool, 
 }  // namespace
 
 // ---- serial MH sampler (mh_batch = .false.) ---------------------------------------------
-// The pair sum of F_z at one cathode point over the diode's first n
-// particles, summed by the whole block (every thread gets the total, before
-// z0_finish).
+// Thread 0 gets the pair sum of F_z at one cathode point over the diode's first n
+// particles (before z0_finish).  FP32: every thread's share in particle order as a
+// float pair, the pairs added over the block (pair_add, ~44 bits; FP64 additions take
+// some hundred clocks each here); FP64: the shares' tree in FP64.
+struct SerialSum {
+  float h, l;   // FP32
+  double s;     // FP64
+};
 template <int PREC>
-__device__ double block_field_sum(const DiodeParams& p, const Pool& pool, int n, double px, double py,
-                                  double* red) {
-  const int tid = threadIdx.x, nt = blockDim.x, off = p.off;
+__device__ __forceinline__ double serial_value(const SerialSum& v) {
+  return PREC == 1 ? (double)v.h + (double)v.l : v.s;
+}
+template <int PREC>
+__device__ __forceinline__ SerialSum serial_field_sum(const DiodeParams& p, const Pool& pool, int n, double px,
+                                                      double py, float4 pp, float2* red_f, double* red_d) {
+  const int tid = threadIdx.x, lane = tid & 31, off = p.off;
   const int nic = p.image_charge ? p.N_ic_max : 0;
-  double s;
+  SerialSum r = {0.0f, 0.0f, 0.0};
   if (PREC == 1) {
-    const float4 pp = z0_point(p, px, py);
     const float dnm = (float)(p.d * 1.0e9);
     float hi = 0.f, lo = 0.f;
-    for (int j = tid; j < n; j += nt) {
-      float4 h = pool.zk_hi[off + j], l = pool.zk_lo[off + j];
-      two_sum_acc(hi, lo, nic == 0 ? z0_tile_f32<true>(&h, &l, 1, pp, 0, dnm)
-                                   : z0_tile_f32<false>(&h, &l, 1, pp, nic, dnm));
+    for (int j0 = tid; j0 < n; j0 += 256 * 4) {   // four particles' loads in flight
+      float4 h[4], l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = min(j0 + 256 * q, n - 1);
+        h[q] = pool.zk_hi[off + j];
+        l[q] = pool.zk_lo[off + j];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (j0 + 256 * q < n)
+          two_sum_acc(hi, lo, nic == 0 ? z0_tile_f32<true>(&h[q], &l[q], 1, pp, 0, dnm)
+                                       : z0_tile_f32<false>(&h[q], &l[q], 1, pp, nic, dnm));
     }
-    s = (double)hi + (double)lo;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      pair_add(hi, lo, __shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o));
+    if (lane == 0) red_f[tid >> 5] = make_float2(hi, lo);
+    __syncthreads();
+    if (tid < 32) {
+      const float2 v = red_f[lane & 7];
+      r.h = v.x;
+      r.l = v.y;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+        pair_add(r.h, r.l, __shfl_down_sync(0xffffffffu, r.h, o), __shfl_down_sync(0xffffffffu, r.l, o));
+    }
   } else {
-    s = 0.0;
-    for (int j = tid; j < n; j += nt) {
-      rd_d4 pj = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
+    double s = 0.0;
+    for (int j = tid; j < n; j += 256) {
+      const rd_d4 pj = make_d4(pool.x[off + j], pool.y[off + j], pool.z[off + j], pool.q[off + j]);
       s += z0_tile_f64(&pj, 1, px, py, nic, p.d, c_k.L2);
     }
+    red_d[tid] = s;
+    __syncthreads();
+    if (tid < 32) {
+      double v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = red_d[tid + 32 * k];
+#pragma unroll
+      for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+        for (int k = 0; k < h; ++k) v[k] += v[k + h];
+      for (int h = 16; h > 0; h >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], h);
+      r.s = v[0];
+    }
   }
-  return block_sum(s, red);
+  return r;
+}
+
+// x > y for finite doubles by their bits (an FP64 comparison waits for the FP64 pipe)
+__device__ __forceinline__ bool above(double x, double y) {
+  const long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+  return (a ^ ((a >> 63) & 0x7fffffffffffffffll)) > (b ^ ((b >> 63) & 0x7fffffffffffffffll));
+}
+
+// The accept / reject decision of a serial chain: s_n >= s_c or log u <= s_n - s_c
+// with the FP64 targets, as mh_decide_f takes it for the batched FP32 chains: FP32
+// estimates decide outside mh_guard, the FP64 targets inside.
+__device__ __noinline__ bool serial_take_fp64(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
+                                              double F, double ln, double cx, double cy, double Fc, double lc,
+                                              double lu) {
+  const double sn = supply_log_xy(p, wtab, wx, wy, F) + ln, sc = supply_log_xy(p, wtab, cx, cy, Fc) + lc;
+  return sn >= sc || lu <= sn - sc;
+}
+__device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
+                                            double F, double cx, double cy, double Fc, double lu) {
+  if (p.work_model != 2) {
+    const int cn = work_cell(p, wx, wy), cc = work_cell(p, cx, cy);
+    const double *tn = wtab + 3 * (p.work_off + cn), *tc = wtab + 3 * (p.work_off + cc);
+    const float Ff = (float)F, Fcf = (float)Fc;
+    const float rn = rho_entry_f(p, (float)tn[0], (float)tn[2], Ff), rc = rho_entry_f(p, (float)tc[0], (float)tc[2], Fcf);
+    const float l2 = 2.0f * logf(Ff / Fcf), df = l2 - (rn - rc), S = fabsf(l2) + fabsf(rn) + fabsf(rc);
+    if (isfinite(df)) {
+      if (df >= mh_guard(S)) return true;
+      if (cn == cc && __double_as_longlong(F) == __double_as_longlong(Fc)) return true;   // equal targets
+      const float luf = (float)lu, g = mh_guard(S + fabsf(luf));
+      if (luf <= df - g) return true;
+      if (luf > df + g) return false;
+    }
+  }
+  return serial_take_fp64(p, wtab, wx, wy, F, 0.0, cx, cy, Fc, 0.0, lu);
 }
 
 // The serial branch of Do_Field_Emission_Planar_rectangle (:322-333, 338-383)
@@ -2168,31 +2244,44 @@ __device__ double block_field_sum(const DiodeParams& p, const Pool& pool, int n,
 // with 10 % of the emitter as the step, then MH_std), updates MH_std once from
 // its own acceptance rate after the warm-up, and its electron, if the escape
 // test passes, is added before the next chain starts, so later chains see it.
-// Same Philox counters as the batched sampler.  The whole block sums the field
-// at each point (block_field_sum); thread 0 alone holds the chain and does the
-// rest (draws, proposals, targets, decisions: FP64 work, which every warp
-// would otherwise repeat on the part's narrow FP64 pipe) and hands the block
-// the next point through shared memory.
+// Same Philox counters as the batched sampler.
+//
+// A chain of dependent jumps: latency is all there is.  The whole block sums the
+// field at each point; thread 0 alone holds the chain and hands the block the next
+// point through shared memory.  What does not depend on the chain's state is not on
+// its path: the block draws the Gaussian pairs and the accept tests' log u of up to
+// RD_SER_DRAWS jumps at once, and the FP64 targets are formed only where FP32
+// estimates leave a decision open.  33 chains of 100 jumps over 400 electrons:
+// 25.9 -> 6.7 ms (7.8 -> 2.0 us a jump).
+#define RD_SER_DRAWS 256
 template <int PREC>
 __global__ void __launch_bounds__(256)
 k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool,
             const double* __restrict__ work, const double* __restrict__ wtab,
             const int* __restrict__ step_ptr, double kscale, EventLog ev) {
-  __shared__ double red[256];
+  __shared__ double red_d[PREC == 1 ? 1 : 256];
+  __shared__ float2 red_f[8];
+  __shared__ double s_g[RD_SER_DRAWS][2], s_lu[RD_SER_DRAWS];   // Gaussian pairs and log u of the next jumps
+  __shared__ float s_luf[RD_SER_DRAWS];
   // thread 0 -> block, one slot per jump parity (a slot is rewritten only after a
   // barrier that every reader of its last value has passed)
   __shared__ double s_pt[2][2];   // the point whose field the block sums next
+  __shared__ float4 s_pp[2];      // the same in the FP32 frame
   __shared__ int s_sum[2];        // the block sums a field this jump (a ring proposal off the ring: no)
   __shared__ int s_found, s_add, s_stop;   // the chain started; a particle was added; the chains stop
+  __shared__ DiodeParams sp;   // thread 0's loads of it are on the jumps' path
   const int d = blockIdx.x;
-  const DiodeParams& p = P[d];
-  if (!p.active || !p.emission || !p.mh_serial || p.geometry != RD_G_PLANAR) return;
+  if (!P[d].active || !P[d].emission || !P[d].mh_serial || P[d].geometry != RD_G_PLANAR) return;
   DiodeDyn& y = Dy[d];
   if (y.ser_done) {   // k_mh_serial_vacuum sampled this step's chains
     __syncthreads();
     if (threadIdx.x == 0) y.ser_done = 0;
     return;
   }
+  for (int k = threadIdx.x; k < (int)(sizeof(DiodeParams) / sizeof(int)); k += blockDim.x)
+    reinterpret_cast<int*>(&sp)[k] = reinterpret_cast<const int*>(P + d)[k];
+  __syncthreads();
+  const DiodeParams& p = sp;
   const bool t0 = threadIdx.x == 0;
   const uint32_t step = (uint32_t)(*step_ptr - y.step_offset);
   const int M = y.chains, n0 = y.n, id0 = y.nrID;
@@ -2202,11 +2291,19 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
   int emitted = 0, dropped = 0, failed = 0;
   double mhs = y.MH_std, a_rate = y.a_rate, df_sum = 0.0;
   const bool ring = p.emitter_type == 4;
+  // FP32: the decisions are taken from float fields where those are certain
+  const bool est = PREC == 1 && !ring && p.work_model != 2;
+  const float A0 = (float)((p.image_charge ? -2.0 : -1.0) * kscale), Ezf = (float)p.E_z;
+  const bool one_cell = p.work_model == 1 && p.work_nx == 1 && p.work_ny == 1;
+  float t0e = 0.0f, t2e = 0.0f;   // the work-function entry of the only cell
+  if (one_cell) { const double* e = wtab + 3 * p.work_off; t0e = (float)e[0]; t2e = (float)e[2]; }
+  const double hx = p.em_x0 + p.em_Lx, hy = p.em_y0 + p.em_Ly;
   const double twopi = 2.0 * c_k.pi, rmin = p.ring_rmin, rmax = p.ring_rmin + p.ring_thick;
   for (int c = 0; c < M; ++c) {
     double cx = p.em_x0, cy = p.em_y0, F = 1.0;
     double ca = 0.0, cr = rmin;   // ring: (angle, radius) of the chain (Metropolis_Hastings_ring_J)
     bool found = false;
+    SerialSum cur = {0.0f, 0.0f, 0.0};   // the sum at the chain's point
     if (t0) s_found = 0;
     for (int r = 0; r < p.init_rounds; ++r) {
       if (t0) {
@@ -2222,11 +2319,12 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
           cy = u2 * p.em_Ly + p.em_y0;
         }
         s_pt[0][0] = cx; s_pt[0][1] = cy;
+        if (PREC == 1) s_pp[0] = z0_point(p, cx, cy);
       }
       __syncthreads();
-      const double sum = block_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], red);
+      cur = serial_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], s_pp[0], red_f, red_d);
       if (t0) {
-        F = z0_finish<PREC>(p, sum, kscale);
+        F = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
         found = F < 0.0;
         s_found = found;
       }
@@ -2235,7 +2333,8 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
     }
     __syncthreads();   // s_found final (also with no start rounds)
     double D = -1.79769313486231570e308, Fout = 1.0;
-    double sup_cur = 0.0, sx = 0.0, sy = 0.0;
+    double sx = 0.0, sy = 0.0, sx1 = 0.0, sy1 = 0.0;   // step sizes: warm-up, then MH_std's
+    float Fc = 0.0f, fe = 0.0f, rc = 0.0f;               // est: the chain's field, its bound, its rho
     int ja = 0, jr = 0;
     if (t0) {
       if (!found) {
@@ -2243,20 +2342,40 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         cy = ring ? 0.0 : p.em_y0;
         ++failed;
       } else {
-        Fout = F;
-        // ring: log(radius) is the Jacobian of the (angle, radius) parametrisation (:1592-1596)
-        sup_cur = supply_log_xy(p, wtab, cx, cy, F) + (ring ? log(cr) : 0.0);
         sx = (ring ? twopi : p.em_Lx) * 0.10;
         sy = (ring ? p.ring_thick : p.em_Ly) * 0.10;
+        sx1 = (ring ? twopi : p.em_Lx) * mhs;
+        sy1 = (ring ? p.ring_thick : p.em_Ly) * mhs;
+        if (est) {
+          float te = t0e, ue = t2e;
+          if (!one_cell) {
+            const double* e = wtab + 3 * (p.work_off + work_cell(p, cx, cy));
+            te = (float)e[0]; ue = (float)e[2];
+          }
+          Fc = (float)F;
+          fe = 1.2e-7f * fabsf(Fc);
+          rc = rho_entry_f(p, te, ue, Fc);
+        }
       }
     }
     const bool walk = s_found != 0;   // every thread: the chain found a start
     for (int i = 1; walk && i <= ndim; ++i) {
       double wx = 0.0, wy = 0.0, na = 0.0, nr = 0.0;
+      const int draw = (i - 1) % RD_SER_DRAWS;
+      if (draw == 0) {
+        if (i > 1) __syncthreads();   // thread 0 is done with the last draws
+        for (int k = threadIdx.x; k < min(RD_SER_DRAWS, ndim - i + 1); k += blockDim.x) {
+          gauss2(p.seed, (uint32_t)c, (uint32_t)(i + k), step, &s_g[k][0], &s_g[k][1]);
+          double u1, u2;
+          rng2(p.seed, (uint32_t)c, (uint32_t)(i + k), step, RNG_ACCEPT, &u1, &u2);
+          s_lu[k] = log(u1);
+          s_luf[k] = (float)s_lu[k];
+        }
+        __syncthreads();
+      }
       if (t0) {
-        if (i > ndim_first) { sx = (ring ? twopi : p.em_Lx) * mhs; sy = (ring ? p.ring_thick : p.em_Ly) * mhs; }
-        double g1, g2;
-        gauss2(p.seed, (uint32_t)c, (uint32_t)i, step, &g1, &g2);
+        if (i == ndim_first + 1) { sx = sx1; sy = sy1; }
+        const double g1 = s_g[draw][0], g2 = s_g[draw][1];
         int sum_it = 1;
         if (ring) {   // angle wrapped (Fortran MODULO), radius outside the ring rejected
           const double a = g1 * sx + ca;
@@ -2272,37 +2391,54 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         } else {
           wx = g1 * sx + cx;
           wy = g2 * sy + cy;
-          const double hx = p.em_x0 + p.em_Lx, hy = p.em_y0 + p.em_Ly;
-          if (wx > hx) wx = hx - (wx - hx); else if (wx < p.em_x0) wx = (p.em_x0 - wx) + p.em_x0;
-          if (wy > hy) wy = hy - (wy - hy); else if (wy < p.em_y0) wy = (p.em_y0 - wy) + p.em_y0;
+          if (above(wx, hx)) wx = hx - (wx - hx); else if (above(p.em_x0, wx)) wx = (p.em_x0 - wx) + p.em_x0;
+          if (above(wy, hy)) wy = hy - (wy - hy); else if (above(p.em_y0, wy)) wy = (p.em_y0 - wy) + p.em_y0;
         }
         s_pt[i & 1][0] = wx; s_pt[i & 1][1] = wy;
+        if (PREC == 1) s_pp[i & 1] = z0_point(p, wx, wy);
         s_sum[i & 1] = sum_it;
       }
       __syncthreads();
       if (!s_sum[i & 1]) continue;   // block-uniform: a ring proposal off the ring, no field needed
-      const double sum = block_field_sum<PREC>(p, pool, n, s_pt[i & 1][0], s_pt[i & 1][1], red);
+      const SerialSum sum = serial_field_sum<PREC>(p, pool, n, s_pt[i & 1][0], s_pt[i & 1][1], s_pp[i & 1], red_f, red_d);
       if (t0) {
-        const double Fw = z0_finish<PREC>(p, sum, kscale);
-        if (Fw >= 0.0) {
-          if (i > ndim_first) ++jr;
-        } else {
-          const double sn = supply_log_xy(p, wtab, wx, wy, Fw) + (ring ? log(nr) : 0.0);
-          bool take = sn >= sup_cur;
-          if (!take) {
-            double u1, u2;
-            rng2(p.seed, (uint32_t)c, (uint32_t)i, step, RNG_ACCEPT, &u1, &u2);
-            take = log(u1) <= sn - sup_cur;
+        // ring: log(radius) is the Jacobian of the (angle, radius) parametrisation (:1592-1596)
+        const double lu = s_lu[draw];
+        int take = -1;
+        float Fn = 0.0f, dF = 0.0f, rn = 0.0f;
+        if (est) {
+          float te = t0e, ue = t2e;
+          if (!one_cell) {
+            const double* e = wtab + 3 * (p.work_off + work_cell(p, wx, wy));
+            te = (float)e[0]; ue = (float)e[2];
           }
-          if (take) {
-            cx = wx; cy = wy; sup_cur = sn; Fout = Fw; ca = na; cr = nr;
-            if (i > ndim_first) ++ja;
-          } else if (i > ndim_first) {
-            ++jr;
+          const float S = sum.h + sum.l;
+          Fn = fmaf(A0, S, Ezf);
+          dF = 2.4e-7f * (fabsf(Ezf) + fabsf(A0 * S));
+          take = near_decide(p, Fn, dF, Fc, fe, rc, te, ue, s_luf[draw], &rn);
+        }
+        if (take < 0) {   // the FP64 targets
+          const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
+          const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+          if (Fw >= 0.0) take = 0;
+          else if (ring) take = serial_take_fp64(p, wtab, wx, wy, Fw, log(nr), cx, cy, Fd, log(cr), lu);
+          else if (PREC == 0) take = serial_take(p, wtab, wx, wy, Fw, cx, cy, Fd, lu);
+          else take = serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, lu);
+          if (est) {
+            const double* e = wtab + 3 * (p.work_off + work_cell(p, wx, wy));
+            rn = rho_entry_f(p, (float)e[0], (float)e[2], Fn);
           }
+        }
+        if (take) {
+          cx = wx; cy = wy; cur = sum; ca = na; cr = nr;
+          Fc = Fn; fe = dF; rc = rn;
+          if (i > ndim_first) ++ja;
+        } else if (i > ndim_first) {
+          ++jr;
         }
       }
     }
+    if (t0 && found) Fout = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
     // the chain's end: MH_std, the escape test and its electron (thread 0)
     if (t0) {
       s_add = 0;
