@@ -73,10 +73,11 @@ cudaError_t rd_launch_mh_jump(int prec, int geometry_mask, int grid, cudaStream_
 cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
                                  const Pool& pool, const PlanEntry* sup_plan, const PlanHeader* sup_ph,
                                  const float4* qpp, const double* qF, const NearState& nr, double kscale);
-cudaError_t rd_launch_mh_jumps_near(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
-                                    const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
-                                    const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
-                                    int jumps, const NearState& nr, double kscale, int* gave_up, bool lone);
+cudaError_t rd_launch_mh_jumps_near(int prec, int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
+                                    const Pool& pool, const PlanEntry* plan, const PlanHeader* ph,
+                                    const PlanEntry* plan_mh, const ChainState& cs, const int* ch_off,
+                                    const double* wtab, const int* step_ptr, int jumps, const NearState& nr,
+                                    double kscale, int* gave_up, bool lone);
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                            const Pool& pool, const ChainState& cs, const int* ch_off,
                            const double* work, const int* step_ptr, const EventLog& ev);
@@ -506,7 +507,7 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
     if (slow) pm = PM_MH_SLOW;
   }
   if (near) {
-    CK(rd_launch_mh_jumps_near(e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
+    CK(rd_launch_mh_jumps_near(prec, e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
                                e->plan[PM_MH], e->cs, e->d_choff, e->wtab, e->d_step, s.jumps, e->nr, e->kscale,
                                e->cq + 3, s.mh_near == 1));
     e->kernels_in_step += s.mh_near == 1 ? 2 : 1;
@@ -908,7 +909,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
       e->dalloc(&e->cs.fF, chcap) || e->dalloc(&e->cs.fe, chcap) ||
       e->dalloc(&e->cs.fgx, chcap) || e->dalloc(&e->cs.fgy, chcap) ||
       e->dalloc(&e->cs.pph, chcap) || e->dalloc(&e->cs.pih, chcap) ||
-      (cfg->precision == RD_PREC_FP32C && alloc_near(e, cap, qcap, S)) ||
+      alloc_near(e, cap, qcap, S) ||
       e->dalloc(&e->d_choff, S) || e->dalloc(&e->d_qoff, S) ||
       e->dalloc(&e->d_npts, S) || e->dalloc(&e->d_zero_off, S) ||
       e->dalloc(&e->partial, (size_t)e->max_items * 3 * RD_ITILE) ||
@@ -1062,15 +1063,15 @@ static int flush_admissions(rd_engine* e) {
   return RD_OK;
 }
 
-// The near / far split of the FP32 chains' field for a new planar diode.  It wants
+// The near / far split of the chains' field (rd_near.cuh) for a new planar diode.  It wants
 // the 4-node supply rule (its panels carry the far part), one image partner
 // (every term of the sum has one sign), panels that are about square (the two
 // axes share the near region) and enough of them that the near region is a
 // part of the emitter (P >= 16; the default rule gives that).  Everything else
 // keeps the pair-sum jumps, as do diodes that are given ions or atoms later.
-static void near_params(const rd_engine* e, DiodeParams& p, int P, int Q) {
+static void near_params(DiodeParams& p, int P, int Q) {
   p.mh_fast = 0;
-  if (e->cfg.precision != RD_PREC_FP32C || p.geometry != RD_G_PLANAR || p.mh_serial || p.emitter_type == 4 ||
+  if (p.geometry != RD_G_PLANAR || p.mh_serial || p.emitter_type == 4 ||
       !p.image_charge || p.N_ic_max != 0 || Q != 4 || P < 16 || P > 1024 || p.max_chains >= 1 << 22)
     return;
   const double ax = 0.5e9 * p.em_Lx / P, ay = 0.5e9 * p.em_Ly / P;
@@ -1247,7 +1248,7 @@ static int diode_add_impl(rd_engine* e, const rd_diode_config* c, int* diode, cu
     qs.ring_rmin = p.ring_rmin; qs.ring_thick = p.ring_thick; qs.org_x = p.org_x; qs.org_y = p.org_y;
     qs.a_foci = p.a_foci; qs.eta_1 = p.eta_1; qs.max_xi = p.max_xi; qs.shift_z = p.shift_z;
     if (c->geometry == RD_GEOM_PLANAR) gauss_legendre(Q, qs.gx, qs.gw);
-    near_params(e, p, P_, Q);
+    near_params(p, P_, Q);
     CK(rd_launch_quad_fill(us, qs, e->qx, e->qy, e->qz, e->qw, e->qpp));
   }
   CK(upload(e, e->work + sl.w_off, wv.data(), sl.w_len * sizeof(double), us, deferred));
@@ -1819,9 +1820,10 @@ int rd_do_emission(rd_engine* e, int step) {
   NvtxRange nvtx_range("rd_do_emission");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   CK(rd_launch_step_set(e->st, e->d_step, step));
-  e->packs_stale = true;
-  int rc = launch_emission(e);
+  int rc = fresh_packs(e);   // of an emission just before this one
   if (rc) return rc;
+  e->packs_stale = true;
+  if ((rc = launch_emission(e))) return rc;
   CK(cudaStreamSynchronize(e->st));
   return compaction_check(e);
 }

@@ -273,6 +273,31 @@ __device__ __forceinline__ void work_entry_f(const DiodeParams& p, const double*
   *t0 = (float)log(phi); *t2 = (float)(c_k.l_const / (phi * phi));
 }
 
+// The same at a point in metres.
+__device__ __forceinline__ void work_entry_d(const DiodeParams& p, const double* __restrict__ wtab, double x, double y,
+                                             float* t0, float* t2) {
+  const int cell = work_cell(p, x, y);
+  if (cell >= 0) {
+    const double* t = wtab + 3 * (p.work_off + cell);
+    *t0 = (float)t[0]; *t2 = (float)t[2];
+    return;
+  }
+  const double phi = gaussian_work(p, p.work_data, x, y);
+  *t0 = (float)log(phi); *t2 = (float)(c_k.l_const / (phi * phi));
+}
+
+// What the near / far split (rd_near.cuh) keeps of an FP64 chain's field.
+__device__ __forceinline__ void near_start_d(const DiodeParams& p, const ChainState& cs, const double* __restrict__ wtab,
+                                             int k, double x, double y, double F) {
+  if (!p.mh_fast) return;
+  float t0, t2;
+  work_entry_d(p, wtab, x, y, &t0, &t2);
+  const float Ff = (float)F;
+  cs.fF[k] = Ff;
+  cs.fe[k] = 1.2e-7f * fabsf(Ff);
+  cs.fsup[k] = rho_entry_f(p, t0, t2, Ff);
+}
+
 // rho of an FP32 chain's point for the field F < 0 (as a float).
 __device__ __forceinline__ float rho_xy_f(const DiodeParams& p, const double* __restrict__ wtab, float x,
                                           float y, float F) {
@@ -881,6 +906,7 @@ __global__ void k_mh_init(const DiodeParams* __restrict__ P, DiodeDyn* __restric
             double g1, g2;
             gauss2(p.seed, (uint32_t)c, 1u, step, &g1, &g2);
             cs.gx[k] = g1; cs.gy[k] = g2;
+            near_start_d(p, cs, wtab, k, X, Y, F);
           }
         }
       }
@@ -1134,6 +1160,7 @@ __device__ __forceinline__ void mh_start_f64(const DiodeParams& p, ChainState& c
   if (F < 0.0 && p.init_rounds > 0) {
     cs.ok[k] = 1; cs.F[k] = F; cs.x[k] = x; cs.y[k] = y;
     cs.sup[k] = supply_log_xy(p, wtab, x, y, F);
+    near_start_d(p, cs, wtab, k, x, y, F);
     double g1, g2;
     gauss2(p.seed, (uint32_t)c, 1u, step, &g1, &g2);
     cs.gx[k] = g1; cs.gy[k] = g2;
@@ -1210,7 +1237,7 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
         const int c = it.i0 + tid + q * nt;
         kk[q] = ch_off[it.d] + c;
         ok[q] = (c < M) ? (init ? 1 : cs.ok[kk[q]]) : 0;
-        mh_propose_f64(p, cs, kk[q], c, ok[q], init, dry, step, sx, sy, &wx[q], &wy[q]);
+        mh_propose_f64(p, cs, kk[q], c, ok[q], init, dry || fin, step, sx, sy, &wx[q], &wy[q]);
       }
     }
     double s[CPT];
@@ -1236,16 +1263,16 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
     }
     // epilogue of the completed tile
     if (dry) continue;
-    if constexpr (PREC == 1) {
-      if (fin) {   // the field and the point in metres that the emission test reads
-        for (int q = 0; q < CPT; ++q) {
-          if (!ok[q]) continue;
-          cs.F[kk[q]] = z0_finish<PREC>(p, s[q], kscale);
+    if (fin) {   // the field and the point in metres that the emission test reads
+      for (int q = 0; q < CPT; ++q) {
+        if (!ok[q]) continue;
+        cs.F[kk[q]] = z0_finish<PREC>(p, s[q], kscale);
+        if constexpr (PREC == 1) {
           cs.x[kk[q]] = p.org_x + (double)fwx[q] * 1.0e-9;
           cs.y[kk[q]] = p.org_y + (double)fwy[q] * 1.0e-9;
         }
-        continue;
       }
+      continue;
     }
     if (init) {   // a favourable start (F < 0) makes the chain; the others go to k_mh_init
       for (int q = 0; q < CPT; ++q) {
@@ -2655,19 +2682,28 @@ static cudaError_t launch_coop(void (*kernel)(A...), int block, int grid, cudaSt
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kernel, args...);
 }
-cudaError_t rd_launch_mh_jumps_near(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
-                                    const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
-                                    const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
-                                    int jumps, const NearState& nr, double kscale, int* gave_up, bool lone) {
-  const int most = rd_grid(k_mh_jumps_near, 128, 0), most1 = rd_grid(k_mh_jumps_near_one, 256, 0);
+template <int PREC>
+static cudaError_t launch_jumps_near(int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy, const Pool& pool,
+                                     const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
+                                     const ChainState& cs, const int* ch_off, const double* wtab, const int* step_ptr,
+                                     int jumps, const NearState& nr, double kscale, int* gave_up, bool lone) {
+  const int most = rd_grid(k_mh_jumps_near<PREC>, 128, 0), most1 = rd_grid(k_mh_jumps_near_one<PREC>, 256, 0);
   const int g = grid > 0 && grid < most ? grid : most, g1 = grid > 0 && grid < most1 ? grid : most1;
   if (lone) {
-    const cudaError_t e = launch_coop(k_mh_jumps_near_one, 256, g1, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab,
-                                      step_ptr, jumps, nr, kscale, gave_up);
+    const cudaError_t e = launch_coop(k_mh_jumps_near_one<PREC>, 256, g1, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off,
+                                      wtab, step_ptr, jumps, nr, kscale, gave_up);
     if (e != cudaSuccess) return e;
   }
-  return launch_coop(k_mh_jumps_near, 128, g, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr,
-                     kscale, gave_up, lone ? g1 : 0);
+  return launch_coop(k_mh_jumps_near<PREC>, 128, g, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps,
+                     nr, kscale, gave_up, lone ? g1 : 0);
+}
+cudaError_t rd_launch_mh_jumps_near(int prec, int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
+                                    const Pool& pool, const PlanEntry* plan, const PlanHeader* ph,
+                                    const PlanEntry* plan_mh, const ChainState& cs, const int* ch_off,
+                                    const double* wtab, const int* step_ptr, int jumps, const NearState& nr,
+                                    double kscale, int* gave_up, bool lone) {
+  if (prec == 1) return launch_jumps_near<1>(grid, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr, kscale, gave_up, lone);
+  return launch_jumps_near<0>(grid, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr, kscale, gave_up, lone);
 }
 
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,

@@ -1,10 +1,12 @@
-// rd_near.cuh -- the jumps of the FP32 planar Metropolis-Hastings chains from a
-// near / far split of the cathode field (included by rd_field.cu, in its
-// anonymous namespace).
+// rd_near.cuh -- the jumps of the planar Metropolis-Hastings chains from a near /
+// far split of the cathode field (included by rd_field.cu, in its anonymous
+// namespace).
 //
 // A jump needs the field at its proposal only to compare two targets, and the
 // FP32 chains already decide from FP32 estimates of the targets wherever those
-// are certain (mh_decide_f).  The same holds for the field itself: an estimate
+// are certain (mh_decide_f).  (The FP64 form's chains take the same estimates, with
+// FP64 points, draws and pair sums; below u and the pair sum's roundings are the FP32
+// form's, the FP64 form's are smaller.)  The same holds for the field itself: an estimate
 // with a bound on how far it can lie from the value the pair-sum kernel
 // (k_mh_jump_planar) computes decides every jump outside that bound, and the few
 // jumps inside it take the pair sum.  So the decisions, and with them the
@@ -38,6 +40,7 @@
 //   one diode, 4500 electrons, 3800 chains, 100 jumps      6.13 -> 0.79 ms
 //   24 diodes of 256-4096 electrons, 30,000 chains, 200    15.9 -> 2.3 ms
 //   128 diodes of 256-32768 electrons, 353,000 chains, 200  276 -> 26.4 ms
+//   FP64: 1300 electrons, 960 chains, 100                   8.4 -> 1.0 ms
 // Open after the estimate: one jump in 10^5; the estimate lay within 0.08 of its
 // bound in every jump checked.  What is left is latency (one near list, one far
 // record, three logarithms and one counter per jump), not arithmetic.
@@ -150,8 +153,9 @@ k_near_scatter(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ D
   }
 }
 
-__device__ __forceinline__ float near_term(float4 h, float2 l, float px, float py) {
-  const float dx = (px - h.x) - l.x, dy = (py - h.y) - l.y;
+// The term of one electron at a point on the FP32 grid, or (qx, qy) off it.
+__device__ __forceinline__ float near_term(float4 h, float2 l, float px, float py, float qx = 0.0f, float qy = 0.0f) {
+  const float dx = (px - h.x) - (l.x - qx), dy = (py - h.y) - (l.y - qy);
   const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, h.z)));
   return h.w * ((inv * inv) * inv);
 }
@@ -503,6 +507,60 @@ __device__ __noinline__ int near_open(const DiodeParams& p, const Pool& pool, co
   return a;
 }
 
+// The FP64 chains' open jumps: FP64 sums at both points by the block, then the test
+// of mh_accept_one.
+template <int NT>
+__device__ __noinline__ int near_open64(const DiodeParams& p, const Pool& pool, const ChainState& cs,
+                                        const double* __restrict__ wtab, const PlanEntry& e, double kscale, bool mine,
+                                        int c, int k, int it_idx, uint32_t step, double px, double py, double cx,
+                                        double cy, double (*red)[NT / 32]) {
+  const int tid = threadIdx.x, nic = p.image_charge ? p.N_ic_max : 0;
+  double s0 = 0.0, s1 = 0.0;
+  for (int j = tid; j < e.n_j; j += NT) {
+    const int g = p.off + j;
+    const rd_d4 pj = make_d4(pool.x[g], pool.y[g], pool.z[g], pool.q[g]);
+    s0 += z0_tile_f64(&pj, 1, px, py, nic, p.d, c_k.L2);
+    s1 += z0_tile_f64(&pj, 1, cx, cy, nic, p.d, c_k.L2);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  }
+  if ((tid & 31) == 0) { red[0][tid >> 5] = s0; red[1][tid >> 5] = s1; }
+  __syncthreads();
+  int a = 0;
+  if (mine) {
+    s0 = s1 = 0.0;
+    for (int w = 0; w < NT / 32; ++w) { s0 += red[0][w]; s1 += red[1][w]; }
+    const double F = z0_finish<0>(p, s0, kscale), Fc = z0_finish<0>(p, s1, kscale);
+    float t0, t2;
+    work_entry_d(p, wtab, cx, cy, &t0, &t2);
+    cs.fF[k] = (float)Fc;
+    cs.fe[k] = 1.2e-7f * fabsf((float)Fc);
+    cs.fsup[k] = rho_entry_f(p, t0, t2, (float)Fc);
+    if (F < 0.0) {
+      const double sn = supply_log_xy(p, wtab, px, py, F), sc = supply_log_xy(p, wtab, cx, cy, Fc);
+      bool take = sn >= sc;
+      if (!take) {
+        double u1, u2;
+        rng2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, &u1, &u2);
+        take = log(u1) <= sn - sc;
+      }
+      if (take) {
+        work_entry_d(p, wtab, px, py, &t0, &t2);
+        cs.x[k] = px; cs.y[k] = py;
+        cs.fF[k] = (float)F;
+        cs.fe[k] = 1.2e-7f * fabsf((float)F);
+        cs.fsup[k] = rho_entry_f(p, t0, t2, (float)F);
+        a = 1;
+      }
+    }
+  }
+  __syncthreads();
+  return a;
+}
+
 // The plan entry of item g: two rounds of 32 slots each instead of a binary search's
 // chain of loads (more than 1024 slots take decode_item).
 __device__ __forceinline__ int near_entry(const PlanEntry* __restrict__ plan, int nd, int g, int lane) {
@@ -554,15 +612,23 @@ __device__ __forceinline__ void near_counts(const DiodeParams& p, DiodeDyn& y, u
 // each still polls at most RD_NEAR_SPIN times (about a second), after which the
 // block counts in *gave_up and leaves (rd_run reports it).
 // ONE: every block has at most one item; its chains stay in registers.
-template <int NW>
+template <int PREC, int NW>
 struct NearShared {
-  float x[32], y[32], near[32], lu[32], g[2][32];   // proposal, near sum, log u, next Gaussian pair
-  int pan[32];                                      // the chain's panel; -1: no chain
-  float cx[32], cy[32];                             // the chains' points, where a jump is left open
+  using Real = typename std::conditional<PREC == 1, float, double>::type;
+  float x[32], y[32], near[32], lu[32];   // proposal (nm; FP64 chains: high words), near sum, log u
+  float xl[PREC == 1 ? 1 : 32], yl[PREC == 1 ? 1 : 32];   // FP64 chains: low words
+  Real g[2][32];                          // next Gaussian pair
+  int pan[32];                            // the chain's panel; -1: no chain
+  Real ox[32], oy[32], cx[32], cy[32];    // proposals and chains' points, where a jump is left open
   unsigned open;
   int dead;
-  NearExact<32 * NW> ex;
+  typename std::conditional<PREC == 1, NearExact<32 * NW>, double[2][NW]>::type ex;
 };
+
+template <int PREC>
+__device__ __forceinline__ typename std::conditional<PREC == 1, float, double>::type* near_sel(float* f, double* d) {
+  if constexpr (PREC == 1) return f; else return d;
+}
 
 // The far part at a point: a panel's record, then its value and bound (c0.x, c0.y).
 struct NearFar {
@@ -583,18 +649,25 @@ struct NearFar {
   }
 };
 
-template <int NW, bool ONE>
-__device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const Pool& pool,
-                                           const PlanEntry* __restrict__ plan, int total, int nd,
+template <int PREC, int NW, bool ONE>
+__device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const DiodeParams* __restrict__ P,
+                                           DiodeDyn* __restrict__ Dy, const Pool& pool, const PlanEntry* __restrict__ plan, int total, int nd,
                                            const PlanEntry* __restrict__ plan_mh, const ChainState& cs,
                                            const int* __restrict__ ch_off, const double* __restrict__ wtab,
                                            int engine_step, int jumps, const NearState& nr, double kscale, int* gave_up) {
+  using Real = typename NearShared<PREC, NW>::Real;
   constexpr int NT = 32 * NW, ROUNDS = 8 / NW;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   if (tid == 0) sh.dead = 0;
   const float ksc = (float)kscale;
+  // the chains' points and Gaussian pairs in memory: nm from the emitter's centre, or m
+  Real* const ax = near_sel<PREC>(cs.fx, cs.x);
+  Real* const ay = near_sel<PREC>(cs.fy, cs.y);
+  Real* const agx = near_sel<PREC>(cs.fgx, cs.gx);
+  Real* const agy = near_sel<PREC>(cs.fgy, cs.gy);
   // the chains of the block's item (ONE; warp 0)
-  float fx = 0.0f, fy = 0.0f, gx = 0.0f, gy = 0.0f, Fc = 0.0f, rc = 0.0f, fe = 0.0f;
+  Real fx = 0, fy = 0, gx = 0, gy = 0;
+  float Fc = 0.0f, rc = 0.0f, fe = 0.0f;
   int ok = 0, d = 0;
   for (int it = 1; it <= jumps; ++it) {
     for (int g = blockIdx.x; g < total; g += gridDim.x) {
@@ -607,12 +680,14 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
       const uint32_t step = (uint32_t)(engine_step - y.step_offset);
       const float* recs = nr.rec + (size_t)(p.q_off / 16) * RD_NEAR_REC;
       float px = 0.0f, py = 0.0f, t0 = 0.0f, t2 = 0.0f;
+      Real ox = 0, oy = 0;   // the proposal
       NearFar far_part;
       unsigned long long pr = 0;
       if (NW > 1 ? w == NW - 1 : true) {   // the next proposal's Gaussian pair
         if (c < M && it < p.mh_jumps && cs.ok[k]) {
-          float g1, g2;
-          gauss2f(p.seed, (uint32_t)c, (uint32_t)(it + 1), step, &g1, &g2);
+          Real g1, g2;
+          if constexpr (PREC == 1) gauss2f(p.seed, (uint32_t)c, (uint32_t)(it + 1), step, &g1, &g2);
+          else gauss2(p.seed, (uint32_t)c, (uint32_t)(it + 1), step, &g1, &g2);
           sh.g[0][lane] = g1;
           sh.g[1][lane] = g2;
         }
@@ -626,7 +701,7 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
         if (!ONE || it == 1) {
           ok = c < M ? cs.ok[k] : 0;
           if (ok) {
-            fx = cs.fx[k]; fy = cs.fy[k]; gx = cs.fgx[k]; gy = cs.fgy[k];
+            fx = ax[k]; fy = ay[k]; gx = agx[k]; gy = agy[k];
             Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k];
           }
         }
@@ -638,15 +713,35 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
           if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
         }
         pr = __shfl_sync(0xffffffffu, pr, 0);
-        const float mhs = __uint_as_float((unsigned)(pr >> 32));
-        const float sx = (it > ndim_first) ? p.em_wx * mhs : p.em_wx * 0.10f;
-        const float sy = (it > ndim_first) ? p.em_wy * mhs : p.em_wy * 0.10f;
-        if (ok) {   // mh_propose_f32
-          const float hx = p.em_hx, hy = p.em_hy;
-          px = fmaf(gx, sx, fx);
-          py = fmaf(gy, sy, fy);
-          if (px > hx) px = hx - (px - hx); else if (px < -hx) px = -hx - (px + hx);
-          if (py > hy) py = hy - (py - hy); else if (py < -hy) py = -hy - (py + hy);
+        if constexpr (PREC == 1) {   // mh_propose_f32
+          const float mhs = __uint_as_float((unsigned)(pr >> 32));
+          const float sx = (it > ndim_first) ? p.em_wx * mhs : p.em_wx * 0.10f;
+          const float sy = (it > ndim_first) ? p.em_wy * mhs : p.em_wy * 0.10f;
+          if (ok) {
+            const float hx = p.em_hx, hy = p.em_hy;
+            px = fmaf(gx, sx, fx);
+            py = fmaf(gy, sy, fy);
+            if (px > hx) px = hx - (px - hx); else if (px < -hx) px = -hx - (px + hx);
+            if (py > hy) py = hy - (py - hy); else if (py < -hy) py = -hy - (py + hy);
+          }
+          ox = px; oy = py;
+        } else {                     // mh_propose_f64
+          __threadfence();           // MH_std was written before the progress word
+          const double mhs = __ldcg(&y.MH_std);
+          const double sx = (it > ndim_first) ? p.em_Lx * mhs : p.em_Lx * 0.10;
+          const double sy = (it > ndim_first) ? p.em_Ly * mhs : p.em_Ly * 0.10;
+          ox = p.em_x0; oy = p.em_y0;
+          if (ok) {
+            const double hx = p.em_x0 + p.em_Lx, hy = p.em_y0 + p.em_Ly;
+            ox = fma(gx, sx, fx);
+            oy = fma(gy, sy, fy);
+            if (ox > hx) ox = hx - (ox - hx); else if (ox < p.em_x0) ox = (p.em_x0 - ox) + p.em_x0;
+            if (oy > hy) oy = hy - (oy - hy); else if (oy < p.em_y0) oy = (p.em_y0 - oy) + p.em_y0;
+          }
+          float lx, ly;
+          split_nm(ox, p.org_x, &px, &lx);
+          split_nm(oy, p.org_y, &py, &ly);
+          sh.xl[lane] = lx; sh.yl[lane] = ly;
         }
         const int NP = p.nr_P;
         const int ppx = min(max((int)floorf((px + p.em_hx) * p.nr_iwx), 0), NP - 1);
@@ -658,7 +753,10 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
         const float4* rec = reinterpret_cast<const float4*>(recs + (size_t)pan * RD_NEAR_REC);
         far_part.load(rec);
         if (!ONE) far_part.eval(p, px, py);   // (ONE: evaluated after the near sums, the loads in flight meanwhile)
-        if (ok) work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
+        if (ok) {
+          if constexpr (PREC == 1) work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
+          else work_entry_d(p, wtab, ox, oy, &t0, &t2);
+        }
       } else {
         __syncthreads();
       }
@@ -674,7 +772,7 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
           // the list's rows: their ends in it, and what turns an index of it into an electron
           const int4* rt = reinterpret_cast<const int4*>(recs + (size_t)pan * RD_NEAR_REC + 20);
           const int4 end = rt[0], at = rt[1];
-          const float x = sh.x[q], yv = sh.y[q];
+          const float x = sh.x[q], yv = sh.y[q], xl = PREC == 1 ? 0.0f : sh.xl[q], yl = PREC == 1 ? 0.0f : sh.yl[q];
           const float4* nh = nr.hi + p.off;
           const float2* nl = nr.lo + p.off;
           float run = 0.0f;
@@ -691,7 +789,7 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
               lo[u] = in ? nl[k2] : make_float2(0.0f, 0.0f);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) run += near_term(h[u], lo[u], x, yv);
+            for (int u = 0; u < 4; ++u) run += near_term(h[u], lo[u], x, yv, xl, yl);
             if (++m == 8) { s += run; run = 0.0f; m = 0; }   // short runs: the sum stays accurate
           }
           s += run;
@@ -704,7 +802,7 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
       int a = 0;
       if (w == 0) {   // the decisions (mh_decide_f with the field's bound added to its guard)
         int open = 0;
-        const float cx = fx, cy = fy;
+        const Real cx = fx, cy = fy;
         if (ok) {
           if (ONE) far_part.eval(p, px, py);
           const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y;
@@ -713,35 +811,39 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
           const int take = near_decide(p, Fn, dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
           open = take < 0;
           if (take == 1) {
-            fx = px; fy = py; rc = rn; Fc = Fn; fe = dF;
+            fx = ox; fy = oy; rc = rn; Fc = Fn; fe = dF;
             a = 1;
           }
         }
         const unsigned mask = __ballot_sync(0xffffffffu, open);
-        if (mask) { sh.cx[lane] = cx; sh.cy[lane] = cy; }
+        if (mask) { sh.cx[lane] = cx; sh.cy[lane] = cy; sh.ox[lane] = ox; sh.oy[lane] = oy; }
         if (lane == 0) sh.open = mask;
         if (ok && ((!ONE && a) || open)) {
-          cs.fx[k] = fx; cs.fy[k] = fy; cs.fF[k] = Fc; cs.fsup[k] = rc; cs.fe[k] = fe;
+          ax[k] = fx; ay[k] = fy; cs.fF[k] = Fc; cs.fsup[k] = rc; cs.fe[k] = fe;
         }
         if (ok && it < p.mh_jumps) {
           gx = sh.g[0][lane];
           gy = sh.g[1][lane];
-          if (!ONE) { cs.fgx[k] = gx; cs.fgy[k] = gy; }
+          if (!ONE) { agx[k] = gx; agy[k] = gy; }
         }
       }
       if (NW > 1) __syncthreads(); else __syncwarp();
       const unsigned open = sh.open;
       for (unsigned o = open; o; o &= o - 1) {   // block-uniform
         const int q = __ffs(o) - 1;
-        a += near_open<NT>(p, pool, cs, wtab, plan_mh[d], kscale, tid == q, c, k, it, step, sh.x[q], sh.y[q], sh.cx[q],
-                           sh.cy[q], sh.lu[q], &sh.ex);
-        if (ONE && tid == q) { fx = cs.fx[k]; fy = cs.fy[k]; Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k]; }
+        if constexpr (PREC == 1)
+          a += near_open<NT>(p, pool, cs, wtab, plan_mh[d], kscale, tid == q, c, k, it, step, sh.ox[q], sh.oy[q],
+                             sh.cx[q], sh.cy[q], sh.lu[q], &sh.ex);
+        else
+          a += near_open64<NT>(p, pool, cs, wtab, plan_mh[d], kscale, tid == q, c, k, it, step, sh.ox[q], sh.oy[q],
+                               sh.cx[q], sh.cy[q], sh.ex);
+        if (ONE && tid == q) { fx = ax[k]; fy = ay[k]; Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k]; }
       }
       if (w == 0) {
         const int acc = __popc(__ballot_sync(0xffffffffu, a)), rej = __popc(__ballot_sync(0xffffffffu, ok && !a));
         if (lane == 0)
           near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, ndim_first, acc, rej);
-        if (ONE && ok && it == p.mh_jumps) { cs.fx[k] = fx; cs.fy[k] = fy; }   // the last points (RD_MH_FINAL)
+        if (ONE && ok && it == p.mh_jumps) { ax[k] = fx; ay[k] = fy; }   // the last points (RD_MH_FINAL)
       }
     }
   }
@@ -749,30 +851,32 @@ __device__ __forceinline__ void near_jumps(NearShared<NW>& sh, const DiodeParams
 
 // A lone diode's few items: eight warps each, the chains in registers (at most two
 // blocks per SM; leaves larger diodes to k_mh_jumps_near).
+template <int PREC>
 __global__ void __launch_bounds__(256, 2)
 k_mh_jumps_near_one(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const __grid_constant__ Pool pool,
                     const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
                     const PlanEntry* __restrict__ plan_mh, const __grid_constant__ ChainState cs,
                     const int* __restrict__ ch_off, const double* __restrict__ wtab, const int* __restrict__ step_ptr,
                     int jumps, const __grid_constant__ NearState nr, double kscale, int* gave_up) {
-  __shared__ NearShared<8> sh;
+  __shared__ NearShared<PREC, 8> sh;
   const int total = ph->total_items;
   if ((int)blockIdx.x >= total || total > (int)gridDim.x) return;
-  near_jumps<8, true>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
+  near_jumps<PREC, 8, true>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
                       gave_up);
 }
 
 // Any number of items, four warps each; above: leaves plans of at most that many
 // items to k_mh_jumps_near_one.
-__global__ void __launch_bounds__(128, 8)
+template <int PREC>
+__global__ void __launch_bounds__(128, PREC == 1 ? 8 : 4)
 k_mh_jumps_near(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const __grid_constant__ Pool pool,
                 const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
                 const PlanEntry* __restrict__ plan_mh, const __grid_constant__ ChainState cs,
                 const int* __restrict__ ch_off, const double* __restrict__ wtab, const int* __restrict__ step_ptr,
                 int jumps, const __grid_constant__ NearState nr, double kscale, int* gave_up, int above) {
-  __shared__ NearShared<4> sh;
+  __shared__ NearShared<PREC, 4> sh;
   const int total = ph->total_items;
   if ((int)blockIdx.x >= total || total <= above) return;
-  near_jumps<4, false>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
+  near_jumps<PREC, 4, false>(sh, P, Dy, pool, plan, total, ph->n_diodes, plan_mh, cs, ch_off, wtab, *step_ptr, jumps, nr, kscale,
                        gave_up);
 }

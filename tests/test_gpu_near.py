@@ -1,4 +1,4 @@
-"""The near / far split of the FP32 chains' field (rd_near.cuh) against the pair-sum
+"""The near / far split of the chains' field (rd_near.cuh) against the pair-sum
 jumps.  A diode that was given an atom keeps the pair-sum kernel, also after the atom
 has left, so the same diode with and without that history has to run the same
 chains: every electron, counter and step size equal, bit for bit."""
@@ -30,11 +30,11 @@ def _electrons(n, side_x, side_y, gap, seed, low=3):
     return np.column_stack([r.uniform(-0.6, 0.6, n) * side_x, r.uniform(-0.6, 0.6, n) * side_y, z]) * NM
 
 
-def _run(rg, diodes, steps, atom, chunk=None):
+def _run(rg, diodes, steps, atom, chunk=None, fp64=False):
     quad = sum(rg.supply_points(**kw) for kw, _ in diodes) + 64 * len(diodes)
     cap = sum(kw["capacity"] + 64 for kw, _ in diodes)
     chains = sum(max(kw["capacity"], kw.get("max_chains", 0)) + 64 for kw, _ in diodes)
-    with rg.Engine(precision=rg.PREC_FP32C, max_diodes=len(diodes), particle_capacity=cap, chain_capacity=chains,
+    with rg.Engine(precision=rg.PREC_FP64 if fp64 else rg.PREC_FP32C, max_diodes=len(diodes), particle_capacity=cap, chain_capacity=chains,
                    quad_capacity=quad) as eng:
         if chunk:
             eng.set_chunking(*chunk)
@@ -91,6 +91,48 @@ def test_near_far_chains_equal_pair_sum_chains(rg, name, chunk):
     fast, slow = (_run(rg, [(kw, pos)], 3, atom, chunk) for atom in (False, True))
     assert fast[0][1]["emitted_total"] > 0
     _same(fast, slow)
+
+
+@pytest.mark.parametrize("name,chunk", [(name, None) for name in sorted(CASES)] + [("tile-edge", (128, 32))])
+def test_near_far_fp64_chains_equal_pair_sum_chains(rg, name, chunk):
+    n, lx, ly, gap, opt = CASES[name]
+    opt = dict(opt)
+    pos = _electrons(n, lx, ly, gap, 6, opt.pop("low", 3))
+    kw = _kw(lx, ly, n + 6000, gap=gap, **opt)
+    fast, slow = (_run(rg, [(kw, pos)], 3, atom, chunk, fp64=True) for atom in (False, True))
+    assert fast[0][1]["emitted_total"] > 0
+    _same(fast, slow)
+
+
+def test_near_far_fp64_mix_equals_alone(rg):
+    sizes = [(700, 200.0, 300.0), (900, 900.0, 700.0), (60, 1500.0, 1000.0)]
+    diodes = [(dict(_kw(s, s, n + 3000, gap=g), seed=100 + k), _electrons(n, s, s, g, k))
+              for k, (n, s, g) in enumerate(sizes)]
+    mix = _run(rg, diodes, 3, False, fp64=True)
+    for k, d in enumerate(diodes):
+        _same(_run(rg, [d], 3, False, fp64=True), mix[k:k + 1])
+
+
+def test_emission_after_emission(rg):
+    """Two emissions without a position update between them: the second one's
+    chains feel the first one's electrons."""
+    kw = _kw(400.0, 400.0, 4000)
+    pos = _electrons(500, 400.0, 400.0, 1000.0, 3)
+    res = []
+    for atom in (False, True):
+        with rg.Engine(precision=rg.PREC_FP64, max_diodes=1, particle_capacity=4100, chain_capacity=4100,
+                       quad_capacity=rg.supply_points(**kw) + 64) as eng:
+            d = eng.add_diode(**kw)
+            d.add_particles(pos, step=0)
+            if atom:
+                d.add_particle((0.0, 0.0, 500.0 * NM), species=rg.ATOM, step=0)
+                d.mark_particles_remove(len(pos), rg.REMOVE_TOP)
+                eng.remove_particles(0)
+            eng.do_emission(1)
+            eng.do_emission(2)
+            res.append((d.particles(), d.counters()))
+    assert res[0][1]["emitted_total"] > 0
+    _same(res[:1], res[1:])
 
 
 def test_near_far_mix_equals_alone(rg):
