@@ -78,6 +78,10 @@ cudaError_t rd_launch_mh_jumps_near(int prec, int grid, cudaStream_t st, const D
                                     const PlanEntry* plan_mh, const ChainState& cs, const int* ch_off,
                                     const double* wtab, const int* step_ptr, int jumps, const NearState& nr,
                                     double kscale, int* gave_up, bool lone);
+cudaError_t rd_launch_tip_near(int nslots, int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
+                               const Pool& pool, const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
+                               const ChainState& cs, const int* ch_off, const int* step_ptr, int jumps,
+                               const NearState& nr, double kscale, int* gave_up);
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
                            const Pool& pool, const ChainState& cs, const int* ch_off,
                            const double* work, const int* step_ptr, const EventLog& ev);
@@ -229,6 +233,7 @@ struct SlotHost {
   long long ch_off = 0, ch_len = 0;
   long long q_off = 0, q_len = 0;
   long long w_off = 0, w_len = 0;
+  unsigned char* tn_mem = nullptr;   // the tip's panels, lists and expansions (rd_tipnear.cuh)
 };
 
 struct rd_engine {
@@ -422,7 +427,8 @@ struct Sig {
   int jumps = 0;
   int mh_planar = 0;          // planar diodes with batched MH chains
   int mh_near = 0;            // of these, the diodes whose jumps take the near / far split
-  bool mh_slow() const { return mh_planar > mh_near || emit_tip; }
+  bool tip_near = false, tip_slow = false;   // tip diodes whose jumps take the split / the pair sums
+  bool mh_slow() const { return mh_planar > mh_near || tip_slow; }
 };
 static Sig signature(const rd_engine* e) {
   Sig s;
@@ -433,7 +439,12 @@ static Sig signature(const rd_engine* e) {
     if (p.geometry == RD_G_PLANAR && p.image_charge && p.N_ic_max > 0) s.nic = true;
     if (p.tts > 0) s.tts = true;
     if (p.emission) {
-      if (p.geometry == RD_G_TIP) s.emit_tip = true; else s.emit_planar = true;
+      if (p.geometry == RD_G_TIP) {
+        s.emit_tip = true;
+        if (p.tn) s.tip_near = true; else s.tip_slow = true;
+      } else {
+        s.emit_planar = true;
+      }
       if (p.geometry != RD_G_TIP && !p.image_charge) s.emit_lat = true;
       if (p.geometry != RD_G_TIP && p.mh_serial) s.emit_serial = true;
       if (p.geometry != RD_G_TIP && !p.mh_serial) s.mh_planar++;
@@ -446,9 +457,14 @@ static Sig signature(const rd_engine* e) {
 
 // The plans of the batched MH chains (counts of this step's supply).
 static cudaError_t plan_chains(rd_engine* e, const Sig& s) {
-  if (s.mh_near == 0) return plan(e, PM_MH);
-  if (s.mh_planar == s.mh_near) return plans_on(e, {PM_MH, PM_MH_NEAR}, e->st);
-  return plans_on(e, {PM_MH, PM_MH_NEAR, PM_MH_SLOW}, e->st);
+  PlanJobs jobs{};
+  auto add = [&](int m) { jobs.j[jobs.n++] = PlanJob{m, e->plan[m], e->ph[m]}; };
+  add(PM_MH);
+  if (s.mh_near > 0) add(PM_MH_NEAR);
+  if (s.mh_near > 0 && s.mh_planar > s.mh_near) add(PM_MH_SLOW);
+  if (s.tip_near) add(PM_MH_TIP);
+  e->kernels_in_step++;
+  return rd_launch_plan(e->st, e->dP, e->dD, e->nslots_hw(), jobs, chunk_rule(e), e->max_items, nullptr);
 }
 
 // MH launch shape of the planar jumps for the resident mix: parts of the plan
@@ -512,14 +528,14 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
                                e->cq + 3, s.mh_near == 1));
     e->kernels_in_step += s.mh_near == 1 ? 2 : 1;
   }
-  const int tiled_jumps = slow || s.emit_tip ? s.jumps : 0;
+  const int tiled_jumps = slow || s.tip_slow ? s.jumps : 0;
   if ((rc = mh_fork(e, parts, main))) return rc;
   for (int it = 1; it <= tiled_jumps; ++it) {
     if (slow) {
       if ((rc = planar_mh_launch(e, s, it, parts, form, main, pm))) return rc;
       e->kernels_in_step += parts;
     }
-    if (s.emit_tip) {   // tip propose + jump
+    if (s.tip_slow) {   // tip propose + jump
       CK(rd_launch_mh_jump(prec, 2, e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH], e->ph[PM_MH], e->cs,
                            e->d_choff, e->wtab, e->d_step, it, e->partial, e->tickets, e->kscale, e->item_queue));
       e->kernels_in_step += 2;
@@ -529,6 +545,13 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
   if (near) {   // the pair sums at the chains' last points, for the emission test
     if ((rc = planar_mh_launch(e, s, RD_MH_FINAL, 1, form, main))) return rc;
     e->kernels_in_step++;
+  }
+  if (s.tip_near) {
+    CK(rd_launch_tip_near(e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_TIP], e->ph[PM_MH_TIP],
+                          e->plan[PM_MH], e->cs, e->d_choff, e->d_step, s.jumps, e->nr, e->kscale, e->cq + 3));
+    CK(rd_launch_mh_jump(prec, 2, e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH], e->ph[PM_MH], e->cs,
+                         e->d_choff, e->wtab, e->d_step, RD_MH_FINAL, e->partial, e->tickets, e->kscale, e->item_queue));
+    e->kernels_in_step += 4;
   }
   return RD_OK;
 }
@@ -728,9 +751,9 @@ static int launch_step_body(rd_engine* e) {
 static std::string sig_string(rd_engine* e) {
   Sig s = signature(e);
   char b[128];
-  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
+  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
            s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.mh_near > 1 ? 2 : s.mh_near, s.mh_planar > s.mh_near,
-           e->chunk_auto, s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
+           s.tip_near, s.tip_slow, e->chunk_auto, s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
   return b;
 }
 
@@ -965,6 +988,7 @@ int rd_engine_destroy(rd_engine* e) {
   if (e->st) cudaStreamSynchronize(e->st);
   if (e->graph) cudaGraphExecDestroy(e->graph);
   for (void* p : e->allocs) cudaFree(p);
+  for (auto& sl : e->slots) if (sl.tn_mem) cudaFree(sl.tn_mem);
   if (e->stage_d) cudaFree(e->stage_d);
   if (e->stage_i) cudaFree(e->stage_i);
   if (e->stage_hd) cudaFreeHost(e->stage_hd);
@@ -1089,12 +1113,103 @@ static void near_params(DiodeParams& p, int P, int Q) {
   p.nr_iwx = (float)(0.5 / ax); p.nr_iwy = (float)(0.5 / ay);
 }
 
+// The same for the FP32 chains of a new tip diode (rd_tipnear.cuh): its panels, and one
+// allocation for their records and lists, freed with the diode.  Without the memory the
+// diode keeps the pair-sum jumps.
+static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, cudaStream_t us, bool deferred) {
+  p.tn = 0;
+  if (e->cfg.precision != RD_PREC_FP32C || p.geometry != RD_G_TIP || p.max_chains >= 1 << 22) return cudaSuccess;
+  const double a = p.a_foci * 1.0e9, eta = p.eta_1, sh = p.shift_z * 1.0e9, s2 = std::sqrt(1.0 - eta * eta);
+  auto rad = [&](double xi) { return a * std::sqrt((xi * xi - 1.0) * (1.0 - eta * eta)); };
+  auto hgt = [&](double xi) { return a * xi * eta + sh; };
+  // arc length and area along the meridian, in steps of v = sqrt(xi - 1)
+  const int N = 4 * RD_TN_MAP;
+  const double vmax = std::sqrt(p.max_xi - 1.0);
+  std::vector<double> arc(N + 1, 0.0);
+  double area = 0.0;
+  for (int i = 0; i < N; ++i) {
+    const double v0 = vmax * i / N, v1 = vmax * (i + 1) / N, x0 = 1.0 + v0 * v0, x1 = 1.0 + v1 * v1;
+    const double ds = std::hypot(rad(x1) - rad(x0), hgt(x1) - hgt(x0));
+    arc[i + 1] = arc[i] + ds;
+    area += 3.14159265358979323846 * (rad(x0) + rad(x1)) * ds;
+  }
+  if (!(arc[N] > 0.0) || !std::isfinite(area)) return cudaSuccess;
+  const double width = std::sqrt(area / RD_TN_PANELS);
+  const int rings = std::max(1, std::min(RD_TN_RINGS, (int)std::ceil(arc[N] / width)));
+  std::vector<int2> map(RD_TN_MAP);
+  std::vector<float4> pan;
+  auto xi_at = [&](double s) {   // xi at arc length s
+    const int i = (int)(std::lower_bound(arc.begin(), arc.end(), s) - arc.begin());
+    const double v = vmax * std::min(i, N) / N;
+    return 1.0 + v * v;
+  };
+  std::vector<int2> ring(rings);
+  for (int r = 0; r < rings; ++r) {
+    const double sm = arc[N] * (r + 0.5) / rings, xm = xi_at(sm);
+    const int n = std::max(r == 0 ? 1 : 3, (int)std::ceil(2.0 * 3.14159265358979323846 * rad(xm) / width * (r == 0 ? 0.0 : 1.0)));
+    ring[r] = make_int2((int)pan.size(), n);
+    // the ring with a map entry's room on both sides
+    auto wider = [&](double s, double step) {
+      const double v = std::min(std::max(std::sqrt(xi_at(s) - 1.0) + step * 1.5 * vmax / RD_TN_MAP, 0.0), vmax);
+      return 1.0 + v * v;
+    };
+    const double xa = wider(arc[N] * r / rings, -1.0), xb = wider(arc[N] * (r + 1) / rings, 1.0);
+    const double half = 3.14159265358979323846 / n * 1.0001;
+    const double xc = n == 1 ? 1.0 : xm;
+    double rr = 0.0;
+    for (int i = 0; i <= 8; ++i)
+      for (int q = 0; q <= 8; ++q) {
+        const double xi = xa + (xb - xa) * i / 8, ph = half * q / 8;
+        rr = std::max(rr, std::hypot(std::hypot(rad(xi) * std::cos(ph) - rad(xc), rad(xi) * std::sin(ph)), hgt(xi) - hgt(xc)));
+      }
+    for (int q = 0; q < n; ++q) {
+      const double ph = 2.0 * 3.14159265358979323846 * (q + 0.5) / n;
+      pan.push_back(make_float4((float)(rad(xc) * std::cos(ph)), (float)(rad(xc) * std::sin(ph)), (float)hgt(xc),
+                                (float)(rr * 1.002 + 1.0e-3)));
+    }
+  }
+  for (int i = 0; i < RD_TN_MAP; ++i) {
+    const double s = arc[(size_t)(i * 2 + 1) * N / (2 * RD_TN_MAP)];
+    map[i] = ring[std::min(rings - 1, (int)(s / arc[N] * rings))];
+  }
+  const size_t np = pan.size();
+  p.tn_cap = std::min((long long)p.cap * RD_TN_LIST, 1ll << 27);
+  size_t at = 0;
+  auto part = [&](size_t bytes) { const size_t o = at; at += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t o_pan = part(sizeof(float4) * np), o_map = part(sizeof(int2) * RD_TN_MAP), o_rec = part(sizeof(float2) * 64 * np),
+               o_hdr = part(sizeof(float4) * np), o_next = part(sizeof(int)), o_list = part(sizeof(float4) * (size_t)p.tn_cap);
+  unsigned char* base = nullptr;
+  if (cudaMalloc(&base, at) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  sl.tn_mem = base;
+  p.tn_pan = (const float4*)(base + o_pan); p.tn_map = (const int2*)(base + o_map); p.tn_rec = (float2*)(base + o_rec);
+  p.tn_hdr = (float4*)(base + o_hdr); p.tn_next = (int*)(base + o_next); p.tn_list = (float4*)(base + o_list);
+  p.tn_np = (int)np;
+  p.tn_vs = (float)(RD_TN_MAP / vmax);
+  p.tn_nf = (float)(eta / s2);
+  p.tn_c = (float)(a * a * (1.0 - eta * eta));
+  p.tn_v0 = (float)(p.pre_E / s2);
+  p.tn_t0 = (float)std::log(p.tip_phi);
+  p.tn_t2 = (float)(e->k.l_const / (p.tip_phi * p.tip_phi));
+  p.tn_ir = (float)(1.0e-9 / p.r_tip);
+  p.tn_z0 = (float)((p.h_tip - p.r_tip) * 1.0e9);
+  p.tn_e2 = (float)(1.0 - eta * eta);
+  p.tn_ia = (float)(1.0 / a);
+  cudaError_t ce = cudaMemsetAsync(base + o_next, 0, sizeof(int), us);
+  if (ce == cudaSuccess) ce = upload(e, base + o_pan, pan.data(), sizeof(float4) * np, us, deferred);
+  if (ce == cudaSuccess) ce = upload(e, base + o_map, map.data(), sizeof(int2) * RD_TN_MAP, us, deferred);
+  p.tn = ce == cudaSuccess;
+  return ce;
+}
+
 // A diode that holds anything but electrons keeps the pair-sum jumps from now on.
 static int keep_pair_sum(rd_engine* e, int d) {
   DiodeParams& p = e->slots[d].p;
-  if (!p.mh_fast) return RD_OK;
-  p.mh_fast = 0;
-  e->act_P[d].mh_fast = 0;
+  if (!p.mh_fast && !p.tn) return RD_OK;
+  p.mh_fast = p.tn = 0;
+  e->act_P[d].mh_fast = e->act_P[d].tn = 0;
   CK(cudaMemcpyAsync(e->dP + d, &e->act_P[d], sizeof(DiodeParams), cudaMemcpyHostToDevice, e->st));
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
@@ -1249,6 +1364,7 @@ static int diode_add_impl(rd_engine* e, const rd_diode_config* c, int* diode, cu
     qs.a_foci = p.a_foci; qs.eta_1 = p.eta_1; qs.max_xi = p.max_xi; qs.shift_z = p.shift_z;
     if (c->geometry == RD_GEOM_PLANAR) gauss_legendre(Q, qs.gx, qs.gw);
     near_params(p, P_, Q);
+    CK(tip_near_params(e, p, sl, us, deferred));
     CK(rd_launch_quad_fill(us, qs, e->qx, e->qy, e->qz, e->qw, e->qpp));
   }
   CK(upload(e, e->work + sl.w_off, wv.data(), sl.w_len * sizeof(double), us, deferred));
@@ -1309,6 +1425,7 @@ int rd_diode_remove(rd_engine* e, int d) {
   if (sl.ch_len) e->ch_alloc.release(sl.ch_off, sl.ch_len);
   if (sl.q_len) e->q_alloc.release(sl.q_off, sl.q_len);
   if (sl.w_len) e->w_alloc.release(sl.w_off, sl.w_len);
+  if (sl.tn_mem) cudaFree(sl.tn_mem);
   sl = SlotHost();
   return RD_OK;
 }

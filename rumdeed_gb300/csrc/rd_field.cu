@@ -829,6 +829,58 @@ __device__ __forceinline__ double tip_target_log(const DiodeParams& p, double F,
   return log(v) + 0.5 * log(xi * xi - p.eta_1 * p.eta_1);
 }
 
+// Field normal to the tip at a surface point: vacuum field plus the particles' f3.
+__device__ __forceinline__ double tip_normal_field(const DiodeParams& p, double X, double Y, double Z, const double* f3) {
+  double ex, ey, ez, nx, ny, nz;
+  tip_field_E(p, X, Y, Z, &ex, &ey, &ez);
+  ex += f3[0]; ey += f3[1]; ez += f3[2];
+  tip_normal(p, X, Y, &nx, &ny, &nz);
+  return (nx * ex + ny * ey) + nz * ez;
+}
+
+// A component of the particles' field from its FP32 sums (tip_point_tiles_f32): direct
+// part (h, l), image part im, ci = R / dis of the point.
+__device__ __forceinline__ double tip_sum_finish(const DiodeParams& p, float h, float l, float im, float ci, double kscale) {
+  const double K = c_k.tip_K, cd = p.image_charge ? (1.0 + K) * kscale : kscale, ce = K * kscale;
+  const double cq = ce * (double)ci;
+  return ((double)h + (double)l) * cd - (double)im * cq;
+}
+
+// A jump's proposal: Gaussian step in (xi, phi), xi reflected, phi wrapped
+// (Metro_algo_tip_v3, src/mod_emission_tip.f90:1337-1365); false: xi left its range.
+__device__ __forceinline__ int tip_step(const DiodeParams& p, double xi, double phi, double g1, double g2, double sxi,
+                                        double sph, double* nxi, double* nph) {
+  const double twopi = 2.0 * c_k.pi;
+  double x = xi + g1 * sxi;
+  const double a = phi + g2 * sph;
+  double turns = a * (1.0 / twopi);      // Fortran MODULO; the quotient itself only next to a whole number
+  if (fabs(turns - rint(turns)) < 1.0e-9) turns = a / twopi;
+  *nph = a - floor(turns) * twopi;
+  if (x > p.max_xi) x = 2.0 * p.max_xi - x;
+  if (x < 1.0) x = 2.0 - x;
+  *nxi = x;
+  return !(x < 1.0 || x > p.max_xi);
+}
+
+// A surface point of the FP32 chains: at its FP32 nm coordinates (at most 6e-5 nm off
+// the surface).
+__device__ __forceinline__ void tip_grid_xyz(const DiodeParams& p, double xi, double phi, double* X, double* Y, double* Z) {
+  tip_xyz(p, xi, p.eta_1, phi, X, Y, Z);
+  *X = (double)(float)(*X * 1.0e9) * 1.0e-9;
+  *Y = (double)(float)(*Y * 1.0e9) * 1.0e-9;
+  *Z = (double)(float)(*Z * 1.0e9) * 1.0e-9;
+}
+
+// What the near / far split (rd_tipnear.cuh) keeps of a chain that starts at xi.
+__device__ __forceinline__ void tip_start(const DiodeParams& p, const ChainState& cs, int k, double xi, double F) {
+  if (!p.tn) return;
+  const float Ff = (float)F;
+  cs.fF[k] = Ff;
+  cs.fe[k] = 1.2e-7f * fabsf(Ff);
+  cs.fsup[k] = rho_entry_f(p, p.tn_t0 - 0.5f * logf((float)(xi * xi - p.eta_1 * p.eta_1)), p.tn_t2, Ff);
+  cs.em[k] = 0;   // not moved yet
+}
+
 template <int PREC>
 __global__ void k_mh_init(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool,
                           const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
@@ -894,8 +946,10 @@ __global__ void k_mh_init(const DiodeParams* __restrict__ P, DiodeDyn* __restric
         atomicAdd(&Dy[d].chains_failed, 1);
       }
       cs.ok[k] = ok; cs.F[k] = F; cs.sup[k] = sup;
-      if (p.geometry == RD_G_TIP) { cs.x[k] = xi; cs.y[k] = ph_; cs.tx[k] = X; cs.ty[k] = Y; cs.tz[k] = Z; }
-      else {
+      if (p.geometry == RD_G_TIP) {
+        cs.x[k] = xi; cs.y[k] = ph_; cs.tx[k] = X; cs.ty[k] = Y; cs.tz[k] = Z;
+        if (ok) tip_start(p, cs, k, xi, F);
+      } else {
         cs.x[k] = X; cs.y[k] = Y;
         if (ok) {   // Gaussian pair of the first jump
           if constexpr (PREC == 1) {
@@ -1793,11 +1847,11 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
   constexpr int CPT = PREC == 1 ? RD_TIP_CPT : 1;
   const int nt = blockDim.x;
   const int total = ph->total_items, nd = ph->n_diodes, tid = threadIdx.x;
-  const bool init = it_idx == 0;
+  const bool init = it_idx == 0, fin = it_idx == RD_MH_FINAL;
   for (int g = queue_first(0, total); g < total; g = queue_next(queue, &s_item, 0, total)) {
     ItemRef it = decode_item(plan, nd, g);
     const DiodeParams& p = P[it.d];
-    if (p.geometry != RD_G_TIP || it_idx > p.mh_jumps) continue;
+    if (p.geometry != RD_G_TIP || it_idx > p.mh_jumps || (!init && fin != (bool)p.tn)) continue;
     DiodeDyn& y = Dy[it.d];
     const uint32_t step = (uint32_t)(*step_ptr - y.step_offset);
     const int M = plan[it.d].n_i;
@@ -1808,7 +1862,7 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
     for (int q = 0; q < CPT; ++q) {
       const int c = it.i0 + tid + q * nt;
       kk[q] = ch_off[it.d] + c;
-      ok[q] = (c < M) ? (init ? 1 : cs.ok[kk[q]]) : 0;
+      ok[q] = (c < M) ? (init ? 1 : fin ? cs.ok[kk[q]] && cs.em[kk[q]] : cs.ok[kk[q]]) : 0;
     }
     double f3[CPT][3];
     if constexpr (PREC == 1) {
@@ -1857,13 +1911,11 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
           acce[q][0] += te[q][0]; acce[q][1] += te[q][1]; acce[q][2] += te[q][2];
         }
       }
-      const double K = c_k.tip_K, cd = p.image_charge ? (1.0 + K) * kscale : kscale, ce = K * kscale;
 #pragma unroll
       for (int q = 0; q < CPT; ++q) {
-        const double cq = ce * (double)iih[q].w;
-        f3[q][0] = ((double)accd[q].hx + (double)accd[q].lx) * cd - (double)acce[q][0] * cq;
-        f3[q][1] = ((double)accd[q].hy + (double)accd[q].ly) * cd - (double)acce[q][1] * cq;
-        f3[q][2] = ((double)accd[q].hz + (double)accd[q].lz) * cd - (double)acce[q][2] * cq;
+        f3[q][0] = tip_sum_finish(p, accd[q].hx, accd[q].lx, acce[q][0], iih[q].w, kscale);
+        f3[q][1] = tip_sum_finish(p, accd[q].hy, accd[q].ly, acce[q][1], iih[q].w, kscale);
+        f3[q][2] = tip_sum_finish(p, accd[q].hz, accd[q].lz, acce[q][2], iih[q].w, kscale);
       }
     } else {
       __shared__ rd_d4 sj[RD_TILE];
@@ -1905,26 +1957,23 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
       if (!ok[q]) continue;
       const int c = it.i0 + tid + q * nt, k = kk[q];
       const double X = cs.pxx[k], Y = cs.pyy[k], Z = cs.pzz[k], nxi = cs.px[k], nph = cs.py[k];
+      const double F = tip_normal_field(p, X, Y, Z, f3[q]);   // one expression: the last pass repeats a jump's F
+      if (fin) {   // the field and the point that the emission test reads
+        cs.F[k] = F;
+        cs.tx[k] = X; cs.ty[k] = Y; cs.tz[k] = Z;
+        continue;
+      }
       if (init) {   // a favourable start makes the chain; the others go to k_mh_init
-        double ex, ey, ez, nx, ny, nz;
-        tip_field_E(p, X, Y, Z, &ex, &ey, &ez);
-        ex += f3[q][0]; ey += f3[q][1]; ez += f3[q][2];
-        tip_normal(p, X, Y, &nx, &ny, &nz);
-        const double F = (nx * ex + ny * ey) + nz * ez;
         if (F < 0.0 && p.init_rounds > 0) {
           cs.ok[k] = 1; cs.x[k] = nxi; cs.y[k] = nph; cs.F[k] = F; cs.sup[k] = tip_target_log(p, F, nxi);
           cs.tx[k] = X; cs.ty[k] = Y; cs.tz[k] = Z;
+          tip_start(p, cs, k, nxi, F);
         } else {
           cs.ok[k] = 0;
         }
         continue;
       }
       if (!cs.prop_ok[k]) { r += 1; continue; }
-      double ex, ey, ez, nx, ny, nz;
-      tip_field_E(p, X, Y, Z, &ex, &ey, &ez);
-      ex += f3[q][0]; ey += f3[q][1]; ez += f3[q][2];
-      tip_normal(p, X, Y, &nx, &ny, &nz);
-      const double F = (nx * ex + ny * ey) + nz * ez;
       if (F >= 0.0) { r += 1; continue; }
       const double sn = tip_target_log(p, F, nxi), sc = cs.sup[k];
       bool take = sn >= sc;
@@ -1941,7 +1990,7 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
         r += 1;
       }
     }
-    if (init) continue;
+    if (init || fin) continue;
     mh_counts_and_update(p, y, plan[it.d].tiles, it_idx, ndim_first, a, r, red_i);
   }
   queue_leave(queue, 0, total);
@@ -1952,7 +2001,9 @@ k_mh_jump_tip(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool
 // (Metro_algo_tip_v3, src/mod_emission_tip.f90:1334-1350); the step uses the
 // fixed warm-up size for the first quarter of the jumps and MH_std
 // afterwards (MH_std was updated at the end of the previous iteration).
-// it = 0: round 0 of the uniform start of every chain.  The proposal is also
+// it = 0: round 0 of the uniform start of every chain; RD_MH_FINAL: the chain's
+// point itself.  Diodes whose jumps take the near / far split (rd_tipnear.cuh)
+// come here only for those two.  The proposal is also
 // packed into the FP32 frame here, once, for the field tiles of the jump.
 __global__ void k_mh_propose(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy,
                              const PlanEntry* __restrict__ plan, const PlanHeader* __restrict__ ph,
@@ -1966,7 +2017,8 @@ __global__ void k_mh_propose(const DiodeParams* __restrict__ P, const DiodeDyn* 
     while (lo < hi) { int mid = (lo + hi + 1) >> 1; if (plan[mid].pad0 <= g) lo = mid; else hi = mid - 1; }
     const int d = lo, c = g - plan[d].pad0;
     const DiodeParams& p = P[d];
-    if (p.geometry != RD_G_TIP || it_idx > p.mh_jumps) continue;
+    if (p.geometry != RD_G_TIP || it_idx > p.mh_jumps || (it_idx != 0 && (it_idx == RD_MH_FINAL) != (bool)p.tn)) continue;
+    if (it_idx == 0 && p.tn && c == 0) *p.tn_next = 0;   // no panel's list of this step yet (k_tip_panels)
     const int k = ch_off[d] + c;
     const DiodeDyn& y = Dy[d];
     const uint32_t step = (uint32_t)(*step_ptr - y.step_offset);
@@ -1977,27 +2029,21 @@ __global__ void k_mh_propose(const DiodeParams* __restrict__ P, const DiodeDyn* 
       rng2(p.seed, (uint32_t)c, 0u, step, RNG_INIT, &u1, &u2);
       nxi = 1.0 + (p.max_xi - 1.0) * u1;
       nph = twopi * u2;
-    } else {             // Gaussian step in (xi, phi), xi reflected, phi wrapped (:1337-1365)
+    } else if (it_idx == RD_MH_FINAL) {   // the chain's last point
+      if (!cs.ok[k]) continue;
+      nxi = cs.x[k]; nph = cs.y[k];
+    } else {
       if (!cs.ok[k]) continue;
       const int ndim_first = (int)nint_d(p.mh_jumps * 0.25);
       double g1, g2;
       gauss2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, &g1, &g2);
       const double sxi = (it_idx > ndim_first) ? (p.max_xi - 1.0) * y.MH_std : (p.max_xi - 1.0) * 0.10;
       const double sph = (it_idx > ndim_first) ? twopi * y.MH_std : twopi * 0.10;
-      nxi = cs.x[k] + g1 * sxi;
-      const double a = cs.y[k] + g2 * sph;
-      nph = a - floor(a / twopi) * twopi;   // Fortran MODULO
-      if (nxi > p.max_xi) nxi = 2.0 * p.max_xi - nxi;
-      if (nxi < 1.0) nxi = 2.0 - nxi;
-      inside = !(nxi < 1.0 || nxi > p.max_xi);
+      inside = tip_step(p, cs.x[k], cs.y[k], g1, g2, sxi, sph, &nxi, &nph);
     }
     double X, Y, Z;
-    tip_xyz(p, inside ? nxi : 1.5, p.eta_1, nph, &X, &Y, &Z);
-    if (f32_grid) {   // FP32 form: the point at its FP32 nm coordinates (at most 6e-5 nm off the surface)
-      X = (double)(float)(X * 1.0e9) * 1.0e-9;
-      Y = (double)(float)(Y * 1.0e9) * 1.0e-9;
-      Z = (double)(float)(Z * 1.0e9) * 1.0e-9;
-    }
+    if (f32_grid) tip_grid_xyz(p, inside ? nxi : 1.5, nph, &X, &Y, &Z);
+    else tip_xyz(p, inside ? nxi : 1.5, p.eta_1, nph, &X, &Y, &Z);
     cs.px[k] = nxi; cs.py[k] = nph; cs.prop_ok[k] = inside;
     cs.pxx[k] = X; cs.pyy[k] = Y; cs.pzz[k] = Z;
     float4 ih, il, iih, iil;   // FP32 frame of the proposal, once per jump
@@ -2005,6 +2051,8 @@ __global__ void k_mh_propose(const DiodeParams* __restrict__ P, const DiodeDyn* 
     cs.pph[k] = ih; cs.pih[k] = iih;
   }
 }
+
+#include "rd_tipnear.cuh"
 
 // ---- emission decisions and stable append ----------------------------------------------------
 // One CTA per emitting diode.  Candidates are tested in chain order
@@ -2704,6 +2752,17 @@ cudaError_t rd_launch_mh_jumps_near(int prec, int grid, cudaStream_t st, const D
                                     double kscale, int* gave_up, bool lone) {
   if (prec == 1) return launch_jumps_near<1>(grid, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr, kscale, gave_up, lone);
   return launch_jumps_near<0>(grid, st, P, Dy, pool, plan, ph, plan_mh, cs, ch_off, wtab, step_ptr, jumps, nr, kscale, gave_up, lone);
+}
+
+// Tip diodes (rd_tipnear.cuh): lists and expansions of the panels, then all jumps.
+cudaError_t rd_launch_tip_near(int nslots, int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
+                               const Pool& pool, const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
+                               const ChainState& cs, const int* ch_off, const int* step_ptr, int jumps,
+                               const NearState& nr, double kscale, int* gave_up) {
+  k_tip_panels<<<dim3(std::max(16, RD_TN_PANELS / std::max(nslots, 1)), nslots), 256, 0, st>>>(P, Dy, pool, nr);
+  const int most = rd_grid(k_tip_jumps, 256, 0), g = grid > 0 && grid < most ? grid : most;
+  return launch_coop(k_tip_jumps, 256, g, st, P, (DiodeDyn*)Dy, pool, plan, ph, plan_mh, cs, ch_off, step_ptr, jumps, nr,
+                     kscale, gave_up);
 }
 
 cudaError_t rd_launch_emit(int nslots, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,

@@ -58,6 +58,10 @@ inline int rd_chunk_rule(int clen_min, int nch_max, int target) {
 #define RD_NEAR_W (2 * RD_NEAR_M + 1)   // panels across the near region
 #define RD_NEAR_ROWS (RD_NEAR_M + 1)    // rows of bins (two panels high) that cover it
 #define RD_NEAR_REC 32        // words of a panel record (a multiple of 4)
+#define RD_TN_PANELS 768      // panels of a tip, about (rd_tipnear.cuh)
+#define RD_TN_RINGS 128       // at most this many rings of them
+#define RD_TN_MAP 1024        // entries of the ring map
+#define RD_TN_LIST 48         // list entries per particle slot (an electron is near to about 30 panels)
 #define RD_MAX_WORK 4096      // max checkerboard cells per diode (64x64)
 
 enum { RD_G_PLANAR = 1, RD_G_TIP = 2 };
@@ -116,12 +120,28 @@ struct DiodeParams {
   double nr_hx, nr_hy;   // panel half widths (nm)
   float nr_Ez;           // E_z
   float nr_ax, nr_ay, nr_iax, nr_iay, nr_iwx, nr_iwy;   // panel half widths (nm), 1 / half width, 1 / width
+  // the same for the FP32 tip chains (rd_tipnear.cuh); lengths in nm
+  int tn;                // 1: the diode's jumps take it
+  int tn_np;             // panels
+  long long tn_cap;      // electrons that the panels' lists can hold together
+  const float4* tn_pan;  // panel centres and radii
+  const int2* tn_map;    // first panel and sectors of the ring at sqrt(xi - 1) = entry / tn_vs
+  float2* tn_rec;        // expansions, 64 coefficients per panel
+  float4* tn_hdr;        // their bounds; the panels' lists
+  float4* tn_list;
+  int* tn_next;          // entries of tn_list taken
+  float tn_vs;
+  float tn_nf, tn_c;     // surface normal: eta / sqrt(1 - eta^2) and a^2 (1 - eta^2)
+  float tn_v0;           // vacuum field: pre_E / sqrt(1 - eta^2)
+  float tn_t0, tn_t2;    // log phi, l_const / phi^2
+  float tn_ir, tn_z0;    // 1 / apex radius, height of its centre
+  float tn_e2, tn_ia;    // 1 - eta^2, 1 / a
 };
 
 // Planner modes (k_plan): which i-set of each diode a pair-sum plan covers.
 // Modes up to PM_SUPPLY_LAT and PM_MH_SLOW are pair sums (tiles x j-chunks), the
-// two PM_PART modes per-particle index spaces, PM_MH_NEAR tiles of RD_NEAR_CPB
-// chains.  PM_MH: all batched chains of the tiled kernels (start rounds, last
+// two PM_PART modes per-particle index spaces, PM_MH_NEAR and PM_MH_TIP (tip diodes
+// that take rd_tipnear.cuh) tiles of RD_NEAR_CPB chains.  PM_MH: all batched chains of the tiled kernels (start rounds, last
 // points); their jumps split into PM_MH_NEAR (rd_near.cuh) and PM_MH_SLOW.  PM_SUPPLY_PLANAR: the supply points of
 // planar diodes with image charges (F_z only: the lateral components cancel
 // at the cathode); PM_SUPPLY_LAT: those of planar diodes without (all three
@@ -130,7 +150,7 @@ struct DiodeParams {
 // Calculate_Acceleration_Particles pass, which ignores two_time_step).
 enum { PM_FORCE_PLANAR = 0, PM_FORCE_TIP = 1, PM_FIELD = 2, PM_SUPPLY_PLANAR = 3,
        PM_SUPPLY_TIP = 4, PM_MH = 5, PM_FORCE_TTS = 6, PM_SUPPLY_LAT = 7, PM_PART = 8, PM_PART1024 = 9,
-       PM_MH_SLOW = 10, PM_MH_NEAR = 11, PM_COUNT = 12, PM_ALL_DIODES = 0x100 };
+       PM_MH_SLOW = 10, PM_MH_NEAR = 11, PM_MH_TIP = 12, PM_COUNT = 13, PM_ALL_DIODES = 0x100 };
 
 // Supply quadrature grid of one diode, filled on the device (k_quad_fill):
 // planar, quad_n x quad_n Gauss-Legendre nodes (P panels of Q nodes per side)

@@ -118,6 +118,7 @@ __device__ __forceinline__ int plan_ni(const DiodeParams& p, const DiodeDyn& y, 
     // serial diodes: k_mh_serial; diodes with no particle in flight: k_mh_vacuum
     case PM_MH: return (p.emission && !p.mh_serial && !rd_mh_vacuum(p, y)) ? y.chains : 0;
     case PM_MH_SLOW: return (p.emission && !p.mh_serial && !p.mh_fast && !rd_mh_vacuum(p, y)) ? y.chains : 0;
+    case PM_MH_TIP: return (p.emission && p.tn) ? y.chains : 0;
     case PM_MH_NEAR: return (p.emission && p.mh_fast && !rd_mh_vacuum(p, y)) ? y.chains : 0;
     default: return nj;
   }
@@ -162,7 +163,7 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
   __shared__ int s_chains[32];
   const PlanJob job = jobs.j[blockIdx.x];
   const int mode = job.mode, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
-  const int tsize = (mode == PM_PART1024) ? 1024 : (mode == PM_MH_NEAR) ? RD_NEAR_CPB : RD_ITILE;
+  const int tsize = (mode == PM_PART1024) ? 1024 : (mode == PM_MH_NEAR || mode == PM_MH_TIP) ? RD_NEAR_CPB : RD_ITILE;
   const bool pair = (mode & 0xff) <= PM_SUPPLY_LAT || mode == PM_MH_SLOW;
   const bool supply = (mode & 0xff) == PM_SUPPLY_PLANAR, lat = (mode & 0xff) == PM_SUPPLY_LAT;
   int clen_min = chunk_rule & 0xffff, target = (chunk_rule >> 24) * 64;   // rd_chunk_rule
