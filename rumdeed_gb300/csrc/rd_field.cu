@@ -2710,7 +2710,15 @@ cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const Di
   k_near_count<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
   k_near_scan<<<nslots, 1024, 0, st>>>(P, Dy, nr);
   k_near_scatter<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
-  k_near_panels<<<rd_grid(k_near_panels, 64, grid), 64, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
+  // Only a tile's first item has work: a prime number of blocks, so that no number of
+  // chunks gives those items to a part of the blocks only.
+  int blocks = rd_grid(k_near_panels, 256, grid);
+  auto prime = [](int v) {
+    for (int f = 2; f * f <= v; ++f) if (v % f == 0) return false;
+    return true;
+  };
+  while (!prime(blocks)) --blocks;
+  k_near_panels<<<blocks, 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
   return cudaGetLastError();
 }
 

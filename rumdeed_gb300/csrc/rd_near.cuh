@@ -168,23 +168,35 @@ __device__ const float c_gl4_inv[4][4] = {
     {0.798762056f, -0.798762056f, -0.798762056f, 0.798762056f},
     {-0.927567512f, 2.34943118f, -2.34943118f, 0.927567512f}};
 
+#define RD_NEAR_AWAY 24.0f    // electrons this many half widths from eight panels share their term of T
+
 // Panel records, one warp per panel: the far part's interpolation coefficients
 // (powers of t_x fastest), the panel's centre, T and the largest |S| of its
-// nodes, and where its near electrons are.  The supply plan's tiles of 128 points cover eight panels each.
-__global__ void __launch_bounds__(64)
+// nodes, and where its near electrons are.  A block takes the eight panels of a tile of
+// the supply plan (128 points; the items of its first chunk).  T of every electron and
+// panel, about 50 instructions a pair, was most of the set-up (128 diodes of 256-32768
+// electrons, 230,000 panels: 11.2 ms, half of it on a part of the SMs only): electrons
+// RD_NEAR_AWAY half widths from the eight panels' rectangle now add one term for all of
+// them (at the rectangle's distance T is larger by a per cent or so), the others pass
+// through shared memory once for the eight warps: 2.8 ms.
+__global__ void __launch_bounds__(256)
 k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, const PlanEntry* __restrict__ plan,
               const PlanHeader* __restrict__ ph, const float4* __restrict__ qpp, const double* __restrict__ qF,
               NearState nr, double kscale) {
-  const int total = ph->total_items, nd = ph->n_diodes, lane = threadIdx.x & 31;
+  __shared__ float4 low[512];
+  __shared__ float s_gT[8];
+  __shared__ int s_n;
+  const int total = ph->total_items, nd = ph->n_diodes, tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) s_n = 0;
+  __syncthreads();
   const double inv_A0 = 1.0 / (-2.0 * kscale);
   for (int g = blockIdx.x; g < total; g += gridDim.x) {
     const ItemRef it = decode_item(plan, nd, g);
     const DiodeParams& p = P[it.d];
-    if (!near_live(p, Dy[it.d])) continue;
-    const int NP = p.nr_P;
-    // the item's share of the tile's eight panels, one warp each
-    for (int pan = it.tile * 8 + 8 * it.chunk / it.nch + (threadIdx.x >> 5);
-         pan < min(NP * NP, it.tile * 8 + 8 * (it.chunk + 1) / it.nch); pan += 2) {
+    if (it.chunk != 0 || !near_live(p, Dy[it.d])) continue;
+    const int NP = p.nr_P, own = it.tile * 8 + (tid >> 5);
+    const bool live = own < NP * NP;
+    const int pan = live ? own : 0;   // (a warp without a panel helps to load)
     const int ppy = pan / NP, ppx = pan - ppy * NP, nb = p.nr_bx, r0 = ppy >> 1;
     const int* start = nr.start + p.nr_boff;
     // the node of this lane (lanes l and l + 16 share one and take every other near electron)
@@ -216,11 +228,39 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     // T over the far electrons, as seen from the panel's rectangle
     const float ox = (float)((2 * ppx + 1 - NP) * p.nr_hx), oy = (float)((2 * ppy + 1 - NP) * p.nr_hy);
     const float ax = p.nr_ax, ay = p.nr_ay;
-    float Tx = 0.0f, Ty = 0.0f;
+    float Tx = 0.0f, Ty = 0.0f, gT = 0.0f;
     const int n = Dy[it.d].n;
+    // electrons far from all eight panels (a row of them, or parts of two): one term for
+    // all, at the least distance to their rectangle; the others go to every warp
+    const int g0 = it.tile * 8, g1 = min(g0 + 7, NP * NP - 1), ra = g0 / NP, rb = g1 / NP;
+    const int ca = ra == rb ? g0 - ra * NP : 0, cb = ra == rb ? g1 - rb * NP : NP - 1;
+    const float gx = (float)((ca + cb + 1 - NP) * p.nr_hx), gy = (float)((ra + rb + 1 - NP) * p.nr_hy);
+    const float hx = (float)(cb - ca + 1) * ax * 1.0001f, hy = (float)(rb - ra + 1) * ay * 1.0001f;
+    const float away = RD_NEAR_AWAY * fmaxf(ax, ay), away2 = away * away;
+    int here = 0;   // electrons in low
+    for (int j0 = 0; j0 < n; j0 += 256) {
+      float4 e4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      bool close = false;
+      if (j0 + tid < n) {
+        e4 = nr.low[p.off + j0 + tid];
+        const float bx = fmaxf(fabsf(e4.x - gx) - hx, 0.0f), by = fmaxf(fabsf(e4.y - gy) - hy, 0.0f);
+        const float r2 = fmaf(bx, bx, fmaf(by, by, e4.z * e4.z));
+        close = r2 < away2;
+        if (!close) {
+          const float inv = rsqrtf(r2), i2 = inv * inv;
+          gT = fmaf(e4.z * inv, i2 * i2 * i2, gT);
+        }
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, close);
+      int at = 0;
+      if (lane == 0 && mask) at = atomicAdd(&s_n, __popc(mask));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (close) low[at + __popc(mask & ((1u << lane) - 1))] = e4;
+      here += __syncthreads_count(close);
+      if (here <= 256 && j0 + 256 < n) continue;   // room for another 256 (block-uniform)
 #pragma unroll 4
-    for (int j = lane; j < n; j += 32) {
-      const float4 e = nr.low[p.off + j];
+      for (int q = lane; q < here; q += 32) {
+      const float4 e = low[q];
       const int code = __float_as_int(e.w);
       const bool is_near = code >= 0 && (unsigned)((code & 0xffff) - ppx) < RD_NEAR_W &&
                            (unsigned)((code >> 16) - r0) < RD_NEAR_ROWS;
@@ -232,11 +272,25 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
       // c_x^2 <= 0.68 over the panel: 0.32 x^2 <= 0.68 (y^2 + z^2)
       Tx = fmaf(0.32f * tx * tx <= 0.68f * fmaf(by, by, z2) ? 2.5f : 15.0f, v7, Tx);
       Ty = fmaf(0.32f * ty * ty <= 0.68f * fmaf(bx, bx, z2) ? 2.5f : 15.0f, v7, Ty);
+      }
+      here = 0;
+      __syncthreads();
+      if (tid == 0) s_n = 0;
+      __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1) {
       Tx += __shfl_xor_sync(0xffffffffu, Tx, o);
       Ty += __shfl_xor_sync(0xffffffffu, Ty, o);
+      gT += __shfl_xor_sync(0xffffffffu, gT, o);
     }
+    if (lane == 0) s_gT[tid >> 5] = gT;
+    __syncthreads();
+    gT = 0.0f;
+    for (int q = 0; q < 8; ++q) gT += s_gT[q];
+    __syncthreads();
+    Tx = fmaf(15.0f, gT, Tx);
+    Ty = fmaf(15.0f, gT, Ty);
+    if (!live) continue;   // (at the end of the item's work: no barrier is left)
     float* rec = nr.rec + (size_t)(p.q_off / 16 + pan) * RD_NEAR_REC;
     if (lane < 16) rec[lane] = c;
     // the rows of near electrons end to end: what turns a list index into an electron, and the row's end
@@ -257,7 +311,6 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     }
     if (lane == 0) *reinterpret_cast<float4*>(rec + 16) = make_float4(ox, oy, 1.03f * Tx, big);
     if (lane == 1) rec[28] = 1.03f * Ty;
-    }
   }
 }
 
