@@ -48,8 +48,48 @@ __device__ __forceinline__ void point_pack(const DiodeParams& p, double x, doubl
   }
 }
 
+// Field sums of up to 64 particles of a tile (one image partner or none) at two points:
+// the terms of planar_tile_f32<T_UPPER> with one shared load for both points, the floor
+// inside dxy^2 and one lateral factor for a particle and its image (27 FP32 operations
+// and two reciprocal roots a pair; 31 and twice the loads one point at a time).
+template <bool IC, bool ELEC>
+__device__ __forceinline__ void field_tile2_nic0(const float4* __restrict__ sh, const float4* __restrict__ sl, int kmax,
+                                                 const float4* ih, const float4* il, float (*t)[3]) {
+  float x[2] = {0.f, 0.f}, y[2] = {0.f, 0.f}, z[2] = {0.f, 0.f};
+#pragma unroll 2
+  for (int k = 0; k < kmax; ++k) {
+    const float4 h = sh[k], l = sl[k];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float dx = (ih[q].x - h.x) + (il[q].x - l.x), dy = (ih[q].y - h.y) + (il[q].y - l.y);
+      const float dz = (ih[q].z - h.z) + (il[q].z - l.z);
+      const float dxy2 = fmaf(dx, dx, fmaf(dy, dy, 1e-20f));
+      const float inv = rsqrtf(fmaf(dz, dz, dxy2)), c = (inv * inv) * inv, s = ELEC ? c : h.w * c;
+      if (IC) {
+        const float zs = (ih[q].z + h.z) + (il[q].z + l.z);
+        const float ri = rsqrtf(fmaf(zs, zs, dxy2)), ci = (ri * ri) * ri, si = ELEC ? ci : h.w * ci;
+        const float d = s - si;
+        x[q] = fmaf(d, dx, x[q]); y[q] = fmaf(d, dy, y[q]);
+        z[q] = fmaf(s, dz, fmaf(-si, zs, z[q]));
+      } else {
+        x[q] = fmaf(s, dx, x[q]); y[q] = fmaf(s, dy, y[q]); z[q] = fmaf(s, dz, z[q]);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    t[q][0] = ELEC ? -x[q] : x[q]; t[q][1] = ELEC ? -y[q] : y[q]; t[q][2] = ELEC ? -z[q] : z[q];
+  }
+}
+
+// E at points, one tile of 128 points by a chunk of particles per item.  FP32 planar
+// diodes with at most one image partner take two points per thread and half of a tile's
+// particles, eight blocks per SM (64 registers; with 80 the waves of short items cost
+// more than the spills: 4096 points and 20,000 particles 134 us against 120).  Bound by
+// issue: 31 instructions a pair (35 with one point per thread).  4096 points, 65,536
+// particles: 376 -> 353 us with RD_FIELD_NCH, 338 so; 64 points 137 -> 65 us.
 template <int PREC, int GEOM>
-__global__ void __launch_bounds__(RD_ITILE)
+__global__ void __launch_bounds__(RD_ITILE, PREC == 1 && GEOM == RD_G_PLANAR ? 8 : 0)
 k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __restrict__ plan,
                const PlanHeader* __restrict__ ph, PointSet pts, double* __restrict__ partial,
                int* __restrict__ tickets, double kscale) {
@@ -65,7 +105,56 @@ k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __
     double X = valid ? pts.x[po + i] : 0.0, Y = valid ? pts.y[po + i] : 0.0;
     double Z = valid ? pts.z[po + i] : 0.5 * p.d;
     double fx, fy, fz;
-    if (PREC == 1) {
+    bool nic0 = false;
+    if constexpr (PREC == 1 && GEOM == RD_G_PLANAR) nic0 = p.N_ic_max == 0;
+    if (PREC == 1 && nic0) {   // two points per thread, half of a tile's particles each
+      __shared__ float4 sp[2][RD_ITILE];
+      __shared__ double sf[3][RD_ITILE];
+      const int half = tid >> 6, a0 = tid & 63;
+      {
+        float4 iih, iil;
+        __syncthreads();
+        point_pack(p, X, Y, Z, sp[0][tid], sp[1][tid], iih, iil);
+        __syncthreads();
+      }
+      const float4 ih[2] = {sp[0][a0], sp[0][64 + a0]}, il[2] = {sp[1][a0], sp[1][64 + a0]};
+      F32Acc acc[2];
+      acc[0].zero(); acc[1].zero();
+      for (int jt = it.j0; jt < it.j1; jt += RD_TILE) {
+        __syncthreads();
+        int elec = 1;   // every charge of the tile is an electron's
+        if (jt + tid < it.j1) {
+          const float4 hj = pool.pk_hi[off + jt + tid];
+          sh[tid] = hj; sl[tid] = pool.pk_lo[off + jt + tid];
+          elec = (hj.w == -1.0f);
+        }
+        elec = __syncthreads_and(elec);
+        const int kmax = min(RD_TILE, it.j1 - jt), mid = (kmax + 1) >> 1, k0 = half ? mid : 0, m2 = half ? kmax - mid : mid;
+        float t[2][3];
+        if (p.image_charge) {
+          if (elec) field_tile2_nic0<true, true>(sh + k0, sl + k0, m2, ih, il, t);
+          else field_tile2_nic0<true, false>(sh + k0, sl + k0, m2, ih, il, t);
+        } else {
+          if (elec) field_tile2_nic0<false, true>(sh + k0, sl + k0, m2, ih, il, t);
+          else field_tile2_nic0<false, false>(sh + k0, sl + k0, m2, ih, il, t);
+        }
+        acc[0].add(t[0][0], t[0][1], t[0][2]);
+        acc[1].add(t[1][0], t[1][1], t[1][2]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {   // the first half's sums, then the second's on top
+        if (half == h)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int k = a0 + 64 * q;
+            const double x = (double)acc[q].hx + (double)acc[q].lx, y = (double)acc[q].hy + (double)acc[q].ly,
+                         z = (double)acc[q].hz + (double)acc[q].lz;
+            sf[0][k] = h ? sf[0][k] + x : x; sf[1][k] = h ? sf[1][k] + y : y; sf[2][k] = h ? sf[2][k] + z : z;
+          }
+        __syncthreads();
+      }
+      fx = sf[0][tid] * kscale; fy = sf[1][tid] * kscale; fz = sf[2][tid] * kscale;
+    } else if (PREC == 1) {
       float4 ih, il, iih, iil;
       point_pack(p, X, Y, Z, ih, il, iih, iil);
       const float dnm = (float)(p.d * 1.0e9);
@@ -91,9 +180,6 @@ k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __
           if (elec) tip_tile_split_f32<T_UPPER, true>(sh, sl, sih, kmax, ih, il, iih, -1, p.image_charge, ts);
           else tip_tile_split_f32<T_UPPER>(sh, sl, sih, kmax, ih, il, iih, -1, p.image_charge, ts);
           tx = ts.dx; ty = ts.dy; tz = ts.dz;
-        } else if (p.N_ic_max == 0) {
-          if (elec) planar_tile_f32<T_UPPER, true, true>(sh, sl, kmax, ih, il, -1, 0, dnm, p.image_charge, tx, ty, tz);
-          else planar_tile_f32<T_UPPER, true>(sh, sl, kmax, ih, il, -1, 0, dnm, p.image_charge, tx, ty, tz);
         } else {
           if (elec) planar_tile_f32<T_UPPER, false, true>(sh, sl, kmax, ih, il, -1, p.N_ic_max, dnm, p.image_charge, tx, ty, tz);
           else planar_tile_f32<T_UPPER, false>(sh, sl, kmax, ih, il, -1, p.N_ic_max, dnm, p.image_charge, tx, ty, tz);
@@ -127,6 +213,7 @@ k_field_points(const DiodeParams* __restrict__ P, Pool pool, const PlanEntry* __
       pp[tid] = fx; pp[RD_ITILE + tid] = fy; pp[2 * RD_ITILE + tid] = fz;
       if (!tile_ticket(tickets, it)) continue;
       fx = fy = fz = 0.0;
+#pragma unroll 8
       for (int c = 0; c < it.nch; ++c) {
         const double* q = partial + (size_t)(it.base + c) * 3 * RD_ITILE;
         fx += __ldcg(q + tid); fy += __ldcg(q + RD_ITILE + tid); fz += __ldcg(q + 2 * RD_ITILE + tid);

@@ -171,6 +171,7 @@ k_plan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, int n
   // the supply points are many tiles already: few chunks per tile.  k_z0_points keeps one
   // sum per point, a third of an item's scratch: three times the items fit.
   if (lat) nch_max = min(nch_max, RD_SUP_NCH);
+  if (mode == PM_FIELD && target > 0) nch_max *= RD_FIELD_NCH;
   if (supply) {
     nch_max = min(nch_max, 3 * RD_SUP_NCH);
     target *= 4;   // its items are single warps
