@@ -2369,6 +2369,56 @@ __device__ __forceinline__ bool above(double x, double y) {
   return (a ^ ((a >> 63) & 0x7fffffffffffffffll)) > (b ^ ((b >> 63) & 0x7fffffffffffffffll));
 }
 
+// A coordinate's jump from c, reflected once at the emitter's edges a and b.
+__device__ __forceinline__ double serial_jump(double g, double step, double c, double a, double b) {
+  double w = g * step + c;
+  if (above(w, b)) w = b - (w - b); else if (above(a, w)) w = (a - w) + a;
+  return w;
+}
+
+// serial_field_sum<1> at three points: lanes 0, 8 and 16 of warp 0 get their sums.
+__device__ __forceinline__ void serial_field_sum3(const DiodeParams& p, const Pool& pool, int n, const float4* pp3,
+                                                  float2 (*red)[8], float* sh, float* sl) {
+  const int tid = threadIdx.x, lane = tid & 31, off = p.off;
+  const int nic = p.image_charge ? p.N_ic_max : 0;
+  const float dnm = (float)(p.d * 1.0e9);
+  const float4 pp[3] = {pp3[0], pp3[1], pp3[2]};
+  float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
+  for (int j0 = tid; j0 < n; j0 += 256 * 4) {
+    float4 h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = min(j0 + 256 * q, n - 1);
+      h[q] = pool.zk_hi[off + j];
+      l[q] = pool.zk_lo[off + j];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j0 + 256 * q < n)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          two_sum_acc(hi[k], lo[k], nic == 0 ? z0_tile_f32<true>(&h[q], &l[q], 1, pp[k], 0, dnm)
+                                             : z0_tile_f32<false>(&h[q], &l[q], 1, pp[k], nic, dnm));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      pair_add(hi[k], lo[k], __shfl_down_sync(0xffffffffu, hi[k], o), __shfl_down_sync(0xffffffffu, lo[k], o));
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) red[k][tid >> 5] = make_float2(hi[k], lo[k]);
+  __syncthreads();
+  if (tid < 32) {
+    const float2 v = red[min(lane >> 3, 2)][lane & 7];
+    *sh = v.x;
+    *sl = v.y;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+      pair_add(*sh, *sl, __shfl_down_sync(0xffffffffu, *sh, o, 8), __shfl_down_sync(0xffffffffu, *sl, o, 8));
+  }
+}
+
 // The accept / reject decision of a serial chain: s_n >= s_c or log u <= s_n - s_c
 // with the FP64 targets, as mh_decide_f takes it for the batched FP32 chains: FP32
 // estimates decide outside mh_guard, the FP64 targets inside.
@@ -2413,11 +2463,15 @@ __device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* 
 // point through shared memory.  What does not depend on the chain's state is not on
 // its path: the block draws the Gaussian pairs and the accept tests' log u of up to
 // RD_SER_DRAWS jumps at once, and the FP64 targets are formed only where FP32
-// estimates leave a decision open.  33 chains of 100 jumps over 400 electrons:
-// 25.9 -> 6.7 ms (7.8 -> 2.0 us a jump).
+// estimates leave a decision open.  The FP32 chains go two jumps at a time: a jump's
+// proposal is known up to the last jump's answer, so lanes 0 to 2 of warp 0 take jump i
+// and jump i + 1 from either point, the block sums the field at all three, and one
+// comparison each answers both.  33 chains of 100 jumps over 400 electrons: 25.9 ->
+// 6.7 ms one at a time, 5.1 ms so (7.8 -> 2.0 -> 1.6 us a jump); over 4000 electrons 9.3
+// -> 6.9 ms (30 chains).
 #define RD_SER_DRAWS 256
 template <int PREC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 1)
 k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool,
             const double* __restrict__ work, const double* __restrict__ wtab,
             const int* __restrict__ step_ptr, double kscale, EventLog ev) {
@@ -2429,6 +2483,8 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
   // barrier that every reader of its last value has passed)
   __shared__ double s_pt[2][2];   // the point whose field the block sums next
   __shared__ float4 s_pp[2];      // the same in the FP32 frame
+  __shared__ float4 s_pp3[2][3];  // two jumps at once: their three possible points, by parity of the pair
+  __shared__ float2 red_f3[3][8];
   __shared__ int s_sum[2];        // the block sums a field this jump (a ring proposal off the ring: no)
   __shared__ int s_found, s_add, s_stop;   // the chain started; a particle was added; the chains stop
   __shared__ DiodeParams sp;   // thread 0's loads of it are on the jumps' path
@@ -2535,6 +2591,71 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         }
         __syncthreads();
       }
+      if constexpr (PREC == 1) {
+        if (est && i < ndim && draw + 1 < RD_SER_DRAWS) {   // jumps i and i + 1 (block-uniform)
+          const int par = (i >> 1) & 1;
+          double x = 0.0, y2 = 0.0, wx0 = 0.0, wy0 = 0.0;
+          if (threadIdx.x < 32) {   // lane 0: jump i; 1, 2: jump i + 1 from its point, from the chain's
+            const int lane = threadIdx.x;
+            cx = __shfl_sync(0xffffffffu, cx, 0); cy = __shfl_sync(0xffffffffu, cy, 0);
+            sx = __shfl_sync(0xffffffffu, sx, 0); sy = __shfl_sync(0xffffffffu, sy, 0);
+            sx1 = __shfl_sync(0xffffffffu, sx1, 0); sy1 = __shfl_sync(0xffffffffu, sy1, 0);
+            if (i == ndim_first + 1) { sx = sx1; sy = sy1; }
+            wx0 = serial_jump(s_g[draw][0], sx, cx, p.em_x0, hx);
+            wy0 = serial_jump(s_g[draw][1], sy, cy, p.em_y0, hy);
+            if (i == ndim_first) { sx = sx1; sy = sy1; }   // of jump i + 1
+            x = serial_jump(s_g[draw + 1][0], sx, lane == 1 ? wx0 : cx, p.em_x0, hx);
+            y2 = serial_jump(s_g[draw + 1][1], sy, lane == 1 ? wy0 : cy, p.em_y0, hy);
+            if (lane == 0) { x = wx0; y2 = wy0; }
+            if (lane < 3) s_pp3[par][lane] = z0_point(p, x, y2);
+          }
+          __syncthreads();
+          float h = 0.0f, l = 0.0f;
+          serial_field_sum3(p, pool, n, s_pp3[par], red_f3, &h, &l);
+          if (threadIdx.x < 32) {
+            const int lane = threadIdx.x, src = 8 * min(lane, 2);
+            h = __shfl_sync(0xffffffffu, h, src);
+            l = __shfl_sync(0xffffffffu, l, src);
+            float te = t0e, ue = t2e;
+            if (!one_cell && lane < 3) {
+              const double* e = wtab + 3 * (p.work_off + work_cell(p, x, y2));
+              te = (float)e[0]; ue = (float)e[2];
+            }
+            const float S = h + l, Fn = fmaf(A0, S, Ezf), dF = 2.4e-7f * (fabsf(Ezf) + fabsf(A0 * S));
+            const float rn = rho_entry_f(p, te, ue, Fn);
+            Fc = __shfl_sync(0xffffffffu, Fc, 0); fe = __shfl_sync(0xffffffffu, fe, 0);
+            rc = __shfl_sync(0xffffffffu, rc, 0);
+            const float F0 = __shfl_sync(0xffffffffu, Fn, 0), d0 = __shfl_sync(0xffffffffu, dF, 0);
+            const float r0 = __shfl_sync(0xffffffffu, rn, 0);
+            float again;
+            const int take = near_decide(p, Fn, dF, lane == 1 ? F0 : Fc, lane == 1 ? d0 : fe, lane == 1 ? r0 : rc, te, ue,
+                                         s_luf[draw + (lane > 0)], &again);
+            // a jump's answer, from the FP64 targets where the estimates leave it open
+            auto settle = [&](int from, int j) {
+              int tk = __shfl_sync(0xffffffffu, take, from);
+              const double wx = __shfl_sync(0xffffffffu, x, from), wy = __shfl_sync(0xffffffffu, y2, from);
+              const float wh = __shfl_sync(0xffffffffu, h, from), wl = __shfl_sync(0xffffffffu, l, from);
+              const float wF = __shfl_sync(0xffffffffu, Fn, from), wd = __shfl_sync(0xffffffffu, dF, from);
+              const float wr = __shfl_sync(0xffffffffu, rn, from);
+              if (tk < 0) {
+                if (t0) {
+                  const SerialSum sum = {wh, wl, 0.0};
+                  const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
+                  const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+                  tk = Fw < 0.0 && serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
+                }
+                tk = __shfl_sync(0xffffffffu, tk, 0);
+              }
+              if (tk) { cx = wx; cy = wy; cur.h = wh; cur.l = wl; Fc = wF; fe = wd; rc = wr; }
+              if (i + j > ndim_first) { if (tk) ++ja; else ++jr; }
+              return tk;
+            };
+            settle(settle(0, 0) ? 1 : 2, 1);
+          }
+          ++i;
+          continue;
+        }
+      }
       if (t0) {
         if (i == ndim_first + 1) { sx = sx1; sy = sy1; }
         const double g1 = s_g[draw][0], g2 = s_g[draw][1];
@@ -2551,10 +2672,8 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
             wy = nr * sin(na);
           }
         } else {
-          wx = g1 * sx + cx;
-          wy = g2 * sy + cy;
-          if (above(wx, hx)) wx = hx - (wx - hx); else if (above(p.em_x0, wx)) wx = (p.em_x0 - wx) + p.em_x0;
-          if (above(wy, hy)) wy = hy - (wy - hy); else if (above(p.em_y0, wy)) wy = (p.em_y0 - wy) + p.em_y0;
+          wx = serial_jump(g1, sx, cx, p.em_x0, hx);
+          wy = serial_jump(g2, sy, cy, p.em_y0, hy);
         }
         s_pt[i & 1][0] = wx; s_pt[i & 1][1] = wy;
         if (PREC == 1) s_pp[i & 1] = z0_point(p, wx, wy);
