@@ -302,12 +302,6 @@ def reduce_ranks(world, maxes, sums):
     return [float(x) for x in mx] + [float(x) for x in sm]
 
 
-# DRAM bytes (read + write) of one planar MH jump, both halves of the plan, on the 128
-# resident requests of the stream: the mean of jumps 2 and 3 of a one-pass ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum), profiles/k_mh_jump_planar_serve128.md.
-MH_JUMP_DRAM_BYTES = 35.05e6
-
-
 # Serving-iteration time of the 128-slot mix, used only to pace the stream's
 # arrivals in the admission schedule below.
 STEP_S_EST = 0.245
@@ -464,21 +458,18 @@ def run_ours(args, rank, world):
     e2e = e2e_all / e2e_wall if e2e_wall > 0 else 0.0
     if rank != 0:
         return
-    # dominant kernel roofline (FP32 pipe; 20 flops per Coulomb-like term).  The unit is one
-    # MH jump: the mh_parts concurrent launches of k_mh_jump_planar<1> (one per part of the
-    # plan, on their own streams), timed together by CUDA events that bracket the fork and
-    # the join.
+    # roofline of the largest kernel (FP32 pipe; 20 flops per Coulomb-like term): the supply
+    # integral's pair sum, the CUDA-event time of the whole phase charged to it.  The jumps no
+    # longer evaluate every (chain, electron) pair (rd_near.cuh), so their pair count over
+    # their time is a rate of jumps, not of arithmetic.
     jumps = max(prof["mh_jump_launches"], 1)
-    avg_ms = prof["mh_jumps_ms"] / jumps
-    flops_per_jump = 20.0 * prof["mh_pair_evals"] / jumps
-    achieved = flops_per_jump / (avg_ms / 1e3) / 1e12 if avg_ms > 0 else 0.0
+    sup_s = prof["supply_ms"] / 1e3
+    achieved = 20.0 * prof["supply_pair_evals"] / sup_s / 1e12 if sup_s > 0 else 0.0
     peak = measure_fp32_peak()
     peak_src = "measured: cuBLAS SGEMM 8192^3, TF32 off"
     if peak is None:
         peak = 152 * 128 * 2 * 2.07e9 / 1e12
         peak_src = "nominal: 152 SMs x 128 lanes x 2 x 2.07 GHz"
-    # the ncu figure was taken on the 128-slot resident set; other mixes report none
-    traffic = MH_JUMP_DRAM_BYTES if args.slots == 128 else None
     plain_v, plain_caps, plain_n = plain_fp64_all(rg, resident, budget_s=args.plain_budget)
     cpu_v, cpu_desc, cores, cpu_t = cpu_sample(resident, rank=rank)
     line = {
@@ -525,22 +516,21 @@ def run_ours(args, rank, world):
                                            "covered": "%d of the %d resident requests" % (len(plain_caps), plain_n),
                                            "served_over_plain": value / plain_v if plain_v else None},
         "gpu_launches": 2 * args.steps * (kps + 1) + 3 * (admitted + len(burst)),
-        "roofline": {"bound": "fp32", "kernel": "k_mh_jump_planar<1>",
+        "roofline": {"bound": "fp32", "kernel": "k_z0_points<1>",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                     "frac": achieved / peak if peak else None, "traffic": traffic,
+                     "frac": achieved / peak if peak else None, "traffic": None,
                      "peak_source": peak_src,
-                     "unit_of_work": "one MH jump of every chain: the %d concurrent launches "
-                                     "(parts of the plan) of k_mh_jump_planar<1>" % tune["mh_parts"],
-                     "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the "
-                                        "launches of a jump on the burst case (the same 128 resident "
-                                        "requests)" if traffic else "not captured for this mix"),
+                     "unit_of_work": "the supply integral of every resident diode (one step)",
+                     "traffic_source": "not captured for this mix",
                      "flops_convention": "20 flops per Coulomb-like term (Nyland et al.); "
-                                         "1 term per (chain, particle) at the cathode"},
+                                         "1 term per (supply point, particle) at the cathode"},
+        "mh_jump": {"ms": prof["mh_jumps_ms"] / jumps,
+                    "pairs_per_jump": prof["mh_pair_evals"] / jumps,
+                    "note": "pairs a jump stands for; near / far split, most of them in panel expansions"},
         "phase_ms": {k: prof[k] for k in ("supply_ms", "mh_init_ms", "mh_jumps_ms", "emit_ms",
                                           "position_ms", "force_ms", "velocity_ms", "compact_ms",
                                           "total_ms")},
-        "supply_TFLOPs": (20.0 * prof["supply_pair_evals"] / (prof["supply_ms"] / 1e3) / 1e12
-                          if prof["supply_ms"] > 0 else None),
+        "supply_TFLOPs": achieved if sup_s > 0 else None,
         "cpu_baseline": {"value": cpu_v, "unit": METRIC, "cores": cores, "kind": "port",
                          "sample": cpu_desc, "seconds": cpu_t},
         "clocks": clk,

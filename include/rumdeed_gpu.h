@@ -52,7 +52,8 @@ typedef struct {
   long long chain_capacity;     /* MH chain pool size (sum of per-diode chain caps) */
   long long quad_capacity;      /* supply quadrature points over all diodes */
   int chunk_min;                /* j-chunk length floor of the pair sums, particles, a
-                                   multiple of 128 (0 = 1024); see rd_autotune */
+                                   multiple of 128 (0 = 1024, shorter for small systems); see
+                                   rd_autotune */
   int grid_blocks;              /* persistent grid size (0 = per kernel: resident blocks per
                                    SM at its occupancy x SM count) */
   int chunk_count_max;          /* at most this many j-chunks per i-tile, 1..32 (0 = 32) */
@@ -197,7 +198,9 @@ int rd_mark_remove(rd_engine* e, int diode, int index, int why);
  * number of polls, until the earlier tiles it overwrites have read their
  * particles.  Those waits always end in a working run; if one ever gave up,
  * rd_remove_particles, rd_run, rd_serve, rd_profile_step and rd_time_remove
- * return RD_ERR_STATE, and the particle state is no longer valid. */
+ * return RD_ERR_STATE, and the particle state is no longer valid.  The same holds for
+ * the Metropolis-Hastings jumps, whose blocks wait (bounded) for one another's
+ * acceptance counts: rd_do_emission and the calls above return RD_ERR_STATE. */
 int rd_do_emission(rd_engine* e, int step);
 int rd_update_position(rd_engine* e, int step);
 int rd_remove_particles(rd_engine* e, int step);
@@ -333,7 +336,10 @@ int rd_events_take(rd_engine* e, int cap, rd_event* out, int* n_out, long long* 
  * chain's current point, nothing written) weighted by the jump count --
  * keeps the fastest, then times the MH launch shapes (rd_set_mh_launch) under
  * it, rebuilds the step graph and leaves the particle state as it was.
- * rd_set_chunking sets one directly (0 = default).  The i-tile width (128
+ * rd_set_chunking sets one directly; 0, 0 brings the default back: 1024 and 32,
+ * but shorter chunks (down to 128) for a diode whose tiles alone would not fill
+ * the GPU, and up to 96 of them per tile of a field evaluation.  The jumps of
+ * most planar and tip diodes do not depend on it (near / far split).  The i-tile width (128
  * particles, points or chains per work item) is fixed. */
 typedef struct {
   int chunk_min, chunk_count_max;   /* the chosen chunking */
@@ -344,7 +350,9 @@ typedef struct {
 int rd_autotune(rd_engine* e, rd_tune_result* out);
 int rd_set_chunking(rd_engine* e, int chunk_min, int chunk_count_max);
 int rd_get_chunking(rd_engine* e, int* chunk_min, int* chunk_count_max);
-/* Launch shape of the planar MH jumps, which changes no result: `parts`
+/* Launch shape of the planar MH jumps that take pair sums (diodes with a longer
+ * image series, without image charges, or that have held ions or atoms), which
+ * changes no result: `parts`
  * launches per jump on as many streams, each over a part of the work plan cut
  * at diode boundaries (1..4; 0 = 2, used only when two or more diodes run
  * batched chains), and the FP32 thread form (0: 32 threads x 4 chains per

@@ -375,7 +375,7 @@ static cudaError_t alloc_near(rd_engine* e, long long cap, long long qcap, int S
   const size_t low = part(sizeof(float4) * cap), hi = part(sizeof(float4) * cap), lo = part(sizeof(float2) * cap),
                rank = part(sizeof(int) * cap), cnt = part(sizeof(int) * near_bins(qcap)),
                start = part(sizeof(int) * near_bins(qcap)), count = part(sizeof(unsigned long long) * S),
-               progress = part(sizeof(unsigned long long) * S),
+               progress = part(sizeof(unsigned long long) * S), ring = part(sizeof(unsigned long long) * 4 * S),
                rec = part(sizeof(float) * RD_NEAR_REC * ((size_t)qcap / 16 + 1));
   unsigned char* base = nullptr;
   const cudaError_t ce = e->dalloc(&base, at);
@@ -385,6 +385,7 @@ static cudaError_t alloc_near(rd_engine* e, long long cap, long long qcap, int S
   n.rank = (int*)(base + rank); n.cnt = (int*)(base + cnt); n.start = (int*)(base + start);
   n.count = (unsigned long long*)(base + count); n.progress = (unsigned long long*)(base + progress);
   n.rec = (float*)(base + rec);
+  n.ring = (unsigned long long*)(base + ring);
   return cudaSuccess;
 }
 

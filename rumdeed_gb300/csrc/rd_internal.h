@@ -115,7 +115,7 @@ struct DiodeParams {
   double planes_z[10];
   int tts;               // two-time-step interval T (atom_time_interval); 0 off
   double ramo_uz;        // -1 / d: z of the planar unit field E_zunit_planar
-  // near / far split of the FP32 chains' field (rd_near.cuh)
+  // near / far split of the planar chains' field (rd_near.cuh)
   int mh_fast;           // 1: the diode's jumps take it
   int nr_P;              // panels per side of the supply rule
   int nr_boff;           // first bin of this diode
@@ -278,6 +278,7 @@ struct NearState {
   float* rec;
   unsigned long long *count, *progress;   // per slot: tiles done, accepted, rejected of a jump; jumps
                                           // done and step size (near_counts)
+  unsigned long long* ring;               // a lone diode's counts, four jumps per slot (near_wait_counts)
 };
 
 // Where k_rows_out puts a diode's particles in the host buffer (byte offsets; -1: not

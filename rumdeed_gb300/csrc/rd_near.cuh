@@ -37,10 +37,10 @@
 // ions or atoms keep the pair-sum kernel).  nr_guard has the multiples.
 //
 // Measured (GB300, jumps of one step, the split's set-up and last pass included):
-//   one diode, 4500 electrons, 3800 chains, 100 jumps      6.13 -> 0.79 ms
-//   24 diodes of 256-4096 electrons, 30,000 chains, 200    15.9 -> 2.3 ms
-//   128 diodes of 256-32768 electrons, 353,000 chains, 200  276 -> 26.4 ms
-//   FP64: 1300 electrons, 960 chains, 100                   8.4 -> 1.0 ms
+//   one diode, 4500 electrons, 3800 chains, 100 jumps      6.13 -> 0.67 ms
+//   24 diodes of 256-4096 electrons, 30,000 chains, 200    15.9 -> 1.9 ms
+//   128 diodes of 256-32768 electrons, 353,000 chains, 200  276 -> 22.3 ms
+//   FP64: 1300 electrons, 960 chains, 100                   8.4 -> 0.85 ms
 // Open after the estimate: one jump in 10^5; the estimate lay within 0.08 of its
 // bound in every jump checked.  What is left is latency (one near list, one far
 // record, three logarithms and one counter per jump), not arithmetic.
@@ -133,6 +133,7 @@ k_near_scan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, 
   }
   if (tid == 1023) start[bins] = at;   // the last thread's range ends at the last bin
   if (tid == 0) nr.progress[d] = near_progress(p, 0, Dy[d].MH_std);   // no jump of this step done
+  if (tid < 4) nr.ring[4 * d + tid] = 0;
 }
 
 // The near electrons in bin order: (x_hi, y_hi, z^2, q z) and (x_lo, y_lo).
@@ -652,6 +653,23 @@ __device__ __forceinline__ void near_counts(const DiodeParams& p, DiodeDyn& y, u
   *reinterpret_cast<volatile unsigned long long*>(progress) = next;
 }
 
+// A lone diode's form of near_counts without a second hop: jump it's tiles add to ring
+// word it & 3, every block reads the words itself and forms the same step size from
+// them.  A word is cleared two jumps before its next use by the block of the diode's
+// first tile, which then knows that every block has read it (all of them have counted
+// in the jump after).  Returns false if the wait gave up.  Without the fence and the
+// second word a jump of 121 blocks takes 0.1 us less (FP32, 4.5 us) and 1.6 us less
+// (FP64, whose step size was read from memory, 8.7 us); 1.6 us from the last block's
+// count to the last block's start are left.
+__device__ __forceinline__ bool near_wait_counts(const unsigned long long* word, int tiles, int* A, int* R) {
+  const volatile unsigned long long* v = word;
+  unsigned long long now = *v;
+  for (int spins = 0; (int)(now >> 44) != tiles && spins < RD_NEAR_SPIN; ++spins) now = *v;
+  *A = (int)(now >> 22) & 0x3fffff;
+  *R = (int)now & 0x3fffff;
+  return (int)(now >> 44) == tiles;
+}
+
 // Every jump of every chain of the diodes with the near / far split, in one
 // cooperative launch.  A block of NW warps takes 32 chains at a time (an item of the
 // PM_MH_NEAR plan) through a jump: warp 0 proposes and evaluates the far part, one
@@ -721,6 +739,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
   // the chains of the block's item (ONE; warp 0)
   Real fx = 0, fy = 0, gx = 0, gy = 0;
   float Fc = 0.0f, rc = 0.0f, fe = 0.0f;
+  double std_ = 0.0;   // (ONE) the step size
   int ok = 0, d = 0;
   for (int it = 1; it <= jumps; ++it) {
     for (int g = blockIdx.x; g < total; g += gridDim.x) {
@@ -759,15 +778,30 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           }
         }
         // the step size: fixed during the warm-up jumps, then MH_std after the last jump
-        if (lane == 0) {
-          const volatile unsigned long long* prog = nr.progress + d;
-          pr = *prog;
-          for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1 && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
-          if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
+        if (ONE) {
+          if (lane == 0) {
+            if (it == 1) {
+              std_ = __ldcg(&y.MH_std);
+            } else {
+              int A, R;
+              if (!near_wait_counts(nr.ring + 4 * d + ((it - 1) & 3), plan[d].tiles, &A, &R)) sh.dead = 1;
+              double rate;
+              if (it - 1 > ndim_first && A + R > 0 && (std_ != p.mh_hi || 20ll * A <= 7ll * (A + R)))
+                std_ = mh_std_clamp(p, std_ * mh_std_gain(A, R, &rate));
+            }
+          }
+          std_ = __shfl_sync(0xffffffffu, std_, 0);
+        } else {
+          if (lane == 0) {
+            const volatile unsigned long long* prog = nr.progress + d;
+            pr = *prog;
+            for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1 && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
+            if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
+          }
+          pr = __shfl_sync(0xffffffffu, pr, 0);
         }
-        pr = __shfl_sync(0xffffffffu, pr, 0);
         if constexpr (PREC == 1) {   // mh_propose_f32
-          const float mhs = __uint_as_float((unsigned)(pr >> 32));
+          const float mhs = ONE ? (float)std_ : __uint_as_float((unsigned)(pr >> 32));
           const float sx = (it > ndim_first) ? p.em_wx * mhs : p.em_wx * 0.10f;
           const float sy = (it > ndim_first) ? p.em_wy * mhs : p.em_wy * 0.10f;
           if (ok) {
@@ -779,8 +813,8 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           }
           ox = px; oy = py;
         } else {                     // mh_propose_f64
-          __threadfence();           // MH_std was written before the progress word
-          const double mhs = __ldcg(&y.MH_std);
+          if (!ONE) __threadfence();   // MH_std was written before the progress word
+          const double mhs = ONE ? std_ : __ldcg(&y.MH_std);
           const double sx = (it > ndim_first) ? p.em_Lx * mhs : p.em_Lx * 0.10;
           const double sy = (it > ndim_first) ? p.em_Ly * mhs : p.em_Ly * 0.10;
           ox = p.em_x0; oy = p.em_y0;
@@ -816,6 +850,10 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
       if (sh.dead) {   // block-uniform
         if (tid == 0) atomicAdd(gave_up, 1);
         return;
+      }
+      if (ONE && tid == NT - 32 && g == plan[d].item_off) {   // the word of jump it + 2 (a barrier before this jump's count)
+        __stcg(nr.ring + 4 * d + ((it + 2) & 3), 0ull);
+        __threadfence();
       }
       // near electrons
       for (int r8 = 0; r8 < ROUNDS; ++r8) {
@@ -894,8 +932,17 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
       }
       if (w == 0) {
         const int acc = __popc(__ballot_sync(0xffffffffu, a)), rej = __popc(__ballot_sync(0xffffffffu, ok && !a));
-        if (lane == 0)
+        if (lane == 0 && !ONE)
           near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, ndim_first, acc, rej);
+        if (lane == 0 && ONE) {
+          atomicAdd(nr.ring + 4 * d + (it & 3), (1ull << 44) | ((unsigned long long)acc << 22) | (unsigned long long)rej);
+          if (it == p.mh_jumps && g == plan[d].item_off) {   // the step's last counts
+            int A, R;
+            if (!near_wait_counts(nr.ring + 4 * d + (it & 3), plan[d].tiles, &A, &R)) atomicAdd(gave_up, 1);
+            else if (it > ndim_first && A + R > 0) y.MH_std = mh_std_clamp(p, std_ * mh_std_gain(A, R, &y.a_rate));
+            else y.MH_std = std_;
+          }
+        }
         if (ONE && ok && it == p.mh_jumps) { ax[k] = fx; ay[k] = fy; }   // the last points (RD_MH_FINAL)
       }
     }
