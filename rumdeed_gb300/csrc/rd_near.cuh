@@ -627,7 +627,8 @@ __device__ __forceinline__ int near_entry(const PlanEntry* __restrict__ plan, in
   return seg * step + __popc(__ballot_sync(0xffffffffu, lane < step && j < nd && plan[j].item_off <= g)) - 1;
 }
 
-// The acceptance counts of one tile; the diode's last tile updates MH_std
+// The acceptance counts of one tile, after the warm-up (whose step size is fixed: its
+// jumps neither count nor wait); the diode's last tile updates MH_std
 // (MH_std_update :603-612, as mh_std_step) and lets the next jump go.  One packed
 // atomic carries the tile count and both sums, so its answer tells the last tile
 // the diode's totals.  At the upper clamp with a rate above 0.35 the product stays
@@ -635,14 +636,14 @@ __device__ __forceinline__ int near_entry(const PlanEntry* __restrict__ plan, in
 // the rate itself is only kept at the last jump (every jump counts the same chains).
 __device__ __forceinline__ void near_counts(const DiodeParams& p, DiodeDyn& y, unsigned long long* count,
                                             unsigned long long* progress, unsigned long long last, int tiles, int it_idx,
-                                            int ndim_first, int a, int r) {
+                                            int a, int r) {
   const unsigned long long add = (1ull << 44) | ((unsigned long long)a << 22) | (unsigned long long)r;
   const unsigned long long now = atomicAdd(count, add) + add;
   if ((int)(now >> 44) != tiles) return;
   __stcg(count, 0ull);
   const int A = (int)(now >> 22) & 0x3fffff, R = (int)now & 0x3fffff;
-  unsigned long long next = last + 1;   // the step size stays
-  if (it_idx > ndim_first && A + R > 0 &&
+  unsigned long long next = (last & ~0x7fffffffull) | (unsigned)it_idx;   // the step size stays
+  if (A + R > 0 &&
       (it_idx == p.mh_jumps || !((unsigned)last & RD_NEAR_CLAMPED) || 20ll * A <= 7ll * (A + R))) {
     const double g = mh_std_gain(A, R, &y.a_rate);
     const double m = mh_std_clamp(p, __ldcg(&y.MH_std) * g);
@@ -782,11 +783,11 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           if (lane == 0) {
             if (it == 1) {
               std_ = __ldcg(&y.MH_std);
-            } else {
+            } else if (it - 1 > ndim_first) {
               int A, R;
               if (!near_wait_counts(nr.ring + 4 * d + ((it - 1) & 3), plan[d].tiles, &A, &R)) sh.dead = 1;
               double rate;
-              if (it - 1 > ndim_first && A + R > 0 && (std_ != p.mh_hi || 20ll * A <= 7ll * (A + R)))
+              if (A + R > 0 && (std_ != p.mh_hi || 20ll * A <= 7ll * (A + R)))
                 std_ = mh_std_clamp(p, std_ * mh_std_gain(A, R, &rate));
             }
           }
@@ -795,8 +796,9 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           if (lane == 0) {
             const volatile unsigned long long* prog = nr.progress + d;
             pr = *prog;
-            for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1 && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
-            if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
+            const int need = it - 1 > ndim_first ? it - 1 : 0;   // the warm-up's step size is fixed: no wait
+            for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < need && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
+            if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < need) sh.dead = 1;
           }
           pr = __shfl_sync(0xffffffffu, pr, 0);
         }
@@ -851,7 +853,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
         if (tid == 0) atomicAdd(gave_up, 1);
         return;
       }
-      if (ONE && tid == NT - 32 && g == plan[d].item_off) {   // the word of jump it + 2 (a barrier before this jump's count)
+      if (ONE && tid == NT - 32 && it > ndim_first && g == plan[d].item_off) {   // the word of jump it + 2 (a barrier before this jump's count)
         __stcg(nr.ring + 4 * d + ((it + 2) & 3), 0ull);
         __threadfence();
       }
@@ -932,14 +934,14 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
       }
       if (w == 0) {
         const int acc = __popc(__ballot_sync(0xffffffffu, a)), rej = __popc(__ballot_sync(0xffffffffu, ok && !a));
-        if (lane == 0 && !ONE)
-          near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, ndim_first, acc, rej);
-        if (lane == 0 && ONE) {
+        if (lane == 0 && !ONE && it > ndim_first)
+          near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, acc, rej);
+        if (lane == 0 && ONE && it > ndim_first) {
           atomicAdd(nr.ring + 4 * d + (it & 3), (1ull << 44) | ((unsigned long long)acc << 22) | (unsigned long long)rej);
           if (it == p.mh_jumps && g == plan[d].item_off) {   // the step's last counts
             int A, R;
             if (!near_wait_counts(nr.ring + 4 * d + (it & 3), plan[d].tiles, &A, &R)) atomicAdd(gave_up, 1);
-            else if (it > ndim_first && A + R > 0) y.MH_std = mh_std_clamp(p, std_ * mh_std_gain(A, R, &y.a_rate));
+            else if (A + R > 0) y.MH_std = mh_std_clamp(p, std_ * mh_std_gain(A, R, &y.a_rate));
             else y.MH_std = std_;
           }
         }

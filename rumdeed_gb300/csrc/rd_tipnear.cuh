@@ -359,8 +359,9 @@ k_tip_jumps(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const 
         if (lane == 0) {   // the step size after the last jump
           const volatile unsigned long long* prog = nr.progress + d;
           pr = *prog;
-          for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1 && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
-          if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < it - 1) sh.dead = 1;
+          const int need = it - 1 > ndim_first ? it - 1 : 0;   // the warm-up's step size is fixed: no wait
+          for (int spins = 0; (int)((unsigned)pr & ~RD_NEAR_CLAMPED) < need && spins < RD_NEAR_SPIN; ++spins) pr = *prog;
+          if ((int)((unsigned)pr & ~RD_NEAR_CLAMPED) < need) sh.dead = 1;
         }
         pr = __shfl_sync(0xffffffffu, pr, 0);
         __threadfence();   // MH_std was written before the progress word
@@ -525,7 +526,7 @@ k_tip_jumps(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const 
       }
       if (w == 0) {
         const int acc = __popc(__ballot_sync(0xffffffffu, a)), rej = __popc(__ballot_sync(0xffffffffu, ok && !a));
-        if (lane == 0) near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, ndim_first, acc, rej);
+        if (lane == 0 && it > ndim_first) near_counts(p, y, nr.count + d, nr.progress + d, pr, plan[d].tiles, it, acc, rej);
       }
       __syncthreads();   // the shared proposals are free for the next item
     }
