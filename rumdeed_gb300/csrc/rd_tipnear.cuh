@@ -201,12 +201,14 @@ __device__ __forceinline__ void tip_entry(const DiodeParams& p, double xi, float
 // A jump that the estimate leaves open (rare): the pair sums at the proposal (point 0)
 // and at the chain's point (1), as k_mh_jump_tip forms them, by the whole block -- a
 // thread per tile and point's 128 terms, then each component's tiles in order -- and its
-// test.  A chain that has not moved keeps the field of its start.  mine decides.
+// test.  FP64 latency on few threads, so log u is drawn by another warp meanwhile; with
+// one thread for both points of a tile and log u at the end a step with eight open jumps
+// took 3.23 ms, so 3.15.  A chain that has not moved keeps the field of its start.  mine decides.
 template <int NT>
 struct TipExact {
-  float t[2][6][NT];            // a pass's tile sums
+  float t[2][6][NT / 2];        // a pass's tile sums
   float4 ih[2], iih[2];
-  double X[2], Y[2], Z[2], f[2][3], F[2], s[2];
+  double X[2], Y[2], Z[2], f[2][3], F[2], s[2], lu;
 };
 template <int NT>
 __device__ __noinline__ int tip_open(const DiodeParams& p, const Pool& pool, const ChainState& cs, const PlanEntry& e,
@@ -219,28 +221,31 @@ __device__ __noinline__ int tip_open(const DiodeParams& p, const Pool& pool, con
     float4 il, iil;
     point_pack(p, X, Y, Z, s->ih[tid], il, s->iih[tid], iil);
     s->X[tid] = X; s->Y[tid] = Y; s->Z[tid] = Z;
+  } else if (tid == 32) {   // log u of the accept test
+    double u1, u2;
+    rng2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, &u1, &u2);
+    s->lu = log(u1);
   }
   __syncthreads();
   const int pt = tid / 3, i = tid % 3;   // threads 0..5: component i of point pt
   float h = 0.0f, l = 0.0f, im = 0.0f;
   double acc = 0.0;
   int in_chunk = 0, chunk = 0;
-  for (int base = 0; base < tiles; base += NT) {
-    const int tile = base + tid;
+  for (int base = 0; base < tiles; base += NT / 2) {
+    const int q = tid / (NT / 2), slot = tid % (NT / 2), tile = base + slot;   // a thread per point and tile
     if (tile < tiles) {
       const int j = tile * RD_TILE;
-      const float4 ih[2] = {s->ih[0], s->ih[1]}, iih[2] = {s->iih[0], s->iih[1]};
-      float td[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, te[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+      const float4 ih[1] = {s->ih[q]}, iih[1] = {s->iih[q]};
+      float td[1][3] = {{0.f, 0.f, 0.f}}, te[1][3] = {{0.f, 0.f, 0.f}};
       const float4 *sh = pool.pk_hi + p.off + j, *sl = pool.pk_lo + p.off + j;
       const int kmax = min(RD_TILE, n - j);
-      if (p.image_charge) tip_point_tiles_f32<2, false, true>(sh, sl, kmax, ih, iih, td, te);
-      else tip_point_tiles_f32<2, false, false>(sh, sl, kmax, ih, iih, td, te);
-      for (int q = 0; q < 2; ++q)
-        for (int a = 0; a < 3; ++a) { s->t[q][a][tid] = td[q][a]; s->t[q][3 + a][tid] = te[q][a]; }
+      if (p.image_charge) tip_point_tiles_f32<1, false, true>(sh, sl, kmax, ih, iih, td, te);
+      else tip_point_tiles_f32<1, false, false>(sh, sl, kmax, ih, iih, td, te);
+      for (int a = 0; a < 3; ++a) { s->t[q][a][slot] = td[0][a]; s->t[q][3 + a][slot] = te[0][a]; }
     }
     __syncthreads();
     if (tid < 6)
-      for (int t = 0; t < min(NT, tiles - base); ++t) {
+      for (int t = 0; t < min(NT / 2, tiles - base); ++t) {
         two_sum_acc(h, l, s->t[pt][i][t]);
         im += s->t[pt][3 + i][t];
         if (++in_chunk == tpc || base + t + 1 == tiles) {
@@ -266,13 +271,7 @@ __device__ __noinline__ int tip_open(const DiodeParams& p, const Pool& pool, con
     float t0, t2;
     const double F = s->F[0], Fc = cs.em[k] ? s->F[1] : cs.F[k], sn = s->s[0], sc = cs.em[k] ? s->s[1] : cs.sup[k];
     if (F < 0.0) {
-      bool take = sn >= sc;
-      if (!take) {
-        double u1, u2;
-        rng2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, &u1, &u2);
-        take = log(u1) <= sn - sc;
-      }
-      a = take;
+      a = sn >= sc || s->lu <= sn - sc;
     }
     const double xi = a ? nxi : cxi;
     const float Ff = (float)(a ? F : Fc);
@@ -304,9 +303,9 @@ struct TipShared {
 // decides; eight lanes per chain sum its near electrons, four loads in flight each, and
 // evaluate the expansion, an order m per lane.  em marks a chain that has moved.
 // Measured (GB300, 8900 chains, 12,500 electrons, 80 jumps): 17.1 ms with the pair-sum
-// jumps, 1.9 ms so, the panels and the last pass included.  Bound by the latency of a
+// jumps, 1.7 ms so, the panels and the last pass included.  Bound by the latency of a
 // jump, about 10 us: FP64 sine and cosine 3, the step 1.5, the sums 3, the decision 1.4,
-// the rest loads and the progress word.  One jump in 10^5 is left open and takes 60 us;
+// the rest loads and the progress word.  One jump in 10^5 is left open (tip_open);
 // the estimate lay within 0.16 of its bound in every jump checked.
 __global__ void __launch_bounds__(256, 2)
 k_tip_jumps(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const __grid_constant__ Pool pool,
@@ -521,7 +520,7 @@ k_tip_jumps(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const 
       __syncthreads();
       for (unsigned o = sh.open; o; o &= o - 1) {   // block-uniform
         const int q = __ffs(o) - 1;
-        a += tip_open<256>(p, pool, cs, plan_mh[d], kscale, tid == q, c, k, it, step, sh.oxi[q], sh.oph[q], sh.cxi[q],
+        a += tip_open<256>(p, pool, cs, plan_mh[d], kscale, tid == q, c - lane + q, k, it, step, sh.oxi[q], sh.oph[q], sh.cxi[q],
                            sh.cph[q], &sh.ex);
       }
       if (w == 0) {
