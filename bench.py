@@ -499,7 +499,7 @@ def run_ours(args, rank, world):
                     "step_ms_max": float(max(step_ms)),
                     "queueing_delay_s_p50": float(np.percentile(qd, 50)) if qd else None,
                     "queueing_delay_s_p99": float(np.percentile(qd, 99)) if qd else None,
-                    "simulation_latency": "a simulation lasts minutes (500-20000 steps at ~0.25 s): "
+                    "simulation_latency": "a simulation lasts up to a quarter of an hour (500-20000 steps at ~0.05 s): "
                                           "measured with step counts / 100 by --case serve-latency"},
         "e2e": {"value": e2e, "unit": METRIC, "h2d_bytes_per_step": e2e_h2d / max(args.steps, 1),
                 "d2h_bytes_per_step": e2e_d2h / max(args.steps, 1),

@@ -952,9 +952,11 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
   for (auto p : chd) if (e->dalloc(p, chcap)) return bail(fail(RD_ERR_NOMEM, "chain pool allocation failed"));
   if (e->dalloc(&e->cs.ok, chcap) || e->dalloc(&e->cs.prop_ok, chcap) || e->dalloc(&e->cs.em, chcap))
     return bail(fail(RD_ERR_NOMEM, "chain pool allocation failed"));
-  for (int m = 0; m < PM_COUNT; ++m)
-    if (e->dalloc(&e->plan[m], S) || e->dalloc(&e->ph[m], 1))
-      return bail(fail(RD_ERR_NOMEM, "plan allocation failed"));
+  PlanEntry* plans = nullptr;   // one allocation each: a cudaMalloc takes some 10 us
+  PlanHeader* heads = nullptr;
+  if (e->dalloc(&plans, (size_t)PM_COUNT * S) || e->dalloc(&heads, PM_COUNT))
+    return bail(fail(RD_ERR_NOMEM, "plan allocation failed"));
+  for (int m = 0; m < PM_COUNT; ++m) { e->plan[m] = plans + (size_t)m * S; e->ph[m] = heads + m; }
   cudaMemsetAsync(e->dP, 0, sizeof(DiodeParams) * S, e->st);
   cudaMemsetAsync(e->dD, 0, sizeof(DiodeDyn) * S, e->st);
   cudaMemsetAsync(e->tickets, 0, 3 * sizeof(int) * (size_t)e->max_items, e->st);
