@@ -303,7 +303,8 @@ def reduce_ranks(world, maxes, sums):
 
 
 # Serving-iteration time of the 128-slot mix, used only to pace the stream's
-# arrivals in the admission schedule below.
+# arrivals in the admission schedule below (the pace that fixes the workload's window; a
+# step of that mix takes 0.05 s now).
 STEP_S_EST = 0.245
 # The timed window starts at least this many serving iterations (~100 s) into the stream.
 WINDOW_AFTER = 400
