@@ -70,7 +70,7 @@ cudaError_t rd_launch_mh_jump(int prec, int geometry_mask, int grid, cudaStream_
                               const int* ch_off, const double* wtab, const int* step_ptr,
                               int it_idx, double* partial, int* tickets, double kscale, int* queue,
                               int part = 0, int nparts = 1, int form = 0);
-cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
+cudaError_t rd_launch_near_setup(int prec, int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
                                  const Pool& pool, const PlanEntry* sup_plan, const PlanHeader* sup_ph,
                                  const float4* qpp, const double* qF, const NearState& nr, double kscale);
 cudaError_t rd_launch_mh_jumps_near(int prec, int grid, cudaStream_t st, const DiodeParams* P, DiodeDyn* Dy,
@@ -518,7 +518,7 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
   const int parts = slow ? mh_parts_for(e, s) : 1, form = mh_form_for(e, s);
   int pm = PM_MH, rc;
   if (near) {
-    CK(rd_launch_near_setup(e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_SUPPLY_PLANAR],
+    CK(rd_launch_near_setup(prec, e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_SUPPLY_PLANAR],
                             e->ph[PM_SUPPLY_PLANAR], e->qpp, e->qF, e->nr, e->kscale));
     e->kernels_in_step += 4;
     if (slow) pm = PM_MH_SLOW;

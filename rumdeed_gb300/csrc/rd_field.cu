@@ -2910,7 +2910,7 @@ cudaError_t rd_launch_mh_jump(int prec, int geometry_mask, int grid, cudaStream_
 
 // Bins, near electrons and panel records of the step's chains (rd_near.cuh), from the
 // supply field qF.
-cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
+cudaError_t rd_launch_near_setup(int prec, int nslots, int grid, cudaStream_t st, const DiodeParams* P, const DiodeDyn* Dy,
                                  const Pool& pool, const PlanEntry* sup_plan, const PlanHeader* sup_ph,
                                  const float4* qpp, const double* qF, const NearState& nr, double kscale) {
   k_near_count<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
@@ -2918,13 +2918,14 @@ cudaError_t rd_launch_near_setup(int nslots, int grid, cudaStream_t st, const Di
   k_near_scatter<<<dim3(32, nslots), 256, 0, st>>>(P, Dy, pool, nr);
   // Only a tile's first item has work: a prime number of blocks, so that no number of
   // chunks gives those items to a part of the blocks only.
-  int blocks = rd_grid(k_near_panels, 256, grid);
+  int blocks = prec == 1 ? rd_grid(k_near_panels<1>, 256, grid) : rd_grid(k_near_panels<0>, 256, grid);
   auto prime = [](int v) {
     for (int f = 2; f * f <= v; ++f) if (v % f == 0) return false;
     return true;
   };
   while (!prime(blocks)) --blocks;
-  k_near_panels<<<blocks, 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
+  if (prec == 1) k_near_panels<1><<<blocks, 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
+  else k_near_panels<0><<<blocks, 256, 0, st>>>(P, Dy, sup_plan, sup_ph, qpp, qF, nr, kscale);
   return cudaGetLastError();
 }
 

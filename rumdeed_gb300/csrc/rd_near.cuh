@@ -180,6 +180,10 @@ __device__ const float c_gl4_inv[4][4] = {
 // RD_NEAR_AWAY half widths from the eight panels' rectangle now add one term for all of
 // them (at the rectangle's distance T is larger by a per cent or so), the others pass
 // through shared memory once for the eight warps: 2.8 ms.
+// S is the FP32 pair sum at the nodes' high words, or the FP64 one at the nodes
+// themselves (high and low words); the near terms taken off it are at the same points:
+// beside a node half an ulp of its coordinate is worth many of the bound's u.
+template <int PREC>
 __global__ void __launch_bounds__(256)
 k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, const PlanEntry* __restrict__ plan,
               const PlanHeader* __restrict__ ph, const float4* __restrict__ qpp, const double* __restrict__ qF,
@@ -211,7 +215,8 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
       for (int e0 = start[row]; e0 < e1; e0 += 64) {   // short runs: the sums stay accurate
         float s = 0.0f;
         for (int e = e0 + (lane >> 4); e < min(e0 + 64, e1); e += 2)
-          s += near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z);
+          s += PREC == 1 ? near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z)
+                         : near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z, pp.y, pp.w);
         near += s;
       }
     }
