@@ -1978,6 +1978,7 @@ int rd_run(rd_engine* e, int first_step, int nsteps) {
   if (nsteps < 0) return fail(RD_ERR_INVALID, "nsteps < 0");
   int rc = ensure_graph(e);
   if (rc) return rc;
+  if (nsteps > 0 && (rc = fresh_packs(e))) return rc;   // of a lone emission before this step's
   CK(rd_launch_step_set(e->st, e->d_step, first_step));
   CK(cudaEventRecord(e->ev0, e->st));
   for (int s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(e->graph, e->st));
@@ -1986,7 +1987,6 @@ int rd_run(rd_engine* e, int first_step, int nsteps) {
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
   e->last_ms = ms;
-  if (nsteps > 0) e->packs_stale = false;
   return compaction_check(e);
 }
 
@@ -2208,6 +2208,8 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   Sig s = signature(e);
   const int prec = e->cfg.precision;
   std::vector<DiodeDyn> dyn(S);
+  int rc = fresh_packs(e);
+  if (rc) return rc;
   CK(rd_launch_step_set(e->st, e->d_step, step));
   CK(cudaEventRecord(ev[0], e->st));
   if (s.emit_planar || s.emit_tip) {
@@ -2269,7 +2271,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   CK(rd_launch_position(e->grid, e->st, e->dP, e->dD, e->pool, e->plan[PM_PART], e->ph[PM_PART], e->evlog,
                         e->d_step));
   CK(cudaEventRecord(ev[5], e->st));
-  int rc = launch_force(e, true);
+  rc = launch_force(e, true);
   if (rc) return rc;
   CK(cudaEventRecord(ev[6], e->st));
   CK(rd_launch_velocity(e->grid, S, e->st, e->dP, e->dD, e->pool, e->plan[PM_PART], e->ph[PM_PART], e->ramo,
@@ -2420,7 +2422,7 @@ int rd_serve(rd_engine* e, int iterations, rd_serve_stats* out) {
     if (e->running.empty() && (rc = serve_admit(e, out, e->gstep))) return rc;
     if ((rc = activate_pending(e))) return rc;
     if (e->running.empty()) break;
-    if ((rc = ensure_graph(e))) return rc;
+    if ((rc = ensure_graph(e)) || (rc = fresh_packs(e))) return rc;
     CK(rd_launch_step_set(e->st, e->d_step, e->gstep));
     CK(cudaEventRecord(e->ev0, e->st));
     CK(cudaGraphLaunch(e->graph, e->st));
