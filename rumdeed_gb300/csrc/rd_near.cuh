@@ -161,6 +161,24 @@ __device__ __forceinline__ float near_term(float4 h, float2 l, float px, float p
   return h.w * ((inv * inv) * inv);
 }
 
+// FP64 chains: how far a term can lie from the FP64 pair sum's, added to *wide.  The
+// reference's r + l^2 (l^2 = 1e-9 nm) makes a term smaller by at most 3 l^2 / r of it.
+// The packs and the split point hold a coordinate to 2^-48 of it and their difference
+// loses as much again: 2^-45 of the emitter's half width together, which is at most
+// 4 times that over r of the term as long as r is ten times larger; closer (and where
+// l^2 shows in the first digit) nothing is promised.  At r = 1 nm this is 0.05 u of the
+// term, at 1e-3 nm 50 u.
+__device__ __forceinline__ float near_wide(const DiodeParams& p) {
+  return 3.0e-9f + 1.2e-13f * (float)p.nr_P * fmaxf(p.nr_ax, p.nr_ay);
+}
+__device__ __forceinline__ float near_term(float4 h, float2 l, float px, float py, float qx, float qy, float kw,
+                                           float* wide) {
+  const float dx = (px - h.x) - (l.x - qx), dy = (py - h.y) - (l.y - qy);
+  const float inv = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, h.z))), g = h.w * ((inv * inv) * inv), k = kw * inv;
+  *wide = fmaf(fabsf(g), k < 0.25f ? k : INFINITY, *wide);
+  return g;
+}
+
 // Inverse Vandermonde matrix of the four Gauss-Legendre nodes: coefficients of
 // the interpolating cubic from the node values.
 __device__ const float c_gl4_inv[4][4] = {
@@ -208,7 +226,8 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     const int k = p.q_off + (ppy * 4 + ((lane >> 2) & 3)) * p.quad_n + ppx * 4 + (lane & 3);
     const float4 pp = qpp[k];
     const float S = (float)((qF[k] - p.E_z) * inv_A0);
-    float near = 0.0f;
+    float near = 0.0f, wide = 0.0f;
+    const float kw = near_wide(p);
     for (int r = 0; r < RD_NEAR_ROWS; ++r) {
       const int row = (r0 + r) * nb + ppx;   // bins ppx .. ppx + 2 M of this row
       const int e1 = start[row + RD_NEAR_W];
@@ -216,12 +235,17 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
         float s = 0.0f;
         for (int e = e0 + (lane >> 4); e < min(e0 + 64, e1); e += 2)
           s += PREC == 1 ? near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z)
-                         : near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z, pp.y, pp.w);
+                         : near_term(nr.hi[p.off + e], nr.lo[p.off + e], pp.x, pp.z, pp.y, pp.w, kw, &wide);
         near += s;
       }
     }
     near += __shfl_xor_sync(0xffffffffu, near, 16);
     float big = fabsf(S);
+    if (PREC == 0) {   // the node's near terms too, in the units of the bound's 250 u of `big`
+      wide += __shfl_xor_sync(0xffffffffu, wide, 16);
+      big = fmaf(wide, 6.7e4f, big);
+      if (!(big < INFINITY)) big = INFINITY;
+    }
     for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
     // tensor coefficients of the far part, about the value at the first node
     const float far = S - near, base = __shfl_sync(0xffffffffu, far, 0), v = far - base;
@@ -694,6 +718,7 @@ struct NearShared {
   using Real = typename std::conditional<PREC == 1, float, double>::type;
   float x[32], y[32], near[32], lu[32];   // proposal (nm; FP64 chains: high words), near sum, log u
   float xl[PREC == 1 ? 1 : 32], yl[PREC == 1 ? 1 : 32];   // FP64 chains: low words
+  float wide[PREC == 1 ? 1 : 32];                         // and how far the near sum may be off (near_wide)
   Real g[2][32];                          // next Gaussian pair
   int pan[32];                            // the chain's panel; -1: no chain
   Real ox[32], oy[32], cx[32], cy[32];    // proposals and chains' points, where a jump is left open
@@ -865,8 +890,9 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
       // near electrons
       for (int r8 = 0; r8 < ROUNDS; ++r8) {
         const int l = lane & 7, q = (w * ROUNDS + r8) * 4 + (lane >> 3), pan = sh.pan[q];
-        float s = 0.0f;
+        float s = 0.0f, wide = 0.0f;
         if (pan >= 0) {
+          const float kw = near_wide(p);
           // the list's rows: their ends in it, and what turns an index of it into an electron
           const int4* rt = reinterpret_cast<const int4*>(recs + (size_t)pan * RD_NEAR_REC + 20);
           const int4 end = rt[0], at = rt[1];
@@ -887,14 +913,21 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
               lo[u] = in ? nl[k2] : make_float2(0.0f, 0.0f);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) run += near_term(h[u], lo[u], x, yv, xl, yl);
+            for (int u = 0; u < 4; ++u)
+              run += PREC == 1 ? near_term(h[u], lo[u], x, yv) : near_term(h[u], lo[u], x, yv, xl, yl, kw, &wide);
             if (++m == 8) { s += run; run = 0.0f; m = 0; }   // short runs: the sum stays accurate
           }
           s += run;
         }
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (l == 0) sh.near[q] = s;
+        for (int o = 4; o > 0; o >>= 1) {
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (PREC == 0) wide += __shfl_xor_sync(0xffffffffu, wide, o);
+        }
+        if (l == 0) {
+          sh.near[q] = s;
+          if (PREC == 0) sh.wide[q] = wide;
+        }
       }
       if (NW > 1) __syncthreads(); else __syncwarp();
       int a = 0;
@@ -903,7 +936,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
         const Real cx = fx, cy = fy;
         if (ok) {
           if (ONE) far_part.eval(p, px, py);
-          const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y;
+          const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y + (PREC == 1 ? 0.0f : sh.wide[lane]);
           float dF, rn;
           const float Fn = near_field(p, ksc, S, fmaf(near_boundA(p), 1.01f * fabsf(S), b0), &dF);
           const int take = near_decide(p, Fn, dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
