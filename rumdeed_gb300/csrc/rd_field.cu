@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "rd_bounds.h"
 #include "rd_tiles.cuh"
 
 

@@ -228,9 +228,11 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     const float S = (float)((qF[k] - p.E_z) * inv_A0);
     float near = 0.0f, wide = 0.0f;
     const float kw = near_wide(p);
+    int cnt = 0;   // near electrons
     for (int r = 0; r < RD_NEAR_ROWS; ++r) {
       const int row = (r0 + r) * nb + ppx;   // bins ppx .. ppx + 2 M of this row
       const int e1 = start[row + RD_NEAR_W];
+      cnt += e1 - start[row];
       for (int e0 = start[row]; e0 < e1; e0 += 64) {   // short runs: the sums stay accurate
         float s = 0.0f;
         for (int e = e0 + (lane >> 4); e < min(e0 + 64, e1); e += 2)
@@ -241,12 +243,13 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
     }
     near += __shfl_xor_sync(0xffffffffu, near, 16);
     float big = fabsf(S);
-    if (PREC == 0) {   // the node's near terms too, in the units of the bound's 250 u of `big`
+    if (PREC == 0) {   // the node's near terms too, in the units of the bound on `big`'s
       wide += __shfl_xor_sync(0xffffffffu, wide, 16);
-      big = fmaf(wide, 6.7e4f, big);
+      big = fmaf(wide, 1.0f / (RD_U24 * RD_NEAR_UNITS), big);
       if (!(big < INFINITY)) big = INFINITY;
     }
     for (int o = 8; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+    big *= rd_near_node_factor(cnt);
     // tensor coefficients of the far part, about the value at the first node
     const float far = S - near, base = __shfl_sync(0xffffffffu, far, 0), v = far - base;
     float cx = 0.0f, c = 0.0f;
@@ -340,26 +343,27 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
       reinterpret_cast<int*>(rec)[20 + RD_NEAR_ROWS + lane] = a0 - (end - len);
     }
     if (lane == 0) *reinterpret_cast<float4*>(rec + 16) = make_float4(ox, oy, 1.03f * Tx, big);
-    if (lane == 1) rec[28] = 1.03f * Ty;
+    if (lane == 1) *reinterpret_cast<float2*>(rec + 28) = make_float2(1.03f * Ty, RD_U24 * rd_near_units(NP, cnt));
   }
 }
 
 // Bound on |estimate - pair sum| at (tx, ty) of a panel: the interpolation's
 // error, and the roundings of the pair sum (153 u of the sum of magnitudes A at
 // the point, the same of the nodes' `big` carried through the interpolation),
-// of the near sums (at most ~60 u each), of the points' own coordinates (half
+// of the near sums (a run of 32 terms, the lanes' sums, and one more addition for
+// every further run: rd_bounds.h, which k_near_panels has put into `big` and the
+// record's last word), of the points' own coordinates (half
 // an ulp of the emitter's half width, against the distance 5 a to the nearest
 // far electron: 0.6 P u) and of the evaluation (~30 u).
-// near_bound0 is the part that does not depend on A (factor near_boundA).
+// near_bound0 is the part that does not depend on A (factor: the record's last word).
 __device__ __forceinline__ float near_bound0(const DiodeParams& p, float tx, float ty, float Tx, float Ty, float big) {
   const float x2 = tx * tx, y2 = ty * ty;
   const float wx = fabsf((x2 - 0.741555748f) * (x2 - 0.115587109f)), wy = fabsf((y2 - 0.741555748f) * (y2 - 0.115587109f));
   const float lx = 1.48f + 14.0f * fmaxf(fabsf(tx) - 0.9f, 0.0f), ly = 1.48f + 14.0f * fmaxf(fabsf(ty) - 0.9f, 0.0f);
   const float ax2 = p.nr_ax * p.nr_ax, ay2 = p.nr_ay * p.nr_ay;
-  const float u = 5.97e-8f, c = 0.6f * (float)p.nr_P;
-  return Tx * ((wx + 1e-5f) * (ax2 * ax2)) + Ty * (lx * (wy + 1e-5f) * (ay2 * ay2)) + u * (lx * ly * (250.0f + c) * big);
+  return Tx * ((wx + 1e-5f) * (ax2 * ax2)) + Ty * (lx * (wy + 1e-5f) * (ay2 * ay2)) +
+         RD_U24 * (lx * ly * rd_near_units(p.nr_P, 0) * big);
 }
-__device__ __forceinline__ float near_boundA(const DiodeParams& p) { return 5.97e-8f * (250.0f + 0.6f * (float)p.nr_P); }
 
 // The pair sums of k_mh_jump_planar at two points, by the NT threads of a block,
 // bit for bit.  A warp takes two j-tiles at a time: its lanes form the factors
@@ -490,8 +494,8 @@ __device__ __forceinline__ float near_field(const DiodeParams& p, float ksc, flo
 // A jump that the interpolated estimate leaves open (rare; out of line so that it
 // costs the others no registers).  First the direct sums at the proposal (px, py)
 // and at the chain's point (cx, cy) by the whole block, in any order: they lie
-// within the roundings of the two sums (153 u for the pair sum, 25 u a term and at
-// most 60 u for the order here) of the pair sums, some twenty times closer than the
+// within the roundings of the two sums (153 u for the pair sum, 25 u a term and the
+// order here: rd_near_direct_units) of the pair sums, some twenty times closer than the
 // estimate, and let the targets be compared in FP64; what even they leave open takes
 // the pair sums (near_exact2) and
 // mh_accept_one_f's test.  The thread that holds the chain (mine) decides and
@@ -532,13 +536,13 @@ __device__ __noinline__ int near_open(const DiodeParams& p, const Pool& pool, co
   if (mine) {
     sn = sc = 0.0f;
     for (int w = 0; w < NT / 32; ++w) { sn += s->t[0][w]; sc += s->t[1][w]; }
-    const float u = 5.97e-8f;
+    const float eu = RD_U24 * rd_near_direct_units(n, NT);
     float dFn, dFc, t0, t2, r;
-    const float Fn = near_field(p, (float)kscale, sn, 250.0f * u * fabsf(sn), &dFn);
+    const float Fn = near_field(p, (float)kscale, sn, eu * fabsf(sn), &dFn);
     work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
     float Fc = cs.fF[k], fe = cs.fe[k], rho = cs.fsup[k];
     if (fe != 0.0f) {
-      const float F2 = near_field(p, (float)kscale, sc, 250.0f * u * fabsf(sc), &dFc);
+      const float F2 = near_field(p, (float)kscale, sc, eu * fabsf(sc), &dFc);
       if (dFc < fe && F2 < 0.0f && 4.0f * dFc <= -F2) {
         Fc = F2; fe = dFc;
         rho = rho_xy_f(p, wtab, cx, cy, F2);
@@ -548,7 +552,7 @@ __device__ __noinline__ int near_open(const DiodeParams& p, const Pool& pool, co
     int take = near_decide(p, Fn, dFn, Fc, fe, rho, t0, t2, lu, &r);
     const double Dn = p.E_z - 2.0 * kscale * (double)sn, Dc = p.E_z - 2.0 * kscale * (double)sc;
     if (take < 0 && Dn < 0.0 && Dc < 0.0) {   // the targets in FP64: only the sums' own bounds remain
-      const double en = 2.0 * kscale * 250.0 * (double)u * fabs((double)sn), ec = 2.0 * kscale * 250.0 * (double)u * fabs((double)sc);
+      const double en = 2.0 * kscale * (double)eu * fabs((double)sn), ec = 2.0 * kscale * (double)eu * fabs((double)sc);
       if (4.0 * en <= -Dn && 4.0 * ec <= -Dc) {
         uint32_t o[4];
         philox4x32((uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), o);
@@ -735,10 +739,10 @@ __device__ __forceinline__ typename std::conditional<PREC == 1, float, double>::
 // The far part at a point: a panel's record, then its value and bound (c0.x, c0.y).
 struct NearFar {
   float4 c0, c1, c2, c3, cm;
-  float ty;
+  float2 ty;   // and the rounding per |S|
   __device__ __forceinline__ void load(const float4* rec) {
     c0 = rec[0]; c1 = rec[1]; c2 = rec[2]; c3 = rec[3]; cm = rec[4];
-    ty = reinterpret_cast<const float*>(rec)[28];
+    ty = reinterpret_cast<const float2*>(rec)[14];
   }
   __device__ __forceinline__ void eval(const DiodeParams& p, float px, float py) {
     const float x = (px - cm.x) * p.nr_iax, y = (py - cm.y) * p.nr_iay;
@@ -746,7 +750,7 @@ struct NearFar {
     const float r1 = fmaf(fmaf(fmaf(c1.w, x, c1.z), x, c1.y), x, c1.x);
     const float r2 = fmaf(fmaf(fmaf(c2.w, x, c2.z), x, c2.y), x, c2.x);
     const float r3 = fmaf(fmaf(fmaf(c3.w, x, c3.z), x, c3.y), x, c3.x);
-    c0.y = near_bound0(p, x, y, cm.z, ty, cm.w);
+    c0.y = near_bound0(p, x, y, cm.z, ty.x, cm.w);
     c0.x = fmaf(fmaf(fmaf(r3, y, r2), y, r1), y, r0);
   }
 };
@@ -938,7 +942,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           if (ONE) far_part.eval(p, px, py);
           const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y + (PREC == 1 ? 0.0f : sh.wide[lane]);
           float dF, rn;
-          const float Fn = near_field(p, ksc, S, fmaf(near_boundA(p), 1.01f * fabsf(S), b0), &dF);
+          const float Fn = near_field(p, ksc, S, fmaf(far_part.ty.y, 1.01f * fabsf(S), b0), &dF);
           const int take = near_decide(p, Fn, dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
           open = take < 0;
           if (take == 1) {
