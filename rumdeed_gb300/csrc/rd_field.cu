@@ -382,7 +382,7 @@ __device__ __forceinline__ void near_start_d(const DiodeParams& p, const ChainSt
   work_entry_d(p, wtab, x, y, &t0, &t2);
   const float Ff = (float)F;
   cs.fF[k] = Ff;
-  cs.fe[k] = 1.2e-7f * fabsf(Ff);
+  cs.fe[k] = 0.0f;   // F is the pair sum's (its rounding to a float is in near_guard, as the FP32 chains')
   cs.fsup[k] = rho_entry_f(p, t0, t2, Ff);
 }
 
@@ -1408,7 +1408,7 @@ k_mh_jump_planar(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, P
     if (fin) {   // the field and the point in metres that the emission test reads
       for (int q = 0; q < CPT; ++q) {
         if (!ok[q]) continue;
-        cs.F[kk[q]] = z0_finish<PREC>(p, s[q], kscale);
+        if (cs.fe[kk[q]] != 0.0f) cs.F[kk[q]] = z0_finish<PREC>(p, s[q], kscale);   // (0: cs.F is the pair sum already)
         if constexpr (PREC == 1) {
           cs.x[kk[q]] = p.org_x + (double)fwx[q] * 1.0e-9;
           cs.y[kk[q]] = p.org_y + (double)fwy[q] * 1.0e-9;

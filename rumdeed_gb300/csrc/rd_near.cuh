@@ -987,7 +987,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
             else y.MH_std = std_;
           }
         }
-        if (ONE && ok && it == p.mh_jumps) { ax[k] = fx; ay[k] = fy; }   // the last points (RD_MH_FINAL)
+        if (ONE && ok && it == p.mh_jumps) { ax[k] = fx; ay[k] = fy; cs.fe[k] = fe; }   // the last points (RD_MH_FINAL)
       }
     }
   }
