@@ -526,21 +526,23 @@ __device__ __forceinline__ void z0_item_sumN(const DiodeParams& p, const Pool& p
   for (int i = 0; i < CPT; ++i) { out_hi[i] = hi[i]; out_lo[i] = lo[i]; }
 }
 
-// The FP64 tile sum of q_j sum_h h / (r_h + l^2)^3: 13 FP64 operations a term.
+// s plus the FP64 term q_j sum_h h / (r_h + l^2)^3: 13 FP64 operations for one h.
+__device__ __forceinline__ double z0_add_f64(double s, const rd_d4& pj, double px, double py, int nic, double d,
+                                             double L2, float L2x3) {
+  const double dx = px - pj.x, dy = py - pj.y, dxy2 = fma(dx, dx, dy * dy);
+  s = fma(pj.w * pj.z, planar_inv_f64(fma(pj.z, pj.z, dxy2), L2, L2x3), s);
+  for (int n = 1; n <= nic; ++n) {
+    const double h1 = pj.z + (2.0 * n) * d, h2 = pj.z - (2.0 * n) * d;
+    s = fma(pj.w * h1, planar_inv_f64(fma(h1, h1, dxy2), L2, L2x3), s);
+    s = fma(pj.w * h2, planar_inv_f64(fma(h2, h2, dxy2), L2, L2x3), s);
+  }
+  return s;
+}
 __device__ __forceinline__ double z0_tile_f64(const rd_d4* __restrict__ sj, int kmax, double px,
                                               double py, int nic, double d, double L2) {
   const float L2x3 = (float)(3.0 * L2);
   double s = 0.0;
-  for (int k = 0; k < kmax; ++k) {
-    const rd_d4 pj = sj[k];
-    const double dx = px - pj.x, dy = py - pj.y, dxy2 = fma(dx, dx, dy * dy);
-    s = fma(pj.w * pj.z, planar_inv_f64(fma(pj.z, pj.z, dxy2), L2, L2x3), s);
-    for (int n = 1; n <= nic; ++n) {
-      const double h1 = pj.z + (2.0 * n) * d, h2 = pj.z - (2.0 * n) * d;
-      s = fma(pj.w * h1, planar_inv_f64(fma(h1, h1, dxy2), L2, L2x3), s);
-      s = fma(pj.w * h2, planar_inv_f64(fma(h2, h2, dxy2), L2, L2x3), s);
-    }
-  }
+  for (int k = 0; k < kmax; ++k) s = z0_add_f64(s, sj[k], px, py, nic, d, L2, L2x3);
   return s;
 }
 

@@ -594,51 +594,132 @@ __device__ __noinline__ int near_open(const DiodeParams& p, const Pool& pool, co
   return a;
 }
 
-// The FP64 chains' open jumps: FP64 sums at both points by the block, then the test
-// of mh_accept_one.
+// The FP64 chains' open jumps, in the two stages of near_open.  First FP64 sums at both
+// points by the block in any order: with nt threads they lie within n / nt + 200
+// additions' and 8 terms' roundings (v = 2^-53) of the pair sums, and compare the targets
+// to 1e-11.  What even they leave open takes the pair sums of k_mh_jump_planar bit for bit
+// -- a thread per point and tile, the tiles of a chunk and then the chunks in order -- and
+// the test of mh_accept_one.  A point whose field is a pair sum already (fe = 0) keeps it,
+// and its target.  1200 electrons: 2 us an open jump, 25 us with the pair sums at once.
+template <int NT>
+struct NearExact64 {
+  double t[2][NT / 2];   // a pass's tile sums
+  double out[2];
+  int still;
+};
+template <int NT>
+__device__ __noinline__ void near_exact64(const DiodeParams& p, const Pool& pool, const PlanEntry& e, double px,
+                                          double py, double cx, double cy, NearExact64<NT>* s) {
+  const int tid = threadIdx.x, n = e.n_j, tiles = (n + RD_TILE - 1) / RD_TILE, tpc = e.clen / RD_TILE;
+  const float L2x3 = (float)(3.0 * c_k.L2);
+  const int q = tid / (NT / 2), slot = tid % (NT / 2);
+  const double x = q ? cx : px, y = q ? cy : py;
+  double chunk = 0.0, all = 0.0;   // threads 0 and 1: a point each
+  int in_chunk = 0;
+  for (int base = 0; base < tiles; base += NT / 2) {
+    const int j0 = (base + slot) * RD_TILE;
+    double a = 0.0;
+#pragma unroll 4
+    for (int j = j0; j < min(j0 + RD_TILE, n); ++j) {
+      const int g = p.off + j;
+      a = z0_add_f64(a, make_d4(pool.x[g], pool.y[g], pool.z[g], pool.q[g]), x, y, 0, p.d, c_k.L2, L2x3);
+    }
+    s->t[q][slot] = a;
+    __syncthreads();
+    if (tid < 2)
+      for (int i = 0; i < min(NT / 2, tiles - base); ++i) {
+        chunk += s->t[tid][i];
+        if (++in_chunk == tpc || base + i + 1 == tiles) {
+          all = e.nch > 1 ? all + chunk : chunk;
+          chunk = 0.0;
+          in_chunk = 0;
+        }
+      }
+    __syncthreads();
+  }
+  if (tid < 2) s->out[tid] = all;
+  __syncthreads();
+}
+
 template <int NT>
 __device__ __noinline__ int near_open64(const DiodeParams& p, const Pool& pool, const ChainState& cs,
                                         const double* __restrict__ wtab, const PlanEntry& e, double kscale, bool mine,
                                         int c, int k, int it_idx, uint32_t step, double px, double py, double cx,
-                                        double cy, double (*red)[NT / 32]) {
-  const int tid = threadIdx.x, nic = p.image_charge ? p.N_ic_max : 0;
+                                        double cy, NearExact64<NT>* s) {
+  const int tid = threadIdx.x, n = e.n_j;
+  const float L2x3 = (float)(3.0 * c_k.L2);
   double s0 = 0.0, s1 = 0.0;
-  for (int j = tid; j < e.n_j; j += NT) {
+  for (int j = tid; j < n; j += NT) {
     const int g = p.off + j;
     const rd_d4 pj = make_d4(pool.x[g], pool.y[g], pool.z[g], pool.q[g]);
-    s0 += z0_tile_f64(&pj, 1, px, py, nic, p.d, c_k.L2);
-    s1 += z0_tile_f64(&pj, 1, cx, cy, nic, p.d, c_k.L2);
+    s0 = z0_add_f64(s0, pj, px, py, 0, p.d, c_k.L2, L2x3);
+    s1 = z0_add_f64(s1, pj, cx, cy, 0, p.d, c_k.L2, L2x3);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     s0 += __shfl_xor_sync(0xffffffffu, s0, o);
     s1 += __shfl_xor_sync(0xffffffffu, s1, o);
   }
-  if ((tid & 31) == 0) { red[0][tid >> 5] = s0; red[1][tid >> 5] = s1; }
+  if ((tid & 31) == 0) { s->t[0][tid >> 5] = s0; s->t[1][tid >> 5] = s1; }
   __syncthreads();
   int a = 0;
+  float t0, t2;
+  double lu = 0.0;
   if (mine) {
     s0 = s1 = 0.0;
-    for (int w = 0; w < NT / 32; ++w) { s0 += red[0][w]; s1 += red[1][w]; }
-    const double F = z0_finish<0>(p, s0, kscale), Fc = z0_finish<0>(p, s1, kscale);
-    float t0, t2;
-    work_entry_d(p, wtab, cx, cy, &t0, &t2);
-    cs.fF[k] = (float)Fc;
-    cs.fe[k] = 1.2e-7f * fabsf((float)Fc);
-    cs.fsup[k] = rho_entry_f(p, t0, t2, (float)Fc);
+    for (int w = 0; w < NT / 32; ++w) { s0 += s->t[0][w]; s1 += s->t[1][w]; }
+    const double v = 1.12e-16 * (n / NT + 208), E = fabs(p.E_z);
+    const bool exact = cs.fe[k] == 0.0f;
+    const double F = z0_finish<0>(p, s0, kscale), Fc = exact ? cs.F[k] : z0_finish<0>(p, s1, kscale);
+    const double en = v * (fabs(F) + 2.0 * E), ec = exact ? 0.0 : v * (fabs(Fc) + 2.0 * E);   // |S| <= |F| + |E|
+    double u1, u2;
+    rng2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, &u1, &u2);
+    lu = log(u1);
+    int take = F > en ? 0 : -1;
+    if (F < 0.0 && Fc < 0.0 && 4.0 * en <= -F && 4.0 * ec <= -Fc) {
+      const double sc = exact ? cs.sup[k] : supply_log_xy(p, wtab, cx, cy, Fc);
+      const double d = (supply_log_xy(p, wtab, px, py, F) - sc) - lu;
+      const double eps = 2.5 * (en / -F + ec / -Fc) + 1.0e-11;   // take iff d >= 0 (log u <= 0)
+      take = d > eps ? 1 : d < -eps ? 0 : -1;
+    }
+    if (!exact) {
+      work_entry_d(p, wtab, cx, cy, &t0, &t2);
+      cs.fF[k] = (float)Fc;
+      cs.fe[k] = 1.2e-7f * fabsf((float)Fc);
+      cs.fsup[k] = rho_entry_f(p, t0, t2, (float)Fc);
+    }
+    if (take == 1) {
+      work_entry_d(p, wtab, px, py, &t0, &t2);
+      cs.x[k] = px; cs.y[k] = py;
+      cs.fF[k] = (float)F;
+      cs.fe[k] = 1.2e-7f * fabsf((float)F);
+      cs.fsup[k] = rho_entry_f(p, t0, t2, (float)F);
+      a = 1;
+    }
+    s->still = take < 0;
+  }
+  __syncthreads();
+  const int still = s->still;
+  __syncthreads();   // (read before the next call writes it)
+  if (!still) return a;   // block-uniform
+  near_exact64<NT>(p, pool, e, px, py, cx, cy, s);
+  if (mine) {
+    if (cs.fe[k] != 0.0f) {   // the chain's field was an estimate
+      const double Fc = z0_finish<0>(p, s->out[1], kscale);
+      cs.F[k] = Fc;
+      cs.sup[k] = supply_log_xy(p, wtab, cx, cy, Fc);
+      cs.fF[k] = (float)Fc;
+      cs.fe[k] = 0.0f;
+    }
+    const double F = z0_finish<0>(p, s->out[0], kscale);
     if (F < 0.0) {
-      const double sn = supply_log_xy(p, wtab, px, py, F), sc = supply_log_xy(p, wtab, cx, cy, Fc);
-      bool take = sn >= sc;
-      if (!take) {
-        double u1, u2;
-        rng2(p.seed, (uint32_t)c, (uint32_t)it_idx, step, RNG_ACCEPT, &u1, &u2);
-        take = log(u1) <= sn - sc;
-      }
-      if (take) {
+      const double sn = supply_log_xy(p, wtab, px, py, F), sc = cs.sup[k];
+      if (sn >= sc || lu <= sn - sc) {
         work_entry_d(p, wtab, px, py, &t0, &t2);
         cs.x[k] = px; cs.y[k] = py;
+        cs.F[k] = F; cs.sup[k] = sn;
         cs.fF[k] = (float)F;
-        cs.fe[k] = 1.2e-7f * fabsf((float)F);
+        cs.fe[k] = 0.0f;
         cs.fsup[k] = rho_entry_f(p, t0, t2, (float)F);
         a = 1;
       }
@@ -728,7 +809,7 @@ struct NearShared {
   Real ox[32], oy[32], cx[32], cy[32];    // proposals and chains' points, where a jump is left open
   unsigned open;
   int dead;
-  typename std::conditional<PREC == 1, NearExact<32 * NW>, double[2][NW]>::type ex;
+  typename std::conditional<PREC == 1, NearExact<32 * NW>, NearExact64<32 * NW>>::type ex;
 };
 
 template <int PREC>
@@ -971,7 +1052,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
                              sh.cx[q], sh.cy[q], sh.lu[q], &sh.ex);
         else
           a += near_open64<NT>(p, pool, cs, wtab, plan_mh[d], kscale, tid == q, c, k, it, step, sh.ox[q], sh.oy[q],
-                               sh.cx[q], sh.cy[q], sh.ex);
+                               sh.cx[q], sh.cy[q], &sh.ex);
         if (ONE && tid == q) { fx = ax[k]; fy = ay[k]; Fc = cs.fF[k]; rc = cs.fsup[k]; fe = cs.fe[k]; }
       }
       if (w == 0) {
