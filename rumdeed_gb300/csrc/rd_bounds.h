@@ -27,3 +27,18 @@ RD_HD float rd_near_node_factor(int cnt) { return 1.0f + (float)cnt * (1.0f / (2
 
 // Direct sums over all n electrons by nt threads, runs of eight terms (near_open).
 RD_HD float rd_near_direct_units(int n, int nt) { return RD_NEAR_UNITS + (float)n / (float)(8 * nt); }
+
+// Guard of a decision from FP32 targets (near_decide): how far
+//   df = 2 log(F_n / F_c) - (rho_n - rho_c)  and  log u
+// as FP32 forms them can lie from what the same fields give in FP64, S the sum of
+// their magnitudes.  With e = 2^-24, logf and log1pf within 1 ulp (2e of the result):
+//   the fields rounded to floats 4e, their quotient 2e, its logarithm 2e |2 log|;
+//   each rho 1.95e + 2e |rho| (mh_guard has the terms);
+//   at a tip rho also has -1/2 log v, v = xi^2 - eta^2: v rounded 0.5e, its logarithm
+//   e |log v|, and log phi rounded (the same in both) and the sum e |rho| more;
+//   log u 2.01e + 2e |log u|, three sums rounded.
+// Planar: 12.2e + 5e S.  A tip adds 1.5e + e (|log v_n| + |log v_c|) + e S, and
+// |log v| / 2 <= |rho| + 2.3 (phi below 8 eV): 23e + 8e S at most.  The guard is a quarter
+// above that, twice the planar value.  (With a tenth above the planar value a step of
+// 10,000 electrons at a tip took 3.11 ms, so 3.15; planar steps 0 to 0.5 % more.)
+RD_HD float rd_near_guard(float S) { return 1.7e-6f + 6.6e-7f * S; }

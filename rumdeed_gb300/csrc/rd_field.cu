@@ -382,7 +382,7 @@ __device__ __forceinline__ void near_start_d(const DiodeParams& p, const ChainSt
   work_entry_d(p, wtab, x, y, &t0, &t2);
   const float Ff = (float)F;
   cs.fF[k] = Ff;
-  cs.fe[k] = 0.0f;   // F is the pair sum's (its rounding to a float is in near_guard, as the FP32 chains')
+  cs.fe[k] = 0.0f;   // F is the pair sum's (its rounding to a float is in rd_near_guard, as the FP32 chains')
   cs.fsup[k] = rho_entry_f(p, t0, t2, Ff);
 }
 

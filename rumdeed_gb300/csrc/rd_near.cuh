@@ -34,7 +34,7 @@
 // node values carried through I (L(t_x) L(t_y) times theirs), and of this
 // kernel's own sums is bounded by multiples of u = 2^-24 times the sum of
 // magnitudes, which is |S| because every charge has one sign (diodes that hold
-// ions or atoms keep the pair-sum kernel).  nr_guard has the multiples.
+// ions or atoms keep the pair-sum kernel).  near_bound0 and rd_bounds.h have the multiples.
 //
 // Measured (GB300, jumps of one step, the split's set-up and last pass included):
 //   one diode, 4500 electrons, 3800 chains, 100 jumps      6.13 -> 0.67 ms
@@ -461,10 +461,6 @@ __device__ __forceinline__ void near_exact2(const float4* __restrict__ zhi, cons
   __syncthreads();
 }
 
-// The bound on mh_decide_f's FP32 evaluation (7.3e-7 + 3.0e-7 S, see mh_guard, which
-// takes ten times it) and a tenth more.
-__device__ __forceinline__ float near_guard(float S) { return 8.0e-7f + 3.3e-7f * S; }
-
 // The decision of mh_decide_f from estimated fields: the proposal's Fn within dF of
 // the pair sum's, the chain's Fc within fe; t0, t2 the proposal's work-function
 // entry, lu the accept test's log u.  The fields' errors widen the guard: each
@@ -479,8 +475,8 @@ __device__ __forceinline__ int near_decide(const DiodeParams& p, float Fn, float
   const float St = fabsf(l2) + fabsf(*rn) + fabsf(rc);
   const float eps = 2.5f * (dF / -Fn + fe / -Fc);
   if (!(isfinite(df) && isfinite(eps) && isfinite(lu))) return -1;
-  const float gd = near_guard(St + fabsf(lu)) + eps;
-  if (df >= near_guard(St) + eps || lu <= df - gd) return 1;
+  const float gd = rd_near_guard(St + fabsf(lu)) + eps;
+  if (df >= rd_near_guard(St) + eps || lu <= df - gd) return 1;
   return lu > df + gd ? 0 : -1;
 }
 

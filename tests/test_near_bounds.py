@@ -1,6 +1,8 @@
 """The rounding bounds of the planar near / far split (rumdeed_gb300/csrc/rd_bounds.h)
 hold for near lists of any length: sums of up to a million terms in the kernels' order,
-with terms whose roundings agree.  Compiled for the host with g++."""
+with terms whose roundings agree.  And the guard of its decisions from FP32 targets holds
+with every logarithm an ulp off either way, at a tip with parts that cancel too.  Compiled
+for the host with g++."""
 import os
 import shutil
 import subprocess
