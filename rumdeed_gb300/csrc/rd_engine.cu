@@ -234,6 +234,11 @@ struct SlotHost {
   long long q_off = 0, q_len = 0;
   long long w_off = 0, w_len = 0;
   unsigned char* tn_mem = nullptr;   // the tip's panels, lists and expansions (rd_tipnear.cuh)
+  // Route of the MH jumps (settle_split): whether the diode can take the near / far split
+  // at all, and what keeps it on the pair sums.
+  bool near_ok = false, tip_ok = false;
+  bool foreign = false;   // it holds, or has held, ions or atoms
+  bool marked = false;    // electrons may be marked for removal and not yet removed (charge 0)
 };
 
 struct rd_engine {
@@ -1207,15 +1212,29 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
   return ce;
 }
 
-// A diode that holds anything but electrons keeps the pair-sum jumps from now on.
-static int keep_pair_sum(rd_engine* e, int d) {
-  DiodeParams& p = e->slots[d].p;
-  if (!p.mh_fast && !p.tn) return RD_OK;
-  p.mh_fast = p.tn = 0;
-  e->act_P[d].mh_fast = e->act_P[d].tn = 0;
-  CK(cudaMemcpyAsync(e->dP + d, &e->act_P[d], sizeof(DiodeParams), cudaMemcpyHostToDevice, e->st));
-  CK(cudaStreamSynchronize(e->st));
+// The jumps' route of every diode, before an emission: the near / far split where the
+// diode can take it and nothing it holds stands against it.  Ions and atoms do, for good;
+// at a tip also electrons whose charge a removal mark has set to 0, until they are
+// removed (the split of rd_tipnear.cuh would leave every jump open).
+static int settle_split(rd_engine* e) {
+  bool moved = false;
+  for (size_t d = 0; d < e->slots.size(); ++d) {
+    SlotHost& sl = e->slots[d];
+    if (!sl.used) continue;
+    const int near = sl.near_ok && !sl.foreign, tip = sl.tip_ok && !sl.foreign && !sl.marked;
+    if (sl.p.mh_fast == near && sl.p.tn == tip) continue;
+    sl.p.mh_fast = e->act_P[d].mh_fast = near;
+    sl.p.tn = e->act_P[d].tn = tip;
+    CK(cudaMemcpyAsync(e->dP + d, &e->act_P[d], sizeof(DiodeParams), cudaMemcpyHostToDevice, e->st));
+    moved = true;
+  }
+  if (moved) CK(cudaStreamSynchronize(e->st));
   return RD_OK;
+}
+
+// A removal has taken the marked electrons.
+static void marks_gone(rd_engine* e) {
+  for (auto& sl : e->slots) sl.marked = false;
 }
 
 // rd_diode_add on stream `us`.  deferred: the slot is written inactive and
@@ -1403,6 +1422,8 @@ static int diode_add_impl(rd_engine* e, const rd_diode_config* c, int* diode, cu
   else CK(cudaStreamSynchronize(us));
   sl.used = true;
   sl.p = p;
+  sl.near_ok = p.mh_fast;
+  sl.tip_ok = p.tn;
   e->slots[s] = sl;
   *diode = s;
   return RD_OK;
@@ -1466,9 +1487,8 @@ int rd_add_particles(rd_engine* e, int d, int n, const double* pos, const double
   if (n < 0 || (n > 0 && !pos)) return fail(RD_ERR_INVALID, "bad particle arrays");
   int rc = stage(e, 6LL * n, n);
   if (rc) return rc;
-  if (species && std::any_of(species, species + n, [](int s) { return s != RD_SPECIES_ELEC; }) &&
-      (rc = keep_pair_sum(e, d)))
-    return rc;
+  if (species && std::any_of(species, species + n, [](int s) { return s != RD_SPECIES_ELEC; }))
+    e->slots[d].foreign = true;
   if (n > 0) {
     // the previous upload from the pinned stage has completed (every call ends with a
     // stream synchronize), so the stage can be refilled
@@ -1693,6 +1713,7 @@ int rd_time_remove(rd_engine* e, double* position_ms, double* remove_ms, long lo
   CK(cudaEventRecord(e->ev1, e->st));
   CK(cudaEventSynchronize(e->ev1));
   CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+  marks_gone(e);
   *remove_ms = ms;
   return compaction_check(e);
 }
@@ -1798,7 +1819,7 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   out->chunk_count_max = e->nch_max;
   if (e->nslots_hw() == 0) return RD_OK;
   int rc = repack(e);
-  if (rc) return rc;
+  if (rc || (rc = settle_split(e))) return rc;
   // the force passes overwrite the current accelerations: keep them in the compaction pool
   const size_t bytes = sizeof(double) * (size_t)e->cfg.particle_capacity;
   CK(cudaMemcpyAsync(e->save_ax, e->pool.ax, bytes, cudaMemcpyDeviceToDevice, e->st));
@@ -1932,6 +1953,7 @@ int rd_mark_remove(rd_engine* e, int d, int i, int why) {
   if (why != RD_REMOVE_TOP && why != RD_REMOVE_BOT) return fail(RD_ERR_INVALID, "unknown removal flag");
   CK(rd_launch_mark(e->st, e->dP, e->dD, e->pool, d, i, why));
   CK(cudaStreamSynchronize(e->st));
+  e->slots[d].marked = true;
   return RD_OK;
 }
 
@@ -1940,8 +1962,8 @@ int rd_do_emission(rd_engine* e, int step) {
   NvtxRange nvtx_range("rd_do_emission");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   CK(rd_launch_step_set(e->st, e->d_step, step));
-  int rc = fresh_packs(e);   // of an emission just before this one
-  if (rc) return rc;
+  int rc = settle_split(e);
+  if (rc || (rc = fresh_packs(e))) return rc;   // of an emission just before this one
   e->packs_stale = true;
   if ((rc = launch_emission(e))) return rc;
   CK(cudaStreamSynchronize(e->st));
@@ -1956,6 +1978,7 @@ int rd_update_position(rd_engine* e, int step) {
   int rc = launch_update_position(e);   // packs every particle
   if (rc) return rc;
   e->packs_stale = false;
+  for (auto& sl : e->slots) sl.marked = true;   // those that left their diode
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }
@@ -1967,6 +1990,7 @@ int rd_remove_particles(rd_engine* e, int step) {
   CK(rd_launch_step_set(e->st, e->d_step, step));
   int rc = launch_remove(e, false);
   if (rc) return rc;
+  marks_gone(e);
   CK(cudaStreamSynchronize(e->st));
   return compaction_check(e);
 }
@@ -1976,12 +2000,16 @@ int rd_run(rd_engine* e, int first_step, int nsteps) {
   NvtxRange nvtx_range("rd_run");
   if (!e) return fail(RD_ERR_INVALID, "null engine");
   if (nsteps < 0) return fail(RD_ERR_INVALID, "nsteps < 0");
-  int rc = ensure_graph(e);
-  if (rc) return rc;
+  int rc = settle_split(e);
+  if (rc || (rc = ensure_graph(e))) return rc;
   if (nsteps > 0 && (rc = fresh_packs(e))) return rc;   // of a lone emission before this step's
   CK(rd_launch_step_set(e->st, e->d_step, first_step));
   CK(cudaEventRecord(e->ev0, e->st));
-  for (int s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(e->graph, e->st));
+  for (int s = 0; s < nsteps; ++s) {
+    if (s == 1 && ((rc = settle_split(e)) || (rc = ensure_graph(e)))) return rc;   // what the first step's removal allows
+    CK(cudaGraphLaunch(e->graph, e->st));
+    if (s == 0) marks_gone(e);
+  }
   CK(cudaEventRecord(e->ev1, e->st));
   CK(cudaStreamSynchronize(e->st));
   float ms = 0.f;
@@ -2063,6 +2091,7 @@ struct StateHeader {
   int pad;
 };
 constexpr int kStateDoubles = 17;   // x y z vx vy vz, a, a_prev, a_prev2 (9), q, m
+constexpr int kChargeArray = 15;
 constexpr int kStateInts = 5;       // species id step0 section mask
 
 double* state_dbl(Pool& p, int k) {
@@ -2144,13 +2173,18 @@ int rd_diode_load(rd_engine* e, int d, const void* buf, long long size) {
   in += sizeof y;
   const char* ints = in + kStateDoubles * sizeof(double) * (size_t)h.n;
   const char* life = ints + kStateInts * sizeof(int) * (size_t)h.n;
-  int rc = RD_OK;   // species is the first of the integer arrays
-  for (int i = 0; i < h.n; ++i) {
-    int sp;
-    std::memcpy(&sp, ints + sizeof(int) * (size_t)i, sizeof sp);
-    if (sp != RD_SPECIES_ELEC) {
-      if ((rc = keep_pair_sum(e, d))) return rc;
-      break;
+  int rc = RD_OK;
+  SlotHost& sl = e->slots[d];
+  if (sl.near_ok || sl.tip_ok) {   // what the state means for the jumps' route (settle_split)
+    const char* charges = in + kChargeArray * sizeof(double) * (size_t)h.n;   // species is the first integer array
+    sl.marked = false;
+    for (int i = 0; i < h.n; ++i) {
+      int sp;
+      double q;
+      std::memcpy(&sp, ints + sizeof(int) * (size_t)i, sizeof sp);
+      std::memcpy(&q, charges + sizeof(double) * (size_t)i, sizeof q);
+      sl.foreign |= sp != RD_SPECIES_ELEC;
+      sl.marked |= q != -e->k.q0;
     }
   }
   const size_t row = kStateDoubles * sizeof(double) + kStateInts * sizeof(int);
@@ -2210,6 +2244,8 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   std::vector<DiodeDyn> dyn(S);
   int rc = fresh_packs(e);
   if (rc) return rc;
+  if ((rc = settle_split(e))) return rc;
+  s = signature(e);
   CK(rd_launch_step_set(e->st, e->d_step, step));
   CK(cudaEventRecord(ev[0], e->st));
   if (s.emit_planar || s.emit_tip) {
@@ -2280,6 +2316,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
   rc = launch_remove(e, true);
   if (rc) return rc;
+  marks_gone(e);
   CK(rd_launch_step_inc(e->st, e->d_step));
   CK(cudaEventRecord(ev[8], e->st));
   CK(cudaStreamSynchronize(e->st));
@@ -2422,10 +2459,11 @@ int rd_serve(rd_engine* e, int iterations, rd_serve_stats* out) {
     if (e->running.empty() && (rc = serve_admit(e, out, e->gstep))) return rc;
     if ((rc = activate_pending(e))) return rc;
     if (e->running.empty()) break;
-    if ((rc = ensure_graph(e)) || (rc = fresh_packs(e))) return rc;
+    if ((rc = settle_split(e)) || (rc = ensure_graph(e)) || (rc = fresh_packs(e))) return rc;
     CK(rd_launch_step_set(e->st, e->d_step, e->gstep));
     CK(cudaEventRecord(e->ev0, e->st));
     CK(cudaGraphLaunch(e->graph, e->st));
+    marks_gone(e);
     CK(cudaEventRecord(e->ev1, e->st));
     CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
     // while the step runs: admit queued requests into the slots free now, for the next step
