@@ -239,6 +239,7 @@ struct SlotHost {
   bool near_ok = false, tip_ok = false;
   bool foreign = false;   // it holds, or has held, ions or atoms
   bool marked = false;    // electrons may be marked for removal and not yet removed (charge 0)
+  bool misplaced = false; // electrons where the split's bounds do not hold (electron_misplaced)
 };
 
 struct rd_engine {
@@ -1215,13 +1216,15 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
 // The jumps' route of every diode, before an emission: the near / far split where the
 // diode can take it and nothing it holds stands against it.  Ions and atoms do, for good;
 // at a tip also electrons whose charge a removal mark has set to 0, until they are
-// removed (the split of rd_tipnear.cuh would leave every jump open).
+// removed (the split of rd_tipnear.cuh would leave every jump open); and electrons that a
+// caller put where no emitted one gets, until a position update has marked them.
 static int settle_split(rd_engine* e) {
   bool moved = false;
   for (size_t d = 0; d < e->slots.size(); ++d) {
     SlotHost& sl = e->slots[d];
     if (!sl.used) continue;
-    const int near = sl.near_ok && !sl.foreign, tip = sl.tip_ok && !sl.foreign && !sl.marked;
+    const int near = sl.near_ok && !sl.foreign && !sl.misplaced;
+    const int tip = sl.tip_ok && !sl.foreign && !sl.misplaced && !sl.marked;
     if (sl.p.mh_fast == near && sl.p.tn == tip) continue;
     sl.p.mh_fast = e->act_P[d].mh_fast = near;
     sl.p.tn = e->act_P[d].tn = tip;
@@ -1232,9 +1235,43 @@ static int settle_split(rd_engine* e) {
   return RD_OK;
 }
 
+// A position update has marked every electron that lies outside its diode.
+static void electrons_moved(rd_engine* e) {
+  for (auto& sl : e->slots) { sl.marked = true; sl.misplaced = false; }
+}
 // A removal has taken the marked electrons.
 static void marks_gone(rd_engine* e) {
   for (auto& sl : e->slots) sl.marked = false;
+}
+// A whole step has done both.
+static void step_done(rd_engine* e) {
+  electrons_moved(e);
+  marks_gone(e);
+}
+
+// Whether one of n electrons lies where the bounds of the diode's near / far split do not
+// hold: below the cathode, where its term has the other sign (rd_near.cuh takes |S| for the
+// sum of magnitudes), or inside the tip's apex sphere, whose image then lies outside.
+// Coordinates `stride` bytes apart, at any alignment.
+static bool electron_misplaced(const SlotHost& sl, int n, const void* x, const void* y, const void* z,
+                               size_t stride) {
+  auto at = [stride](const void* a, int i) {
+    double v;
+    std::memcpy(&v, (const char*)a + stride * (size_t)i, sizeof v);
+    return v;
+  };
+  const DiodeParams& p = sl.p;
+  int bad = 0;
+  if (sl.tip_ok) {
+    const double zc = p.h_tip - p.r_tip, R2 = p.r_tip * p.r_tip;
+    for (int i = 0; i < n; ++i) {
+      const double a = at(x, i), b = at(y, i), c = at(z, i) - zc;
+      bad |= !(a * a + b * b + c * c > R2);
+    }
+  } else if (sl.near_ok) {
+    for (int i = 0; i < n; ++i) bad |= !(at(z, i) >= 0.0);
+  }
+  return bad != 0;
 }
 
 // rd_diode_add on stream `us`.  deferred: the slot is written inactive and
@@ -1489,6 +1526,7 @@ int rd_add_particles(rd_engine* e, int d, int n, const double* pos, const double
   if (rc) return rc;
   if (species && std::any_of(species, species + n, [](int s) { return s != RD_SPECIES_ELEC; }))
     e->slots[d].foreign = true;
+  e->slots[d].misplaced |= electron_misplaced(e->slots[d], n, pos, pos + 1, pos + 2, 3 * sizeof(double));
   if (n > 0) {
     // the previous upload from the pinned stage has completed (every call ends with a
     // stream synchronize), so the stage can be refilled
@@ -1559,6 +1597,7 @@ int rd_set_particles(rd_engine* e, int d, int n, const double* pos, const double
   if (rc) return rc;
   if (n < 0 || n > y.n) return fail(RD_ERR_INVALID, "n exceeds the particles in flight");
   const int off = e->slots[d].p.off;
+  if (pos) e->slots[d].misplaced |= electron_misplaced(e->slots[d], n, pos, pos + 1, pos + 2, 3 * sizeof(double));
   std::vector<double> buf(std::max(n, 1));
   auto put3 = [&](const double* srcv, double* a, double* b, double* c2) -> int {
     double* dst[3] = {a, b, c2};
@@ -1978,7 +2017,7 @@ int rd_update_position(rd_engine* e, int step) {
   int rc = launch_update_position(e);   // packs every particle
   if (rc) return rc;
   e->packs_stale = false;
-  for (auto& sl : e->slots) sl.marked = true;   // those that left their diode
+  electrons_moved(e);
   CK(cudaStreamSynchronize(e->st));
   return RD_OK;
 }
@@ -2008,7 +2047,7 @@ int rd_run(rd_engine* e, int first_step, int nsteps) {
   for (int s = 0; s < nsteps; ++s) {
     if (s == 1 && ((rc = settle_split(e)) || (rc = ensure_graph(e)))) return rc;   // what the first step's removal allows
     CK(cudaGraphLaunch(e->graph, e->st));
-    if (s == 0) marks_gone(e);
+    if (s == 0) step_done(e);
   }
   CK(cudaEventRecord(e->ev1, e->st));
   CK(cudaStreamSynchronize(e->st));
@@ -2178,6 +2217,8 @@ int rd_diode_load(rd_engine* e, int d, const void* buf, long long size) {
   if (sl.near_ok || sl.tip_ok) {   // what the state means for the jumps' route (settle_split)
     const char* charges = in + kChargeArray * sizeof(double) * (size_t)h.n;   // species is the first integer array
     sl.marked = false;
+    const size_t column = sizeof(double) * (size_t)h.n;
+    sl.misplaced = electron_misplaced(sl, h.n, in, in + column, in + 2 * column, sizeof(double));
     for (int i = 0; i < h.n; ++i) {
       int sp;
       double q;
@@ -2316,7 +2357,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
   rc = launch_remove(e, true);
   if (rc) return rc;
-  marks_gone(e);
+  step_done(e);
   CK(rd_launch_step_inc(e->st, e->d_step));
   CK(cudaEventRecord(ev[8], e->st));
   CK(cudaStreamSynchronize(e->st));
@@ -2427,6 +2468,8 @@ static int serve_admit(rd_engine* e, rd_serve_stats* st, int first_step) {
     // the slot exists on the host now; its device slot stays inactive until activation
     e->slots[slot].used = true;
     const int n = (int)(r.pos.size() / 3);
+    SlotHost& sl = e->slots[slot];
+    sl.misplaced = electron_misplaced(sl, n, r.pos.data(), r.pos.data() + 1, r.pos.data() + 2, 3 * sizeof(double));
     if (n > 0 || true) {
       rc = add_particles_deferred(e, slot, n, r.pos.data(), r.vel.empty() ? nullptr : r.vel.data(), 0, 1);
       if (rc) return rc;
@@ -2463,7 +2506,7 @@ int rd_serve(rd_engine* e, int iterations, rd_serve_stats* out) {
     CK(rd_launch_step_set(e->st, e->d_step, e->gstep));
     CK(cudaEventRecord(e->ev0, e->st));
     CK(cudaGraphLaunch(e->graph, e->st));
-    marks_gone(e);
+    step_done(e);
     CK(cudaEventRecord(e->ev1, e->st));
     CK(cudaMemcpyAsync(dyn.data(), e->dD, sizeof(DiodeDyn) * S, cudaMemcpyDeviceToHost, e->st));
     // while the step runs: admit queued requests into the slots free now, for the next step
