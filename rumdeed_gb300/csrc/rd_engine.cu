@@ -237,7 +237,7 @@ struct SlotHost {
   // Route of the MH jumps (settle_split): whether the diode can take the near / far split
   // at all, and what keeps it on the pair sums.
   bool near_ok = false, tip_ok = false;
-  bool foreign = false;   // it holds, or has held, ions or atoms
+  bool foreign = false;   // it holds, or has held since its last checkpoint was loaded, ions or atoms
   bool marked = false;    // electrons may be marked for removal and not yet removed (charge 0)
   bool misplaced = false; // electrons where the split's bounds do not hold (electron_misplaced)
 };
@@ -1214,8 +1214,8 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
 }
 
 // The jumps' route of every diode, before an emission: the near / far split where the
-// diode can take it and nothing it holds stands against it.  Ions and atoms do, for good;
-// at a tip also electrons whose charge a removal mark has set to 0, until they are
+// diode can take it and nothing it holds stands against it.  Ions and atoms do, until a
+// checkpoint without them replaces the state; at a tip also electrons whose charge a removal mark has set to 0, until they are
 // removed (the split of rd_tipnear.cuh would leave every jump open); and electrons that a
 // caller put where no emitted one gets, until a position update has marked them.
 static int settle_split(rd_engine* e) {
@@ -2216,7 +2216,7 @@ int rd_diode_load(rd_engine* e, int d, const void* buf, long long size) {
   SlotHost& sl = e->slots[d];
   if (sl.near_ok || sl.tip_ok) {   // what the state means for the jumps' route (settle_split)
     const char* charges = in + kChargeArray * sizeof(double) * (size_t)h.n;   // species is the first integer array
-    sl.marked = false;
+    sl.marked = sl.foreign = false;
     const size_t column = sizeof(double) * (size_t)h.n;
     sl.misplaced = electron_misplaced(sl, h.n, in, in + column, in + 2 * column, sizeof(double));
     for (int i = 0; i < h.n; ++i) {
