@@ -2298,7 +2298,9 @@ k_emit(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool, 
 // Thread 0 gets the pair sum of F_z at one cathode point over the diode's first n
 // particles (before z0_finish).  FP32: every thread's share in particle order as a
 // float pair, the pairs added over the block (pair_add, ~44 bits; FP64 additions take
-// some hundred clocks each here); FP64: the shares' tree in FP64.
+// some hundred clocks each here), which decides a jump where 1e-10 of the field is
+// enough.  Where it is not, and for the field that the emission test reads, the shares
+// are added in FP64 (serial_tree_sum, serial_tree_warp).  FP64: the shares' tree in FP64.
 struct SerialSum {
   float h, l;   // FP32
   double s;     // FP64
@@ -2307,6 +2309,37 @@ template <int PREC>
 __device__ __forceinline__ double serial_value(const SerialSum& v) {
   return PREC == 1 ? (double)v.h + (double)v.l : v.s;
 }
+// The FP64 tree over 256 shares by one warp: lane l has those of threads l + 32 k.
+__device__ __forceinline__ double serial_tree(double* v) {
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int k = 0; k < h; ++k) v[k] += v[k + h];
+  for (int h = 16; h > 0; h >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], h);
+  return v[0];
+}
+
+// Thread tid's share of the FP32 sum: every 256th particle in order, as a float pair.
+__device__ __forceinline__ void serial_share(const DiodeParams& p, const Pool& pool, int n, float4 pp, int tid, float* hi,
+                                             float* lo) {
+  const int nic = p.image_charge ? p.N_ic_max : 0;
+  const float dnm = (float)(p.d * 1.0e9);
+  *hi = *lo = 0.0f;
+  for (int j0 = tid; j0 < n; j0 += 256 * 4) {   // four particles' loads in flight
+    float4 h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = min(j0 + 256 * q, n - 1);
+      h[q] = pool.zk_hi[p.off + j];
+      l[q] = pool.zk_lo[p.off + j];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j0 + 256 * q < n)
+        two_sum_acc(*hi, *lo, nic == 0 ? z0_tile_f32<true>(&h[q], &l[q], 1, pp, 0, dnm)
+                                       : z0_tile_f32<false>(&h[q], &l[q], 1, pp, nic, dnm));
+  }
+}
 template <int PREC>
 __device__ __forceinline__ SerialSum serial_field_sum(const DiodeParams& p, const Pool& pool, int n, double px,
                                                       double py, float4 pp, float2* red_f, double* red_d) {
@@ -2314,22 +2347,8 @@ __device__ __forceinline__ SerialSum serial_field_sum(const DiodeParams& p, cons
   const int nic = p.image_charge ? p.N_ic_max : 0;
   SerialSum r = {0.0f, 0.0f, 0.0};
   if (PREC == 1) {
-    const float dnm = (float)(p.d * 1.0e9);
-    float hi = 0.f, lo = 0.f;
-    for (int j0 = tid; j0 < n; j0 += 256 * 4) {   // four particles' loads in flight
-      float4 h[4], l[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = min(j0 + 256 * q, n - 1);
-        h[q] = pool.zk_hi[off + j];
-        l[q] = pool.zk_lo[off + j];
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (j0 + 256 * q < n)
-          two_sum_acc(hi, lo, nic == 0 ? z0_tile_f32<true>(&h[q], &l[q], 1, pp, 0, dnm)
-                                       : z0_tile_f32<false>(&h[q], &l[q], 1, pp, nic, dnm));
-    }
+    float hi, lo;
+    serial_share(p, pool, n, pp, tid, &hi, &lo);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
       pair_add(hi, lo, __shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, lo, o));
@@ -2355,15 +2374,38 @@ __device__ __forceinline__ SerialSum serial_field_sum(const DiodeParams& p, cons
       double v[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = red_d[tid + 32 * k];
-#pragma unroll
-      for (int h = 4; h > 0; h >>= 1)
-#pragma unroll
-        for (int k = 0; k < h; ++k) v[k] += v[k + h];
-      for (int h = 16; h > 0; h >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], h);
+      v[0] = serial_tree(v);
       r.s = v[0];
     }
   }
   return r;
+}
+
+// The same FP32 sum with an FP64 tree over the shares, for thread 0: the value that the
+// emission test reads.
+__device__ __forceinline__ double serial_tree_sum(const DiodeParams& p, const Pool& pool, int n, float4 pp, double* red_d) {
+  const int tid = threadIdx.x;
+  float hi, lo;
+  serial_share(p, pool, n, pp, tid, &hi, &lo);
+  red_d[tid] = (double)hi + (double)lo;
+  __syncthreads();
+  double v[8] = {0.0};
+  if (tid < 32) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = red_d[tid + 32 * k];
+    v[0] = serial_tree(v);
+  }
+  return v[0];
+}
+// The same by warp 0 alone (lane 0 gets it), for a decision that the float pairs leave open.
+__device__ __noinline__ double serial_tree_warp(const DiodeParams& p, const Pool& pool, int n, float4 pp) {
+  double v[8];
+  for (int k = 0; k < 8; ++k) {
+    float hi, lo;
+    serial_share(p, pool, n, pp, (threadIdx.x & 31) + 32 * k, &hi, &lo);
+    v[k] = (double)hi + (double)lo;
+  }
+  return serial_tree(v);
 }
 
 // x > y for finite doubles by their bits (an FP64 comparison waits for the FP64 pipe)
@@ -2431,6 +2473,18 @@ __device__ __noinline__ bool serial_take_fp64(const DiodeParams& p, const double
   const double sn = supply_log_xy(p, wtab, wx, wy, F) + ln, sc = supply_log_xy(p, wtab, cx, cy, Fc) + lc;
   return sn >= sc || lu <= sn - sc;
 }
+// The same from fields that are within 1e-10 of |F| and the vacuum field (float pairs):
+// -1 where that leaves the answer open.
+__device__ __noinline__ int serial_take_pairs(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
+                                              double F, double ln, double cx, double cy, double Fc, double lc,
+                                              double lu) {
+  const double E2 = 2.0 * fabs(p.E_z), en = 1.0e-10 * (fabs(F) + E2), ec = 1.0e-10 * (fabs(Fc) + E2);
+  if (F > en) return 0;
+  if (!(F < 0.0 && Fc < 0.0 && 4.0 * en <= -F && 4.0 * ec <= -Fc)) return -1;
+  const double d = ((supply_log_xy(p, wtab, wx, wy, F) + ln) - (supply_log_xy(p, wtab, cx, cy, Fc) + lc)) - lu;
+  const double eps = 2.5 * (en / -F + ec / -Fc) + 1.0e-11;   // take iff d >= 0 (log u <= 0)
+  return d > eps ? 1 : d < -eps ? 0 : -1;
+}
 __device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
                                             double F, double cx, double cy, double Fc, double lu) {
   if (p.work_model != 2) {
@@ -2470,15 +2524,15 @@ __device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* 
 // proposal is known up to the last jump's answer, so lanes 0 to 2 of warp 0 take jump i
 // and jump i + 1 from either point, the block sums the field at all three, and one
 // comparison each answers both.  33 chains of 100 jumps over 400 electrons: 25.9 ->
-// 6.7 ms one at a time, 5.1 ms so (7.8 -> 2.0 -> 1.6 us a jump); over 4000 electrons 9.3
-// -> 6.9 ms (30 chains).
+// 6.7 ms one at a time, 5.1 ms so (7.8 -> 2.0 -> 1.6 us a jump), 5.2 with the FP64 sums at
+// a chain's two ends; over 4000 electrons 9.3 -> 6.9 ms (30 chains).
 #define RD_SER_DRAWS 256
 template <int PREC>
 __global__ void __launch_bounds__(256, 1)
 k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool pool,
             const double* __restrict__ work, const double* __restrict__ wtab,
             const int* __restrict__ step_ptr, double kscale, EventLog ev) {
-  __shared__ double red_d[PREC == 1 ? 1 : 256];
+  __shared__ double red_d[256];
   __shared__ float2 red_f[8];
   __shared__ double s_g[RD_SER_DRAWS][2], s_lu[RD_SER_DRAWS];   // Gaussian pairs and log u of the next jumps
   __shared__ float s_luf[RD_SER_DRAWS];
@@ -2490,6 +2544,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
   __shared__ float2 red_f3[3][8];
   __shared__ int s_sum[2];        // the block sums a field this jump (a ring proposal off the ring: no)
   __shared__ int s_found, s_add, s_stop;   // the chain started; a particle was added; the chains stop
+  __shared__ int s_moved;   // the chain has left its start
   __shared__ DiodeParams sp;   // thread 0's loads of it are on the jumps' path
   const int d = blockIdx.x;
   if (!P[d].active || !P[d].emission || !P[d].mh_serial || P[d].geometry != RD_G_PLANAR) return;
@@ -2525,6 +2580,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
     double ca = 0.0, cr = rmin;   // ring: (angle, radius) of the chain (Metropolis_Hastings_ring_J)
     bool found = false;
     SerialSum cur = {0.0f, 0.0f, 0.0};   // the sum at the chain's point
+    bool moved = false;   // (thread 0) the chain has left its start
     if (t0) s_found = 0;
     for (int r = 0; r < p.init_rounds; ++r) {
       if (t0) {
@@ -2543,9 +2599,11 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         if (PREC == 1) s_pp[0] = z0_point(p, cx, cy);
       }
       __syncthreads();
-      cur = serial_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], s_pp[0], red_f, red_d);
+      if constexpr (PREC == 1) cur.s = serial_tree_sum(p, pool, n, s_pp[0], red_d);
+      else cur = serial_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], s_pp[0], red_f, red_d);
       if (t0) {
-        F = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+        if (PREC == 1) { cur.h = (float)cur.s; cur.l = (float)(cur.s - (double)cur.h); }
+        F = z0_finish<PREC>(p, cur.s, kscale);
         found = F < 0.0;
         s_found = found;
       }
@@ -2645,11 +2703,17 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
                   const SerialSum sum = {wh, wl, 0.0};
                   const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
                   const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
-                  tk = Fw < 0.0 && serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
+                  tk = serial_take_pairs(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
                 }
                 tk = __shfl_sync(0xffffffffu, tk, 0);
               }
-              if (tk) { cx = wx; cy = wy; cur.h = wh; cur.l = wl; Fc = wF; fe = wd; rc = wr; }
+              if (tk < 0) {   // (about one jump in 10^9)
+                const double Fw = z0_finish<PREC>(p, serial_tree_warp(p, pool, n, z0_point(p, wx, wy)), kscale);
+                const double Fd = z0_finish<PREC>(p, serial_tree_warp(p, pool, n, z0_point(p, cx, cy)), kscale);
+                if (t0) tk = Fw < 0.0 && serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
+                tk = __shfl_sync(0xffffffffu, tk, 0);
+              }
+              if (tk) { cx = wx; cy = wy; cur.h = wh; cur.l = wl; Fc = wF; fe = wd; rc = wr; moved = true; }
               if (i + j > ndim_first) { if (tk) ++ja; else ++jr; }
               return tk;
             };
@@ -2685,11 +2749,11 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
       __syncthreads();
       if (!s_sum[i & 1]) continue;   // block-uniform: a ring proposal off the ring, no field needed
       const SerialSum sum = serial_field_sum<PREC>(p, pool, n, s_pt[i & 1][0], s_pt[i & 1][1], s_pp[i & 1], red_f, red_d);
+      int take = -1;
+      float Fn = 0.0f, dF = 0.0f, rn = 0.0f;
       if (t0) {
         // ring: log(radius) is the Jacobian of the (angle, radius) parametrisation (:1592-1596)
         const double lu = s_lu[draw];
-        int take = -1;
-        float Fn = 0.0f, dF = 0.0f, rn = 0.0f;
         if (est) {
           float te = t0e, ue = t2e;
           if (!one_cell) {
@@ -2704,25 +2768,49 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         if (take < 0) {   // the FP64 targets
           const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
           const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
-          if (Fw >= 0.0) take = 0;
+          if (PREC == 1) {
+            take = serial_take_pairs(p, wtab, wx, wy, Fw, ring ? log(nr) : 0.0, cx, cy, Fd, ring ? log(cr) : 0.0, lu);
+          } else if (Fw >= 0.0) take = 0;
           else if (ring) take = serial_take_fp64(p, wtab, wx, wy, Fw, log(nr), cx, cy, Fd, log(cr), lu);
-          else if (PREC == 0) take = serial_take(p, wtab, wx, wy, Fw, cx, cy, Fd, lu);
-          else take = serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, lu);
+          else take = serial_take(p, wtab, wx, wy, Fw, cx, cy, Fd, lu);
           if (est) {
             const double* e = wtab + 3 * (p.work_off + work_cell(p, wx, wy));
             rn = rho_entry_f(p, (float)e[0], (float)e[2], Fn);
           }
         }
+      }
+      if (PREC == 1 && threadIdx.x < 32 && __shfl_sync(0xffffffffu, take, 0) < 0) {
+        const double x = __shfl_sync(0xffffffffu, wx, 0), y2 = __shfl_sync(0xffffffffu, wy, 0);
+        const double bx = __shfl_sync(0xffffffffu, cx, 0), by = __shfl_sync(0xffffffffu, cy, 0);
+        const double Fw = z0_finish<PREC>(p, serial_tree_warp(p, pool, n, z0_point(p, x, y2)), kscale);
+        const double Fd = z0_finish<PREC>(p, serial_tree_warp(p, pool, n, z0_point(p, bx, by)), kscale);
+        if (t0)
+          take = Fw < 0.0 && serial_take_fp64(p, wtab, wx, wy, Fw, ring ? log(nr) : 0.0, cx, cy, Fd,
+                                              ring ? log(cr) : 0.0, s_lu[draw]);
+      }
+      if (t0) {
         if (take) {
           cx = wx; cy = wy; cur = sum; ca = na; cr = nr;
           Fc = Fn; fe = dF; rc = rn;
+          moved = true;
           if (i > ndim_first) ++ja;
         } else if (i > ndim_first) {
           ++jr;
         }
       }
     }
-    if (t0 && found) Fout = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+    if (t0 && found) Fout = PREC == 1 ? F : z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+    if constexpr (PREC == 1) {   // the field at the chain's last point
+      if (t0) {
+        s_pp[0] = z0_point(p, cx, cy);
+        s_moved = moved;
+      }
+      __syncthreads();
+      if (s_moved) {   // block-uniform
+        const double sum = serial_tree_sum(p, pool, n, s_pp[0], red_d);
+        if (t0) Fout = z0_finish<PREC>(p, sum, kscale);
+      }
+    }
     // the chain's end: MH_std, the escape test and its electron (thread 0)
     if (t0) {
       s_add = 0;
