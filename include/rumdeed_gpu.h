@@ -198,9 +198,11 @@ int rd_mark_remove(rd_engine* e, int diode, int index, int why);
  * number of polls, until the earlier tiles it overwrites have read their
  * particles.  Those waits always end in a working run; if one ever gave up,
  * rd_remove_particles, rd_run, rd_serve, rd_profile_step and rd_time_remove
- * return RD_ERR_STATE, and the particle state is no longer valid.  The same holds for
- * the Metropolis-Hastings jumps, whose blocks wait (bounded) for one another's
- * acceptance counts: rd_do_emission and the calls above return RD_ERR_STATE. */
+ * return RD_ERR_STATE from then on: the particle state is no longer valid and the
+ * engine has to be destroyed.  The blocks of the Metropolis-Hastings jumps wait
+ * (bounded) for one another's acceptance counts; if one of those waits gave up,
+ * rd_do_emission and the calls above return RD_ERR_STATE once.  That step's emission is
+ * not valid; a checkpoint loaded with rd_diode_load goes on as ever. */
 int rd_do_emission(rd_engine* e, int step);
 int rd_update_position(rd_engine* e, int step);
 int rd_remove_particles(rd_engine* e, int step);

@@ -723,12 +723,13 @@ static int launch_update_position(rd_engine* e) {
 
 // Waits of the in-place compaction (k_compact_move) that gave up: each is a
 // tile that stored nothing, so the particle state is no longer valid; and waits
-// of the Metropolis-Hastings jumps (k_mh_jumps_near).  Read after the engine stream
-// has drained.
+// of the Metropolis-Hastings jumps (k_mh_jumps_near), which are reported once: the next
+// emission starts afresh (near_reset).  Read after the engine stream has drained.
 static int compaction_check(rd_engine* e) {
   int gave_up[2] = {0, 0};
   CK(cudaMemcpyAsync(gave_up, e->cq + 2, sizeof gave_up, cudaMemcpyDeviceToHost, e->st));
   CK(cudaStreamSynchronize(e->st));
+  if (gave_up[1]) CK(cudaMemsetAsync(e->cq + 3, 0, sizeof(int), e->st));
   if (gave_up[1]) return fail(RD_ERR_STATE, "emission: a wait on a diode's last jump gave up; the chain state is not valid");
   if (gave_up[0]) return fail(RD_ERR_STATE, "compaction: a wait on an earlier tile gave up; the particle state is not valid");
   return RD_OK;

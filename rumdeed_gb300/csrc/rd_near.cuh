@@ -77,6 +77,13 @@ __device__ __forceinline__ unsigned long long near_progress(const DiodeParams& p
          ((unsigned)done | (mh_std == p.mh_hi ? RD_NEAR_CLAMPED : 0u));
 }
 
+// Before the first jump of a step: none done and none counted, also if a wait of the last
+// step gave up half way through a jump.
+__device__ __forceinline__ void near_reset(const DiodeParams& p, const NearState& nr, int d, double mh_std) {
+  nr.progress[d] = near_progress(p, 0, mh_std);
+  nr.count[d] = 0;
+}
+
 // Electrons into bins: each electron's bin and its rank among the bin's.
 __global__ void __launch_bounds__(256)
 k_near_count(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, NearState nr) {
@@ -132,7 +139,7 @@ k_near_scan(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, 
     at += c;
   }
   if (tid == 1023) start[bins] = at;   // the last thread's range ends at the last bin
-  if (tid == 0) nr.progress[d] = near_progress(p, 0, Dy[d].MH_std);   // no jump of this step done
+  if (tid == 0) near_reset(p, nr, d, Dy[d].MH_std);
   if (tid < 4) nr.ring[4 * d + tid] = 0;
 }
 

@@ -59,7 +59,7 @@ k_tip_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy,
   const DiodeParams& p = P[d];
   if (!tip_live(p, Dy[d])) return;
   const int n = Dy[d].n;
-  if (blockIdx.x == 0 && tid == 0) nr.progress[d] = near_progress(p, 0, Dy[d].MH_std);   // no jump of this step done
+  if (blockIdx.x == 0 && tid == 0) near_reset(p, nr, d, Dy[d].MH_std);
   const float4* hi = pool.pk_hi + p.off;
   const float4* lo = pool.pk_lo + p.off;
   const float R = (float)(p.r_tip * 1.0e9), z0 = (float)((p.h_tip - p.r_tip) * 1.0e9);
