@@ -334,13 +334,16 @@ int rd_events_take(rd_engine* e, int cap, rd_event* out, int* n_out, long long* 
  * counts and these two numbers, so a diode's results are the same alone and
  * in any mix under the same chunking; different chunkings differ in the last
  * FP32 bits.  rd_autotune times every candidate chunking on the diodes
- * resident now -- the force pass and a dry MH pass (the field at every
- * chain's current point, nothing written) weighted by the jump count --
- * keeps the fastest, then times the MH launch shapes (rd_set_mh_launch) under
+ * resident now -- the force pass, the supply points and a dry MH pass (the
+ * field at every chain's current point, nothing written) weighted by the jumps
+ * that take it -- keeps the fastest, then times the MH launch shapes (rd_set_mh_launch) under
  * it, rebuilds the step graph and leaves the particle state as it was.
  * rd_set_chunking sets one directly; 0, 0 brings the default back: 1024 and 32,
- * but shorter chunks (down to 128) for a diode whose tiles alone would not fill
- * the GPU, and up to 96 of them per tile of a field evaluation.  The jumps of
+ * which stand for shorter chunks (down to 128) where a diode's tiles alone would
+ * not fill the GPU, and up to 96 of them per tile of a field evaluation.  That
+ * rule is one of the tuner's candidates, and field evaluations keep it unless a
+ * chunking is set by hand; setting what rd_get_chunking gives changes nothing.
+ * The jumps of
  * most planar and tip diodes do not depend on it (near / far split).  The i-tile width (128
  * particles, points or chains per work item) is fixed. */
 typedef struct {

@@ -255,7 +255,9 @@ struct rd_engine {
   double kscale = 0.0;
   int max_items = 0;
   int clen_min = RD_CLEN_MIN, nch_max = RD_NCH_MAX;   // chunk rule of the pair sums
-  bool chunk_auto = true;                             // no chunking set: shorter chunks for small systems
+  bool chunk_hand = false;                            // set by hand: field evaluations take it too
+  // 1024 and 32 stand for the default rule: shorter chunks for small systems
+  bool chunk_auto() const { return clen_min == RD_CLEN_MIN && nch_max == RD_NCH_MAX; }
   // device memory
   DiodeParams* dP = nullptr;
   DiodeDyn* dD = nullptr;
@@ -408,7 +410,12 @@ static int alloc_pool(rd_engine* e, Pool& P, long long cap) {
 
 // ---- pipeline pieces ----------------------------------------------------------------
 static int chunk_rule(const rd_engine* e) {
-  return rd_chunk_rule(e->clen_min, e->nch_max, e->chunk_auto ? RD_ITEMS : 0);
+  return rd_chunk_rule(e->clen_min, e->nch_max, e->chunk_auto() ? RD_ITEMS : 0);
+}
+// Field evaluations at points: the tuner does not time them, so only a chunking set by
+// hand takes them off the default rule.
+static int field_chunk_rule(const rd_engine* e) {
+  return e->chunk_hand ? chunk_rule(e) : rd_chunk_rule(RD_CLEN_MIN, RD_NCH_MAX, RD_ITEMS);
 }
 
 // The plans of `modes` in one launch.
@@ -417,7 +424,8 @@ static cudaError_t plans_on(rd_engine* e, std::initializer_list<int> modes, cuda
   e->kernels_in_step++;
   PlanJobs jobs{};
   for (int m : modes) jobs.j[jobs.n++] = PlanJob{m, e->plan[m & 0xff], e->ph[m & 0xff]};
-  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), jobs, chunk_rule(e), e->max_items, npts);
+  const int rule = npts ? field_chunk_rule(e) : chunk_rule(e);   // (points only for PM_FIELD, alone)
+  return rd_launch_plan(st, e->dP, e->dD, e->nslots_hw(), jobs, rule, e->max_items, npts);
 }
 static cudaError_t plan(rd_engine* e, int mode, const int* npts = nullptr) { return plans_on(e, {mode}, e->st, npts); }
 
@@ -618,11 +626,9 @@ static int launch_mh_tiled_if(rd_engine* e, const Sig& s) {
   return RD_OK;
 }
 
-static int launch_emission(rd_engine* e) {
-  Sig s = signature(e);
-  if (!s.emit_planar && !s.emit_tip) return RD_OK;
+// The particles' field at the supply points of every emitting diode.
+static int launch_supply_sums(rd_engine* e, const Sig& s) {
   const int prec = e->cfg.precision;
-  const int ns = e->nslots_hw();
   if (s.emit_planar) {
     CK(plan(e, PM_SUPPLY_PLANAR));
     CK(rd_launch_z0_points(prec, e->grid, e->st, e->dP, e->pool, e->plan[PM_SUPPLY_PLANAR],
@@ -644,6 +650,16 @@ static int launch_emission(rd_engine* e) {
                               e->ph[PM_SUPPLY_TIP], pts, e->partial, e->tickets, e->kscale));
     e->kernels_in_step++;
   }
+  return RD_OK;
+}
+
+static int launch_emission(rd_engine* e) {
+  Sig s = signature(e);
+  if (!s.emit_planar && !s.emit_tip) return RD_OK;
+  const int prec = e->cfg.precision;
+  const int ns = e->nslots_hw();
+  int rc = launch_supply_sums(e, s);
+  if (rc) return rc;
   CK(rd_launch_supply_reduce(ns, e->st, e->dP, e->dD, e->qx, e->qy, e->qw, e->qF, e->qfx, e->qfy,
                              e->qS, e->work, e->d_step, e->sup_part));
   e->kernels_in_step += 2;
@@ -652,7 +668,7 @@ static int launch_emission(rd_engine* e) {
     CK(rd_launch_mh_vacuum(prec, ns, e->st, e->dP, e->dD, e->cs, e->d_choff, e->wtab, e->d_step, e->kscale));
     e->kernels_in_step += 2;   // uniform work functions, and the others
   }
-  int rc = launch_mh_tiled_if(e, s);
+  rc = launch_mh_tiled_if(e, s);
   if (rc) return rc;
   CK(rd_launch_emit(ns, e->st, e->dP, e->dD, e->pool, e->cs, e->d_choff, e->work, e->d_step, e->evlog));
   e->kernels_in_step += 2;
@@ -761,7 +777,7 @@ static std::string sig_string(rd_engine* e) {
   char b[128];
   snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
            s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.mh_near > 1 ? 2 : s.mh_near, s.mh_planar > s.mh_near,
-           s.tip_near, s.tip_slow, e->chunk_auto, s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
+           s.tip_near, s.tip_slow, e->chunk_auto(), s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
   return b;
 }
 
@@ -865,7 +881,7 @@ int rd_engine_view(rd_engine* e, int diode, const DiodeParams** P, const DiodeDy
 }
 
 int rd_engine_repack(rd_engine* e) { return repack(e); }
-int rd_engine_chunk_rule(rd_engine* e) { return chunk_rule(e); }
+int rd_engine_chunk_rule(rd_engine* e) { return field_chunk_rule(e); }
 
 // ---- C ABI ----------------------------------------------------------------------------
 extern "C" {
@@ -895,7 +911,7 @@ int rd_engine_create(const rd_engine_config* cfg, rd_engine** out) {
   e->grid = cfg->grid_blocks > 0 ? cfg->grid_blocks : 0;   // 0: occupancy-based per kernel
   e->clen_min = cfg->chunk_min > 0 ? cfg->chunk_min : RD_CLEN_MIN;
   e->nch_max = cfg->chunk_count_max > 0 ? cfg->chunk_count_max : RD_NCH_MAX;
-  e->chunk_auto = cfg->chunk_min <= 0 && cfg->chunk_count_max <= 0;
+  e->chunk_hand = !e->chunk_auto();
   if ((ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking)) != cudaSuccess ||
       (ce = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming)) != cudaSuccess)
     return bail(fail(RD_ERR_CUDA, cudaGetErrorString(ce)));
@@ -1813,17 +1829,18 @@ int rd_events_take(rd_engine* e, int cap, rd_event* out, int* n_out, long long* 
 
 // ---- autotuner ------------------------------------------------------------------------
 // Device time of the pair-sum passes of one step under the current chunking:
-// the force pass and, if planar diodes emit, a dry MH jump pass (field at
-// every chain's current point; nothing written but scratch), each averaged
-// over `reps` launches after one warm-up.
+// the force pass and the supply points' (each step's emission evaluates them afresh),
+// and, if planar diodes emit, a dry MH jump pass (field at every chain's current
+// point; nothing written but scratch), each averaged over `reps` launches after one
+// warm-up.
 static int time_pair_passes(rd_engine* e, int reps, double* force_ms, double* mh_ms) {
   Sig s = signature(e);
   float ms = 0.f;
   int rc = launch_force(e);
-  if (rc) return rc;
+  if (rc || (rc = launch_supply_sums(e, s))) return rc;
   CK(cudaEventRecord(e->ev0, e->st));
   for (int r = 0; r < reps; ++r)
-    if ((rc = launch_force(e))) return rc;
+    if ((rc = launch_force(e)) || (rc = launch_supply_sums(e, s))) return rc;
   CK(cudaEventRecord(e->ev1, e->st));
   CK(cudaEventSynchronize(e->ev1));
   CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
@@ -1868,9 +1885,11 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   // jumps that take the pair sums (near / far split: only the start and the last points)
   const int jumps = signature(e).mh_slow() ? std::max(signature(e).jumps, 1) : 2;
   const int saved_min = e->clen_min, saved_max = e->nch_max;
-  const bool saved_auto = e->chunk_auto;
-  e->chunk_auto = false;
   const int user_parts = e->mh_parts, user_form = e->mh_form;
+  auto give_up = [&](int code) {   // as the tuner found it
+    e->clen_min = saved_min; e->nch_max = saved_max; e->mh_parts = user_parts; e->mh_form = user_form;
+    return code;
+  };
   e->mh_parts = 0;    // the chunking is searched at the default launch shape
   e->mh_form = -1;
   double best = 1e300, at_default = 0.0, best_fms = 0.0;
@@ -1882,10 +1901,7 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
       e->clen_min = a;
       e->nch_max = b;
       double fms = 0.0, mms = 0.0;
-      if ((rc = time_pair_passes(e, 2, &fms, &mms))) {
-        e->clen_min = saved_min; e->nch_max = saved_max; e->chunk_auto = saved_auto; e->mh_parts = user_parts; e->mh_form = user_form;
-        return rc;
-      }
+      if ((rc = time_pair_passes(e, 2, &fms, &mms))) return give_up(rc);
       const double est = fms + jumps * mms;
       if (a == RD_CLEN_MIN && b == RD_NCH_MAX) at_default = est;
       if (est < best) { best = est; best_min = a; best_max = b; best_fms = fms; }
@@ -1896,7 +1912,6 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   // the MH launch shape under the chosen chunking: plan parts (with two or more
   // diodes running batched chains) and the FP32 thread form; both bit-identical
   const Sig sg = signature(e);
-  const int saved_parts = user_parts, saved_form = user_form;
   int best_parts = mh_parts_for(e, sg), best_form = mh_form_for(e, sg);
   double best_mh_ms = 1e300;
   if (sg.emit_planar) {
@@ -1908,7 +1923,7 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
         e->mh_parts = parts;
         e->mh_form = form;
         double fms = 0.0, mms = 0.0;
-        if ((rc = time_pair_passes(e, 6, &fms, &mms))) { e->mh_parts = saved_parts; e->mh_form = saved_form; return rc; }
+        if ((rc = time_pair_passes(e, 6, &fms, &mms))) return give_up(rc);
         if (mms < best_mh) { best_mh = mms; best_parts = parts; best_form = form; }
         out->candidates++;
       }
@@ -1920,6 +1935,7 @@ int rd_autotune(rd_engine* e, rd_tune_result* out) {
   CK(cudaMemcpyAsync(e->pool.ay, e->save_ay, bytes, cudaMemcpyDeviceToDevice, e->st));
   CK(cudaMemcpyAsync(e->pool.az, e->save_az, bytes, cudaMemcpyDeviceToDevice, e->st));
   CK(cudaStreamSynchronize(e->st));
+  e->chunk_hand = false;
   out->chunk_min = best_min;
   out->chunk_count_max = best_max;
   out->mh_parts = best_parts;
@@ -1974,9 +1990,10 @@ int rd_set_chunking(rd_engine* e, int chunk_min, int chunk_count_max) {
   const int a = chunk_min > 0 ? chunk_min : RD_CLEN_MIN, b = chunk_count_max > 0 ? chunk_count_max : RD_NCH_MAX;
   if (!valid_chunking(a, b))
     return fail(RD_ERR_INVALID, "chunk_min must be a multiple of 128 in [128, 65536], chunk_count_max in [1, 32]");
+  if (a == e->clen_min && b == e->nch_max) return RD_OK;   // what rd_get_chunking gave changes nothing
   e->clen_min = a;
   e->nch_max = b;
-  e->chunk_auto = chunk_min <= 0 && chunk_count_max <= 0;
+  e->chunk_hand = !e->chunk_auto();
   return RD_OK;
 }
 
@@ -2292,23 +2309,7 @@ int rd_profile_step(rd_engine* e, int step, rd_phase_times* out) {
   CK(cudaEventRecord(ev[0], e->st));
   if (s.emit_planar || s.emit_tip) {
     // supply integral
-    if (s.emit_planar) {
-      CK(plan(e, PM_SUPPLY_PLANAR));
-      CK(rd_launch_z0_points(prec, e->grid, e->st, e->dP, e->pool, e->plan[PM_SUPPLY_PLANAR],
-                             e->ph[PM_SUPPLY_PLANAR], e->qx, e->qy, e->qpp, e->qF, e->partial, e->tickets, e->kscale, e->item_queue + 6));
-    }
-    if (s.emit_lat) {
-      CK(plan(e, PM_SUPPLY_LAT));
-      PointSet lp{e->qx, e->qy, e->qz, e->qfx, e->qfy, e->qF, e->d_qoff};
-      CK(rd_launch_field_points(prec, RD_G_PLANAR, e->grid, e->st, e->dP, e->pool, e->plan[PM_SUPPLY_LAT],
-                                e->ph[PM_SUPPLY_LAT], lp, e->partial, e->tickets, e->kscale));
-    }
-    if (s.emit_tip) {
-      CK(plan(e, PM_SUPPLY_TIP));
-      PointSet pts{e->qx, e->qy, e->qz, e->qfx, e->qfy, e->qF, e->d_qoff};
-      CK(rd_launch_field_points(prec, RD_G_TIP, e->grid, e->st, e->dP, e->pool, e->plan[PM_SUPPLY_TIP],
-                                e->ph[PM_SUPPLY_TIP], pts, e->partial, e->tickets, e->kscale));
-    }
+    if ((rc = launch_supply_sums(e, s))) return rc;
     CK(rd_launch_supply_reduce(S, e->st, e->dP, e->dD, e->qx, e->qy, e->qw, e->qF, e->qfx, e->qfy, e->qS,
                                e->work, e->d_step, e->sup_part));
     CK(cudaEventRecord(ev[1], e->st));
