@@ -443,10 +443,15 @@ struct Sig {
   int mh_planar = 0;          // planar diodes with batched MH chains
   int mh_near = 0;            // of these, the diodes whose jumps take the near / far split
   bool tip_near = false, tip_slow = false;   // tip diodes whose jumps take the split / the pair sums
+  // Blocks that the cooperative launches of the split's jumps can use: the chains that a
+  // lone diode can have, so that they start beside other work on the GPU; 0 (any number)
+  // with more diodes, whose admissions would change the number at every turn.
+  int near_blocks = 0, tip_blocks = 0;
   bool mh_slow() const { return mh_planar > mh_near || tip_slow; }
 };
 static Sig signature(const rd_engine* e) {
   Sig s;
+  int tips = 0;
   for (auto& sl : e->slots) {
     if (!sl.used) continue;
     const DiodeParams& p = sl.p;
@@ -457,17 +462,22 @@ static Sig signature(const rd_engine* e) {
       if (p.geometry == RD_G_TIP) {
         s.emit_tip = true;
         if (p.tn) s.tip_near = true; else s.tip_slow = true;
+        if (p.tn) s.tip_blocks = tips++ ? 0 : (p.max_chains + RD_NEAR_CPB - 1) / RD_NEAR_CPB;
       } else {
         s.emit_planar = true;
       }
       if (p.geometry != RD_G_TIP && !p.image_charge) s.emit_lat = true;
       if (p.geometry != RD_G_TIP && p.mh_serial) s.emit_serial = true;
       if (p.geometry != RD_G_TIP && !p.mh_serial) s.mh_planar++;
-      if (p.mh_fast) s.mh_near++;
+      if (p.mh_fast) s.near_blocks = s.mh_near++ ? 0 : (p.max_chains + RD_NEAR_CPB - 1) / RD_NEAR_CPB;
       s.jumps = std::max(s.jumps, p.mh_jumps);
     }
   }
   return s;
+}
+
+static int jump_grid(const rd_engine* e, int blocks) {
+  return e->grid > 0 && blocks > 0 ? std::min(e->grid, blocks) : std::max(e->grid, blocks);
 }
 
 // The plans of the batched MH chains (counts of this step's supply).
@@ -538,7 +548,7 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
     if (slow) pm = PM_MH_SLOW;
   }
   if (near) {
-    CK(rd_launch_mh_jumps_near(prec, e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
+    CK(rd_launch_mh_jumps_near(prec, jump_grid(e, s.near_blocks), main, e->dP, e->dD, e->pool, e->plan[PM_MH_NEAR], e->ph[PM_MH_NEAR],
                                e->plan[PM_MH], e->cs, e->d_choff, e->wtab, e->d_step, s.jumps, e->nr, e->kscale,
                                e->cq + 3, s.mh_near == 1));
     e->kernels_in_step += s.mh_near == 1 ? 2 : 1;
@@ -562,7 +572,7 @@ static int launch_mh_jumps(rd_engine* e, const Sig& s, cudaStream_t main) {
     e->kernels_in_step++;
   }
   if (s.tip_near) {
-    CK(rd_launch_tip_near(e->nslots_hw(), e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH_TIP], e->ph[PM_MH_TIP],
+    CK(rd_launch_tip_near(e->nslots_hw(), jump_grid(e, s.tip_blocks), main, e->dP, e->dD, e->pool, e->plan[PM_MH_TIP], e->ph[PM_MH_TIP],
                           e->plan[PM_MH], e->cs, e->d_choff, e->d_step, s.jumps, e->nr, e->kscale, e->cq + 3));
     CK(rd_launch_mh_jump(prec, 2, e->grid, main, e->dP, e->dD, e->pool, e->plan[PM_MH], e->ph[PM_MH], e->cs,
                          e->d_choff, e->wtab, e->d_step, RD_MH_FINAL, e->partial, e->tickets, e->kscale, e->item_queue));
@@ -774,10 +784,11 @@ static int launch_step_body(rd_engine* e) {
 
 static std::string sig_string(rd_engine* e) {
   Sig s = signature(e);
-  char b[128];
-  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
+  char b[160];
+  snprintf(b, sizeof b, "%d%d%d%d%d%d%d%d%d%d%d%d%d%d:%d:%d:%d:%d:%d:%d:%d", s.planar, s.tip, s.emit_planar, s.emit_tip, s.nic,
            s.emit_serial, s.tts, s.mh_planar > 1 ? 2 : s.mh_planar, s.emit_lat, s.mh_near > 1 ? 2 : s.mh_near, s.mh_planar > s.mh_near,
-           s.tip_near, s.tip_slow, e->chunk_auto(), s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s));
+           s.tip_near, s.tip_slow, e->chunk_auto(), s.jumps, e->clen_min, e->nch_max, mh_parts_for(e, s), mh_form_for(e, s),
+           s.near_blocks, s.tip_blocks);
   return b;
 }
 
