@@ -1025,7 +1025,8 @@ int rd_engine_destroy(rd_engine* e) {
   if (e->st) cudaStreamSynchronize(e->st);
   if (e->graph) cudaGraphExecDestroy(e->graph);
   for (void* p : e->allocs) cudaFree(p);
-  for (auto& sl : e->slots) if (sl.tn_mem) cudaFree(sl.tn_mem);
+  for (auto& sl : e->slots) if (sl.tn_mem) cudaFreeAsync(sl.tn_mem, e->st);
+  if (e->st) cudaStreamSynchronize(e->st);   // gives them back to the GPU
   if (e->stage_d) cudaFree(e->stage_d);
   if (e->stage_i) cudaFree(e->stage_i);
   if (e->stage_hd) cudaFreeHost(e->stage_hd);
@@ -1216,7 +1217,8 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
   const size_t o_pan = part(sizeof(float4) * np), o_map = part(sizeof(int2) * RD_TN_MAP), o_rec = part(sizeof(float2) * 64 * np),
                o_hdr = part(sizeof(float4) * np), o_next = part(sizeof(int)), o_list = part(sizeof(float4) * (size_t)p.tn_cap);
   unsigned char* base = nullptr;
-  if (cudaMalloc(&base, at) != cudaSuccess) {
+  // stream-ordered: neither an admission nor a removal waits for the GPU (cudaFree does)
+  if (cudaMallocAsync((void**)&base, at, us) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }
@@ -1509,12 +1511,13 @@ int rd_diode_remove(rd_engine* e, int d) {
   DiodeDyn y{};
   CK(cudaMemcpyAsync(e->dP + d, &p, sizeof p, cudaMemcpyHostToDevice, e->st));
   CK(cudaMemcpyAsync(e->dD + d, &y, sizeof y, cudaMemcpyHostToDevice, e->st));
+  if (sl.tn_mem) CK(cudaFreeAsync(sl.tn_mem, e->st));
+  sl.tn_mem = nullptr;
   CK(cudaStreamSynchronize(e->st));
   e->pool_alloc.release(sl.pool_off, sl.pool_len);
   if (sl.ch_len) e->ch_alloc.release(sl.ch_off, sl.ch_len);
   if (sl.q_len) e->q_alloc.release(sl.q_off, sl.q_len);
   if (sl.w_len) e->w_alloc.release(sl.w_off, sl.w_len);
-  if (sl.tn_mem) cudaFree(sl.tn_mem);
   sl = SlotHost();
   return RD_OK;
 }
