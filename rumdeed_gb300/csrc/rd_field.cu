@@ -961,13 +961,20 @@ __device__ __forceinline__ void tip_grid_xyz(const DiodeParams& p, double xi, do
   *Z = (double)(float)(*Z * 1.0e9) * 1.0e-9;
 }
 
+// log phi less half the logarithm of v = xi^2 - eta^2: rho_entry_f's t0 at a tip.
+__device__ __forceinline__ float tip_log_phi(const DiodeParams& p, float v) {
+  float kf;
+  const float m = rd_log_parts(v, &kf);
+  return rd_less_half_log(p.tn_t0, kf, logf(m));
+}
+
 // What the near / far split (rd_tipnear.cuh) keeps of a chain that starts at xi.
 __device__ __forceinline__ void tip_start(const DiodeParams& p, const ChainState& cs, int k, double xi, double F) {
   if (!p.tn) return;
   const float Ff = (float)F;
   cs.fF[k] = Ff;
   cs.fe[k] = 1.2e-7f * fabsf(Ff);
-  cs.fsup[k] = rho_entry_f(p, p.tn_t0 - 0.5f * logf((float)(xi * xi - p.eta_1 * p.eta_1)), p.tn_t2, Ff);
+  cs.fsup[k] = rho_entry_f(p, tip_log_phi(p, (float)(xi * xi - p.eta_1 * p.eta_1)), p.tn_t2, Ff);
   cs.em[k] = 0;   // not moved yet
 }
 

@@ -39,6 +39,16 @@ RD_HD double rd_float64_of_bits(uint64_t b) {
 #endif
 }
 
+RD_HD uint32_t rd_bits_of_float(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(f);
+#else
+  uint32_t b;
+  memcpy(&b, &f, sizeof b);
+  return b;
+#endif
+}
+
 RD_HD float rd_float_of_bits(uint32_t b) {
 #ifdef __CUDA_ARCH__
   return __uint_as_float(b);

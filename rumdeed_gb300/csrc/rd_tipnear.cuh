@@ -194,7 +194,7 @@ k_tip_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy,
 
 // The entry (t0, t2) of rho_entry_f at a tip point.
 __device__ __forceinline__ void tip_entry(const DiodeParams& p, double xi, float* t0, float* t2) {
-  *t0 = p.tn_t0 - 0.5f * logf((float)(xi * xi - p.eta_1 * p.eta_1));
+  *t0 = tip_log_phi(p, (float)(xi * xi - p.eta_1 * p.eta_1));
   *t2 = p.tn_t2;
 }
 
@@ -383,7 +383,7 @@ k_tip_jumps(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, const 
           const float4 ct = p.tn_pan[pan];
           r = make_float4(px - ct.x, py - ct.y, pz - ct.z, ct.w);
           const float v = (float)(nxi * nxi - p.eta_1 * p.eta_1), iv = 1.0f / v;
-          t0 = p.tn_t0 - 0.5f * logf(v);
+          t0 = tip_log_phi(p, v);
           t2 = p.tn_t2;
           // the normal
           const float rho2 = fmaf(px, px, py * py), gn = p.tn_nf * rsqrtf(rho2 + p.tn_c);

@@ -59,7 +59,11 @@ struct Target {
 static float ulp(float x, unsigned move, int bit) { return std::nextafterf(x, (move >> bit & 1) ? INFINITY : -INFINITY); }
 static float rho_f(const Target& t, float F, unsigned move, int bit) {
   const float lphi = (float)t.logphi;
-  const float t0 = t.tip ? lphi - 0.5f * ulp(std::log((float)t.v), move, bit) : lphi;
+  float t0 = lphi, kf;
+  if (t.tip) {
+    const float m = rd_log_parts((float)t.v, &kf);
+    t0 = rd_less_half_log(lphi, kf, ulp(std::log(m), move, bit));
+  }
   const float l = (float)t.lcoef * (-F);
   float tau = 0.0f;
   if (l > 1.0f) tau = 1.0f / 9.0f;
