@@ -714,12 +714,13 @@ k_supply_points(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ 
                 const double* __restrict__ qx, const double* __restrict__ qy,
                 const double* __restrict__ qw, const double* __restrict__ qF,
                 const double* __restrict__ qfx, const double* __restrict__ qfy,
-                const double* __restrict__ work, const int* __restrict__ step_ptr, double* __restrict__ qS) {
-  const int d = blockIdx.y;
+                const double* __restrict__ work, const int* __restrict__ step_ptr, double* __restrict__ qS,
+                int per) {
+  const int d = blockIdx.x / per, b = blockIdx.x % per;
   const DiodeParams& p = P[d];
   if (!supply_live(p, Dy[d], step_ptr)) return;
   const int npt = (p.geometry == RD_G_TIP) ? 10000 : p.quad_n * p.quad_n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npt; i += gridDim.x * blockDim.x) {
+  for (int i = b * blockDim.x + threadIdx.x; i < npt; i += per * blockDim.x) {
     const int k = p.q_off + i;
     double F = qF[k], S = 0.0;
     if (p.geometry == RD_G_TIP) {   // Field_normal :105-112
@@ -2944,8 +2945,9 @@ cudaError_t rd_launch_supply_reduce(int nslots, cudaStream_t st, const DiodePara
                                     const double* qF, const double* qfx, const double* qfy, double* qS,
                                     const double* work, const int* step_ptr, double* sup_part) {
   // one diode: a thread per point of the default rules; many: a few points per thread
+  // (all along x: a grid's y ends at 65535)
   const int blocks = std::max(8, 1216 / std::max(nslots, 1));
-  k_supply_points<<<dim3(blocks, nslots), 128, 0, st>>>(P, Dy, qx, qy, qw, qF, qfx, qfy, work, step_ptr, qS);
+  k_supply_points<<<nslots * blocks, 128, 0, st>>>(P, Dy, qx, qy, qw, qF, qfx, qfy, work, step_ptr, qS, blocks);
   k_supply_reduce<<<dim3(nslots, RD_SUP_SPLIT), 256, 0, st>>>(P, Dy, qS, qw, qF, qfx, qfy, step_ptr, sup_part);
   return cudaGetLastError();
 }
@@ -3072,7 +3074,8 @@ cudaError_t rd_launch_tip_near(int nslots, int grid, cudaStream_t st, const Diod
                                const Pool& pool, const PlanEntry* plan, const PlanHeader* ph, const PlanEntry* plan_mh,
                                const ChainState& cs, const int* ch_off, const int* step_ptr, int jumps,
                                const NearState& nr, double kscale, int* gave_up) {
-  k_tip_panels<<<dim3(std::max(16, RD_TN_PANELS / std::max(nslots, 1)), nslots), 256, 0, st>>>(P, Dy, pool, nr);
+  const int per = std::max(16, RD_TN_PANELS / std::max(nslots, 1));
+  k_tip_panels<<<nslots * per, 256, 0, st>>>(P, Dy, pool, nr, per);
   const int most = rd_grid(k_tip_jumps, 256, 0), g = grid > 0 && grid < most ? grid : most;
   return launch_coop(k_tip_jumps, 256, g, st, P, (DiodeDyn*)Dy, pool, plan, ph, plan_mh, cs, ch_off, step_ptr, jumps, nr,
                      kscale, gave_up);

@@ -51,19 +51,19 @@ __device__ __forceinline__ bool tip_live(const DiodeParams& p, const DiodeDyn& y
 // 5000 electrons close to the tip and 14,000 chains takes 4.7 / 4.2 / 4.0 ms with 256 / 512
 // / 768 panels, one of 9000 spread electrons and 12,100 chains 3.9 / 3.6 / 3.6 ms.
 __global__ void __launch_bounds__(256)
-k_tip_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, NearState nr) {
+k_tip_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy, Pool pool, NearState nr, int per) {
   constexpr int D = RD_TN_DEG;
   __shared__ float red[8][68];
   __shared__ int s_n, s_at, s_bad;
-  const int d = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int d = blockIdx.x / per, b = blockIdx.x % per, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const DiodeParams& p = P[d];
   if (!tip_live(p, Dy[d])) return;
   const int n = Dy[d].n;
-  if (blockIdx.x == 0 && tid == 0) near_reset(p, nr, d, Dy[d].MH_std);
+  if (b == 0 && tid == 0) near_reset(p, nr, d, Dy[d].MH_std);
   const float4* hi = pool.pk_hi + p.off;
   const float4* lo = pool.pk_lo + p.off;
   const float R = (float)(p.r_tip * 1.0e9), z0 = (float)((p.h_tip - p.r_tip) * 1.0e9);
-  for (int k = blockIdx.x; k < p.tn_np; k += gridDim.x) {
+  for (int k = b; k < p.tn_np; k += per) {
     const float4 c = p.tn_pan[k];
     const float near2 = (RD_TN_NEAR * c.w) * (RD_TN_NEAR * c.w), ia = 1.0f / c.w;
     // the near electrons' number, a place for their list, and whether the bound holds
