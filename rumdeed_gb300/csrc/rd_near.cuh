@@ -871,6 +871,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
       const uint32_t step = (uint32_t)(engine_step - y.step_offset);
       const float* recs = nr.rec + (size_t)(p.q_off / 16) * RD_NEAR_REC;
       float px = 0.0f, py = 0.0f, t0 = 0.0f, t2 = 0.0f;
+      bool off = false;      // no panel's expansion holds there
       Real ox = 0, oy = 0;   // the proposal
       NearFar far_part;
       unsigned long long pr = 0;
@@ -960,6 +961,8 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
         const float4* rec = reinterpret_cast<const float4*>(recs + (size_t)pan * RD_NEAR_REC);
         far_part.load(rec);
         if (!ONE) far_part.eval(p, px, py);   // (ONE: evaluated after the near sums, the loads in flight meanwhile)
+        // a step size above the clamp (from a checkpoint) can reflect a proposal off the emitter
+        off = fmaxf(fabsf(px) - p.em_hx, fabsf(py) - p.em_hy) > 0.005f * fminf(p.nr_ax, p.nr_ay);
         if (ok) {
           if constexpr (PREC == 1) work_entry_f(p, wtab, chain_cell_f(p, px, py), px, py, &t0, &t2);
           else work_entry_d(p, wtab, ox, oy, &t0, &t2);
@@ -1027,7 +1030,7 @@ __device__ __forceinline__ void near_jumps(NearShared<PREC, NW>& sh, const Diode
           const float S = far_part.c0.x + sh.near[lane], b0 = far_part.c0.y + (PREC == 1 ? 0.0f : sh.wide[lane]);
           float dF, rn;
           const float Fn = near_field(p, ksc, S, fmaf(far_part.ty.y, 1.01f * fabsf(S), b0), &dF);
-          const int take = near_decide(p, Fn, dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
+          const int take = near_decide(p, Fn, off ? INFINITY : dF, Fc, fe, rc, t0, t2, sh.lu[lane], &rn);
           open = take < 0;
           if (take == 1) {
             fx = ox; fy = oy; rc = rn; Fc = Fn; fe = dF;
