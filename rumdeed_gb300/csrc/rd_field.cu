@@ -2481,17 +2481,44 @@ __device__ __noinline__ bool serial_take_fp64(const DiodeParams& p, const double
   const double sn = supply_log_xy(p, wtab, wx, wy, F) + ln, sc = supply_log_xy(p, wtab, cx, cy, Fc) + lc;
   return sn >= sc || lu <= sn - sc;
 }
-// The same from fields that are within 1e-10 of |F| and the vacuum field (float pairs):
-// -1 where that leaves the answer open.
-__device__ __noinline__ int serial_take_pairs(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
-                                              double F, double ln, double cx, double cy, double Fc, double lc,
-                                              double lu) {
-  const double E2 = 2.0 * fabs(p.E_z), en = 1.0e-10 * (fabs(F) + E2), ec = 1.0e-10 * (fabs(Fc) + E2);
-  if (F > en) return 0;
-  if (!(F < 0.0 && Fc < 0.0 && 4.0 * en <= -F && 4.0 * ec <= -Fc)) return -1;
-  const double d = ((supply_log_xy(p, wtab, wx, wy, F) + ln) - (supply_log_xy(p, wtab, cx, cy, Fc) + lc)) - lu;
-  const double eps = 2.5 * (en / -F + ec / -Fc) + 1.0e-11;   // take iff d >= 0 (log u <= 0)
+// The error of a field from float pairs (1e-10 of |F| and the vacuum field) over |F|;
+// infinite where that leaves its sign open.
+__device__ __forceinline__ double serial_rel(const DiodeParams& p, double F) {
+  const double en = 1.0e-10 * (fabs(F) + 2.0 * fabs(p.E_z));
+  return 4.0 * en <= fabs(F) ? en / fabs(F) : __longlong_as_double(0x7ff0000000000000ll);
+}
+// A point's FP64 target (F < 0), with the ring's log radius (1: no ring); open: the
+// field's sign is not certain.
+struct SerialTarget {
+  double s, e;
+  bool open;
+};
+template <int PREC>
+__device__ __noinline__ SerialTarget serial_own_target(const DiodeParams& p, const double* __restrict__ wtab, double x,
+                                                       double y, double F, double r) {
+  SerialTarget t = {0.0, 0.0, false};
+  if (PREC == 1) {
+    t.e = serial_rel(p, F);
+    t.open = !(t.e < 1.0);
+  }
+  if (F < 0.0 && !t.open) {
+    t.s = supply_log_xy(p, wtab, x, y, F);
+    if (r != 1.0) t.s += log(r);
+  }
+  return t;
+}
+// A decision from targets whose fields have the relative errors en, ec: -1 where those
+// leave it open.
+__device__ __forceinline__ int serial_decide(double sn, double en, double sc, double ec, double lu) {
+  const double d = (sn - sc) - lu, eps = 2.5 * (en + ec) + 1.0e-11;   // take iff d >= 0 (log u <= 0)
   return d > eps ? 1 : d < -eps ? 0 : -1;
+}
+__device__ __noinline__ int serial_take_pairs(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
+                                              double F, double cx, double cy, double Fc, double lu) {
+  const double en = serial_rel(p, F), ec = serial_rel(p, Fc);
+  if (!(en + ec < 1.0) || Fc > 0.0) return -1;
+  if (F > 0.0) return 0;
+  return serial_decide(supply_log_xy(p, wtab, wx, wy, F), en, supply_log_xy(p, wtab, cx, cy, Fc), ec, lu);
 }
 __device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* __restrict__ wtab, double wx, double wy,
                                             double F, double cx, double cy, double Fc, double lu) {
@@ -2645,6 +2672,8 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         }
       }
     }
+    SerialTarget tc = {};   // the chain's FP64 target, if have_sc
+    bool have_sc = false;
     const bool walk = s_found != 0;   // every thread: the chain found a start
     for (int i = 1; walk && i <= ndim; ++i) {
       double wx = 0.0, wy = 0.0, na = 0.0, nr = 0.0;
@@ -2663,6 +2692,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
       if constexpr (PREC == 1) {
         if (est && i < ndim && draw + 1 < RD_SER_DRAWS) {   // jumps i and i + 1 (block-uniform)
           const int par = (i >> 1) & 1;
+          have_sc = false;
           double x = 0.0, y2 = 0.0, wx0 = 0.0, wy0 = 0.0;
           if (threadIdx.x < 32) {   // lane 0: jump i; 1, 2: jump i + 1 from its point, from the chain's
             const int lane = threadIdx.x;
@@ -2711,7 +2741,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
                   const SerialSum sum = {wh, wl, 0.0};
                   const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
                   const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
-                  tk = serial_take_pairs(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
+                  tk = serial_take_pairs(p, wtab, wx, wy, Fw, cx, cy, Fd, s_lu[draw + j]);
                 }
                 tk = __shfl_sync(0xffffffffu, tk, 0);
               }
@@ -2759,6 +2789,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
       const SerialSum sum = serial_field_sum<PREC>(p, pool, n, s_pt[i & 1][0], s_pt[i & 1][1], s_pp[i & 1], red_f, red_d);
       int take = -1;
       float Fn = 0.0f, dF = 0.0f, rn = 0.0f;
+      SerialTarget tn = {};   // the proposal's FP64 target
       if (t0) {
         // ring: log(radius) is the Jacobian of the (angle, radius) parametrisation (:1592-1596)
         const double lu = s_lu[draw];
@@ -2775,12 +2806,19 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         }
         if (take < 0) {   // the FP64 targets
           const double Fw = z0_finish<PREC>(p, serial_value<PREC>(sum), kscale);
-          const double Fd = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
-          if (PREC == 1) {
-            take = serial_take_pairs(p, wtab, wx, wy, Fw, ring ? log(nr) : 0.0, cx, cy, Fd, ring ? log(cr) : 0.0, lu);
-          } else if (Fw >= 0.0) take = 0;
-          else if (ring) take = serial_take_fp64(p, wtab, wx, wy, Fw, log(nr), cx, cy, Fd, log(cr), lu);
-          else take = serial_take(p, wtab, wx, wy, Fw, cx, cy, Fd, lu);
+          if (PREC == 1 || ring) {
+            if (!have_sc) {   // the chain's target, kept until it moves
+              tc = serial_own_target<PREC>(p, wtab, cx, cy, z0_finish<PREC>(p, serial_value<PREC>(cur), kscale), ring ? cr : 1.0);
+              have_sc = true;
+            }
+            tn = serial_own_target<PREC>(p, wtab, wx, wy, Fw, ring ? nr : 1.0);
+            take = PREC == 1 ? (Fw > 0.0 && !tn.open ? 0 : tn.open || tc.open ? -1 : serial_decide(tn.s, tn.e, tc.s, tc.e, lu))
+                             : (Fw < 0.0 && (tn.s >= tc.s || lu <= tn.s - tc.s));
+          } else if (Fw >= 0.0) {
+            take = 0;
+          } else {
+            take = serial_take(p, wtab, wx, wy, Fw, cx, cy, z0_finish<PREC>(p, serial_value<PREC>(cur), kscale), lu);
+          }
           if (est) {
             const double* e = wtab + 3 * (p.work_off + work_cell(p, wx, wy));
             rn = rho_entry_f(p, (float)e[0], (float)e[2], Fn);
@@ -2800,6 +2838,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         if (take) {
           cx = wx; cy = wy; cur = sum; ca = na; cr = nr;
           Fc = Fn; fe = dF; rc = rn;
+          tc = tn; have_sc = !est;
           moved = true;
           if (i > ndim_first) ++ja;
         } else if (i > ndim_first) {
