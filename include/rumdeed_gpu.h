@@ -149,8 +149,9 @@ int rd_sync(rd_engine* e);
  * (src/mod_field_emission_v2.F90:113-135) or Init_Emission_Tip
  * (src/mod_emission_tip.f90:81-127) for the new slot.  An emitting FP32 tip takes
  * GPU memory of its own beside the engine's pools, 768 B per particle of its
- * capacity (2 GiB at most), in stream order and given back by rd_diode_remove;
- * without it the tip's jumps are slower (pair sums) and all else is the same. */
+ * capacity (2 GiB at most), in stream order; rd_diode_remove gives it back, but for
+ * 256 MiB in all that the engine keeps for its next tips.  Without that memory the
+ * tip's jumps are slower (pair sums) and all else is the same. */
 int rd_diode_add(rd_engine* e, const rd_diode_config* cfg, int* diode);
 int rd_diode_remove(rd_engine* e, int diode);
 int rd_diode_count(rd_engine* e, int* active);

@@ -297,6 +297,7 @@ struct rd_engine {
   long long stage_cap = 0;
   unsigned char* io_h = nullptr;   // pinned buffer of the particle and point transfers
   size_t io_cap = 0;
+  cudaMemPool_t tn_pool = nullptr; // the tips' panels and lists (tip_pool)
   bool packs_stale = false;        // electrons emitted since the last pack (rd_do_emission alone)
   // overlapped admission (rd_serve): uploads on stream sa from a pinned arena into a device
   // arena, slots activated on st before the next step (activate_pending)
@@ -1026,7 +1027,8 @@ int rd_engine_destroy(rd_engine* e) {
   if (e->graph) cudaGraphExecDestroy(e->graph);
   for (void* p : e->allocs) cudaFree(p);
   for (auto& sl : e->slots) if (sl.tn_mem) cudaFreeAsync(sl.tn_mem, e->st);
-  if (e->st) cudaStreamSynchronize(e->st);   // gives them back to the GPU
+  if (e->st) cudaStreamSynchronize(e->st);
+  if (e->tn_pool) cudaMemPoolDestroy(e->tn_pool);
   if (e->stage_d) cudaFree(e->stage_d);
   if (e->stage_i) cudaFree(e->stage_i);
   if (e->stage_hd) cudaFreeHost(e->stage_hd);
@@ -1151,6 +1153,25 @@ static void near_params(DiodeParams& p, int P, int Q) {
   p.nr_iwx = (float)(0.5 / ax); p.nr_iwy = (float)(0.5 / ay);
 }
 
+// The engine's pool of the tips' memory: it keeps RD_TN_KEEP bytes of what removed tips
+// gave back for the next ones (a new mapping of 15 MB takes some 0.1 ms), until the engine
+// is destroyed.
+static bool tip_pool(rd_engine* e) {
+  if (e->tn_pool) return true;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = e->cfg.device;
+  if (cudaMemPoolCreate(&e->tn_pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    e->tn_pool = nullptr;
+    return false;
+  }
+  uint64_t keep = RD_TN_KEEP;
+  cudaMemPoolSetAttribute(e->tn_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return true;
+}
+
 // The same for the FP32 chains of a new tip diode (rd_tipnear.cuh): its panels, and one
 // allocation for their records and lists, freed with the diode.  Without the memory the
 // diode keeps the pair-sum jumps.
@@ -1164,12 +1185,13 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
   const int N = 4 * RD_TN_MAP;
   const double vmax = std::sqrt(p.max_xi - 1.0);
   std::vector<double> arc(N + 1, 0.0);
-  double area = 0.0;
+  double area = 0.0, r0 = rad(1.0), h0 = hgt(1.0);
   for (int i = 0; i < N; ++i) {
-    const double v0 = vmax * i / N, v1 = vmax * (i + 1) / N, x0 = 1.0 + v0 * v0, x1 = 1.0 + v1 * v1;
-    const double ds = std::hypot(rad(x1) - rad(x0), hgt(x1) - hgt(x0));
+    const double v1 = vmax * (i + 1) / N, x1 = 1.0 + v1 * v1, r1 = rad(x1), h1 = hgt(x1);
+    const double ds = std::sqrt((r1 - r0) * (r1 - r0) + (h1 - h0) * (h1 - h0));
     arc[i + 1] = arc[i] + ds;
-    area += 3.14159265358979323846 * (rad(x0) + rad(x1)) * ds;
+    area += 3.14159265358979323846 * (r0 + r1) * ds;
+    r0 = r1; h0 = h1;
   }
   if (!(arc[N] > 0.0) || !std::isfinite(area)) return cudaSuccess;
   const double width = std::sqrt(area / RD_TN_PANELS);
@@ -1194,15 +1216,20 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
     const double xa = wider(arc[N] * r / rings, -1.0), xb = wider(arc[N] * (r + 1) / rings, 1.0);
     const double half = 3.14159265358979323846 / n * 1.0001;
     const double xc = n == 1 ? 1.0 : xm;
-    double rr = 0.0;
-    for (int i = 0; i <= 8; ++i)
+    double cs[9], sn[9], rr = 0.0;   // the largest distance from the centre, squared
+    for (int q = 0; q <= 8; ++q) { cs[q] = std::cos(half * q / 8); sn[q] = std::sin(half * q / 8); }
+    const double rc = rad(xc), hc = hgt(xc);
+    for (int i = 0; i <= 8; ++i) {
+      const double xi = xa + (xb - xa) * i / 8, ri = rad(xi), dh = hgt(xi) - hc;
       for (int q = 0; q <= 8; ++q) {
-        const double xi = xa + (xb - xa) * i / 8, ph = half * q / 8;
-        rr = std::max(rr, std::hypot(std::hypot(rad(xi) * std::cos(ph) - rad(xc), rad(xi) * std::sin(ph)), hgt(xi) - hgt(xc)));
+        const double dx = ri * cs[q] - rc, dy = ri * sn[q];
+        rr = std::max(rr, dx * dx + dy * dy + dh * dh);
       }
+    }
+    rr = std::sqrt(rr);
     for (int q = 0; q < n; ++q) {
       const double ph = 2.0 * 3.14159265358979323846 * (q + 0.5) / n;
-      pan.push_back(make_float4((float)(rad(xc) * std::cos(ph)), (float)(rad(xc) * std::sin(ph)), (float)hgt(xc),
+      pan.push_back(make_float4((float)(rc * std::cos(ph)), (float)(rc * std::sin(ph)), (float)hc,
                                 (float)(rr * 1.002 + 1.0e-3)));
     }
   }
@@ -1218,7 +1245,7 @@ static cudaError_t tip_near_params(rd_engine* e, DiodeParams& p, SlotHost& sl, c
                o_hdr = part(sizeof(float4) * np), o_next = part(sizeof(int)), o_list = part(sizeof(float4) * (size_t)p.tn_cap);
   unsigned char* base = nullptr;
   // stream-ordered: neither an admission nor a removal waits for the GPU (cudaFree does)
-  if (cudaMallocAsync((void**)&base, at, us) != cudaSuccess) {
+  if (!tip_pool(e) || cudaMallocFromPoolAsync((void**)&base, at, e->tn_pool, us) != cudaSuccess) {
     cudaGetLastError();
     return cudaSuccess;
   }

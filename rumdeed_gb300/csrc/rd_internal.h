@@ -66,6 +66,7 @@ inline int rd_chunk_rule(int clen_min, int nch_max, int target) {
 #define RD_TN_RINGS 128       // at most this many rings of them
 #define RD_TN_MAP 1024        // entries of the ring map
 #define RD_TN_LIST 48         // list entries per particle slot (an electron is near to about 30 panels)
+#define RD_TN_KEEP (256ll << 20)   // bytes of removed tips' memory that an engine keeps
 #define RD_MAX_WORK 4096      // max checkerboard cells per diode (64x64)
 
 enum { RD_G_PLANAR = 1, RD_G_TIP = 2 };
