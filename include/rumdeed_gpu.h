@@ -364,7 +364,7 @@ int rd_get_chunking(rd_engine* e, int* chunk_min, int* chunk_count_max);
  * changes no result: `parts`
  * launches per jump on as many streams, each over a part of the work plan cut
  * at diode boundaries (1..4; 0 = 2, used only when two or more diodes run
- * batched chains), and the FP32 thread form (0: 32 threads x 4 chains per
+ * batched chains and no tip takes pair sums), and the FP32 thread form (0: 32 threads x 4 chains per
  * 128-chain tile, 1: 64 threads x 2 chains; -1 = form 1 for a single emitting
  * planar diode, else form 0).  rd_autotune searches both after the chunking;
  * rd_get_mh_launch reports what the next step uses. */

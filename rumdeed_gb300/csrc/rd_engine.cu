@@ -496,9 +496,12 @@ static cudaError_t plan_chains(rd_engine* e, const Sig& s) {
 // MH launch shape of the planar jumps for the resident mix: parts of the plan
 // (one launch and one stream each; one diode cannot be split) and the FP32
 // thread form.  (Jumps by the near / far split have one shape.)  Neither changes a result: each diode's chains and counters sit
-// in one part, and both forms do the same lane arithmetic in the same order.
+// in one part, and both forms do the same lane arithmetic in the same order.  With tips
+// that take the pair sums too there is one part: their kernel lays an item's partial sums
+// out over three times the scratch (and its plan may be another), so a planar part on a
+// second stream would run into them.
 static int mh_parts_for(const rd_engine* e, const Sig& s) {
-  if (s.mh_planar <= 1) return 1;
+  if (s.mh_planar <= 1 || s.tip_slow) return 1;
   return e->mh_parts > 0 ? e->mh_parts : RD_MH_PARTS;
 }
 static int mh_form_for(const rd_engine* e, const Sig& s) {
