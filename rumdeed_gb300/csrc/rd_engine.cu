@@ -874,7 +874,7 @@ static bool valid_diode(rd_engine* e, int d) {
   return e && d >= 0 && d < (int)e->slots.size() && e->slots[d].used;
 }
 
-// ---- helpers for rd_noalloc.cu (C++ linkage, not part of the C ABI) -----------------
+// ---- helpers for rd_noalloc.cu and tests (C++ linkage, not part of the C ABI) ------
 int rd_set_error(int code, const char* msg) { return fail(code, msg); }
 int rd_noalloc_prepare(int device, int prec);   // rd_noalloc.cu
 
@@ -892,6 +892,15 @@ int rd_engine_view(rd_engine* e, int diode, const DiodeParams** P, const DiodeDy
   *kscale = e->kscale;
   *st = e->st;
   *device = e->cfg.device;
+  return RD_OK;
+}
+
+// The chains of a diode's last emission, in device memory from *first on (tests compare the
+// kept estimates and bounds with the pair sums).
+int rd_engine_chains(rd_engine* e, int diode, ChainState* cs, long long* first) {
+  if (!valid_diode(e, diode)) return fail(RD_ERR_NOTFOUND, "unknown diode");
+  *cs = e->cs;
+  *first = e->slots[diode].ch_off;
   return RD_OK;
 }
 
