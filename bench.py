@@ -459,10 +459,10 @@ def run_ours(args, rank, world):
     e2e = e2e_all / e2e_wall if e2e_wall > 0 else 0.0
     if rank != 0:
         return
-    # roofline of the largest kernel (FP32 pipe; 20 flops per Coulomb-like term): the supply
-    # integral's pair sum, the CUDA-event time of the whole phase charged to it.  The jumps no
-    # longer evaluate every (chain, electron) pair (rd_near.cuh), so their pair count over
-    # their time is a rate of jumps, not of arithmetic.
+    # roofline of the largest pair sum (FP32 pipe; 20 flops per Coulomb-like term): the supply
+    # integral's, the CUDA-event time of the whole phase charged to it.  The jumps, the step's
+    # largest kernel, no longer evaluate every (chain, electron) pair (rd_near.cuh): they are
+    # bound by the latency of a jump and have no arithmetic roofline.
     jumps = max(prof["mh_jump_launches"], 1)
     sup_s = prof["supply_ms"] / 1e3
     achieved = 20.0 * prof["supply_pair_evals"] / sup_s / 1e12 if sup_s > 0 else 0.0
@@ -525,9 +525,11 @@ def run_ours(args, rank, world):
                      "traffic_source": "not captured for this mix",
                      "flops_convention": "20 flops per Coulomb-like term (Nyland et al.); "
                                          "1 term per (supply point, particle) at the cathode"},
-        "mh_jump": {"ms": prof["mh_jumps_ms"] / jumps,
+        "mh_jump": {"kernel": "k_mh_jumps_near<1>", "bound": "latency of a jump",
+                    "ms": prof["mh_jumps_ms"] / jumps, "ms_per_step": prof["mh_jumps_ms"],
                     "pairs_per_jump": prof["mh_pair_evals"] / jumps,
-                    "note": "pairs a jump stands for; near / far split, most of them in panel expansions"},
+                    "note": "the phase with its set-up and last pass; pairs a jump stands for: near / far "
+                            "split, most of them in panel expansions"},
         "phase_ms": {k: prof[k] for k in ("supply_ms", "mh_init_ms", "mh_jumps_ms", "emit_ms",
                                           "position_ms", "force_ms", "velocity_ms", "compact_ms",
                                           "total_ms")},

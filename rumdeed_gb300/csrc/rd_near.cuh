@@ -6,13 +6,14 @@
 // FP32 chains already decide from FP32 estimates of the targets wherever those
 // are certain (mh_decide_f).  (The FP64 form's chains take the same estimates, with
 // FP64 points, draws and pair sums; below u and the pair sum's roundings are the FP32
-// form's, the FP64 form's are smaller.)  The same holds for the field itself: an estimate
+// form's, the FP64 form's are smaller, but for what near_wide adds.)  The same holds for the field itself: an estimate
 // with a bound on how far it can lie from the value the pair-sum kernel
 // (k_mh_jump_planar) computes decides every jump outside that bound, and the few
-// jumps inside it take the pair sum.  So the decisions, and with them the
-// chains, are those of the pair-sum kernel, bit for bit, and the field that
-// emission reads is the pair sum at each chain's last point (one pass after the
-// last jump, RD_MH_FINAL).
+// jumps inside it take sums over all electrons: first in any order, with a bound of
+// their own, then as the pair-sum kernel forms them.  So the decisions, and with them
+// the chains, are those of the pair-sum kernel, bit for bit, and the field that
+// emission reads is the pair sum at the last point of each chain that has moved (one
+// pass after the last jump, RD_MH_FINAL) and the start's field of the others.
 //
 // The estimate.  The step's supply integral has just evaluated the pair sum S at
 // 4 x 4 Gauss-Legendre nodes of each of the emitter's P x P panels.  Electrons
@@ -41,14 +42,14 @@
 //   24 diodes of 256-4096 electrons, 30,000 chains, 200    15.9 -> 1.9 ms
 //   128 diodes of 256-32768 electrons, 353,000 chains, 200  276 -> 22.3 ms
 //   FP64: 1300 electrons, 960 chains, 100                   8.4 -> 0.85 ms
-// Open after the estimate: one jump in 10^5; the estimate lay within 0.08 of its
-// bound in every jump checked.  What is left is latency (one near list, one far
-// record, three logarithms and one counter per jump), not arithmetic.
+// Open after the estimate: one jump in 10^5; the estimate lies within 0.13 (FP32) and
+// 0.30 (FP64) of its bound at the chains' last points (tests/near_bound.cu).  What is
+// left is latency (one near list, one far record, three logarithms and one counter per
+// jump), not arithmetic.
 //
 // Near region: RD_NEAR_M = 3 panels and nr_Z = 5 half widths.  5 panels and 8 half
 // widths make the bound's T ten times smaller and leave half as many jumps open,
 // but the near list more than twice as long: 31 -> 42 ms on the 128 diodes.
-
 
 // Does the diode's step run its jumps here?  (planner mode PM_MH_NEAR)
 __device__ __forceinline__ bool near_live(const DiodeParams& p, const DiodeDyn& y) {
@@ -300,18 +301,18 @@ k_near_panels(const DiodeParams* __restrict__ P, const DiodeDyn* __restrict__ Dy
       if (here <= 256 && j0 + 256 < n) continue;   // room for another 256 (block-uniform)
 #pragma unroll 4
       for (int q = lane; q < here; q += 32) {
-      const float4 e = low[q];
-      const int code = __float_as_int(e.w);
-      const bool is_near = code >= 0 && (unsigned)((code & 0xffff) - ppx) < RD_NEAR_W &&
-                           (unsigned)((code >> 16) - r0) < RD_NEAR_ROWS;
-      // least and largest lateral distances to the panel's points
-      const float ux = fabsf(e.x - ox), uy = fabsf(e.y - oy), z2 = fmaf(e.z, e.z, 1e-20f);
-      const float bx = fmaxf(ux - ax, 0.0f), by = fmaxf(uy - ay, 0.0f), tx = ux + ax, ty = uy + ay;
-      const float inv = rsqrtf(fmaf(bx, bx, fmaf(by, by, z2)));
-      const float i2 = inv * inv, v7 = is_near ? 0.0f : (e.z * inv) * (i2 * i2 * i2);
-      // c_x^2 <= 0.68 over the panel: 0.32 x^2 <= 0.68 (y^2 + z^2)
-      Tx = fmaf(0.32f * tx * tx <= 0.68f * fmaf(by, by, z2) ? 2.5f : 15.0f, v7, Tx);
-      Ty = fmaf(0.32f * ty * ty <= 0.68f * fmaf(bx, bx, z2) ? 2.5f : 15.0f, v7, Ty);
+        const float4 e = low[q];
+        const int code = __float_as_int(e.w);
+        const bool is_near = code >= 0 && (unsigned)((code & 0xffff) - ppx) < RD_NEAR_W &&
+                             (unsigned)((code >> 16) - r0) < RD_NEAR_ROWS;
+        // least and largest lateral distances to the panel's points
+        const float ux = fabsf(e.x - ox), uy = fabsf(e.y - oy), z2 = fmaf(e.z, e.z, 1e-20f);
+        const float bx = fmaxf(ux - ax, 0.0f), by = fmaxf(uy - ay, 0.0f), tx = ux + ax, ty = uy + ay;
+        const float inv = rsqrtf(fmaf(bx, bx, fmaf(by, by, z2)));
+        const float i2 = inv * inv, v7 = is_near ? 0.0f : (e.z * inv) * (i2 * i2 * i2);
+        // c_x^2 <= 0.68 over the panel: 0.32 x^2 <= 0.68 (y^2 + z^2)
+        Tx = fmaf(0.32f * tx * tx <= 0.68f * fmaf(by, by, z2) ? 2.5f : 15.0f, v7, Tx);
+        Ty = fmaf(0.32f * ty * ty <= 0.68f * fmaf(bx, bx, z2) ? 2.5f : 15.0f, v7, Ty);
       }
       here = 0;
       __syncthreads();
