@@ -2560,7 +2560,7 @@ __device__ __forceinline__ bool serial_take(const DiodeParams& p, const double* 
 // and jump i + 1 from either point, the block sums the field at all three, and one
 // comparison each answers both.  33 chains of 100 jumps over 400 electrons: 25.9 ->
 // 6.7 ms one at a time, 5.1 ms so (7.8 -> 2.0 -> 1.6 us a jump), 5.2 with the FP64 sums at
-// a chain's two ends; over 4000 electrons 9.3 -> 6.9 ms (30 chains).
+// a chain's end; over 4000 electrons 9.3 -> 6.9 ms (30 chains).
 #define RD_SER_DRAWS 256
 template <int PREC>
 __global__ void __launch_bounds__(256, 1)
@@ -2579,7 +2579,6 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
   __shared__ float2 red_f3[3][8];
   __shared__ int s_sum[2];        // the block sums a field this jump (a ring proposal off the ring: no)
   __shared__ int s_found, s_add, s_stop;   // the chain started; a particle was added; the chains stop
-  __shared__ int s_moved;   // the chain has left its start
   __shared__ DiodeParams sp;   // thread 0's loads of it are on the jumps' path
   const int d = blockIdx.x;
   if (!P[d].active || !P[d].emission || !P[d].mh_serial || P[d].geometry != RD_G_PLANAR) return;
@@ -2615,7 +2614,6 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
     double ca = 0.0, cr = rmin;   // ring: (angle, radius) of the chain (Metropolis_Hastings_ring_J)
     bool found = false;
     SerialSum cur = {0.0f, 0.0f, 0.0};   // the sum at the chain's point
-    bool moved = false;   // (thread 0) the chain has left its start
     if (t0) s_found = 0;
     for (int r = 0; r < p.init_rounds; ++r) {
       if (t0) {
@@ -2634,11 +2632,11 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
         if (PREC == 1) s_pp[0] = z0_point(p, cx, cy);
       }
       __syncthreads();
-      if constexpr (PREC == 1) cur.s = serial_tree_sum(p, pool, n, s_pp[0], red_d);
-      else cur = serial_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], s_pp[0], red_f, red_d);
+      cur = serial_field_sum<PREC>(p, pool, n, s_pt[0][0], s_pt[0][1], s_pp[0], red_f, red_d);
+      if (t0) F = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
+      if (PREC == 1 && threadIdx.x < 32 && __shfl_sync(0xffffffffu, !(serial_rel(p, F) < 1.0), 0))
+        F = z0_finish<PREC>(p, serial_tree_warp(p, pool, n, s_pp[0]), kscale);   // the pairs leave the sign open
       if (t0) {
-        if (PREC == 1) { cur.h = (float)cur.s; cur.l = (float)(cur.s - (double)cur.h); }
-        F = z0_finish<PREC>(p, cur.s, kscale);
         found = F < 0.0;
         s_found = found;
       }
@@ -2751,7 +2749,7 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
                 if (t0) tk = Fw < 0.0 && serial_take_fp64(p, wtab, wx, wy, Fw, 0.0, cx, cy, Fd, 0.0, s_lu[draw + j]);
                 tk = __shfl_sync(0xffffffffu, tk, 0);
               }
-              if (tk) { cx = wx; cy = wy; cur.h = wh; cur.l = wl; Fc = wF; fe = wd; rc = wr; moved = true; }
+              if (tk) { cx = wx; cy = wy; cur.h = wh; cur.l = wl; Fc = wF; fe = wd; rc = wr; }
               if (i + j > ndim_first) { if (tk) ++ja; else ++jr; }
               return tk;
             };
@@ -2839,24 +2837,21 @@ k_mh_serial(const DiodeParams* __restrict__ P, DiodeDyn* __restrict__ Dy, Pool p
           cx = wx; cy = wy; cur = sum; ca = na; cr = nr;
           Fc = Fn; fe = dF; rc = rn;
           tc = tn; have_sc = !est;
-          moved = true;
           if (i > ndim_first) ++ja;
         } else if (i > ndim_first) {
           ++jr;
         }
       }
     }
-    if (t0 && found) Fout = PREC == 1 ? F : z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
     if constexpr (PREC == 1) {   // the field at the chain's last point
-      if (t0) {
-        s_pp[0] = z0_point(p, cx, cy);
-        s_moved = moved;
-      }
-      __syncthreads();
-      if (s_moved) {   // block-uniform
+      if (walk) {   // block-uniform
+        if (t0) s_pp[0] = z0_point(p, cx, cy);
+        __syncthreads();
         const double sum = serial_tree_sum(p, pool, n, s_pp[0], red_d);
         if (t0) Fout = z0_finish<PREC>(p, sum, kscale);
       }
+    } else if (t0 && found) {
+      Fout = z0_finish<PREC>(p, serial_value<PREC>(cur), kscale);
     }
     // the chain's end: MH_std, the escape test and its electron (thread 0)
     if (t0) {
